@@ -1038,25 +1038,21 @@ struct Plan {
     bool want_aexp = false;              // PlusTimes fp64, exact accumulation (k_numeric_x)
     int64_t *fb_items = nullptr;         // big columns the exact kernel hands to the ordered one
     unsigned long long *fb_cnt = nullptr;
-    XSeg *xscratch = nullptr;            // exact kernel: bucketing scratch, kXScap segments per block
+    XSeg *xscratch = nullptr;            // exact kernel: bucketing scratch, xscap segments per block
+    int64_t xscap = 0;                   // (no column has more than its A has tile list entries)
     int x_blocks = 0;                    // exact kernel: its grid (resident blocks)
     SpgemmArgs &a() { return h[0]; }
 };
 
 // PlusTimes fp64 under GBC_FOLD_EXACT: every admitted column is summed
-// exactly (big columns by k_numeric_x).  Its accumulator tile is kXRows
-// high by default (8192-row tiles, one 1024-thread block per SM, made the
-// scale-20 product 19 % slower) and kXRowsBig at most; the tile height is a
-// tuning knob only, so a larger request is lowered.
+// exactly (big columns by k_numeric_x).  Its row tiles are kXRows high; the
+// tile height is a tuning knob only, so a larger request is lowered.
 template <class SR>
 static void plan_fold(Context *ctx, Plan &P)
 {
     if (std::is_same<SR, PlusTimes<double>>::value && ctx->fold == GBC_FOLD_EXACT) {
         P.want_aexp = true;
-        if (P.tile_rows == 0)
-            P.tile_rows = kXRows;
-        else if (P.tile_rows > kXRowsBig)
-            P.tile_rows = kXRowsBig;
+        P.tile_rows = kXRows;
         // columns of more than kSmallMid multiplications go to the exact
         // block kernel (R-MAT s14: 2.1x faster than the larger warp kernel)
         if (!P.s2_set) P.s2 = std::min<int64_t>(P.s2, kSmallMid);
@@ -1066,11 +1062,8 @@ static void plan_fold(Context *ctx, Plan &P)
 template <class SR>
 static bool use_exact(const Plan &P)
 {
-    return std::is_same<SR, PlusTimes<double>>::value && P.want_aexp && P.max_R <= kXRowsBig;
+    return std::is_same<SR, PlusTimes<double>>::value && P.want_aexp;
 }
-
-// shared memory of k_numeric_x for a tile of RS rows
-static size_t x_smem(int RS) { return (size_t)kXW * RS * 4 + RS; }
 
 struct Lists {
     // [0, kWarpClasses): the warp-kernel classes (up to s1, kSmallMid,
@@ -1130,7 +1123,7 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
             note_launch();
         }
         a.aexp = aexp;
-        if (a.T <= (1 << 20) / std::max(a.R, kXRows) && A.ncol > 0) {
+        if (a.T <= kXTMax && A.ncol > 0) {
             // per-column tile lists of A (bucketing in the exact kernel)
             int64_t *kptr = nullptr;
             GBC_TRY(ws.alloc_n(&kptr, (size_t)A.ncol + 1));
@@ -1139,6 +1132,7 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
             GBC_TRY(exclusive_scan_i64(ws, kptr, kptr, A.ncol, s));
             int64_t nent = 0;
             GBC_TRY(read_i64(ctx, kptr + A.ncol, &nent));
+            P.xscap = std::max(P.xscap, std::min(nent, kXScap));
             uint32_t *kst = nullptr;
             uint16_t *ktt = nullptr;
             GBC_TRY(ws.alloc_n(&kst, (size_t)nent + 1));
@@ -1174,18 +1168,10 @@ static int plan_finalize(Workspace &ws, Plan &P)
     if (P.want_aexp) {
         GBC_TRY(ws.alloc_n(&P.fb_items, (size_t)P.total_cols + 1));
         GBC_TRY(ws.alloc_n(&P.fb_cnt, 1));
-        // bucketing scratch of the exact kernel: kXScap segments per resident block
-        if (P.max_R > kXRows) {
-            const size_t smem = x_smem(kXRowsBig);
-            GBC_TRY(set_smem(k_numeric_x<kXThreadsBig, kXRowsBig>, smem));
-            P.x_blocks = ws.ctx->num_sms *
-                         resident_blocks(k_numeric_x<kXThreadsBig, kXRowsBig>, kXThreadsBig, smem, 1);
-        } else {
-            const size_t smem = x_smem(kXRows);
-            GBC_TRY(set_smem(k_numeric_x<kXThreads, kXRows>, smem));
-            P.x_blocks = ws.ctx->num_sms * resident_blocks(k_numeric_x<kXThreads, kXRows>, kXThreads, smem, 2);
-        }
-        GBC_TRY(ws.alloc_n(&P.xscratch, (size_t)P.x_blocks * kXScap));
+        // bucketing scratch of the exact kernel, per resident block
+        GBC_TRY(set_smem(k_numeric_x, sizeof(XSmem)));
+        P.x_blocks = ws.ctx->num_sms * resident_blocks(k_numeric_x, kXThreads, sizeof(XSmem), 2);
+        GBC_TRY(ws.alloc_n(&P.xscratch, (size_t)P.x_blocks * P.xscap + 1));
     }
     GBC_CUDA_TRY(cudaMemcpyAsync(P.d, P.h.data(), P.h.size() * sizeof(SpgemmArgs), cudaMemcpyHostToDevice,
                                  ws.ctx->stream));
@@ -1353,14 +1339,9 @@ static int launch_big_exact(Context *ctx, Plan &P, const Lists &L, const int64_t
     const int grid = (int)std::min<int64_t>(P.x_blocks, L.n[kBigList]);  // the scratch holds P.x_blocks blocks
     GBC_CUDA_TRY(cudaMemsetAsync(P.work + 1, 0, 3 * sizeof(unsigned long long), s));
     GBC_CUDA_TRY(cudaMemsetAsync(P.fb_cnt, 0, sizeof(unsigned long long), s));
-    if (P.max_R > kXRows)
-        k_numeric_x<kXThreadsBig, kXRowsBig><<<grid, kXThreadsBig, x_smem(kXRowsBig), s>>>(
-            P.d, L.l[kBigList], L.n[kBigList], ccp, ccp_base, cap, out_cnt, overflow, cir, static_cast<double *>(cval),
-            P.work + 1, P.fb_items, P.fb_cnt, P.xscratch);
-    else
-        k_numeric_x<kXThreads, kXRows><<<grid, kXThreads, x_smem(kXRows), s>>>(
-            P.d, L.l[kBigList], L.n[kBigList], ccp, ccp_base, cap, out_cnt, overflow, cir, static_cast<double *>(cval),
-            P.work + 1, P.fb_items, P.fb_cnt, P.xscratch);
+    k_numeric_x<<<grid, kXThreads, sizeof(XSmem), s>>>(P.d, L.l[kBigList], L.n[kBigList], ccp, ccp_base, cap, out_cnt,
+                                                       overflow, cir, static_cast<double *>(cval), P.work + 1,
+                                                       P.fb_items, P.fb_cnt, P.xscratch, P.xscap);
     note_launch();
     GBC_CUDA_TRY(cudaGetLastError());
     return launch_big_ordered<SR>(ctx, P, P.fb_items, L.n[kBigList], P.fb_cnt, ccp, ccp_base, cap, out_cnt, overflow, cir,

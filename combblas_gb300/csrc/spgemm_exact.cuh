@@ -15,14 +15,13 @@
 // rounded sum of the reference's own products, within the reference's own
 // summation error of its hash-path and heap-path results.
 //
-// Dense accumulator: kXW signed 32-bit words per row, word i holding a
-// signed multiple of 2^(kXP * i); a product's 53-bit mantissa is split into
-// at most four kXP-bit pieces added with 32-bit shared atomics (about five
-// times the rate of 64-bit shared atomics on this GPU).  Words are
-// normalised (carries moved up) after at most kXNorm B entries, so no word
-// overflows.  A column is admitted when all its products are normal and
-// finite and
-//   span + 53 <= kXP * kXW               (every piece has a word)
+// Accumulator: one signed 128-bit integer per output row, in four 32-bit words
+// of shared memory (word i the multiples of 2^(32 i)); a product's 53-bit
+// mantissa covers at most three words, added with 32-bit shared atomics whose
+// returned old value says whether a carry (a borrow, for a negative product)
+// goes on to the next word.  A column is admitted when all its products are
+// normal and finite and
+//   span <= kXOMax                       (every product has its words)
 //   span + 53 + lg(nnz(B(:,j))) <= 125   (the exact sum fits 126 bits)
 // with span = (largest - smallest product exponent) bounded from per-column
 // exponent ranges of A and the B values; other columns (subnormal values,
@@ -32,23 +31,16 @@
 
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "semiring.cuh"
 #include "spgemm_kernels.cuh"
 
 namespace gbc {
 
-constexpr int kXP = 19;                      // payload bits per accumulator word
-constexpr int kXW = 6;                       // words per row
-constexpr uint32_t kXMask = (1u << kXP) - 1;
-constexpr int kXOMax = kXP * kXW - 53;       // largest product exponent above the base (61)
-constexpr int kXNorm = 2047;                 // B entries between carry normalisations
-// Accumulator tiles and block shapes of k_numeric_x: RS rows (24 B of words
-// + 1 flag byte each) in shared memory; 4096 rows with 512 threads (two
-// blocks per SM) or 8192 rows with 1024 threads (one block per SM).
-constexpr int kXRows = 4096;
-constexpr int kXThreads = 512;
-constexpr int kXRowsBig = 8192;
-constexpr int kXThreadsBig = 1024;
+constexpr int kXOMax = 61;       // largest product exponent above the base
+constexpr int kXRows = 4096;     // rows of a row tile, and output rows of one accumulator pass
+constexpr int kXThreads = 512;   // two blocks per SM
 
 // Phase clocks of k_numeric_x for profiling builds (-DGBC_XPROF): thread 0
 // of every block adds the cycles between two block barriers to a counter.
@@ -83,21 +75,27 @@ extern "C" int gbc_xprof_read(unsigned long long *out, int reset)
 #endif
 
 // Per column of A: smallest and largest biased exponent of its nonzero
-// values, packed as (int16 min) | (int16 max << 16).  Subnormal values count
-// as exponent -64 (their products can underflow: such columns take the
-// ordered kernel); a column without nonzero values gets min > max.
+// values, each plus kXBias in 12 bits, and kXMixed when a value is negative or
+// zero.  Subnormal values count as exponent -64 (their products can
+// underflow: such columns take the ordered kernel); a column without nonzero
+// values gets min > max.
+constexpr int kXBias = 64;
+constexpr uint32_t kXMixed = 1u << 24;
+
 static __global__ void k_aexp_f64(int64_t ncol, const int64_t *acp, const double *aval, int32_t *aexp)
 {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
     for (int64_t c = warp; c < ncol; c += nwarps) {
-        int lo = 32767, hi = -32768;
+        int lo = 4095 - kXBias, hi = -kXBias;
+        bool mixed = false;
         for (int64_t p = acp[c] + lane; p < acp[c + 1]; p += 32) {
             const uint64_t bits = (uint64_t)__double_as_longlong(aval ? aval[p] : 1.0);
             int e = (int)((bits >> 52) & 0x7ff);
             const bool zero = (bits << 1) == 0;
-            if (e == 0) e = -64;
+            mixed |= zero || (bits >> 63);
+            if (e == 0) e = -kXBias;
             if (!zero) {
                 lo = min(lo, e);
                 hi = max(hi, e);
@@ -105,104 +103,57 @@ static __global__ void k_aexp_f64(int64_t ncol, const int64_t *acp, const double
         }
         lo = __reduce_min_sync(0xffffffffu, lo);
         hi = __reduce_max_sync(0xffffffffu, hi);
-        if (lane == 0) aexp[c] = (int32_t)(((uint32_t)(uint16_t)(int16_t)lo) | ((uint32_t)(uint16_t)(int16_t)hi << 16));
+        mixed = __any_sync(0xffffffffu, mixed);
+        if (lane == 0)
+            aexp[c] = (int32_t)((uint32_t)(lo + kXBias) | ((uint32_t)(hi + kXBias) << 12) | (mixed ? kXMixed : 0u));
     }
 }
 
-// Round-to-nearest-even product of two nonzero normal doubles whose exact
-// product is normal and finite (what admitted columns hold), restated in
-// integer arithmetic from IEEE 754: the 53-bit mantissas are multiplied
-// exactly (106 bits), rounded to 53 bits, ties to even.  Returns the 53-bit
-// mantissa q (2^52 <= q < 2^53) and the biased exponent e, so that
-// |a * b| rounds to q * 2^(e - 1075).  (GB300's fp64 pipe issues about two
-// multiplies per SM clock; the integer units do this several times faster,
-// and the accumulator needs the integer mantissa anyway.)
-__device__ __forceinline__ void x_mul(uint64_t abits, uint64_t bbits, uint64_t &q, int &e)
+// Add the nonzero product with bit pattern `bits` (normal, of an admitted
+// column) to the 128-bit integer whose word i is acc[i * stride].  Words that
+// overflow pass their carry on, so no word is ever normalised: the integer is
+// exact modulo 2^128 once every thread has finished.  POS: the product is
+// positive.  Returns false when the product lies outside the column's
+// exponent window (cannot happen for admitted columns; nothing is added then).
+template <bool POS>
+__device__ __forceinline__ bool x_add128(uint32_t *acc, int stride, uint64_t bits, int ebase)
 {
-    const uint64_t ma = (abits & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-    const uint64_t mb = (bbits & 0xFFFFFFFFFFFFFull) | (1ull << 52);
-    e = (int)((abits >> 52) & 0x7ff) + (int)((bbits >> 52) & 0x7ff) - 1023;
-    const uint64_t lo = ma * mb, hi = __umul64hi(ma, mb);  // 2^104 <= ma * mb < 2^106
-    const int top = (int)(hi >> 41);                        // 1 when bit 105 is set
-    const int sh = 52 + top;                                // bits below the kept 53
-    q = (hi << (64 - sh)) | (lo >> sh);
-    const uint64_t rem = lo & ((1ull << sh) - 1), half = 1ull << (sh - 1);
-    q += (rem > half || (rem == half && (q & 1))) ? 1ull : 0ull;
-    e += top;
-    if (q >> 53) {  // rounded up to 2^53
-        q >>= 1;
-        ++e;
+    const uint32_t ml = (uint32_t)bits, h = (uint32_t)(bits >> 32);
+    const uint32_t mh = (h & 0xFFFFFu) | 0x100000u;
+    const uint32_t o = (POS ? h >> 20 : (h >> 20) & 0x7ffu) - (uint32_t)ebase;
+    if (o > (uint32_t)kXOMax) return false;
+    const uint32_t p0 = ml << (o & 31);
+    const uint32_t p1 = __funnelshift_l(ml, mh, o);
+    const uint32_t p2 = __funnelshift_l(mh, 0u, o);  // below 2^21
+    uint32_t *w = acc + (o >> 5) * stride;
+    if (POS || !(h >> 31)) {
+        uint32_t old = atomicAdd(w, p0), t1, wrap, t2, c;
+        // t1 = p1 + carry (wrap: p1 was all ones and the carry goes on)
+        asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %2, %3;\n\taddc.cc.u32 %0, %4, 0;\n\taddc.u32 %1, 0, 0;\n\t}"
+            : "=r"(t1), "=r"(wrap)
+            : "r"(old), "r"(p0), "r"(p1));
+        old = atomicAdd(w + stride, t1);
+        asm("{\n\t.reg .u32 t;\n\tadd.cc.u32 t, %1, %2;\n\taddc.u32 %0, %3, %4;\n\t}"
+            : "=r"(t2)
+            : "r"(old), "r"(t1), "r"(p2), "r"(wrap));
+        if (t2) {
+            old = atomicAdd(w + 2 * stride, t2);
+            c = old > ~t2;
+            if (c && o < 32) atomicAdd(w + 3 * stride, 1u);
+        }
+    } else {
+        uint32_t old = atomicAdd(w, 0u - p0);
+        uint32_t c = old < p0;
+        const uint32_t t1 = p1 + c, wrap = t1 < c;
+        old = atomicAdd(w + stride, 0u - t1);
+        c = wrap | (uint32_t)(old < t1);
+        const uint32_t t2 = p2 + c;
+        if (t2) {
+            old = atomicAdd(w + 2 * stride, 0u - t2);
+            if (old < t2 && o < 32) atomicAdd(w + 3 * stride, ~0u);
+        }
     }
-}
-
-// The product's double (bit pattern): +-0 when a factor is zero.
-__device__ __forceinline__ uint64_t x_mul_bits(uint64_t abits, uint64_t bbits)
-{
-    const uint64_t sign = (abits ^ bbits) & (1ull << 63);
-    if ((abits << 1) == 0 || (bbits << 1) == 0) return sign;
-    uint64_t q;
-    int e;
-    x_mul(abits, bbits, q, e);
-    return sign | ((uint64_t)e << 52) | (q & 0xFFFFFFFFFFFFFull);
-}
-
-// Add the product a * b (bit patterns of two values of an admitted column:
-// zero or normal, product normal) to row r of the accumulator (words at
-// acc[i * stride + r]) and mark the row touched in its flag byte (bit 0
-// touched, bit 1 touched by something other than -0.0, which decides the
-// sign of an exact zero sum); a row's first touch counts it in band[r / 256]
-// (touched rows per 256-row band, the write-out's offsets).  Returns false when the product lies outside
-// the column's admitted exponent window (cannot happen for admitted
-// columns; nothing is added then).
-__device__ __forceinline__ bool x_add(int32_t *acc, int stride, uint32_t *tw, int32_t *band, int r, uint64_t abits,
-                                      uint64_t bbits, int ebase)
-{
-    const bool neg = ((abits ^ bbits) >> 63) != 0;
-    const int sh8 = (r & 3) << 3;
-    const bool zero = (abits << 1) == 0 || (bbits << 1) == 0;  // a zero product: +0.0 or -0.0
-    const uint32_t old = atomicOr(&tw[r >> 2], ((zero && neg) ? 1u : 3u) << sh8);
-    if (((old >> sh8) & 0xff) == 0) atomicAdd(&band[r >> 8], 1);  // first touch: count the row in its band
-    if (zero) return true;
-    uint64_t m;
-    int ex;
-    x_mul(abits, bbits, m, ex);
-    const int o = ex - ebase;
-    if ((unsigned)o > (unsigned)kXOMax) return false;
-    const int w0 = o / kXP;
-    const int bsh = o - kXP * w0;
-    const uint64_t lo = m << bsh;
-    const uint64_t hi = bsh ? (m >> (64 - bsh)) : 0ull;
-    int32_t q0 = (int32_t)(lo & kXMask);
-    int32_t q1 = (int32_t)((lo >> kXP) & kXMask);
-    int32_t q2 = (int32_t)((lo >> (2 * kXP)) & kXMask);
-    int32_t q3 = (int32_t)((lo >> (3 * kXP)) | (hi << (64 - 3 * kXP)));
-    if (neg) {
-        q0 = -q0;
-        q1 = -q1;
-        q2 = -q2;
-        q3 = -q3;
-    }
-    // the top nonzero piece is in word (o + 52) / kXP <= kXW - 1
-    int32_t *base = acc + w0 * stride + r;
-    if (q0) atomicAdd(base, q0);
-    if (q1) atomicAdd(base + stride, q1);
-    if (q2) atomicAdd(base + 2 * stride, q2);
-    if (q3) atomicAdd(base + 3 * stride, q3);
     return true;
-}
-
-// Move the carries of row r's words up (word i keeps its value mod 2^kXP,
-// the top word keeps the rest).
-__device__ __forceinline__ void x_normalise(int32_t *acc, int stride, int r)
-{
-    int32_t carry = 0;
-#pragma unroll
-    for (int i = 0; i < kXW - 1; ++i) {
-        const int32_t v = acc[i * stride + r] + carry;
-        acc[i * stride + r] = (int32_t)((uint32_t)v & kXMask);
-        carry = v >> kXP;
-    }
-    acc[(kXW - 1) * stride + r] += carry;
 }
 
 // Round a signed 128-bit integer M (two's complement hi:lo), times
@@ -219,57 +170,22 @@ __device__ __forceinline__ double x_round(uint64_t hi, uint64_t lo, uint32_t fla
         hi = ~hi + (lo == 0 ? 1ull : 0ull);
     }
     if ((hi | lo) == 0) return (flag & 2) ? 0.0 : -0.0;
-    const int tb = hi ? 127 - __clzll((long long)hi) : 63 - __clzll((long long)lo);  // top bit of |M|
-    const int e = tb + ebase - 52;  // biased exponent when the result is normal
+    const int n = hi ? __clzll((long long)hi) : 64 + __clzll((long long)lo);  // zeros above |M|'s top bit
+    const int e = 127 - n + ebase - 52;  // biased exponent when the result is normal
     uint64_t bits;
     if (e <= 0) {
         // subnormal: |M| * 2^(ebase - 1) < 2^52 is the exact subnormal mantissa
         bits = lo << (ebase - 1);
-    } else if (tb <= 52) {
-        bits = ((uint64_t)e << 52) + ((lo << (52 - tb)) & 0xFFFFFFFFFFFFFull);  // exact
     } else {
-        const int sh = tb - 52;  // 1..73 bits below the 53 kept
-        uint64_t m, rnd, sticky;
-        if (sh < 64) {
-            m = (lo >> sh) | (sh ? (hi << (64 - sh)) : 0ull);
-            rnd = (lo >> (sh - 1)) & 1;
-            sticky = (sh > 1 && (lo << (65 - sh)) != 0) ? 1 : 0;
-        } else {
-            m = hi >> (sh - 64);
-            rnd = sh == 64 ? (lo >> 63) : ((hi >> (sh - 65)) & 1);
-            sticky = (lo & (sh == 64 ? 0x7FFFFFFFFFFFFFFFull : ~0ull)) != 0 ||
-                     (sh > 65 && (hi << (129 - sh)) != 0);
-        }
-        m += (rnd && (sticky || (m & 1))) ? 1 : 0;  // may carry into 2^53: the exponent field absorbs it
+        // |M| shifted to bit 127: 53 bits kept, 11 in `rem`, the others in `rest`
+        const uint64_t top = n < 64 ? (hi << n) | ((lo >> 1) >> (63 - n)) : lo << (n - 64);
+        const uint64_t rest = n < 64 ? lo << n : 0ull;
+        const uint32_t rem = (uint32_t)top & 0x7FFu;
+        uint64_t m = top >> 11;
+        m += (rem > 0x400u || (rem == 0x400u && (rest != 0 || (m & 1)))) ? 1 : 0;  // 2^53 carries into the exponent
         bits = ((uint64_t)(e - 1) << 52) + m;
     }
     return __longlong_as_double((long long)(bits | (neg ? (1ull << 63) : 0ull)));
-}
-
-// The exact sum of row r's words, rounded (x_round); clears the words.
-__device__ __forceinline__ double x_value(int32_t *acc, int stride, int r, uint32_t flag, int ebase)
-{
-    uint64_t lo = 0, hi = 0;
-#pragma unroll
-    for (int i = 0; i < kXW; ++i) {
-        const int64_t s = acc[i * stride + r];
-        acc[i * stride + r] = 0;
-        const int sh = kXP * i;
-        uint64_t pl, ph;
-        if (sh == 0) {
-            pl = (uint64_t)s;
-            ph = (uint64_t)(s >> 63);
-        } else if (sh < 64) {
-            pl = (uint64_t)s << sh;
-            ph = (uint64_t)(s >> (64 - sh));
-        } else {
-            pl = 0;
-            ph = (uint64_t)s << (sh - 64);
-        }
-        lo += pl;
-        hi += ph + (lo < pl ? 1ull : 0ull);
-    }
-    return x_round(hi, lo, flag, ebase);
 }
 
 // Add product p (a double of an admitted column) exactly to a register
@@ -302,7 +218,7 @@ __device__ __forceinline__ bool x_acc128(uint64_t &hi, uint64_t &lo, uint32_t &f
 // allowing for rounding up).  Entries whose products are all zero are skipped.
 __device__ __forceinline__ void x_window(int32_t ae, double b, bool has_b, int &emin, int &emax)
 {
-    const int amin = (int16_t)(ae & 0xffff), amax = (int16_t)((uint32_t)ae >> 16);
+    const int amin = (int)(ae & 0xfff) - kXBias, amax = (int)((ae >> 12) & 0xfff) - kXBias;
     const uint64_t bb = has_b ? (uint64_t)__double_as_longlong(b) : 0x3FF0000000000000ull;
     int eb = (int)((bb >> 52) & 0x7ff);
     if (amin > amax || (bb << 1) == 0) return;
@@ -373,12 +289,71 @@ struct XSeg {
 };
 
 constexpr int kXTMax = 256;                   // row tiles of a bucketed column
-constexpr int kXRange = 4096;                 // products of one sorted range visit (at most; RS for smaller tiles)
-#ifndef GBC_XDENSE
-#define GBC_XDENSE 512
+constexpr int kXSegs = 1024;                  // segments of one chunk table
+constexpr int kXWins = 512;                   // 32-product windows of one round
+constexpr int kXSpanTiles = 16;               // row tiles of one ranked visit (a 64 K-row bitmap)
+constexpr int kXSort = 4096;                  // products of one sorted range visit (at most)
+#ifndef GBC_XLIGHT
+#define GBC_XLIGHT 512
 #endif
-constexpr int kXDense = GBC_XDENSE;           // a tile with more products is a dense visit
-constexpr int64_t kXScap = int64_t(1) << 18;  // bucketed segments of one column (per-block scratch)
+constexpr int kXLight = GBC_XLIGHT;           // runs of at most this many products go to sorted ranges
+constexpr int kXDirect = 8192;                // a tile of more products is a visit of its own
+constexpr int64_t kXScap = int64_t(1) << 20;  // bucketed segments of one column, at most (per-block scratch)
+
+// Shared memory of one k_numeric_x block.
+struct XSmem {
+    uint32_t acc[4 * kXRows];              // accumulator words, plane by plane
+    uint32_t bm[kXSpanTiles * kXRows / 32];   // touched rows of the visit
+    uint16_t pre[kXSpanTiles * kXRows / 32];  // touched rows before each bitmap word
+    uint16_t rows[kXRows];                 // row (from the visit's first) of every accumulator
+    double bv[kXSegs];                     // chunk table: B value of each segment,
+    uint32_t base[kXSegs];                 //   segment start - products before it (modulo 2^32),
+    int32_t off[kXSegs + 1];               //   products before each segment
+    int32_t nseg;                          //   segments
+    uint2 win[kXWins];                     // per 32 products: bit i set where a segment starts at the i-th, and
+                                           //   the segments that start before the window
+    int32_t segcnt[kXTMax], prodcnt[kXTMax], tend[kXTMax];
+    int32_t wsum[2][kXThreads / 32];
+    int32_t emin[kXThreads / 32], emax[kXThreads / 32];
+    int64_t col;
+    int32_t negzero;  // a product of the visit was -0.0
+    int32_t ebase;    // the column's smallest product exponent
+    int64_t bs, be;   // its B entries
+    int64_t *oir;     // its output
+    double *oval;
+    int32_t lim;      // output entries it may write
+    SpgemmArgs a;
+};
+
+// Does row r of column [bs, be) of B receive a term other than -0.0?
+static __device__ __noinline__ bool x_has_term(const SpgemmArgs &a, int64_t bs, int64_t be, int r)
+{
+    const double *aval = static_cast<const double *>(a.aval), *bval = static_cast<const double *>(a.bval);
+    for (int64_t b = bs; b < be; ++b) {
+        const int k = a.brow[b];
+        int64_t lo = a.acp[k], hi = a.acp[k + 1];
+        const int64_t end = hi;
+        while (lo < hi) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (a.arow[mid] < r)
+                lo = mid + 1;
+            else
+                hi = mid;
+        }
+        if (lo < end && a.arow[lo] == r &&
+            __double_as_longlong(__dmul_rn(aval ? aval[lo] : 1.0, bval ? bval[b] : 1.0)) != (long long)(1ull << 63))
+            return true;
+    }
+    return false;
+}
+
+// Output entries [q0, q1) of the column: sums of exactly zero that got no term
+// other than -0.0 become -0.0.  Called when the visit met a -0.0 product.
+static __device__ __noinline__ void x_fix_zeros(const XSmem &sm, int q0, int q1)
+{
+    for (int q = q0 + threadIdx.x; q < q1; q += kXThreads)
+        if (sm.oval[q] == 0.0 && !x_has_term(sm.a, sm.bs, sm.be, (int)sm.oir[q])) sm.oval[q] = -0.0;
+}
 
 // Numeric pass for the columns of the big list, one block per column
 // (dynamic counter).  After the column's exponent window is admitted:
@@ -387,60 +362,59 @@ constexpr int64_t kXScap = int64_t(1) << 18;  // bucketed segments of one column
 //     into the block's scratch grouped by tile (a counting sort; the exact
 //     sum makes the order irrelevant).  Each tile is then visited with its
 //     own segments only, instead of looking up every B entry per tile.
-//  2. visits in row order -- a tile with more than kXDense products is a
-//     dense visit: products added with x_add into the shared-memory word
-//     accumulator, touched rows written in row order.  Consecutive lighter
-//     tiles are merged into one range of at most kXRange products (RS for
-//     smaller tiles): the
-//     products (x_mul) are staged in shared memory with (row, slot) keys,
-//     radix sorted by row (stable LSD, 7-bit digits), and each run of one
-//     row is summed exactly (x_acc128) and rounded (x_round).
-// Columns with more than kXScap segments, or matrices with more than
-// 2^20 / RS tiles, visit every touched tile and look up their B entries' A
-// segments per tile (tptr) instead of step 1.  Columns outside the exact
-// window are appended to fb_items for the ordered kernel.
-template <int NT, int RS>
-__global__ void __launch_bounds__(NT, 1024 / NT)
+//  2. visits in row order, each a chunk table of its segments over which the
+//     products are spread evenly:
+//      * direct: a tile of more than kXDirect products (or too many segments)
+//        is visited alone, the accumulator of a product is its row's;
+//      * ranked: a run of consecutive tiles (at most kXSpanTiles) whose output
+//        is expected to fit kXRows rows: the products' rows are marked in a
+//        bitmap, a prefix of its popcounts ranks the touched rows, and the
+//        accumulator of a product is its row's rank, so consecutive threads
+//        write consecutive output entries.  A run whose output turns out
+//        larger is cut at a tile boundary.  Ranking is what lets one visit take
+//        several sparse tiles: at scale 20 half of all products lie in tiles
+//        of less than 8192 products and 500 output rows on average;
+//      * sorted: a run of at most kXLight products is merged with the light
+//        tiles that follow into a range of at most kXSort products, staged in
+//        shared memory with (row, slot) keys, radix sorted by row (stable LSD,
+//        7-bit digits); each run of one row is summed exactly (x_acc128).
+// Columns with more than scap segments, or matrices with more than kXTMax
+// tiles, visit every touched tile and look up their B entries' A segments per
+// tile (tptr) instead of step 1.  Columns outside the exact window are
+// appended to fb_items for the ordered kernel.
+//
+// Bound by instruction issue and by the latency of a visit's chain of
+// barriers, not by memory (DRAM 9 %).  Against one tile a visit with the
+// segments found by searches and 24-byte accumulators behind flag bytes (322
+// instead of 498 warp instructions per 32 products), R-MAT scale 20 A*A in
+// phases went from 1656 to 998 ms, all passes included (2^14: 1.94 to 1.51 ms).
+static __global__ void __launch_bounds__(kXThreads, 2)
     k_numeric_x(const SpgemmArgs *args, const int64_t *items, int64_t nitems, const int64_t *ccp, int64_t ccp_base,
                 const int64_t *cap, int64_t *out_cnt, int32_t *overflow, int64_t *cir, double *cval,
-                unsigned long long *work, int64_t *fb_items, unsigned long long *fb_count, XSeg *scratch_all)
+                unsigned long long *work, int64_t *fb_items, unsigned long long *fb_count, XSeg *scratch_all, int64_t scap)
 {
-    constexpr int NW = NT / 32;  // RS: rows of the tile = word stride
-    constexpr int TM = (1 << 20) / RS;             // tiles of a bucketed column
-    constexpr int XR = RS < kXRange ? RS : kXRange;  // products of one range visit
-    // TM <= NT: the bucketing's block-wide prefix gives every tile its offset
-    static_assert(XR <= 4096 && XR >= kXDense && (NW * 128) % NT == 0 && RS % (32 * NW) == 0 &&
-                      TM * RS <= (1 << 20) && TM <= kXTMax && TM <= NT,
-                  "range keys: 20-bit row offset and 12-bit slot; eight sorted keys per thread");
-    extern __shared__ __align__(16) int32_t xsm[];
-    int32_t *acc = xsm;                                           // [kXW][RS]
-    uint32_t *tw = reinterpret_cast<uint32_t *>(xsm + kXW * RS);  // [RS/4] flag bytes
-    uint8_t *tfb = reinterpret_cast<uint8_t *>(tw);
-    // range visits reuse the word area (it is cleared again before a dense visit)
-    uint32_t *rk0 = reinterpret_cast<uint32_t *>(xsm);          // [XR] keys
-    uint32_t *rk1 = rk0 + XR;                                   // [XR] keys (sort buffer)
-    uint64_t *rval = reinterpret_cast<uint64_t *>(rk1 + XR);    // [XR] products
-    uint32_t *rwh = reinterpret_cast<uint32_t *>(rval + XR);    // [NW][128] digit counts per warp
-    static_assert(2 * XR * 4 + XR * 8 + NW * 128 * 4 <= kXW * RS * 4, "range area inside the words");
-    __shared__ ChunkSmemN<NT> ch;
-    static_assert(sizeof(ChunkSmemN<NT>) >= NW * 128 * 2, "write-out row lists fit the chunk table");
-    __shared__ uint32_t ch_e[NT];
-    __shared__ int32_t s_segcnt[TM], s_prodcnt[TM], s_off[TM + 1];
-    __shared__ int32_t s_wsum[NW];
-    __shared__ int32_t s_band[RS / 256];  // touched rows per 256-row band of the dense tile
-    __shared__ int32_t s_emin[NW], s_emax[NW];
-    __shared__ int64_t s_col;
-    __shared__ SpgemmArgs sa;
+    constexpr int NT = kXThreads, NW = NT / 32, R = kXRows;
+    static_assert(kXTMax <= NT && kXSegs == 2 * NT && kXWins == NT && kXSort <= 4096 && kXSort <= 8 * NT, "block shape");
+    extern __shared__ __align__(16) unsigned char xsm[];
+    XSmem &sm = *reinterpret_cast<XSmem *>(xsm);
+    // a sorted range reuses the accumulator (cleared again before a ranked visit)
+    uint32_t *rk0 = sm.acc, *rk1 = rk0 + kXSort;                  // [kXSort] keys, sort buffer
+    uint64_t *rval = reinterpret_cast<uint64_t *>(rk1 + kXSort);  // [kXSort] products
+    uint32_t *rwh = reinterpret_cast<uint32_t *>(sm.rows);        // [NW][128] digit counts per warp
+    static_assert(kXSort * 16 <= (int)sizeof(sm.acc) && NW * 128 * 4 <= (int)sizeof(sm.rows), "range area");
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned lt = (1u << lane) - 1;
-    XSeg *scratch = scratch_all + (int64_t)blockIdx.x * kXScap;
-    for (int u = tid; u < kXW * RS + RS / 4; u += NT) xsm[u] = 0;
-    for (int u = tid; u < RS / 256; u += NT) s_band[u] = 0;
-    bool dirty = false;  // the word area holds a range visit's data
+    XSeg *scratch = scratch_all + (int64_t)blockIdx.x * scap;
+    for (int u = tid; u < 4 * R; u += NT) sm.acc[u] = 0;
+    for (int u = tid; u < kXSpanTiles * R / 32; u += NT) sm.bm[u] = 0;
+    if (tid == 0) sm.negzero = 0;
+    bool dirty = false;  // the accumulator holds a sorted range's data
     bool first_item = true;
+    int par = 0;  // which wsum the next prefix uses
     XPROF_T0;
 
-    // block-wide exclusive prefix of v over the threads (two barriers); *tot the sum
+    // block-wide exclusive prefix of v over the threads (one barrier: two
+    // prefixes in a row use different sums); *tot the total
     auto block_prefix = [&](int v, int *tot) -> int {
         int x = v;
 #pragma unroll
@@ -448,320 +422,494 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
             const int y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= o) x += y;
         }
-        if (lane == 31) s_wsum[warp] = x;
+        if (lane == 31) sm.wsum[par][warp] = x;
         __syncthreads();
-        int before = 0, all = 0;
+        int w = lane < NW ? sm.wsum[par][lane] : 0;
+        par ^= 1;
+        const int own = w;
 #pragma unroll
-        for (int u = 0; u < NW; ++u) {
-            const int ws = s_wsum[u];
-            before += u < warp ? ws : 0;
-            all += ws;
+        for (int o = 1; o < NW; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, w, o);
+            if (lane >= o) w += y;
+        }
+        *tot = __shfl_sync(0xffffffffu, w, NW - 1);
+        return __shfl_sync(0xffffffffu, w - own, warp) + x - v;
+    };
+    // The chunk table.  Every thread brings two consecutive segments (start,
+    // length, B value); empty ones are dropped when `compact` (elsewhere only
+    // the last ones are empty).  Product p of the chunk then belongs to
+    // segment win[p / 32].y - 1 + (starts up to p in win[p / 32].x), so a warp
+    // finds its products' segments with one popcount and no search.  A table
+    // covers rounds of kXWins windows; rounds() moves it to another one.
+    // segment i holds products [p, p + len) from the round's first on
+    auto set_windows = [&](int i, int p, int len) {
+        if (len > 0) {
+            if (p >= 0 && p < kXWins * 32) atomicOr(&sm.win[p >> 5].x, 1u << (p & 31));
+            // windows that start inside this segment or right behind it
+            for (int w = max(0, (p >> 5) + 1); w <= min(kXWins - 1, (p + len) >> 5); ++w) sm.win[w].y = i + 1;
+        }
+    };
+    auto fill_table = [&](const uint32_t (&st)[2], const int (&ln)[2], const double (&bv)[2], bool compact) -> int {
+        int tot, cnt = kXSegs;
+        sm.win[tid] = make_uint2(0u, 0u);
+        int p = block_prefix(ln[0] + ln[1], &tot);
+        int c = compact ? block_prefix((ln[0] > 0) + (ln[1] > 0), &cnt) : 2 * tid;
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+            if (ln[u] > 0 || !compact) {
+                sm.off[c] = p;
+                sm.base[c] = st[u] - (uint32_t)p;
+                sm.bv[c] = bv[u];
+                set_windows(c, p, ln[u]);
+                p += ln[u];
+                ++c;
+            }
+        if (tid == 0) {
+            sm.off[cnt] = tot;
+            sm.nseg = cnt;
         }
         __syncthreads();
-        *tot = all;
-        return before + x - v;
+        return tot;
     };
-
-    // products of one chunk of segments (ch, ch_e) flattened over the warps:
-    // f(b, idx, p) for product p of segment b at A position idx
-    auto for_products = [&](int L, int nseg, auto &&f) {
-        const int span = (((L + NW - 1) / NW) + 31) & ~31;
-        const int wb = warp * span, we = min(L, wb + span);
-        if (wb < we) {
-            int bcur = chunk_find_nz(ch, nseg, wb);
-            for (int p0 = wb; p0 < we; p0 += 32) {
-                const int p = p0 + lane;
-                const int b = window_seg(ch, nseg, bcur, p);
-                if (p < we) f(b, (int64_t)(uint32_t)(ch.base[b] + (uint32_t)p), p);
-                int bn = __shfl_sync(0xffffffffu, b, 31);
-                if (bn + 1 < nseg && ch.off[bn + 1] <= p0 + 32) ++bn;
-                bcur = bn;
+    // step(q0, n) for every round of the chunk's L products (n of them from q0
+    // on); `again`: the table was left at a later round.  A caller's barrier
+    // ends the last round.
+    auto rounds = [&](int L, bool again, auto &&step) {
+        for (int q0 = 0; q0 < L; q0 += kXWins * 32) {
+            if (q0 > 0 || (again && L > kXWins * 32)) {
+                __syncthreads();
+                sm.win[tid] = make_uint2(0u, 0u);
+                __syncthreads();
+                for (int i = 2 * tid; i < min(2 * tid + 2, sm.nseg); ++i)
+                    set_windows(i, sm.off[i] - q0, sm.off[i + 1] - sm.off[i]);
+                __syncthreads();
             }
+            step(q0, min(L - q0, kXWins * 32));
         }
+    };
+    const unsigned le = lt | (1u << lane);
+    // segment of the lane's product in window w of the round
+    auto seg_of = [&](int w) -> int {
+        const uint2 x = sm.win[w];
+        return (int)x.y + __popc(x.x & le) - 1;
+    };
+    // f(b, idx, p) for the chunk's products: segment b, A position idx
+    auto for_products = [&](int L, bool again, auto &&f) {
+        rounds(L, again, [&](int q0, int n) {
+            for (int w = warp; w * 32 < n; w += NW) {
+                const int p = w * 32 + lane;
+                if (p < n) {
+                    const int b = seg_of(w);
+                    f(b, sm.base[b] + (uint32_t)(q0 + p), q0 + p);
+                }
+            }
+        });
     };
 
     for (;;) {
         if (tid == 0) {
-            s_col = next_item(work, first_item);
-            if (s_col < nitems) sa = args[item_pid(items[s_col])];
+            sm.col = next_item(work, first_item);
+            if (sm.col < nitems) sm.a = args[item_pid(items[sm.col])];
         }
         __syncthreads();
-        const int64_t ci = s_col;
+        const int64_t ci = sm.col;
         if (ci >= nitems) break;
-        const SpgemmArgs &a = sa;
+        const SpgemmArgs &a = sm.a;
         const int64_t i = item_col(items[ci]);
         const int64_t g = a.col_base + i;
-        const double *aval = static_cast<const double *>(a.aval);
         const double *bval = static_cast<const double *>(a.bval);
         const int64_t bs = a.bcp[i], be = a.bcp[i + 1];
-        const int64_t out0 = ccp[g - ccp_base];
-        int64_t out = out0;
-        const int64_t lim = cap ? out0 + cap[g] : ccp[g - ccp_base + 1];
+        int out = 0;  // entries written (a column's output fits its row ids: below 2^31)
         bool over = false, bad = false;
+        if (tid == 0) {
+            const int64_t out0 = ccp[g - ccp_base];
+            sm.bs = bs;
+            sm.be = be;
+            sm.oir = cir + out0;
+            sm.oval = cval + out0;
+            sm.lim = (int)min(cap ? cap[g] : ccp[g - ccp_base + 1] - out0, (int64_t)INT32_MAX);
+        }
 
-        // admission: the exponent window of the column's products
+        // admission: the exponent window of the column's products; pos: all
+        // of them are positive
+        bool mixed = false;
         {
             int emin = 1 << 30, emax = -(1 << 30);
-            for (int64_t b = bs + tid; b < be; b += NT)
-                x_window(a.aexp[a.brow[b]], bval ? bval[b] : 1.0, bval != nullptr, emin, emax);
+            for (int64_t b = bs + tid; b < be; b += NT) {
+                const int32_t ae = a.aexp[a.brow[b]];
+                const double bv = bval ? bval[b] : 1.0;
+                x_window(ae, bv, bval != nullptr, emin, emax);
+                mixed |= (ae & kXMixed) || !(bv > 0.0);
+            }
             emin = __reduce_min_sync(0xffffffffu, emin);
             emax = __reduce_max_sync(0xffffffffu, emax);
             if (lane == 0) {
-                s_emin[warp] = emin;
-                s_emax[warp] = emax;
+                sm.emin[warp] = emin;
+                sm.emax[warp] = emax;
             }
         }
-        __syncthreads();
-        int ebase = 1 << 30, etop = -(1 << 30);
-#pragma unroll
-        for (int u = 0; u < NW; ++u) {
-            ebase = min(ebase, s_emin[u]);
-            etop = max(etop, s_emax[u]);
+        for (int u = tid; u < kXTMax; u += NT) {
+            sm.segcnt[u] = 0;
+            sm.prodcnt[u] = 0;
         }
+        const bool pos = !__syncthreads_or(mixed);
+        int ebase = __reduce_min_sync(0xffffffffu, sm.emin[lane & (NW - 1)]);
+        const int etop = __reduce_max_sync(0xffffffffu, sm.emax[lane & (NW - 1)]);
         if (!x_admit(ebase, etop, be - bs)) {
             if (tid == 0) fb_items[atomicAdd(fb_count, 1ull)] = items[ci];
-            __syncthreads();  // s_col / sa / s_emin reuse
+            __syncthreads();  // sm.col / sm.a / sm.emin reuse
             continue;
         }
+        if (tid == 0) sm.ebase = ebase;  // read behind the barriers of the chunk tables
         XPROF_LAP(0);
 
-        // dense visit helpers: products of a chunk into the word accumulator,
-        // and the write-out of tile row0's touched rows
-        // (the loads of the next 32-product window are issued before the
-        // current window's atomics, so their latency overlaps them)
-        auto dense_products = [&](int L, int nseg, int row0) {
-            const int span = (((L + NW - 1) / NW) + 31) & ~31;
-            const int wb = warp * span, we = min(L, wb + span);
-            if (wb >= we) return;
-            int bcur = chunk_find_nz(ch, nseg, wb);
-            int r_n = 0;
-            uint64_t a_n = 0, b_n = 0;
-            bool v_n = false;
-            auto load = [&](int p0) {
-                const int p = p0 + lane;
-                const int b = window_seg(ch, nseg, bcur, p);
-                v_n = p < we;
-                if (v_n) {
-                    const int64_t idx = (uint32_t)(ch.base[b] + (uint32_t)p);
-                    r_n = a.arow[idx] - row0;
-                    a_n = (uint64_t)__double_as_longlong(aval ? aval[idx] : 1.0);
-                    b_n = (uint64_t)__double_as_longlong(bval ? bval[bs + ch_e[b]] : 1.0);
+        // ---- a ranked visit's steps.  Rows are relative to the visit's first row row0.
+        auto mark = [&](int L, int row0) {
+            const int32_t *arow = sm.a.arow;
+            rounds(L, false, [&](int q0, int n) {
+                for (int w = warp; w * 32 < n; w += 2 * NW) {  // two windows at a time
+                    const int p = w * 32 + lane, p2 = p + NW * 32;
+                    int r = -1, r2 = -1;
+                    if (p < n) r = arow[sm.base[seg_of(w)] + (uint32_t)(q0 + p)] - row0;
+                    if (p2 < n) r2 = arow[sm.base[seg_of(w + NW)] + (uint32_t)(q0 + p2)] - row0;
+                    if (r >= 0) atomicOr(&sm.bm[r >> 5], 1u << (r & 31));
+                    if (r2 >= 0) atomicOr(&sm.bm[r2 >> 5], 1u << (r2 & 31));
                 }
-                int bn = __shfl_sync(0xffffffffu, b, 31);
-                if (bn + 1 < nseg && ch.off[bn + 1] <= p0 + 32) ++bn;
-                bcur = bn;
-            };
-            load(wb);
-            for (int p0 = wb; p0 < we; p0 += 32) {
-                const int r = r_n;
-                const uint64_t av = a_n, bv = b_n;
-                const bool v = v_n;
-                if (p0 + 32 < we) load(p0 + 32);  // warp-uniform
-                if (v && !x_add(acc, RS, tw, s_band, r, av, bv, ebase)) bad = true;
-            }
+            });
         };
-        // (callers end the products with a block barrier)
-        auto dense_writeout = [&](int row0) {
-            // warp w writes the rows of 256-row bands w, w + NW, ... in order;
-            // offsets from the bands' first-touch counts
-            static_assert(RS / 256 <= 32, "bands fit one warp");
-            const int nband = (a.R + 255) >> 8;
-            const int bc = lane < nband ? s_band[lane] : 0;
-            int inc = bc;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += y;
-            }
-            const int tot = __shfl_sync(0xffffffffu, inc, 31);
-            __syncthreads();  // every warp has read the band counts before they are reset
-            XPROF_LAP(16);
-            XPROF_ADD(18, tot);
-            for (int bd = warp; bd < nband; bd += NW) {
-                const int before = __shfl_sync(0xffffffffu, inc - bc, bd);
-                if (lane == 0) s_band[bd] = 0;
-                const int g0 = bd * 8, g1 = min(a.R >> 5, g0 + 8);
-                int64_t pos = out + before;
-            // touched rows of 4 groups at a time listed in order (the chunk
-            // table's space, 128 rows per warp), then converted one per lane
-            uint16_t *wl = reinterpret_cast<uint16_t *>(&ch) + warp * 128;
-            for (int gb = g0; gb < g1; gb += 4) {
-                int n = 0;
-                for (int gg = gb; gg < min(g1, gb + 4); ++gg) {
-                    const int r = gg * 32 + lane;
-                    const bool f = tfb[r] != 0;
-                    const unsigned m = __ballot_sync(0xffffffffu, f);
-                    if (f) wl[n + __popc(m & lt)] = (uint16_t)r;
-                    n += __popc(m);
-                }
-                __syncwarp();
-                for (int k = lane; k < n; k += 32) {
-                    const int r = wl[k];
-                    const double v = x_value(acc, RS, r, tfb[r], ebase);
-                    tfb[r] = 0;
-                    const int64_t q = pos + k;
-                    if (q < lim) {
-                        cir[q] = (int64_t)row0 + r;
-                        cval[q] = v;
-                    } else {
-                        over = true;
+        // Products added into the accumulators: of their row's rank, or of
+        // the row itself (DIRECT, one tile: the row is marked here as well).
+        // The loads of the warp's next window are issued before the current
+        // window's atomics.
+        auto accumulate_as = [&](int L, int row0, auto pos_t, auto direct_t) {
+            constexpr bool POS = decltype(pos_t)::value, DIRECT = decltype(direct_t)::value;
+            const int32_t *arow = sm.a.arow;
+            const double *aval = static_cast<const double *>(sm.a.aval);
+            const int ebase = sm.ebase;
+            rounds(L, true, [&](int q0, int n) {
+                int r_n = -1;
+                double a_n = 0, b_n = 0;
+                auto load = [&](int w) {
+                    const int p = w * 32 + lane;
+                    r_n = -1;
+                    if (p < n) {
+                        const int b = seg_of(w);
+                        const uint32_t idx = sm.base[b] + (uint32_t)(q0 + p);
+                        r_n = arow[idx] - row0;
+                        a_n = aval ? aval[idx] : 1.0;
+                        b_n = sm.bv[b];
+                    }
+                };
+                load(warp);
+                for (int w = warp; w * 32 < n; w += NW) {
+                    const int r = r_n;
+                    const double av = a_n, bv = b_n;
+                    load(w + NW);
+                    if (r >= 0) {
+                        const uint64_t bits = (uint64_t)__double_as_longlong(__dmul_rn(av, bv));
+                        int at = r;
+                        if (DIRECT) {
+                            atomicOr(&sm.bm[r >> 5], 1u << (r & 31));
+                        } else {
+                            at = sm.pre[r >> 5] + __popc(sm.bm[r >> 5] & ((1u << (r & 31)) - 1));
+                            sm.rows[at] = (uint16_t)r;  // every product of the row writes the same
+                        }
+                        if (!POS && (bits << 1) == 0) {
+                            if (bits) sm.negzero = 1;
+                        } else if (!x_add128<POS>(sm.acc + at, R, bits, ebase)) {
+                            bad = true;
+                        }
                     }
                 }
-                pos += n;
-                __syncwarp();
-            }
-            }
-            out += tot;
-            XPROF_LAP(17);
-            __syncthreads();
+            });
         };
-        auto clean_words = [&]() {
+        auto accumulate = [&](int L, int row0, auto direct_t) {
+            if (pos)
+                accumulate_as(L, row0, std::true_type{}, direct_t);
+            else
+                accumulate_as(L, row0, std::false_type{}, direct_t);
+        };
+        // ranks of the touched rows among the first nw bitmap words (at most
+        // 4 per thread); *before(t) is left in pre[]; returns the total
+        auto rank_rows = [&](int nw) -> int {
+            constexpr int PER = kXSpanTiles * R / 32 / NT;
+            const int per = (nw + NT - 1) / NT;  // block-uniform
+            int pc[PER], sum = 0;
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                const int w = tid * per + u;
+                pc[u] = (u < per && w < nw) ? __popc(sm.bm[w]) : 0;
+                sum += pc[u];
+            }
+            int tot;
+            int run = block_prefix(sum, &tot);
+#pragma unroll
+            for (int u = 0; u < PER; ++u) {
+                const int w = tid * per + u;
+                if (u < per && w < nw) sm.pre[w] = (uint16_t)run;
+                run += pc[u];
+            }
+            __syncthreads();
+            return tot;
+        };
+        // accumulator `at` (row row0 + r) rounded and written as output entry q of the visit, and cleared
+        auto write_one = [&](int at, int q, int r, int row0) {
+            uint32_t *w = sm.acc + at;
+            const uint64_t lo = w[0] | ((uint64_t)w[R] << 32), hi = w[2 * R] | ((uint64_t)w[3 * R] << 32);
+            w[0] = 0;
+            w[R] = 0;
+            w[2 * R] = 0;
+            w[3 * R] = 0;
+            const double v = x_round(hi, lo, 2, sm.ebase);
+            q += out;
+            if (q < sm.lim) {
+                sm.oir[q] = row0 + r;
+                sm.oval[q] = v;
+            } else {
+                over = true;
+            }
+        };
+        auto end_visit = [&](int n) {
+            __syncthreads();
+            if (sm.negzero) {  // block-uniform
+                x_fix_zeros(sm, out, min(out + n, sm.lim));
+                __syncthreads();
+                if (tid == 0) sm.negzero = 0;  // read again only after another visit's barriers
+            }
+            out += n;
+        };
+        // a ranked visit's n entries; the bitmap's first nw words are cleared
+        auto write_ranks = [&](int n, int nw, int row0) {
+            for (int q = tid; q < n; q += NT) write_one(q, q, sm.rows[q], row0);
+            for (int w = tid; w < nw; w += NT) sm.bm[w] = 0;
+            end_visit(n);
+        };
+        // a direct visit's entries: a warp per bitmap word
+        auto write_direct = [&](int nw, int row0) {
+            const int n = rank_rows(nw);
+            for (int w = warp; w < nw; w += NW) {
+                const uint32_t x = sm.bm[w];
+                if ((x >> lane) & 1) write_one(w * 32 + lane, sm.pre[w] + __popc(x & lt), w * 32 + lane, row0);
+                __syncwarp();
+                if (lane == 0) sm.bm[w] = 0;
+            }
+            end_visit(n);
+        };
+        auto clean = [&]() {
             if (dirty) {
-                for (int u = tid; u < kXW * RS; u += NT) xsm[u] = 0;
+                for (int u = tid; u < 4 * R; u += NT) sm.acc[u] = 0;
                 dirty = false;
                 __syncthreads();
             }
         };
 
         // ------------------------------------------------ 1. bucketing
-        bool bucketed = a.T <= TM && a.ktl_ptr != nullptr;  // block-uniform
+        bool bucketed = a.T <= kXTMax && a.ktl_ptr != nullptr;  // block-uniform
         if (bucketed) {
-            for (int u = tid; u < a.T; u += NT) {
-                s_segcnt[u] = 0;
-                s_prodcnt[u] = 0;
-            }
-            __syncthreads();
             // pass 0 counts, pass 1 scatters: the (entry, tile) pairs of a
-            // chunk of NT entries are flattened over the warps like products
+            // chunk of entries are flattened over the warps like products
             for (int pass = 0; pass < 2; ++pass) {
-                for (int64_t cb = bs; cb < be; cb += NT) {
-                    const int64_t e = cb + tid;
-                    uint32_t s0 = 0;
-                    int len = 0;
-                    if (e < be) {
-                        const int k = a.brow[e];
-                        const int64_t p0 = a.ktl_ptr[k];
-                        s0 = (uint32_t)p0;
-                        len = (int)(a.ktl_ptr[k + 1] - p0) - 1;  // touched tiles (the end marker excluded)
+                for (int64_t cb = bs; cb < be; cb += kXSegs) {
+                    uint32_t st[2];
+                    int ln[2];
+                    double en[2];  // the entry, carried in the table's value slot
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int64_t e = cb + 2 * tid + u;
+                        st[u] = 0;
+                        ln[u] = 0;
+                        en[u] = __longlong_as_double(e - bs);
+                        if (e < be) {
+                            const int k = a.brow[e];
+                            const int64_t p0 = a.ktl_ptr[k];
+                            st[u] = (uint32_t)p0;
+                            ln[u] = (int)(a.ktl_ptr[k + 1] - p0) - 1;  // touched tiles (the end marker excluded)
+                        }
                     }
-                    int nseg;
-                    const int L = compact_chunk<uint32_t, NT>(ch, s0, len, (uint32_t)(e - bs), ch_e, nseg);
-                    for_products(L, nseg, [&](int b, int64_t q, int) {
+                    const int L = fill_table(st, ln, en, true);
+                    for_products(L, false, [&](int b, uint32_t q, int) {
                         const int t = a.ktl_tile[q];
-                        const uint32_t st = a.ktl_start[q];
-                        const int ln = (int)(a.ktl_start[q + 1] - st);
+                        const uint32_t s0 = a.ktl_start[q];
+                        const int len = (int)(a.ktl_start[q + 1] - s0);
                         if (pass == 0) {
-                            atomicAdd(&s_segcnt[t], 1);
-                            atomicAdd(&s_prodcnt[t], ln);
+                            atomicAdd(&sm.segcnt[t], 1);
+                            atomicAdd(&sm.prodcnt[t], len);
                         } else {
-                            const int pos = atomicAdd(&s_off[t], 1);
-                            scratch[pos] = XSeg{st, (uint32_t)ln, ch_e[b]};
+                            const int pos = atomicAdd(&sm.tend[t], 1);
+                            scratch[pos] = XSeg{s0, (uint32_t)len, (uint32_t)__double_as_longlong(sm.bv[b])};
                         }
                     });
+                    __syncthreads();
                 }
-                __syncthreads();
                 if (pass == 0) {
                     // tile offsets; a column with too many segments is not bucketed
                     int tot;
-                    const int ex = block_prefix(tid < a.T ? s_segcnt[tid] : 0, &tot);
-                    if (tot > kXScap) {
+                    const int ex = block_prefix(tid < a.T ? sm.segcnt[tid] : 0, &tot);
+                    if (tot > scap) {
                         bucketed = false;  // block-uniform: tot is
                         break;
                     }
-                    if (tid < a.T) s_off[tid] = ex;
+                    if (tid < a.T) sm.tend[tid] = ex;
                     __syncthreads();
                 }
             }
-            // s_off[t] is now the end of tile t's segments
+            // tend[t] is now the end of tile t's segments
             XPROF_LAP(1);
             XPROF_ADD(bucketed ? 11 : 12, 1);
         }
 
+        // segments [c0, min(c0 + kXSegs, se)) of the scratch: this thread's two
+        auto fetch = [&](XSeg (&sg)[2], int c0, int se) {
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int c = c0 + 2 * tid + u;
+                sg[u] = c < se ? scratch[c] : XSeg{0, 0, 0};
+            }
+        };
+        auto load_bucket = [&](const XSeg (&sg)[2]) -> int {
+            const uint32_t st[2] = {sg[0].start, sg[1].start};
+            const int ln[2] = {(int)sg[0].len, (int)sg[1].len};
+            double bv[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const double *b = static_cast<const double *>(sm.a.bval);
+                bv[u] = b ? b[sm.bs + sg[u].e] : 1.0;
+            }
+            return fill_table(st, ln, bv, false);
+        };
+        // The next run from tile t on (lanes hold one tile each): t its first
+        // touched tile (a.T: none), t1 its end.  Of p products over R rows
+        // about p / (1 + p / R) rows are expected.
+        int t = 0, t1 = 0, segs = 0, prods = 0;
+        bool direct = false;
+        auto next_run = [&]() {
+            for (; t < a.T; t += 32) {
+                const unsigned m = __ballot_sync(0xffffffffu, t + lane < a.T && sm.segcnt[t + lane] > 0);
+                if (m) {
+                    t += __ffs(m) - 1;
+                    break;
+                }
+            }
+            if (t >= a.T) {
+                t = t1 = a.T;
+                return;
+            }
+            const int u = t + lane;
+            const bool in = lane < kXSpanTiles && u < a.T;
+            int s = in ? sm.segcnt[u] : 0, p = in ? sm.prodcnt[u] : 0;
+            const bool some = s > 0, heavy = p > kXDirect;
+            int e = p >= 8 * R ? R : (int)__fdividef((float)p, 1.0f + (float)p * (1.0f / R));
+#pragma unroll
+            for (int o = 1; o < kXSpanTiles; o <<= 1) {
+                const int se = __shfl_up_sync(0xffffffffu, s, o), pe = __shfl_up_sync(0xffffffffu, p, o),
+                          ee = __shfl_up_sync(0xffffffffu, e, o);
+                if (lane >= o) {
+                    s += se;
+                    p += pe;
+                    e += ee;
+                }
+            }
+            const bool fits = in && !heavy && e <= R && s <= kXSegs && p <= kXWins * 32;
+            const unsigned tm = __ballot_sync(0xffffffffu, some);
+            unsigned ok = __ballot_sync(0xffffffffu, fits);
+            direct = !(ok & 1);  // the first tile does not fit a ranked visit: a visit of its own
+            if (direct) ok = 1;
+            // tiles before the first that does not fit, less untouched ones at the end
+            const unsigned run = tm & ((ok + 1) & ~ok) - 1;
+            const int last = 31 - __clz(run);
+            t1 = t + last + 1;
+            segs = __shfl_sync(0xffffffffu, s, last);
+            prods = __shfl_sync(0xffffffffu, p, last);
+        };
+
         if (bucketed) {
             // -------------------------------------------- 2. visits in row order
-            int t = 0;
+            XSeg sg[2];
+            next_run();
             while (t < a.T) {
-                const int nsg = s_segcnt[t];
-                if (nsg == 0) {
-                    ++t;
-                    continue;
-                }
-                if (s_prodcnt[t] > kXDense) {
-                    // dense visit of tile t
-                    clean_words();
-                    const int row0 = t * a.R;
-                    const int sb = s_off[t] - nsg;
-                    int since_norm = 0;
-                    for (int c0 = 0; c0 < nsg; c0 += NT) {
-                        const int nent = min(NT, nsg - c0);
-                        if (since_norm + nent > kXNorm) {
-                            __syncthreads();
-                            for (int r = tid; r < a.R; r += NT)
-                                if (tfb[r]) x_normalise(acc, RS, r);
-                            since_norm = 0;
+                const int row0 = t * R;
+                const int sb = sm.tend[t] - sm.segcnt[t];
+                if (direct || prods > kXLight) {
+                    clean();
+                    int nw = (int)((min(t1 * (int64_t)R, a.m) - row0 + 31) >> 5);
+                    int n = 0;
+                    if (direct) {
+                        for (int c0 = sb; c0 < sb + segs; c0 += kXSegs) {
+                            fetch(sg, c0, sb + segs);
+                            if (c0 > sb) __syncthreads();
+                            accumulate(load_bucket(sg), row0, std::true_type{});
                         }
-                        since_norm += nent;
-                        uint32_t s0 = 0, e0 = 0;
-                        int len = 0;
-                        if (tid < nent) {
-                            const XSeg sg = scratch[sb + c0 + tid];
-                            s0 = sg.start;
-                            len = (int)sg.len;
-                            e0 = sg.e;
+                        XPROF_ADD(20, 1);
+                        XPROF_ADD(21, prods);
+                    } else {
+                        fetch(sg, sb, sb + segs);
+                        int L = load_bucket(sg);
+                        mark(L, row0);
+                        __syncthreads();
+                        XPROF_LAP(2);
+                        n = rank_rows(nw);
+                        if (n > R) {
+                            // too many rows: keep the first tiles that fit
+                            while (n > R) {
+                                --t1;
+                                L -= sm.prodcnt[t1];
+                                n = sm.pre[(t1 - t) * (R / 32)];
+                            }
+                            for (int w = (t1 - t) * (R / 32) + tid; w < nw; w += NT) sm.bm[w] = 0;
+                            nw = (t1 - t) * (R / 32);
                         }
-                        int nseg;
-                        const int L = compact_chunk<uint32_t, NT>(ch, s0, len, e0, ch_e, nseg);
-                        dense_products(L, nseg, row0);
-                        XPROF_ADD(14, L);
+                        XPROF_LAP(3);
+                        accumulate(L, row0, std::false_type{});
+                        XPROF_ADD(8, 1);
+                        XPROF_ADD(18, n);
+                        XPROF_ADD(19, L);
                     }
+                    if (tid == 0) atomicAdd(&work[t1 - t > 1 ? 2 : 1], 1ull);  // visits of one tile / of a run
                     __syncthreads();
-                    XPROF_LAP(2);
-                    dense_writeout(row0);
-                    XPROF_LAP(3);
-                    XPROF_ADD(8, 1);
-                    if (tid == 0) atomicAdd(&work[1], 1ull);  // dense visits (statistics)
-                    ++t;
-                } else {
-                    // range visit of light tiles t .. t1 (at most kXRange products)
-                    int t1 = t, prods = s_prodcnt[t];
-                    while (t1 + 1 < a.T && (s_segcnt[t1 + 1] == 0 ||
-                                            (s_prodcnt[t1 + 1] <= kXDense && prods + s_prodcnt[t1 + 1] <= XR))) {
-                        ++t1;
-                        prods += s_prodcnt[t1];
+                    if (direct) {
+                        XPROF_LAP(22);
+                        write_direct(nw, row0);
+                        XPROF_LAP(23);
+                    } else {
+                        XPROF_LAP(4);
+                        write_ranks(n, nw, row0);
+                        XPROF_LAP(5);
                     }
-                    while (s_segcnt[t1] == 0) --t1;  // end on a touched tile
-                    const int rbase = t * a.R;
-                    const int span_rows = (t1 - t + 1) * a.R;  // <= 2^20
-                    const int sb = s_off[t] - s_segcnt[t], se = s_off[t1];
+                    t = t1;
+                    next_run();
+                } else {
+                    // sorted range of light tiles t .. t1 (at most kXSort products)
+                    t1 = t;
+                    prods = sm.prodcnt[t];
+                    while (t1 + 1 < a.T && (sm.segcnt[t1 + 1] == 0 || (sm.prodcnt[t1 + 1] <= kXLight &&
+                                                                       prods + sm.prodcnt[t1 + 1] <= kXSort))) {
+                        ++t1;
+                        prods += sm.prodcnt[t1];
+                    }
+                    while (sm.segcnt[t1] == 0) --t1;  // end on a touched tile
+                    const int span_rows = (t1 - t + 1) * R;  // <= 2^20
+                    const int se = sm.tend[t1];
                     dirty = true;
-                    // stage: key = (row - rbase) << 12 | slot, value = the product
+                    // stage: key = (row - row0) << 12 | slot, value = the product
                     int pbase = 0;
-                    for (int c0 = sb; c0 < se; c0 += NT) {
-                        uint32_t s0 = 0, e0 = 0;
-                        int len = 0;
-                        if (c0 + tid < se) {
-                            const XSeg sg = scratch[c0 + tid];
-                            s0 = sg.start;
-                            len = (int)sg.len;
-                            e0 = sg.e;
-                        }
-                        int nseg;
-                        const int L = compact_chunk<uint32_t, NT>(ch, s0, len, e0, ch_e, nseg);
-                        for_products(L, nseg, [&](int b, int64_t idx, int p) {
+                    for (int c0 = sb; c0 < se; c0 += kXSegs) {
+                        fetch(sg, c0, se);
+                        const int L = load_bucket(sg);
+                        const int32_t *arow = sm.a.arow;
+                        const double *aval = static_cast<const double *>(sm.a.aval);
+                        for_products(L, false, [&](int b, uint32_t idx, int p) {
                             const int slot = pbase + p;
-                            const double av = aval ? aval[idx] : 1.0;
-                            const double bv = bval ? bval[bs + ch_e[b]] : 1.0;
-                            rk0[slot] = ((uint32_t)(a.arow[idx] - rbase) << 12) | (uint32_t)slot;
-                            rval[slot] = x_mul_bits((uint64_t)__double_as_longlong(av),
-                                                    (uint64_t)__double_as_longlong(bv));
+                            rk0[slot] = ((uint32_t)(arow[idx] - row0) << 12) | (uint32_t)slot;
+                            rval[slot] =
+                                (uint64_t)__double_as_longlong(__dmul_rn(aval ? aval[idx] : 1.0, sm.bv[b]));
                         });
                         pbase += L;
                         __syncthreads();  // chunk table reuse
                     }
-                    XPROF_LAP(4);
+                    XPROF_LAP(6);
                     XPROF_ADD(9, 1);
-                    if (tid == 0) atomicAdd(&work[2], 1ull);  // range visits (statistics)
                     XPROF_ADD(13, prods);
+                    if (tid == 0) atomicAdd(&work[2], 1ull);
                     // stable LSD radix sort of the keys by row, 7-bit digits:
                     // warp w owns a contiguous run of keys, counts its digits,
                     // the (digit, warp) counts are scanned digit-major, and
@@ -818,7 +966,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
                         src = dst;
                         dst = tmp;
                     }
-                    XPROF_LAP(5);
+                    XPROF_LAP(7);
                     // runs of one row, one sorted key per thread and round:
                     // the thread holding a run's first key sums the run
                     // exactly (runs are short: a range's rows rarely repeat)
@@ -831,7 +979,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
                         const uint32_t key = act ? src[u] : 0u;
                         const bool head = act && (u == 0 || (src[u - 1] >> 12) != (key >> 12));
                         int tot;
-                        const int64_t q = out + block_prefix(head ? 1 : 0, &tot);
+                        const int q = out + block_prefix(head ? 1 : 0, &tot);
                         if (head) {
                             const uint32_t row = key >> 12;
                             uint64_t hi = 0, lo = 0;
@@ -842,9 +990,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
                                 if (!x_acc128(hi, lo, fl, __longlong_as_double((long long)rval[kv & 4095]), ebase))
                                     bad = true;
                             }
-                            if (q < lim) {
-                                cir[q] = (int64_t)rbase + (int64_t)row;
-                                cval[q] = x_round(hi, lo, fl, ebase);
+                            if (q < sm.lim) {
+                                sm.oir[q] = (int64_t)row0 + (int64_t)row;
+                                sm.oval[q] = x_round(hi, lo, fl, ebase);
                             } else {
                                 over = true;
                             }
@@ -852,13 +1000,14 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
                         out += tot;
                     }
                     __syncthreads();
-                    XPROF_LAP(6);
+                    XPROF_LAP(10);
                     t = t1 + 1;
+                    next_run();
                 }
             }
         } else {
             // ------------------------- enumeration mode: per tile, all entries
-            clean_words();
+            clean();
             int mwi = 0;
             uint64_t msk = a.tmask[i * a.mask_words];
             auto next_tile = [&]() -> int {
@@ -870,44 +1019,38 @@ __global__ void __launch_bounds__(NT, 1024 / NT)
                 msk &= msk - 1;
                 return tt;
             };
-            int t = next_tile();
-            while (t >= 0) {
-                const int tn = next_tile();
-                const int row0 = t * a.R;
-                int since_norm = 0;
-                for (int64_t cb = bs; cb < be; cb += NT) {
-                    const int nent = (int)min((int64_t)NT, be - cb);
-                    if (since_norm + nent > kXNorm) {
-                        __syncthreads();
-                        for (int r = tid; r < a.R; r += NT)
-                            if (tfb[r]) x_normalise(acc, RS, r);
-                        since_norm = 0;
+            for (t = next_tile(); t >= 0; t = next_tile()) {
+                const int row0 = t * R;
+                const int nw = (int)((min((int64_t)(t + 1) * R, a.m) - row0 + 31) >> 5);
+                for (int64_t cb = bs; cb < be; cb += kXSegs) {
+                    uint32_t st[2];
+                    int ln[2];
+                    double bv[2];
+#pragma unroll
+                    for (int u = 0; u < 2; ++u) {
+                        const int64_t e = cb + 2 * tid + u;
+                        st[u] = 0;
+                        ln[u] = 0;
+                        bv[u] = 1.0;
+                        if (e < be) {
+                            const uint32_t *tp = a.tptr + (int64_t)a.brow[e] * (a.T + 1);
+                            st[u] = tp[t];
+                            ln[u] = (int)(tp[t + 1] - st[u]);
+                            if (bval) bv[u] = bval[e];
+                        }
                     }
-                    since_norm += nent;
-                    const int64_t e = cb + tid;
-                    uint32_t s0 = 0;
-                    int len = 0;
-                    if (e < be) {
-                        const uint32_t *tp = a.tptr + (int64_t)a.brow[e] * (a.T + 1);
-                        s0 = tp[t];
-                        len = (int)(tp[t + 1] - s0);
-                    }
-                    int nseg;
-                    const int L = compact_chunk<uint32_t, NT>(ch, s0, len, (uint32_t)(e - bs), ch_e, nseg);
-                    dense_products(L, nseg, row0);
+                    accumulate(fill_table(st, ln, bv, true), row0, std::true_type{});
+                    __syncthreads();
                 }
-                __syncthreads();
-                dense_writeout(row0);
-                XPROF_LAP(7);
-                XPROF_ADD(10, 1);
-                t = tn;
+                write_direct(nw, row0);
+                XPROF_LAP(12);
             }
         }
         over = __syncthreads_or(over);
         bad = __syncthreads_or(bad);
         XPROF_LAP(15);
         if (tid == 0) {
-            if (out_cnt) out_cnt[g] = out - out0;
+            if (out_cnt) out_cnt[g] = out;
             if (over) {
                 if (overflow)
                     overflow[g] = 1;
