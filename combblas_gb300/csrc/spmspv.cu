@@ -26,7 +26,24 @@ namespace gbc {
 
 constexpr int32_t kNoCand = INT32_MAX;
 
+// State of the multi-source traversals with one bit per root (msbfs_bits.cuh).
+struct MsBits {
+    int form = 0;  // of the graph's pattern: 0 not looked at, 1 symmetric with ascending columns, 2 other
+    int words = 0;                              // 64-bit words per vertex that the arrays are sized for
+    uint64_t *seen = nullptr;                   // [n * words] roots that have reached a vertex
+    uint64_t *bits[2] = {nullptr, nullptr};     // frontier words (current / next)
+    int32_t *list[2] = {nullptr, nullptr};      // vertices with a bit in them
+    uint32_t *touched = nullptr;                // [n / 32] vertices already in the next list (push levels)
+    int32_t *item_v = nullptr;                  // chunks of the vertices with many neighbours
+    uint32_t *item_p = nullptr;
+    int64_t nitems = 0;
+    int64_t *ctl = nullptr, *h_ctl = nullptr;   // control block (MB_*) and its pinned mirror
+    cudaGraphExec_t exec[4] = {};               // a pass for 1, 2, 4, 8 words
+    long long kernels = 0;                      // kernels of one level
+};
+
 struct Graph {
+    MsBits mb;
     Context *ctx = nullptr;
     int64_t n = 0, nnz = 0;
     int64_t *cp = nullptr;   // [n+1] (int64 for the caller-facing degree sums)
@@ -1251,6 +1268,8 @@ static int msbfs_device(Graph *g, const int64_t *d_roots, int64_t nroots, int64_
 
 }  // namespace gbc
 
+#include "msbfs_bits.cuh"
+
 using namespace gbc;
 
 struct gbc_graph : gbc::Graph {};
@@ -1307,6 +1326,7 @@ int gbc_graph_destroy(gbc_graph *g)
     if (g->level_exec) cudaGraphExecDestroy(g->level_exec);
     if (g->loop_exec) cudaGraphExecDestroy(g->loop_exec);
     ms_free(g);
+    mb_free(g);
     device_free(c, g->cp);
     device_free(c, g->cp32);
     device_free(c, g->row);
@@ -1446,7 +1466,15 @@ int gbc_msbfs(gbc_context *ctx, gbc_graph *g, const int64_t *roots, int64_t nroo
     const int64_t cells = nroots * g->n;
     int64_t *dp = parents;
     if (where == GBC_HOST) GBC_TRY(ws.alloc_n(&dp, cells));
-    GBC_TRY(msbfs_device(g, d_roots, nroots, dp, st));
+    // One bit per root needs a symmetric pattern with ascending columns (and
+    // the traversal graph); other patterns expand (root, vertex) pairs.
+    GBC_TRY(mb_prepare(g));
+    const int rc = g->mb.form == 1 ? mb_msbfs(g, d_roots, nroots, dp, st) : GBC_EUNSUPPORTED;
+    if (g->mb.form == 1 && rc != GBC_OK && rc != GBC_ECUDA) return rc;
+    if (rc != GBC_OK) {
+        if (g->mb.form == 1) g->mb.form = 2;  // the driver cannot build the while node
+        GBC_TRY(msbfs_device(g, d_roots, nroots, dp, st));
+    }
     if (where == GBC_HOST) {
         GBC_CUDA_TRY(cudaMemcpyAsync(parents, dp, cells * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
         GBC_CUDA_TRY(cudaStreamSynchronize(s));
