@@ -183,6 +183,100 @@ __device__ __forceinline__ int window_seg(const ChunkSmemN<NT> &ch, int nseg, in
     return bcur + c;
 }
 
+// A chunk of up to 2 NT segments of A without a search per product: product p
+// of the chunk belongs to segment win[w].y - 1 + (starts up to p in win[w].x)
+// of window w = p / 32, and sits at position base[segment] + p of A.  win
+// covers a round of NT windows; longer chunks go through several.
+template <int NT>
+struct SegTable {
+    uint32_t base[2 * NT];    // segment start - products before it (modulo 2^32)
+    int32_t off[2 * NT + 1];  // products before each segment
+    int32_t nseg;
+    uint2 win[NT];            // starts in the window (bit i: at its i-th product); segments that start before it
+    int64_t wsum[NT / 32];
+};
+
+// Segment i holds products [p, p + len), counted from the round's first.
+template <int NT>
+__device__ __forceinline__ void seg_windows(SegTable<NT> &t, int i, int p, int len)
+{
+    if (len <= 0) return;
+    if (p >= 0 && p < NT * 32) atomicOr(&t.win[p >> 5].x, 1u << (p & 31));
+    // windows that start inside this segment or right behind it
+    for (int w = max(0, (p >> 5) + 1); w <= min(NT - 1, (p + len) >> 5); ++w) t.win[w].y = i + 1;
+}
+
+// The table from two consecutive segments per thread, empty ones dropped.
+// Barriers: one inside, one at the end; readers of the last table are behind
+// a barrier of the caller.  Returns the chunk's products.
+template <int NT>
+__device__ __forceinline__ int seg_fill(SegTable<NT> &t, const uint32_t (&st)[2], const int (&ln)[2])
+{
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    t.win[tid] = make_uint2(0u, 0u);
+    // products (high word) and non-empty segments (low word) in one prefix
+    const int64_t v = ((int64_t)(ln[0] + ln[1]) << 32) | (int64_t)((ln[0] > 0) + (ln[1] > 0));
+    int64_t x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) t.wsum[warp] = x;
+    __syncthreads();
+    int64_t before = 0, all = 0;
+#pragma unroll
+    for (int u = 0; u < NT / 32; ++u) {
+        const int64_t ws = t.wsum[u];
+        before += u < warp ? ws : 0;
+        all += ws;
+    }
+    before += x - v;
+    int p = (int)(before >> 32), c = (int)(before & 0xffffffff);
+#pragma unroll
+    for (int u = 0; u < 2; ++u)
+        if (ln[u] > 0) {
+            t.off[c] = p;
+            t.base[c] = st[u] - (uint32_t)p;
+            seg_windows<NT>(t, c, p, ln[u]);
+            p += ln[u];
+            ++c;
+        }
+    if (tid == 0) {
+        t.nseg = (int)(all & 0xffffffff);
+        t.off[t.nseg] = (int)(all >> 32);
+    }
+    __syncthreads();
+    return (int)(all >> 32);
+}
+
+// step(q0, n) for the rounds of the chunk's L products: n of them from q0 on,
+// win set for them.  The caller's barrier ends the last round.
+template <int NT, class F>
+__device__ __forceinline__ void seg_rounds(SegTable<NT> &t, int L, F &&step)
+{
+    for (int q0 = 0; q0 < L; q0 += NT * 32) {
+        if (q0 > 0) {
+            __syncthreads();
+            t.win[threadIdx.x] = make_uint2(0u, 0u);
+            __syncthreads();
+            for (int i = 2 * threadIdx.x; i < min(2 * (int)threadIdx.x + 2, t.nseg); ++i)
+                seg_windows<NT>(t, i, t.off[i] - q0, t.off[i + 1] - t.off[i]);
+            __syncthreads();
+        }
+        step(q0, min(L - q0, NT * 32));
+    }
+}
+
+// A position of the round's product w * 32 + lane (q0 the round's first product).
+template <int NT>
+__device__ __forceinline__ uint32_t seg_pos(const SegTable<NT> &t, int w, int q0)
+{
+    const int lane = threadIdx.x & 31;
+    const uint2 x = t.win[w];
+    return t.base[(int)x.y + __popc(x.x & (0xffffffffu >> (31 - lane))) - 1] + (uint32_t)(q0 + w * 32 + lane);
+}
+
 inline size_t numeric_smem_bytes(int R, size_t vsize, int sub)
 {
     // acc[R] + sval[sub] (values) + bitmap[R/32] + srow[sub] (u16) + tag[R] (u8)
