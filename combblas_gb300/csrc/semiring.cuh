@@ -1,7 +1,9 @@
 // Device semirings: one static-method struct per reference semiring, the same
 // shape as the reference's SR::multiply / SR::add / SR::id (Semirings.h).
 // one() is the value of an entry stored without a value array (a pattern
-// matrix); unit() is the multiplicative identity: mul(unit(), x) == x.
+// matrix); unit() is the multiplicative identity: mul(unit(), x) == x; zero() an
+// accumulator that the first product replaces: add(x, zero()) == x for every x
+// (-0.0 for floating sums, so that a lone -0.0 stays one).
 // Floating-point multiply and add use the _rn intrinsics so that the
 // compiler can never fuse them into an FMA: each product is rounded before
 // it is added, as in the reference's `SR::add(SR::multiply(a, b), acc)`.
@@ -22,6 +24,7 @@ struct PlusTimes<double> {
     static __device__ __forceinline__ V add(V a, V b) { return __dadd_rn(a, b); }
     static __host__ __device__ __forceinline__ V one() { return 1.0; }
     static __host__ __device__ __forceinline__ V unit() { return 1.0; }
+    static __device__ __forceinline__ V zero() { return -0.0; }
 };
 
 template <>
@@ -31,6 +34,7 @@ struct PlusTimes<float> {
     static __device__ __forceinline__ V add(V a, V b) { return __fadd_rn(a, b); }
     static __host__ __device__ __forceinline__ V one() { return 1.0f; }
     static __host__ __device__ __forceinline__ V unit() { return 1.0f; }
+    static __device__ __forceinline__ V zero() { return -0.0f; }
 };
 
 // Integer PlusTimes wraps modulo 2^64 (the reference's signed overflow on
@@ -42,6 +46,7 @@ struct PlusTimes<int64_t> {
     static __device__ __forceinline__ V add(V a, V b) { return (V)((uint64_t)a + (uint64_t)b); }
     static __host__ __device__ __forceinline__ V one() { return 1; }
     static __host__ __device__ __forceinline__ V unit() { return 1; }
+    static __device__ __forceinline__ V zero() { return 0; }
 };
 
 // PlusTimesSRing<bool,bool>: promote_trait<bool,bool> is bool, so add is
@@ -52,6 +57,7 @@ struct BoolOrAnd {
     static __device__ __forceinline__ V add(V a, V b) { return (V)((a != 0) | (b != 0)); }
     static __host__ __device__ __forceinline__ V one() { return 1; }
     static __host__ __device__ __forceinline__ V unit() { return 1; }
+    static __device__ __forceinline__ V zero() { return 0; }
 };
 
 // MinPlusSRing (Semirings.h:235-255) with inf_plus (Semirings.h:40-47):
@@ -67,6 +73,7 @@ struct MinPlus<double> {
     static __device__ __forceinline__ V add(V a, V b) { return (b < a) ? b : a; }  // std::min(a, b)
     static __host__ __device__ __forceinline__ V one() { return 1.0; }
     static __host__ __device__ __forceinline__ V unit() { return 0.0; }
+    static __device__ __forceinline__ V zero() { return __longlong_as_double(0x7ff0000000000000ll); }
 };
 
 template <>
@@ -80,6 +87,7 @@ struct MinPlus<int64_t> {
     static __device__ __forceinline__ V add(V a, V b) { return (b < a) ? b : a; }
     static __host__ __device__ __forceinline__ V one() { return 1; }
     static __host__ __device__ __forceinline__ V unit() { return 0; }
+    static __device__ __forceinline__ V zero() { return INT64_MAX; }
 };
 
 // Select2ndMinSR (Applications/FastSV.h:25-44): multiply returns the second
@@ -91,6 +99,7 @@ struct Select2ndMin {
     static __device__ __forceinline__ V add(V a, V b) { return (b < a) ? b : a; }
     static __host__ __device__ __forceinline__ V one() { return 1; }
     static __host__ __device__ __forceinline__ V unit() { return 0; }  // any value: mul returns b
+    static __device__ __forceinline__ V zero() { return INT64_MAX; }
 };
 
 }  // namespace gbc

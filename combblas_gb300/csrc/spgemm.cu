@@ -35,6 +35,7 @@
 #include "spgemm_kernels.cuh"
 #include "spgemm_small.cuh"
 #include "spgemm_exact.cuh"
+#include "spgemm_own.cuh"
 #include "mlp.cuh"
 
 namespace gbc {
@@ -208,9 +209,14 @@ constexpr int kWarpClasses = 4;
 // 2*10^7 products, most of one block's share of a phase).
 constexpr int kBigBins = 4;
 constexpr int kBigList = kWarpClasses;            // index of the big list in Lists
-constexpr int kLists = kWarpClasses + kBigBins;  // list slots while classifying
+constexpr int kOwnList = kBigList + 1;            // ... of the columns for k_numeric_own
+constexpr int kOwnSlot = kWarpClasses + kBigBins; // its slot while classifying
+constexpr int kLists = kOwnSlot + 1;              // list slots while classifying
 
-__global__ void k_classify(const int64_t *flop, int pid, int64_t col_base, int64_t j0, int64_t j1, int64_t s1,
+// Of the big columns, those with at least own_need products per B entry (0:
+// none), own_min() for every row range, are listed for k_numeric_own: a
+// range's segments then fill a good part of a 32-product window.
+__global__ void k_classify(const int64_t *flop, const int64_t *bcp, int64_t own_need, int pid, int64_t col_base, int64_t j0, int64_t j1, int64_t s1,
                            int64_t s2, int64_t *lbuf, int64_t stride, unsigned long long *counts, int64_t *cnt_zero,
                            const int32_t *only_flagged)
 {
@@ -225,6 +231,8 @@ __global__ void k_classify(const int64_t *flop, int pid, int64_t col_base, int64
             cls = 0;
         } else if (f <= s2) {
             cls = f <= kSmallMid ? 1 : f <= kSmallMid2 ? 2 : 3;
+        } else if (own_need > 0 && f >= own_need * (bcp[i + 1] - bcp[i])) {
+            cls = kOwnSlot;
         } else {
             cls = kWarpClasses + (f > (1ll << 23) ? 0 : f > (1ll << 21) ? 1 : f > (1ll << 19) ? 2 : 3);
         }
@@ -1056,6 +1064,9 @@ struct Plan {
     XSeg *xscratch = nullptr;            // exact kernel: bucketing scratch, xscap segments per block
     int64_t xscap = 0;                   // (no column has more than its A has tile list entries)
     int x_blocks = 0;                    // exact kernel: its grid (resident blocks)
+    int own_vsize = 0;                   // value size for k_numeric_own (0: not used)
+    bool own_built = false;              // its range tables are there
+    Workspace *ws = nullptr;
     SpgemmArgs &a() { return h[0]; }
 };
 
@@ -1065,6 +1076,8 @@ struct Plan {
 template <class SR>
 static void plan_fold(Context *ctx, Plan &P)
 {
+    if (!(std::is_same<SR, PlusTimes<double>>::value && ctx->fold == GBC_FOLD_EXACT))
+        P.own_vsize = (int)sizeof(typename SR::V);
     if (std::is_same<SR, PlusTimes<double>>::value && ctx->fold == GBC_FOLD_EXACT) {
         P.want_aexp = true;
         P.tile_rows = kXRows;
@@ -1082,13 +1095,14 @@ static bool use_exact(const Plan &P)
 
 struct Lists {
     // [0, kWarpClasses): the warp-kernel classes (up to s1, kSmallMid,
-    // kSmallMid2, s2 multiplications); [kBigList]: the big list
-    const int64_t *l[kWarpClasses + 1] = {};
-    int64_t n[kWarpClasses + 1] = {};
+    // kSmallMid2, s2 multiplications); [kBigList]: the big list;
+    // [kOwnList]: big columns for k_numeric_own
+    const int64_t *l[kWarpClasses + 2] = {};
+    int64_t n[kWarpClasses + 2] = {};
     int64_t total() const
     {
         int64_t t = 0;
-        for (int c = 0; c <= kWarpClasses; ++c) t += n[c];
+        for (int c = 0; c <= kOwnList; ++c) t += n[c];
         return t;
     }
 };
@@ -1125,6 +1139,9 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
     GBC_CUDA_TRY(cudaGetLastError());
     a.flop = flop;
     a.tmask = tmask;
+    a.own_T = P.own_vsize ? own_ranges(A.nrow, A.ncol, P.own_vsize) : 0;
+    a.own_ptr = nullptr;
+    a.own_rb = nullptr;
     a.aexp = nullptr;
     a.ktl_ptr = nullptr;
     a.ktl_start = nullptr;
@@ -1173,8 +1190,45 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
     return GBC_OK;
 }
 
+// The range tables of k_numeric_own, built when a column first needs them.
+static int plan_own(Plan &P)
+{
+    Workspace &ws = *P.ws;
+    Context *ctx = ws.ctx;
+    cudaStream_t s = ctx->stream;
+    for (SpgemmArgs &a : P.h) {
+        if (a.own_T == 0 || a.m == 0) continue;
+        int64_t nnz = 0;
+        GBC_TRY(read_i64(ctx, a.acp + a.kdim, &nnz));
+        if (nnz == 0) continue;
+        int64_t *w = nullptr;
+        uint8_t *range = nullptr;
+        int32_t *rb = nullptr;
+        uint32_t *optr = nullptr;
+        GBC_TRY(ws.alloc_n(&w, a.m + 1));
+        GBC_TRY(ws.alloc_n(&range, a.m));
+        GBC_TRY(ws.alloc_n(&rb, a.own_T + 1));
+        GBC_TRY(ws.alloc_n(&optr, (size_t)a.kdim * (a.own_T + 1)));
+        GBC_CUDA_TRY(cudaMemsetAsync(w, 0, (a.m + 1) * sizeof(int64_t), s));
+        k_own_count<<<(unsigned)((nnz + 255) / 256), 256, 0, s>>>(nnz, a.arow,
+                                                                  reinterpret_cast<unsigned long long *>(w));
+        k_own_weight<<<(unsigned)((a.m + 255) / 256), 256, 0, s>>>(a.m, nnz, w);
+        GBC_TRY(exclusive_scan_i64(ws, w, w, a.m, s));
+        k_own_bounds<<<(unsigned)((a.m + 255) / 256), 256, 0, s>>>(a.m, nnz, a.own_T, w, range, rb);
+        k_own_ptr<<<grid_for(ctx, (a.kdim + 7) / 8, 8), 256, 0, s>>>(a.kdim, a.acp, a.arow, range, a.own_T, optr);
+        note_launches(4);
+        GBC_CUDA_TRY(cudaGetLastError());
+        a.own_ptr = optr;
+        a.own_rb = rb;
+    }
+    GBC_CUDA_TRY(cudaMemcpyAsync(P.d, P.h.data(), P.h.size() * sizeof(SpgemmArgs), cudaMemcpyHostToDevice, s));
+    P.own_built = true;
+    return GBC_OK;
+}
+
 static int plan_finalize(Workspace &ws, Plan &P)
 {
+    P.ws = &ws;
     GBC_TRY(ws.alloc_n(&P.d, P.h.size() + 1));
     GBC_TRY(ws.alloc_n(&P.work, 16));
     GBC_CUDA_TRY(cudaMemsetAsync(P.work, 0, 16 * sizeof(unsigned long long), ws.ctx->stream));
@@ -1224,7 +1278,9 @@ static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j
         const SpgemmArgs &a = P.h[q];
         const int64_t lo = pid >= 0 ? j0 : 0, hi = (pid >= 0 && j1 >= 0) ? j1 : a.nb;
         if (hi > lo) {
-            k_classify<<<(unsigned)((hi - lo + 255) / 256), 256, 0, s>>>(a.flop, q, a.col_base, lo, hi, P.s1, P.s2,
+            k_classify<<<(unsigned)((hi - lo + 255) / 256), 256, 0, s>>>(a.flop, a.bcp, (int64_t)a.own_T * own_min(P.own_vsize),
+                                                                         q, a.col_base, lo, hi,
+                                                                         P.s1, P.s2,
                                                                          P.lbuf, stride, P.lcnt, cnt_zero, flagged);
             note_launch();
         }
@@ -1248,6 +1304,9 @@ static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j
     }
     L.l[kBigList] = lbig;
     L.n[kBigList] = nbig;
+    L.l[kOwnList] = P.lbuf + kOwnSlot * stride;
+    L.n[kOwnList] = (int64_t)h[kOwnSlot];
+    if (L.n[kOwnList] > 0 && !P.own_built) GBC_TRY(plan_own(P));
     return GBC_OK;
 }
 
@@ -1287,6 +1346,15 @@ static int run_symbolic(Context *ctx, Plan &P, const Lists &L, int64_t *cnt)
         GBC_CUDA_TRY(cudaMemsetAsync(P.work, 0, sizeof(unsigned long long), s));
         k_symbolic<<<grid_for(ctx, L.n[kBigList], per_sm), kThreads, sym_smem, s>>>(P.d, L.l[kBigList],
                                                                                      L.n[kBigList], cnt, P.work);
+        note_launch();
+    }
+    if (L.n[kOwnList] > 0) {
+        const size_t sym_smem = P.max_sym_smem;
+        GBC_TRY(set_smem(k_symbolic, sym_smem));
+        const int per_sm = resident_blocks(k_symbolic, kThreads, sym_smem, 8);
+        GBC_CUDA_TRY(cudaMemsetAsync(P.work, 0, sizeof(unsigned long long), s));
+        k_symbolic<<<grid_for(ctx, L.n[kOwnList], per_sm), kThreads, sym_smem, s>>>(P.d, L.l[kOwnList], L.n[kOwnList],
+                                                                                     cnt, P.work);
         note_launch();
     }
     GBC_CUDA_TRY(cudaGetLastError());
@@ -1411,6 +1479,15 @@ static int run_numeric(Context *ctx, Plan &P, const Lists &L, const int64_t *ccp
             GBC_TRY(launch_big_ordered<SR>(ctx, P, L.l[kBigList], L.n[kBigList], nullptr, ccp, ccp_base, cap,
                                            out_cnt, overflow,
                                            cir, cval));
+    }
+    if (L.n[kOwnList] > 0) {
+        constexpr size_t sm = (size_t)kOwnWarps * own_rows(sizeof(typename SR::V)) * (sizeof(typename SR::V) + 1);
+        GBC_TRY(set_smem(k_numeric_own<SR>, sm));
+        const int per_sm = resident_blocks(k_numeric_own<SR>, kOwnThreads, sm, 32);
+        GBC_CUDA_TRY(cudaMemsetAsync(P.work + 4, 0, sizeof(unsigned long long), ctx->stream));
+        k_numeric_own<SR><<<grid_for(ctx, L.n[kOwnList], per_sm), kOwnThreads, sm, ctx->stream>>>(
+            P.d, L.l[kOwnList], L.n[kOwnList], ccp, ccp_base, cap, out_cnt, overflow, cir, cval, P.work + 4);
+        note_launch();
     }
     GBC_CUDA_TRY(cudaGetLastError());
     return GBC_OK;

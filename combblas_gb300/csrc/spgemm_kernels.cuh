@@ -40,6 +40,9 @@ struct SpgemmArgs {
     const int64_t *ktl_ptr;      // exact accumulation: per column of A, its touched row tiles (or nullptr)
     const uint32_t *ktl_start;   //   ... first position of the column inside each listed tile, then the column end
     const uint16_t *ktl_tile;    //   ... the tiles (0xFFFF: end marker)
+    int own_T;                   // row ranges of k_numeric_own (0: none)
+    const uint32_t *own_ptr;     //   ... [kdim][own_T + 1] where every column of A enters them
+    const int32_t *own_rb;       //   ... [own_T + 1] their first rows
 };
 
 // A work item names one output column of one product of a batch.
