@@ -21,10 +21,16 @@
 // per product into a per-row key (min through the complemented order-
 // preserving flip, Select2nd through (column << 32 | vector position)),
 // marking a touched-row bitmap.  Rows come out ascending from a popcount
-// scan of the bitmap.  PlusTimes pushes only the marks, then each touched
-// row is pulled by one warp over its row-major entries (ascending column):
-// lanes test 32 entries against a dense column -> vector position map and
-// form the products, and the products that hit are folded in lane order.
+// scan of the bitmap.  PlusTimes pushes the marks and counts the products per
+// row; the same scan then places every row's products.  A second push writes
+// them (column, product) to their row's place in any order, and each row folds
+// its own in ascending column order: in a thread up to kSxThread products, in a
+// warp up to 32, in a block up to kSxSort.  Longer rows, and all rows of a
+// vector that brings more than 1/kSxPullShare of the matrix, are pulled instead:
+// a warp walks the row's row-major entries (ascending column), tests them
+// against a dense column -> vector position map and folds the hits in order.
+// (Pulling every touched row reads nearly the whole matrix for 2000 entries of
+// 2^18; it took 0.59 of the call's 0.69 ms.)
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -46,6 +52,7 @@ struct SpmspvPlan {
     int vt = 0;
     int64_t *cp = nullptr;   // [n+1] dense column pointers
     int32_t *row = nullptr;  // [nnz]
+    void *cval = nullptr;    // [nnz] values, column-major (numeric value types only)
     SpmvPlan rm;             // row-major form (numeric value types only)
     bool have_rm = false;
     // scratch kept between calls: every call leaves it as it found it
@@ -86,6 +93,13 @@ __global__ void k_sx_prep(int64_t nzc, int64_t m, int64_t n, int64_t nnz, const 
     }
 }
 
+template <typename V>
+__global__ void k_sx_ones(int64_t n, V *v)
+{
+    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (i < n) v[i] = V(1);
+}
+
 // Vector positions of the columns; flags columns out of range (1) and
 // repeated columns (2).
 __global__ void k_sx_xpos(int64_t nx, const int32_t *xind, int64_t n, int32_t *xpos, int32_t *err)
@@ -116,63 +130,113 @@ __device__ __forceinline__ unsigned long long sx_key(int64_t x, int32_t c, int64
     return ((unsigned long long)(uint32_t)c << 32) | (uint32_t)f;  // SX_SELECT2ND
 }
 
-// Push: per product one atomicMax of the column's key into spa[r] (not for
-// PlusTimes) and the touched mark.
+// fn(f, p) for every entry p of the columns of the vector's entries f: blocks
+// take kSxChunk entries at a time, whose products their threads share out (few
+// enough that a vector of 2000 entries keeps 63 blocks busy, not 8).
+constexpr int kSxChunk = 32;
+
+template <class F>
+__device__ __forceinline__ void sx_products(const int64_t *cp, const int32_t *xind, int64_t nx, int64_t n,
+                                            unsigned long long *work, F &&fn)
+{
+    __shared__ int64_t s_seg[kSxChunk];
+    __shared__ int64_t s_off[kSxChunk + 1];
+    __shared__ int64_t s_base;
+    const int tid = threadIdx.x;
+    for (;;) {
+        if (tid < 32) {
+            long long base = 0;
+            if (tid == 0) base = (long long)atomicAdd(work, (unsigned long long)kSxChunk);
+            base = __shfl_sync(0xffffffffu, base, 0);
+            int64_t len = 0;
+            if (base + tid < nx) {
+                const int32_t c = xind[base + tid];
+                if (c >= 0 && c < n) {
+                    s_seg[tid] = cp[c];
+                    len = cp[c + 1] - cp[c];
+                }
+            }
+            int64_t x = len;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int64_t y = __shfl_up_sync(0xffffffffu, x, o);
+                if (tid >= o) x += y;
+            }
+            s_off[tid] = x - len;
+            if (tid == 31) {
+                s_off[32] = x;
+                s_base = base;
+            }
+        }
+        __syncthreads();
+        const int64_t base = s_base, tot = s_off[kSxChunk];
+        if (base >= nx) break;  // block-uniform
+        for (int64_t j = tid; j < tot; j += kSxThreads) {
+            int lo = 0;
+#pragma unroll
+            for (int step = kSxChunk / 2; step; step >>= 1)
+                if (s_off[lo + step] <= j) lo += step;
+            fn(base + lo, s_seg[lo] + (j - s_off[lo]));
+        }
+        __syncthreads();
+    }
+}
+
+// Push: per product one atomicMax of the column's key into spa[r] (PlusTimes:
+// a count) and the touched mark.
 template <int SX>
 __global__ void __launch_bounds__(kSxThreads) k_sx_expand(const int64_t *cp, const int32_t *row, const int32_t *xind,
                                                           const int64_t *xval, int64_t nx, int64_t n,
                                                           unsigned long long *spa, uint32_t *mark,
                                                           unsigned long long *work)
 {
-    __shared__ int64_t s_seg[kSxThreads];
-    __shared__ int64_t s_off[kSxThreads + 1];
-    __shared__ unsigned long long s_key[kSxThreads];
-    __shared__ int64_t s_base;
-    const int tid = threadIdx.x;
-    for (;;) {
-        if (tid == 0) s_base = (int64_t)atomicAdd(work, (unsigned long long)kSxThreads);
-        __syncthreads();
-        const int64_t base = s_base;
-        __syncthreads();
-        if (base >= nx) break;
-        const int64_t f = base + tid;
-        int64_t len = 0;
-        if (f < nx) {
-            const int32_t c = xind[f];
-            if (c >= 0 && c < n) {
-                const int64_t s = cp[c];
-                len = cp[c + 1] - s;
-                s_seg[tid] = s;
-                if (SX != SX_PLUSTIMES) s_key[tid] = sx_key<SX>(xval[f], c, f);
-            }
-        }
-        int64_t tot;
-        const int64_t off = block_exclusive_sum64<kSxThreads>(len, &tot);
-        s_off[tid] = off;
-        if (tid == kSxThreads - 1) s_off[kSxThreads] = off + len;
-        __syncthreads();
-        for (int64_t j = tid; j < tot; j += kSxThreads) {
-            int lo = 0, hi = kSxThreads;
-            while (hi - lo > 1) {
-                const int mid = (lo + hi) >> 1;
-                if (s_off[mid] <= j)
-                    lo = mid;
-                else
-                    hi = mid;
-            }
-            const int32_t r = row[s_seg[lo] + (j - s_off[lo])];
-            if (SX != SX_PLUSTIMES) atomicMax(&spa[r], s_key[lo]);
-            const uint32_t bit = 1u << (r & 31);
-            if (!(mark[r >> 5] & bit)) atomicOr(&mark[r >> 5], bit);
-        }
-        __syncthreads();
-    }
+    sx_products(cp, xind, nx, n, work, [&](int64_t f, int64_t p) {
+        const int32_t r = row[p];
+        if (SX == SX_PLUSTIMES)
+            atomicAdd(&spa[r], 1ull);
+        else
+            atomicMax(&spa[r], sx_key<SX>(xval[f], xind[f], f));
+        const uint32_t bit = 1u << (r & 31);
+        if (!(mark[r >> 5] & bit)) atomicOr(&mark[r >> 5], bit);
+    });
 }
 
 __global__ void k_sx_counts(const uint32_t *mark, int64_t words, int64_t *cnt)
 {
     const int64_t w = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (w < words) cnt[w] = __popc(mark[w]);
+}
+
+// PlusTimes: touched rows (low 32 bits) and their products (high 32 bits).
+__global__ void k_sx_counts_sum(const uint32_t *mark, int64_t words, const unsigned long long *spa, int64_t *cnt)
+{
+    const int64_t w = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (w >= words) return;
+    const uint32_t x = mark[w];
+    unsigned long long c = 0;
+    for (uint32_t bits = x; bits; bits &= bits - 1) c += spa[w * 32 + __ffs(bits) - 1];
+    cnt[w] = (int64_t)((c << 32) | (unsigned)__popc(x));
+}
+
+// PlusTimes: touched rows in ascending order and the place of their products
+// (off, and spa as a running cursor); clears the marks.
+__global__ void k_sx_places(uint32_t *mark, int64_t words, const int64_t *pos, unsigned long long *spa, int32_t *yind,
+                            uint32_t *off)
+{
+    const int64_t w = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (w >= words) return;
+    const unsigned long long at = (unsigned long long)pos[w];
+    uint32_t p = (uint32_t)at, o = (uint32_t)(at >> 32);
+    for (uint32_t bits = mark[w]; bits; bits &= bits - 1, ++p) {
+        const int64_t r = w * 32 + __ffs(bits) - 1;
+        const uint32_t c = (uint32_t)spa[r];
+        yind[p] = (int32_t)r;
+        off[p] = o;
+        spa[r] = o;
+        o += c;
+    }
+    mark[w] = 0;
+    if (w == words - 1) off[p] = o;
 }
 
 // Touched rows in ascending order with their values (select semirings);
@@ -184,13 +248,15 @@ __global__ void k_sx_emit(uint32_t *mark, int64_t words, const int64_t *pos, uns
     const int64_t w = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (w >= words) return;
     uint32_t bits = mark[w];
-    int64_t p = pos[w];
+    int64_t p = SX == SX_PLUSTIMES ? pos[w] & 0xffffffff : pos[w];
     while (bits) {
         const int b = __ffs(bits) - 1;
         bits &= bits - 1;
         const int64_t r = w * 32 + b;
         yind[p] = (int32_t)r;
-        if (SX != SX_PLUSTIMES) {
+        if (SX == SX_PLUSTIMES) {
+            spa[r] = 0;
+        } else {
             const unsigned long long k = spa[r];
             spa[r] = 0;
             int64_t v;
@@ -223,8 +289,44 @@ __device__ __forceinline__ V sx_add(V a, V b)
     else return a + b;
 }
 
-// PlusTimes pull: one warp per touched row, entries in ascending column
-// order, hits folded left in that order.
+constexpr int kSxThread = 8;      // products of a row folded by one thread
+constexpr int kSxPullShare = 4;   // pull when the products times this exceed the matrix
+
+// The row's products by one warp over its row-major entries, eight windows of
+// 32 entries in flight; hits are folded left in ascending column order.
+template <typename V>
+__device__ __forceinline__ V sx_pull_row(int64_t b, int64_t e, const int32_t *col, const V *aval, const int32_t *xpos,
+                                         const V *xval)
+{
+    constexpr int U = 8;
+    const int lane = threadIdx.x & 31;
+    V acc = V(0);
+    bool have = false;
+    for (int64_t base = b; base < e; base += 32 * U) {
+        int32_t fx[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) fx[u] = base + u * 32 + lane < e ? col[base + u * 32 + lane] : -1;
+#pragma unroll
+        for (int u = 0; u < U; ++u) fx[u] = fx[u] >= 0 ? xpos[fx[u]] : 0;
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            unsigned bal = __ballot_sync(0xffffffffu, fx[u] != 0);
+            if (!bal) continue;
+            V prod = V(0);
+            if (fx[u]) prod = sx_mul<V>(aval[base + u * 32 + lane], xval[fx[u] - 1]);
+            while (bal) {
+                const int l = __ffs(bal) - 1;
+                bal &= bal - 1;
+                const V pv = __shfl_sync(0xffffffffu, prod, l);
+                acc = have ? sx_add<V>(acc, pv) : pv;
+                have = true;
+            }
+        }
+    }
+    return acc;
+}
+
+// PlusTimes pull: one warp per touched row.
 template <typename V>
 __global__ void __launch_bounds__(256) k_sx_pull(int64_t ny, const int32_t *yind, const int64_t *rowptr,
                                                  const int32_t *col, const V *aval, const int32_t *xpos,
@@ -235,30 +337,139 @@ __global__ void __launch_bounds__(256) k_sx_pull(int64_t ny, const int32_t *yind
     const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
     for (int64_t i = warp; i < ny; i += nwarps) {
         const int32_t r = yind[i];
-        const int64_t b = rowptr[r], e = rowptr[r + 1];
-        V acc = V(0);
-        bool have = false;
-        for (int64_t base = b; base < e; base += 32) {
-            const int64_t idx = base + lane;
-            V prod = V(0);
-            bool hit = false;
-            if (idx < e) {
-                const int32_t fx = xpos[col[idx]];
-                if (fx) {
-                    prod = sx_mul<V>(aval[idx], xval[fx - 1]);
-                    hit = true;
+        const V acc = sx_pull_row<V>(rowptr[r], rowptr[r + 1], col, aval, xpos, xval);
+        if (lane == 0) yval[i] = acc;
+    }
+}
+
+// PlusTimes push: the products of the vector's columns, each at the next place
+// of its row (rows that will be pulled need none).
+template <typename V>
+__global__ void __launch_bounds__(kSxThreads) k_sx_scatter(const int64_t *cp, const int32_t *row, const V *aval,
+                                                           const int32_t *xind, const V *xval, int64_t nx, int64_t n,
+                                                           unsigned long long *spa, int32_t *pcol, V *pval,
+                                                           unsigned long long *work)
+{
+    sx_products(cp, xind, nx, n, work, [&](int64_t f, int64_t p) {
+        const unsigned long long at = atomicAdd(&spa[row[p]], 1ull);
+        pcol[at] = xind[f];
+        pval[at] = sx_mul<V>(aval[p], xval[f]);
+    });
+}
+
+// Every touched row folds its products in ascending column order; the row's
+// cursor goes back to zero.
+template <typename V>
+__global__ void __launch_bounds__(256) k_sx_fold(int64_t ny, const int32_t *yind, const uint32_t *off,
+                                                 const int32_t *pcol, const V *pval, unsigned long long *spa,
+                                                 V *yval, int32_t *longs, unsigned long long *nlong)
+{
+    const int lane = threadIdx.x & 31;
+    for (int64_t i0 = int64_t(blockIdx.x) * blockDim.x; i0 < ny; i0 += int64_t(gridDim.x) * blockDim.x) {
+        const int64_t i = i0 + threadIdx.x;
+        uint32_t o = 0, n = 0;
+        if (i < ny) {
+            o = off[i];
+            n = off[i + 1] - o;
+            spa[yind[i]] = 0;
+            if (n <= kSxThread) {
+                V acc = V(0);
+                int32_t done = -1;  // the columns up to this one are folded
+                for (uint32_t k = 0; k < n; ++k) {
+                    int32_t next = INT32_MAX;
+                    V v = V(0);
+                    for (uint32_t q = 0; q < n; ++q) {
+                        const int32_t c = pcol[o + q];
+                        if (c > done && c < next) {
+                            next = c;
+                            v = pval[o + q];
+                        }
+                    }
+                    acc = k ? sx_add<V>(acc, v) : v;
+                    done = next;
                 }
-            }
-            unsigned bal = __ballot_sync(0xffffffffu, hit);
-            while (bal) {
-                const int l = __ffs(bal) - 1;
-                bal &= bal - 1;
-                const V pv = __shfl_sync(0xffffffffu, prod, l);
-                acc = have ? sx_add<V>(acc, pv) : pv;
-                have = true;
+                yval[i] = acc;
             }
         }
-        if (lane == 0) yval[i] = acc;
+        unsigned more = __ballot_sync(0xffffffffu, n > kSxThread);
+        while (more) {
+            const int l = __ffs(more) - 1;
+            more &= more - 1;
+            const uint32_t ro = __shfl_sync(0xffffffffu, o, l), rn = __shfl_sync(0xffffffffu, n, l);
+            const int64_t ri = i0 + (threadIdx.x & ~31) + l;
+            if (rn > 32) {  // a block's work
+                if (lane == 0) longs[atomicAdd(nlong, 1ull)] = (int32_t)ri;
+                continue;
+            }
+            V acc = V(0);
+            unsigned c = lane < (int)rn ? (unsigned)pcol[ro + lane] : 0xffffffffu;
+            const V v = lane < (int)rn ? pval[ro + lane] : V(0);
+            for (uint32_t k = 0; k < rn; ++k) {
+                const unsigned next = __reduce_min_sync(0xffffffffu, c);
+                const int at = __ffs(__ballot_sync(0xffffffffu, c == next)) - 1;
+                const V pv = __shfl_sync(0xffffffffu, v, at);
+                acc = k ? sx_add<V>(acc, pv) : pv;
+                if (lane == at) c = 0xffffffffu;
+            }
+            if (lane == 0) yval[ri] = acc;
+        }
+    }
+}
+
+// Rows of more than 32 products, a block each: the products are sorted by
+// column in shared memory (bitonic) and folded by one thread, the chain that
+// the order asks for; rows of more than kSxSort are pulled.
+constexpr int kSxSort = 2048;
+
+template <typename V>
+__global__ void __launch_bounds__(256) k_sx_fold_long(const int32_t *longs, const unsigned long long *nlong,
+                                                      const int32_t *yind, const uint32_t *off, const int32_t *pcol,
+                                                      const V *pval, const int64_t *rowptr, const int32_t *col,
+                                                      const V *aval, const int32_t *xpos, const V *xval, V *yval)
+{
+    __shared__ uint64_t key[kSxSort];
+    __shared__ V val[kSxSort];
+    const int tid = threadIdx.x;
+    const int64_t count = (int64_t)*nlong;
+    for (int64_t q = blockIdx.x; q < count; q += gridDim.x) {
+        const int32_t i = longs[q];
+        const uint32_t o = off[i];
+        const int n = (int)(off[i + 1] - o);
+        if (n > kSxSort) {
+            if (tid < 32) {
+                const int32_t r = yind[i];
+                const V acc = sx_pull_row<V>(rowptr[r], rowptr[r + 1], col, aval, xpos, xval);
+                if (tid == 0) yval[i] = acc;
+            }
+            continue;
+        }
+        int N = 64;
+        while (N < n) N <<= 1;
+        for (int k = tid; k < N; k += 256)
+            key[k] = k < n ? ((uint64_t)(uint32_t)pcol[o + k] << 32) | (uint32_t)k : ~0ull;
+        __syncthreads();
+        for (int k2 = 2; k2 <= N; k2 <<= 1) {
+            for (int j = k2 >> 1; j > 0; j >>= 1) {
+                for (int u = tid; u < (N >> 1); u += 256) {
+                    const int lo = ((u & ~(j - 1)) << 1) | (u & (j - 1)), hi = lo + j;
+                    const uint64_t x0 = key[lo], x1 = key[hi];
+                    if ((x0 > x1) == ((lo & k2) == 0)) {
+                        key[lo] = x1;
+                        key[hi] = x0;
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        for (int k = tid; k < n; k += 256) val[k] = pval[o + (uint32_t)key[k]];
+        __syncthreads();
+        if (tid == 0) {
+            V acc = val[0];
+#pragma unroll 8
+            for (int k = 1; k < n; ++k) acc = sx_add<V>(acc, val[k]);
+            yval[i] = acc;
+        }
+        __syncthreads();
     }
 }
 
@@ -270,6 +481,7 @@ static void plan_release(SpmspvPlan *p)
     if (p->have_rm) spmv_plan_release(&p->rm);
     device_free(p->ctx, p->cp);
     device_free(p->ctx, p->row);
+    device_free(p->ctx, p->cval);
     device_free(p->ctx, p->spa);
     device_free(p->ctx, p->mark);
     device_free(p->ctx, p->pos);
@@ -319,6 +531,17 @@ static int plan_build(SpmspvPlan *p, const gbc_matrix *Am)
     if (herr & 1) return fail(GBC_EINVAL, "SpMSpV plan: malformed column pointers or column ids");
     if (herr & 2) return fail(GBC_EINVAL, "SpMSpV plan: row id out of range");
     if (p->vt == GBC_F64 || p->vt == GBC_F32 || p->vt == GBC_I64) {
+        const size_t vs = value_size(p->vt);
+        GBC_TRY(device_alloc(ctx, &p->cval, (p->nnz + 1) * vs));
+        if (A.num) {
+            GBC_CUDA_TRY(cudaMemcpyAsync(p->cval, A.num, p->nnz * vs, cudaMemcpyDeviceToDevice, s));
+        } else if (p->nnz > 0) {
+            const unsigned g = (unsigned)((p->nnz + 255) / 256);
+            if (p->vt == GBC_F64) k_sx_ones<double><<<g, 256, 0, s>>>(p->nnz, static_cast<double *>(p->cval));
+            if (p->vt == GBC_F32) k_sx_ones<float><<<g, 256, 0, s>>>(p->nnz, static_cast<float *>(p->cval));
+            if (p->vt == GBC_I64) k_sx_ones<int64_t><<<g, 256, 0, s>>>(p->nnz, static_cast<int64_t *>(p->cval));
+            note_launch();
+        }
         p->rm.ctx = ctx;
         p->rm.vt = p->vt;
         p->have_rm = true;
@@ -337,7 +560,7 @@ static int sx_run(SpmspvPlan *p, Workspace &ws, const int32_t *dx, const void *d
     GBC_CUDA_TRY(cudaMemsetAsync(p->work, 0, sizeof(unsigned long long), s));
     if (nx > 0) {
         k_sx_xpos<<<(unsigned)((nx + 255) / 256), 256, 0, s>>>(nx, dx, p->n, p->xpos, p->err);
-        const int grid = (int)std::min<int64_t>((int64_t)ctx->num_sms * 4, (nx + kSxThreads - 1) / kSxThreads);
+        const int grid = (int)std::min<int64_t>((int64_t)ctx->num_sms * 8, (nx + kSxChunk - 1) / kSxChunk);
         k_sx_expand<SX><<<grid, kSxThreads, 0, s>>>(p->cp, p->row, dx, static_cast<const int64_t *>(dv), nx, p->n,
                                                     p->spa, p->mark, p->work);
         note_launches(2);
@@ -345,28 +568,58 @@ static int sx_run(SpmspvPlan *p, Workspace &ws, const int32_t *dx, const void *d
     int64_t *cnt = nullptr;
     GBC_TRY(ws.alloc_n(&cnt, p->words + 1));
     if (p->words > 0) {
-        k_sx_counts<<<(unsigned)((p->words + 255) / 256), 256, 0, s>>>(p->mark, p->words, cnt);
+        if (SX == SX_PLUSTIMES)
+            k_sx_counts_sum<<<(unsigned)((p->words + 255) / 256), 256, 0, s>>>(p->mark, p->words, p->spa, cnt);
+        else
+            k_sx_counts<<<(unsigned)((p->words + 255) / 256), 256, 0, s>>>(p->mark, p->words, cnt);
         note_launch();
     }
     GBC_TRY(exclusive_scan_i64(ws, cnt, p->pos, p->words, s));
     GBC_TRY(read_i64(ctx, p->pos + p->words, ny));
+    const int64_t nprod = SX == SX_PLUSTIMES ? (int64_t)((uint64_t)*ny >> 32) : 0;
+    if (SX == SX_PLUSTIMES) *ny &= 0xffffffff;
     if (host_out) {
         GBC_TRY(ws.alloc_n(yi, *ny + 1));
         void *b = nullptr;
         GBC_TRY(ws.alloc(&b, (*ny + 1) * sizeof(V)));
         *yv = b;
     }
-    if (p->words > 0) {
-        k_sx_emit<SX><<<(unsigned)((p->words + 255) / 256), 256, 0, s>>>(
-            p->mark, p->words, p->pos, p->spa, static_cast<const int64_t *>(dv), *yi,
-            SX == SX_PLUSTIMES ? nullptr : static_cast<int64_t *>(*yv));
-        note_launch();
-    }
-    if (SX == SX_PLUSTIMES && *ny > 0) {
-        const int grid = (int)std::min<int64_t>((*ny + 7) / 8, (int64_t)ctx->num_sms * 16);
-        k_sx_pull<V><<<grid, 256, 0, s>>>(*ny, *yi, p->rm.rowptr, p->rm.col, static_cast<const V *>(p->rm.val),
-                                          p->xpos, static_cast<const V *>(dv), static_cast<V *>(*yv));
-        note_launch();
+    if (SX == SX_PLUSTIMES && *ny > 0 && nprod * kSxPullShare <= p->nnz) {
+        uint32_t *off = nullptr;
+        int32_t *pcol = nullptr;
+        V *pval = nullptr;
+        GBC_TRY(ws.alloc_n(&off, *ny + 1));
+        GBC_TRY(ws.alloc_n(&pcol, nprod));
+        GBC_TRY(ws.alloc_n(&pval, nprod));
+        int32_t *longs = nullptr;  // rows of more than 32 products
+        unsigned long long *nlong = nullptr;
+        GBC_TRY(ws.alloc_n(&longs, nprod / 33 + 1));
+        GBC_TRY(ws.alloc_n(&nlong, 1));
+        GBC_CUDA_TRY(cudaMemsetAsync(nlong, 0, sizeof(unsigned long long), s));
+        k_sx_places<<<(unsigned)((p->words + 255) / 256), 256, 0, s>>>(p->mark, p->words, p->pos, p->spa, *yi, off);
+        GBC_CUDA_TRY(cudaMemsetAsync(p->work, 0, sizeof(unsigned long long), s));
+        const int grid = (int)std::min<int64_t>((int64_t)ctx->num_sms * 8, (nx + kSxChunk - 1) / kSxChunk);
+        k_sx_scatter<V><<<grid, kSxThreads, 0, s>>>(p->cp, p->row, static_cast<const V *>(p->cval), dx,
+                                                    static_cast<const V *>(dv), nx, p->n, p->spa, pcol, pval, p->work);
+        k_sx_fold<V><<<(int)std::min<int64_t>((*ny + 255) / 256, (int64_t)ctx->num_sms * 8), 256, 0, s>>>(
+            *ny, *yi, off, pcol, pval, p->spa, static_cast<V *>(*yv), longs, nlong);
+        k_sx_fold_long<V><<<(int)std::min<int64_t>(nprod / 33 + 1, (int64_t)ctx->num_sms * 6), 256, 0, s>>>(
+            longs, nlong, *yi, off, pcol, pval, p->rm.rowptr, p->rm.col, static_cast<const V *>(p->rm.val), p->xpos,
+            static_cast<const V *>(dv), static_cast<V *>(*yv));
+        note_launches(4);
+    } else {
+        if (p->words > 0) {
+            k_sx_emit<SX><<<(unsigned)((p->words + 255) / 256), 256, 0, s>>>(
+                p->mark, p->words, p->pos, p->spa, static_cast<const int64_t *>(dv), *yi,
+                SX == SX_PLUSTIMES ? nullptr : static_cast<int64_t *>(*yv));
+            note_launch();
+        }
+        if (SX == SX_PLUSTIMES && *ny > 0) {
+            const int grid = (int)std::min<int64_t>((*ny + 7) / 8, (int64_t)ctx->num_sms * 16);
+            k_sx_pull<V><<<grid, 256, 0, s>>>(*ny, *yi, p->rm.rowptr, p->rm.col, static_cast<const V *>(p->rm.val),
+                                              p->xpos, static_cast<const V *>(dv), static_cast<V *>(*yv));
+            note_launch();
+        }
     }
     if (nx > 0) {
         k_sx_xpos_clear<<<(unsigned)((nx + 255) / 256), 256, 0, s>>>(nx, dx, p->n, p->xpos);
