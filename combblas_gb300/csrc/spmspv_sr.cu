@@ -544,6 +544,7 @@ static int plan_build(SpmspvPlan *p, const gbc_matrix *Am)
         }
         p->rm.ctx = ctx;
         p->rm.vt = p->vt;
+        p->rm.tiles = false;
         p->have_rm = true;
         GBC_TRY(spmv_plan_build(&p->rm, Am));
     }

@@ -4,17 +4,17 @@
 //
 // GPU form: a plan holds A row-major (rows ascending, each row's entries in
 // ascending column order) built once on the device by a stable LSD radix
-// sort of the column-major entries by row.  Rows of at most 64 entries are
-// taken by eight lanes each (four rows per warp); longer rows are cut into
-// chunks of at most 256 entries, a warp per chunk.  Lanes fold their share
-// of a row or chunk in column order, a fixed shuffle tree combines the
-// lanes, and rows of several chunks fold their chunk results in order before
-// y is folded in.
+// sort of the column-major entries by row.  A thread takes kSpmvPer consecutive
+// entries whatever rows they belong to: it folds them in order, whole rows are
+// done there, and the open sums at its ends are joined by a segmented scan over
+// the block and, for rows that cross blocks, by a second small kernel.
 // The order is fixed, so repeated runs are bit-identical; for min-type,
 // boolean and integer semirings every order gives the reference's result
 // exactly, and for PlusTimes on floating values the sum differs from the
 // reference's column-order sum only by rounding.
 #include <algorithm>
+#include <cstring>
+#include <type_traits>
 
 #include "gbc_internal.cuh"
 #include "semiring.cuh"
@@ -121,6 +121,10 @@ __global__ void __launch_bounds__(kRsThreads) k_rs_scatter(const uint32_t *key_i
     }
 }
 
+constexpr int kSpmvPer = 8;
+constexpr int kSpmvThreads = 128;
+constexpr int kSpmvTile = kSpmvPer * kSpmvThreads;
+
 template <typename V>
 __global__ void k_gather_rowmajor(int64_t n, const int32_t *perm, const int32_t *col_cm, const V *val_cm, V one,
                                   int32_t *col, V *val)
@@ -132,165 +136,198 @@ __global__ void k_gather_rowmajor(int64_t n, const int32_t *perm, const int32_t 
     val[p] = val_cm ? val_cm[e] : one;
 }
 
-// Rows are cut into chunks of at most kChunk entries (fixed at plan time).
-// A warp takes one chunk: lane l folds entries l, l+32, ... (up to 8, loads
-// issued together), then a fixed shuffle tree combines the lanes.  A row of
-// one chunk updates y directly; longer rows leave their chunk partials for
-// k_spmv_rows, which folds them in chunk order.
-constexpr int kChunk = 256;
-
-template <class SR>
-__global__ void __launch_bounds__(256) k_spmv_chunks(int64_t nchunks, const int64_t *chunk_start,
-                                                     const int64_t *chunk_end, const int32_t *chunk_row,
-                                                     const int8_t *partial_slot,
-                                                     const int32_t *col, const typename SR::V *val,
-                                                     const typename SR::V *x, typename SR::V *y,
-                                                     typename SR::V *partial)
-{
-    typedef typename SR::V V;
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t c = warp; c < nchunks; c += nwarps) {
-        const int32_t r = chunk_row[c];
-        const int64_t s = chunk_start[c];
-        const int64_t e = chunk_end[c];
-        V t[kChunk / 32];
-        int cnt = 0;
-#pragma unroll
-        for (int k = 0; k < kChunk / 32; ++k) {
-            const int64_t p = s + k * 32 + lane;
-            if (p < e) {
-                t[k] = SR::mul(val[p], x[col[p]]);
-                cnt = k + 1;
-            }
-        }
-        bool have = cnt > 0;
-        V acc = t[0];
-#pragma unroll
-        for (int k = 1; k < kChunk / 32; ++k)
-            if (k < cnt) acc = SR::add(acc, t[k]);
-        // fixed tree: lane l takes lane l + o's partial, if that lane has one
-#pragma unroll
-        for (int o = 16; o; o >>= 1) {
-            const V other = __shfl_down_sync(0xffffffffu, acc, o);
-            const bool ho = __shfl_down_sync(0xffffffffu, (int)have, o) != 0;
-            if (lane + o < 32 && ho) {
-                acc = have ? SR::add(acc, other) : other;
-                have = true;
-            }
-        }
-        if (lane == 0) {
-            if (partial_slot[c] < 0)
-                y[r] = SR::add(y[r], acc);  // the row is this one chunk
-            else
-                partial[c] = acc;
-        }
-    }
-}
-
-// Rows of at most kShort entries: eight lanes per row, four rows per warp;
-// lane g of a row folds entries g, g+8, ... in column order, then a fixed
-// three-step shuffle tree over the eight lanes.
-constexpr int kShort = 64;
-
-template <class SR>
-__global__ void __launch_bounds__(256) k_spmv_short(int64_t nshort, const int32_t *short_rows,
-                                                    const int64_t *rowptr, const int32_t *col,
-                                                    const typename SR::V *val, const typename SR::V *x,
-                                                    typename SR::V *y)
-{
-    typedef typename SR::V V;
-    const int lane = threadIdx.x & 31, gl = lane & 7;
-    const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t b = warp * 4; b < nshort; b += nwarps * 4) {
-        const int64_t i = b + (lane >> 3);
-        const bool act = i < nshort;
-        const int32_t r = act ? short_rows[i] : 0;
-        const int64_t s = act ? rowptr[r] : 0, e = act ? rowptr[r + 1] : 0;
-        V t[kShort / 8];
-        int cnt = 0;
-#pragma unroll
-        for (int k = 0; k < kShort / 8; ++k) {
-            const int64_t p = s + k * 8 + gl;
-            if (p < e) {
-                t[k] = SR::mul(val[p], x[col[p]]);
-                cnt = k + 1;
-            }
-        }
-        bool have = cnt > 0;
-        V acc = t[0];
-#pragma unroll
-        for (int k = 1; k < kShort / 8; ++k)
-            if (k < cnt) acc = SR::add(acc, t[k]);
-#pragma unroll
-        for (int o = 4; o; o >>= 1) {
-            const V other = __shfl_down_sync(0xffffffffu, acc, o, 8);
-            const bool ho = __shfl_down_sync(0xffffffffu, (int)have, o, 8) != 0;
-            if (gl + o < 8 && ho) {
-                acc = have ? SR::add(acc, other) : other;
-                have = true;
-            }
-        }
-        if (act && gl == 0 && have) y[r] = SR::add(y[r], acc);
-    }
-}
-
-template <class SR>
-__global__ void k_spmv_rows(int64_t nlong, const int32_t *long_row, const int64_t *long_first,
-                            const int64_t *long_end, const typename SR::V *partial, typename SR::V *y)
-{
-    typedef typename SR::V V;
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= nlong) return;
-    const int64_t c0 = long_first[i], c1 = long_end[i];
-    V acc = partial[c0];
-    for (int64_t c = c0 + 1; c < c1; ++c) acc = SR::add(acc, partial[c]);
-    const int32_t r = long_row[i];
-    y[r] = SR::add(y[r], acc);
-}
-
-// chunks per row (0 for an empty row)
-__global__ void k_row_chunks(int64_t m, const int64_t *rowptr, int64_t *nch, int64_t *islong, int64_t *isshort)
+// Rows with entries, their starts, and the row of every group of kSpmvPer entries.
+__global__ void k_spmv_has(int64_t m, const int64_t *rowptr, int64_t *has)
 {
     const int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (r >= m) return;
-    const int64_t len = rowptr[r + 1] - rowptr[r];
-    const bool sh = len > 0 && len <= kShort;
-    nch[r] = sh ? 0 : (len + kChunk - 1) / kChunk;
-    islong[r] = len > kChunk;
-    isshort[r] = sh;
+    if (r < m) has[r] = rowptr[r + 1] > rowptr[r];
 }
 
-__global__ void k_fill_chunks(int64_t m, const int64_t *rowptr, const int64_t *cfirst, const int64_t *lpos,
-                              const int64_t *spos, int64_t *chunk_start, int64_t *chunk_end, int32_t *chunk_row,
-                              int8_t *partial_slot, int32_t *short_rows, int32_t *long_row, int64_t *long_first,
-                              int64_t *long_end)
+__global__ void k_spmv_mark(int64_t m, const int64_t *rowptr, const int64_t *index, int32_t *rows, uint32_t *starts,
+                            int32_t *group_row)
 {
     const int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (r >= m) return;
     const int64_t s = rowptr[r], e = rowptr[r + 1];
-    if (e > s && e - s <= kShort) {
-        short_rows[spos[r]] = (int32_t)r;
-        return;
+    if (e <= s) return;
+    const int32_t i = (int32_t)index[r];
+    rows[i] = (int32_t)r;
+    atomicOr(&starts[s >> 5], 1u << (s & 31));
+    for (int64_t g = (s + kSpmvPer - 1) / kSpmvPer; g * kSpmvPer < e; ++g) group_row[g] = i;
+}
+
+// acc + a * x.  Floating sums use a fused multiply-add: one rounding less, and
+// half the fp64 instructions, which bound this kernel otherwise (GB300 issues
+// two fp64 operations per SM and clock).
+template <class SR>
+__device__ __forceinline__ typename SR::V spmv_axpy(typename SR::V a, typename SR::V x, typename SR::V acc)
+{
+    typedef typename SR::V V;
+    if constexpr (std::is_same<SR, PlusTimes<double>>::value)
+        return __fma_rn(a, x, acc);
+    else if constexpr (std::is_same<SR, PlusTimes<float>>::value)
+        return __fmaf_rn(a, x, acc);
+    else
+        return SR::add(acc, (V)SR::mul(a, x));
+}
+
+// One tile of kSpmvTile entries.  Bound by the latency of the gathers of x (an
+// L2 sector per entry) behind the entries' own loads, and by the fp64 pipe.
+// R-MAT scale 20 fp64, 31 M entries, 386 us by rows (eight lanes or a warp per
+// row and a shuffle tree for each): 182 us with 8 entries a thread and 128
+// threads (64: 189, 256: 214, 512: 276); with 256 threads 205 to 214 us, 263
+// with 16 entries a thread, 255 with 4, 331 with the gathers in entry order and
+// handed over through shared memory.
+template <class SR>
+__global__ void __launch_bounds__(kSpmvThreads) k_spmv_tiles(int64_t nnz, const uint32_t *starts,
+                                                             const int32_t *group_row, const int32_t *rows,
+                                                             const int32_t *col, const typename SR::V *val,
+                                                             const typename SR::V *x, typename SR::V *y,
+                                                             typename SR::V *edge, int32_t *edge_row)
+{
+    typedef typename SR::V V;
+    constexpr int NW = kSpmvThreads / 32;
+    __shared__ V s_row[kSpmvTile + 1];  // whole rows' sums, from the tile's first start on
+    __shared__ V s_sum[NW];
+    __shared__ int s_flag[NW], s_n[NW], s_r0;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t group = int64_t(blockIdx.x) * kSpmvThreads + tid, base = group * kSpmvPer;
+    const int count = (int)max((int64_t)0, min((int64_t)kSpmvPer, nnz - base));
+    unsigned flags = 0;
+    int cur = 0;  // the row that is open (index into rows); before the first entry: the row before it
+    if (count > 0) {
+        flags = (starts[base >> 5] >> (base & 31)) & ((1u << kSpmvPer) - 1);
+        cur = group_row[group] - (int)(flags & 1);
     }
-    int64_t c = cfirst[r];
-    const int8_t slot = (e - s > kChunk) ? 1 : -1;
-    for (int64_t p = s; p < e; p += kChunk, ++c) {
-        chunk_start[c] = p;
-        chunk_end[c] = min(e, p + kChunk);
-        chunk_row[c] = (int32_t)r;
-        partial_slot[c] = slot;
+    V v[kSpmvPer];
+    V xq[kSpmvPer];
+    {
+        int32_t c[kSpmvPer];
+        if (count == kSpmvPer) {
+#pragma unroll
+            for (int k = 0; k < kSpmvPer; k += 4) {
+                const int4 q = *reinterpret_cast<const int4 *>(col + base + k);
+                memcpy(&c[k], &q, 16);
+            }
+            if constexpr (sizeof(V) >= 4) {
+                constexpr int K = 16 / sizeof(V);
+#pragma unroll
+                for (int k = 0; k < kSpmvPer; k += K) {
+                    const int4 q = *reinterpret_cast<const int4 *>(val + base + k);
+                    memcpy(&v[k], &q, 16);
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < kSpmvPer; ++k) v[k] = val[base + k];
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < kSpmvPer; ++k) {
+                c[k] = k < count ? col[base + k] : -1;
+                v[k] = k < count ? val[base + k] : SR::one();
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < kSpmvPer; ++k) xq[k] = c[k] >= 0 ? x[c[k]] : SR::one();
     }
-    if (e - s > kChunk) {
-        const int64_t q = lpos[r];
-        long_row[q] = (int32_t)r;
-        long_first[q] = cfirst[r];
-        long_end[q] = c;
+    if (tid == 0) s_r0 = cur;
+    // rows open before the tile and flags before each thread
+    const int nf = __popc(flags);
+    int before = nf;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, before, o);
+        if (lane >= o) before += u;
+    }
+    if (lane == 31) s_n[warp] = before;
+    before -= nf;
+    __syncthreads();
+    int total = 0;
+#pragma unroll
+    for (int u = 0; u < NW; ++u) {
+        before += u < warp ? s_n[u] : 0;
+        total += s_n[u];
+    }
+    // fold in order: head, the sum up to the thread's first start; whole rows; acc, the open sum at its end
+    V acc = SR::zero(), head = SR::zero();
+    bool seen = false;
+    int at = before;  // starts before the next one: row at of the tile is open
+#pragma unroll
+    for (int k = 0; k < kSpmvPer; ++k) {
+        if ((flags >> k) & 1) {
+            if (seen)
+                s_row[at] = acc;
+            else
+                head = acc;
+            seen = true;
+            ++at;
+            acc = SR::zero();
+        }
+        if (k < count) acc = spmv_axpy<SR>(v[k], xq[k], acc);
+    }
+    // segmented inclusive scan of the open sums
+    V sum = acc;
+    bool flag = seen;
+    if (!__all_sync(0xffffffffu, seen)) {
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const V su = __shfl_up_sync(0xffffffffu, sum, o);
+            const bool fu = __shfl_up_sync(0xffffffffu, (int)flag, o) != 0;
+            if (lane >= o && !flag) {
+                sum = SR::add(su, sum);
+                flag = fu;
+            }
+        }
+    }
+    if (lane == 31) {
+        s_sum[warp] = sum;
+        s_flag[warp] = flag;
+    }
+    V left = __shfl_up_sync(0xffffffffu, sum, 1);
+    const bool left_flag = __shfl_up_sync(0xffffffffu, (int)flag, 1) != 0 && lane > 0;
+    __syncthreads();
+    V carry = SR::zero();
+    for (int u = 0; u < warp; ++u) carry = s_flag[u] ? s_sum[u] : SR::add(carry, s_sum[u]);
+    if (lane == 0)
+        left = carry;
+    else if (!left_flag)
+        left = SR::add(carry, left);
+    if (seen) s_row[before] = SR::add(left, head);  // the row that ends at the thread's first start
+    if (tid == kSpmvThreads - 1) {
+        edge[2 * (int64_t)blockIdx.x + 1] = flag ? sum : SR::add(carry, sum);
+        if (total == 0) edge_row[blockIdx.x] = -2;
+    }
+    __syncthreads();
+    if (tid == 0 && total > 0) {  // row 0 of the tile began before it
+        edge[2 * (int64_t)blockIdx.x] = s_row[0];
+        edge_row[blockIdx.x] = s_r0;
+    }
+    for (int k = 1 + tid; k < total; k += kSpmvThreads) {
+        const int32_t r = rows[s_r0 + k];
+        y[r] = SR::add(y[r], s_row[k]);
     }
 }
 
+// Rows that cross tiles: the open sum behind the last start of an earlier tile,
+// the tiles without a start in between, and what the row has in tile b.  The
+// last row ends behind the last tile (b == ntiles).
+template <class SR>
+__global__ void k_spmv_edges(int64_t ntiles, int64_t nrows, const int32_t *rows, const typename SR::V *edge,
+                             const int32_t *edge_row, typename SR::V *y)
+{
+    typedef typename SR::V V;
+    const int64_t b = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (b > ntiles) return;
+    const int64_t i = b < ntiles ? edge_row[b] : nrows - 1;
+    if (i < 0) return;
+    int64_t u = b - 1;
+    while (edge_row[u] == -2) --u;  // the first tile has a start
+    V sum = edge[2 * u + 1];
+    for (++u; u < b; ++u) sum = SR::add(sum, edge[2 * u + 1]);
+    if (b < ntiles) sum = SR::add(sum, edge[2 * b]);
+    const int32_t r = rows[i];
+    y[r] = SR::add(y[r], sum);
+}
 
 template <typename V>
 static int plan_values(SpmvPlan *p, Workspace &ws, const DevMatrix &A, const int32_t *perm, const int32_t *col_cm)
@@ -358,40 +395,26 @@ int spmv_plan_build(SpmvPlan *p, const gbc_matrix *Am)
             cur ^= 1;
         }
     }
-    // row chunks
-    {
-        int64_t *nch = nullptr, *cfirst = nullptr, *islong = nullptr, *lpos = nullptr, *isshort = nullptr,
-                *spos = nullptr;
-        GBC_TRY(ws.alloc_n(&nch, p->m + 1));
-        GBC_TRY(ws.alloc_n(&cfirst, p->m + 1));
-        GBC_TRY(ws.alloc_n(&islong, p->m + 1));
-        GBC_TRY(ws.alloc_n(&lpos, p->m + 1));
-        GBC_TRY(ws.alloc_n(&isshort, p->m + 1));
-        GBC_TRY(ws.alloc_n(&spos, p->m + 1));
+    // rows with entries, their starts
+    if (p->tiles) {
+        int64_t *index = nullptr;
+        GBC_TRY(ws.alloc_n(&index, p->m + 1));
         const unsigned rg = (unsigned)((p->m + 255) / 256);
         if (p->m > 0) {
-            k_row_chunks<<<rg, 256, 0, s>>>(p->m, p->rowptr, nch, islong, isshort);
+            k_spmv_has<<<rg, 256, 0, s>>>(p->m, p->rowptr, index);
             note_launch();
         }
-        GBC_TRY(exclusive_scan_i64(ws, nch, cfirst, p->m, s));
-        GBC_TRY(exclusive_scan_i64(ws, islong, lpos, p->m, s));
-        GBC_TRY(exclusive_scan_i64(ws, isshort, spos, p->m, s));
-        GBC_TRY(read_i64(ctx, cfirst + p->m, &p->nchunks));
-        GBC_TRY(read_i64(ctx, lpos + p->m, &p->nlong));
-        GBC_TRY(read_i64(ctx, spos + p->m, &p->nshort));
-        GBC_TRY(device_alloc(ctx, (void **)&p->short_rows, (p->nshort + 1) * sizeof(int32_t)));
-        GBC_TRY(device_alloc(ctx, (void **)&p->chunk_end, (p->nchunks + 1) * sizeof(int64_t)));
-        GBC_TRY(device_alloc(ctx, (void **)&p->chunk_start, (p->nchunks + 1) * sizeof(int64_t)));
-        GBC_TRY(device_alloc(ctx, (void **)&p->chunk_row, (p->nchunks + 1) * sizeof(int32_t)));
-        GBC_TRY(device_alloc(ctx, (void **)&p->partial_slot, (p->nchunks + 1) * sizeof(int8_t)));
-        GBC_TRY(device_alloc(ctx, (void **)&p->long_row, (p->nlong + 1) * sizeof(int32_t)));
-        GBC_TRY(device_alloc(ctx, (void **)&p->long_first, (p->nlong + 1) * sizeof(int64_t)));
-        GBC_TRY(device_alloc(ctx, (void **)&p->long_end, (p->nlong + 1) * sizeof(int64_t)));
-        GBC_TRY(device_alloc(ctx, &p->partial, (p->nchunks + 1) * sizeof(int64_t)));  // widest value type
+        GBC_TRY(exclusive_scan_i64(ws, index, index, p->m, s));
+        GBC_TRY(read_i64(ctx, index + p->m, &p->nrows));
+        p->ntiles = (n + kSpmvTile - 1) / kSpmvTile;
+        GBC_TRY(device_alloc(ctx, (void **)&p->rows, (p->nrows + 1) * sizeof(int32_t)));
+        GBC_TRY(device_alloc(ctx, (void **)&p->starts, (n / 32 + 2) * sizeof(uint32_t)));
+        GBC_TRY(device_alloc(ctx, (void **)&p->group_row, (n / kSpmvPer + 1) * sizeof(int32_t)));
+        GBC_TRY(device_alloc(ctx, &p->edge, (2 * p->ntiles + 1) * sizeof(int64_t)));  // widest value type
+        GBC_TRY(device_alloc(ctx, (void **)&p->edge_row, (p->ntiles + 1) * sizeof(int32_t)));
+        GBC_CUDA_TRY(cudaMemsetAsync(p->starts, 0, (n / 32 + 2) * sizeof(uint32_t), s));
         if (p->m > 0) {
-            k_fill_chunks<<<rg, 256, 0, s>>>(p->m, p->rowptr, cfirst, lpos, spos, p->chunk_start, p->chunk_end,
-                                             p->chunk_row, p->partial_slot, p->short_rows, p->long_row,
-                                             p->long_first, p->long_end);
+            k_spmv_mark<<<rg, 256, 0, s>>>(p->m, p->rowptr, index, p->rows, p->starts, p->group_row);
             note_launch();
         }
     }
@@ -415,26 +438,14 @@ static int spmv_run(SpmvPlan *p, const void *x, void *y)
 {
     typedef typename SR::V V;
     cudaStream_t s = p->ctx->stream;
-    if (p->nshort > 0) {
-        const int sg = (int)std::min<int64_t>((p->nshort + 31) / 32, (int64_t)p->ctx->num_sms * 16);
-        k_spmv_short<SR><<<sg, 256, 0, s>>>(p->nshort, p->short_rows, p->rowptr, p->col,
-                                            static_cast<const V *>(p->val), static_cast<const V *>(x),
-                                            static_cast<V *>(y));
-        note_launch();
-    }
-    if (p->nchunks == 0) return GBC_OK;
-    const int grid = (int)std::min<int64_t>((p->nchunks + 7) / 8, (int64_t)p->ctx->num_sms * 16);
-    k_spmv_chunks<SR><<<grid, 256, 0, s>>>(p->nchunks, p->chunk_start, p->chunk_end, p->chunk_row,
-                                           p->partial_slot, p->col,
-                                           static_cast<const V *>(p->val), static_cast<const V *>(x),
-                                           static_cast<V *>(y), static_cast<V *>(p->partial));
-    note_launch();
-    if (p->nlong > 0) {
-        k_spmv_rows<SR><<<(unsigned)((p->nlong + 127) / 128), 128, 0, s>>>(
-            p->nlong, p->long_row, p->long_first, p->long_end, static_cast<const V *>(p->partial),
-            static_cast<V *>(y));
-        note_launch();
-    }
+    if (p->ntiles == 0) return GBC_OK;
+    k_spmv_tiles<SR><<<(unsigned)p->ntiles, kSpmvThreads, 0, s>>>(
+        p->nnz, p->starts, p->group_row, p->rows, p->col, static_cast<const V *>(p->val), static_cast<const V *>(x),
+        static_cast<V *>(y), static_cast<V *>(p->edge), p->edge_row);
+    k_spmv_edges<SR><<<(unsigned)(p->ntiles / 128 + 1), 128, 0, s>>>(p->ntiles, p->nrows, p->rows,
+                                                                     static_cast<const V *>(p->edge), p->edge_row,
+                                                                     static_cast<V *>(y));
+    note_launches(2);
     GBC_CUDA_TRY(cudaGetLastError());
     return GBC_OK;
 }
@@ -447,15 +458,11 @@ void spmv_plan_release(SpmvPlan *p)
     device_free(p->ctx, p->rowptr);
     device_free(p->ctx, p->col);
     device_free(p->ctx, p->val);
-    device_free(p->ctx, p->chunk_start);
-    device_free(p->ctx, p->chunk_row);
-    device_free(p->ctx, p->partial_slot);
-    device_free(p->ctx, p->chunk_end);
-    device_free(p->ctx, p->short_rows);
-    device_free(p->ctx, p->long_row);
-    device_free(p->ctx, p->long_first);
-    device_free(p->ctx, p->long_end);
-    device_free(p->ctx, p->partial);
+    device_free(p->ctx, p->rows);
+    device_free(p->ctx, p->starts);
+    device_free(p->ctx, p->group_row);
+    device_free(p->ctx, p->edge);
+    device_free(p->ctx, p->edge_row);
     cudaStreamSynchronize(p->ctx->stream);
 }
 

@@ -13,16 +13,14 @@ struct SpmvPlan {
     int64_t *rowptr = nullptr;  // [m+1]
     int32_t *col = nullptr;     // [nnz]
     void *val = nullptr;        // [nnz]
-    int64_t nchunks = 0, nlong = 0;
-    int64_t *chunk_start = nullptr;  // [nchunks]
-    int32_t *chunk_row = nullptr;    // [nchunks]
-    int8_t *partial_slot = nullptr;  // [nchunks] -1: the row's only chunk, 1: part of a longer row
-    int64_t *chunk_end = nullptr;    // [nchunks]
-    int64_t nshort = 0;
-    int32_t *short_rows = nullptr;   // [nshort] rows of 1..kShort entries
-    int32_t *long_row = nullptr;     // [nlong] rows of more than one chunk
-    int64_t *long_first = nullptr, *long_end = nullptr;  // their chunk ranges
-    void *partial = nullptr;         // [nchunks] chunk results of long rows
+    bool tiles = true;          // laid out for the dense-vector SpMV (the members below)
+    int64_t nrows = 0;             // rows with entries
+    int32_t *rows = nullptr;       // [nrows] their ids, ascending
+    uint32_t *starts = nullptr;    // [nnz / 32] bit p: entry p is the first of its row
+    int32_t *group_row = nullptr;  // [nnz / kSpmvPer] row (index into rows) of each group's first entry
+    int64_t ntiles = 0;            // blocks of k_spmv_tiles
+    void *edge = nullptr;          // [2 ntiles] sums of the rows that cross tiles: before a tile's first start, behind its last
+    int32_t *edge_row = nullptr;   // [ntiles] the row before a tile's first start; -1 none, -2 the tile has no start
 };
 
 // Build p (p->ctx and p->vt set) from A: rows ascending, each row's entries
