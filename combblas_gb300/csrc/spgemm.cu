@@ -1058,7 +1058,8 @@ struct Plan {
     int64_t *lbuf = nullptr;             // column lists (kLists x (total_cols + 1))
     bool s2_set = false;                 // the caller chose s2
     unsigned long long *lcnt = nullptr;  // list lengths
-    bool want_aexp = false;              // PlusTimes fp64, exact accumulation (k_numeric_x)
+    bool want_x = false;                 // big columns by k_numeric_x
+    bool want_aexp = false;              // ... PlusTimes fp64, exact sums
     int64_t *fb_items = nullptr;         // big columns the exact kernel hands to the ordered one
     unsigned long long *fb_cnt = nullptr;
     XSeg *xscratch = nullptr;            // exact kernel: bucketing scratch, xscap segments per block
@@ -1070,27 +1071,33 @@ struct Plan {
     SpgemmArgs &a() { return h[0]; }
 };
 
-// PlusTimes fp64 under GBC_FOLD_EXACT: every admitted column is summed
-// exactly (big columns by k_numeric_x).  Its row tiles are kXRows high; the
-// tile height is a tuning knob only, so a larger request is lowered.
+// PlusTimes fp64 under GBC_FOLD_EXACT, and the semirings whose add does not
+// depend on the order, take their big columns to k_numeric_x.  Its row tiles
+// are kXRows high; the tile height is a tuning knob only, so a larger request
+// is lowered.  Columns of more than kSmallMid multiplications go there as well
+// (R-MAT s14: 2.1x faster than the larger warp kernels).  The others fold in
+// order, in the columns dense enough for it by k_numeric_own; so do the
+// order-free ones on an A (m x k, the largest of a batch) whose tile pointers
+// kXRows apart would pass 8 GB, where the default tiles need half of that.
 template <class SR>
-static void plan_fold(Context *ctx, Plan &P)
+static void plan_fold(Context *ctx, Plan &P, int64_t m, int64_t k)
 {
-    if (!(std::is_same<SR, PlusTimes<double>>::value && ctx->fold == GBC_FOLD_EXACT))
-        P.own_vsize = (int)sizeof(typename SR::V);
-    if (std::is_same<SR, PlusTimes<double>>::value && ctx->fold == GBC_FOLD_EXACT) {
-        P.want_aexp = true;
+    constexpr bool exact = std::is_same<SR, PlusTimes<double>>::value;
+    const bool fits = m < (int64_t)kXRows * 64 * kMaxMaskWords && k * (m / kXRows + 2) <= int64_t(1) << 31;
+    if (XAcc<SR>::kUse && (exact ? ctx->fold == GBC_FOLD_EXACT : fits)) {
+        P.want_x = true;
+        P.want_aexp = exact;
         P.tile_rows = kXRows;
-        // columns of more than kSmallMid multiplications go to the exact
-        // block kernel (R-MAT s14: 2.1x faster than the larger warp kernel)
         if (!P.s2_set) P.s2 = std::min<int64_t>(P.s2, kSmallMid);
+    } else if (!XAcc<SR>::kUse || exact) {
+        P.own_vsize = (int)sizeof(typename SR::V);
     }
 }
 
 template <class SR>
 static bool use_exact(const Plan &P)
 {
-    return std::is_same<SR, PlusTimes<double>>::value && P.want_aexp;
+    return XAcc<SR>::kUse && P.want_x;
 }
 
 struct Lists {
@@ -1146,10 +1153,10 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
     a.ktl_ptr = nullptr;
     a.ktl_start = nullptr;
     a.ktl_tile = nullptr;
-    if (P.want_aexp) {
+    if (P.want_x) {
         int32_t *aexp = nullptr;
-        GBC_TRY(ws.alloc_n(&aexp, (size_t)A.ncol + 1));
-        if (A.ncol > 0) {
+        if (P.want_aexp) GBC_TRY(ws.alloc_n(&aexp, (size_t)A.ncol + 1));
+        if (P.want_aexp && A.ncol > 0) {
             k_aexp_f64<<<grid_for(ctx, (A.ncol + 7) / 8, 8), 256, 0, s>>>(A.ncol, acp,
                                                                          static_cast<const double *>(A.num), aexp);
             note_launch();
@@ -1234,12 +1241,11 @@ static int plan_finalize(Workspace &ws, Plan &P)
     GBC_CUDA_TRY(cudaMemsetAsync(P.work, 0, 16 * sizeof(unsigned long long), ws.ctx->stream));
     GBC_TRY(ws.alloc_n(&P.lbuf, kLists * ((size_t)P.total_cols + 1)));
     GBC_TRY(ws.alloc_n(&P.lcnt, kLists));
-    if (P.want_aexp) {
+    if (P.want_x) {
         GBC_TRY(ws.alloc_n(&P.fb_items, (size_t)P.total_cols + 1));
         GBC_TRY(ws.alloc_n(&P.fb_cnt, 1));
         // bucketing scratch of the exact kernel, per resident block
-        GBC_TRY(set_smem(k_numeric_x, sizeof(XSmem)));
-        P.x_blocks = ws.ctx->num_sms * resident_blocks(k_numeric_x, kXThreads, sizeof(XSmem), 2);
+        P.x_blocks = ws.ctx->num_sms * 2;  // (the kernels' launch bounds and XSmem)
         GBC_TRY(ws.alloc_n(&P.xscratch, (size_t)P.x_blocks * P.xscap + 1));
     }
     GBC_CUDA_TRY(cudaMemcpyAsync(P.d, P.h.data(), P.h.size() * sizeof(SpgemmArgs), cudaMemcpyHostToDevice,
@@ -1422,9 +1428,10 @@ static int launch_big_exact(Context *ctx, Plan &P, const Lists &L, const int64_t
     const int grid = (int)std::min<int64_t>(P.x_blocks, L.n[kBigList]);  // the scratch holds P.x_blocks blocks
     GBC_CUDA_TRY(cudaMemsetAsync(P.work + 1, 0, 3 * sizeof(unsigned long long), s));
     GBC_CUDA_TRY(cudaMemsetAsync(P.fb_cnt, 0, sizeof(unsigned long long), s));
-    k_numeric_x<<<grid, kXThreads, sizeof(XSmem), s>>>(P.d, L.l[kBigList], L.n[kBigList], ccp, ccp_base, cap, out_cnt,
-                                                       overflow, cir, static_cast<double *>(cval), P.work + 1,
-                                                       P.fb_items, P.fb_cnt, P.xscratch, P.xscap);
+    GBC_TRY(set_smem(k_numeric_x<SR>, sizeof(XSmem)));
+    k_numeric_x<SR><<<grid, kXThreads, sizeof(XSmem), s>>>(P.d, L.l[kBigList], L.n[kBigList], ccp, ccp_base, cap, out_cnt,
+                                                           overflow, cir, cval, P.work + 1, P.fb_items, P.fb_cnt,
+                                                           P.xscratch, P.xscap);
     note_launch();
     GBC_CUDA_TRY(cudaGetLastError());
     return launch_big_ordered<SR>(ctx, P, P.fb_items, L.n[kBigList], P.fb_cnt, ccp, ccp_base, cap, out_cnt, overflow, cir,
@@ -1473,21 +1480,28 @@ static int run_numeric(Context *ctx, Plan &P, const Lists &L, const int64_t *ccp
                                                           overflow, cir, cval)));
     }
     if (L.n[kBigList] > 0) {
-        if (use_exact<SR>(P))
-            GBC_TRY(launch_big_exact<SR>(ctx, P, L, ccp, ccp_base, cap, out_cnt, overflow, cir, cval));
-        else
+        bool done = false;
+        if constexpr (XAcc<SR>::kUse) {
+            if (use_exact<SR>(P)) {
+                GBC_TRY(launch_big_exact<SR>(ctx, P, L, ccp, ccp_base, cap, out_cnt, overflow, cir, cval));
+                done = true;
+            }
+        }
+        if (!done)
             GBC_TRY(launch_big_ordered<SR>(ctx, P, L.l[kBigList], L.n[kBigList], nullptr, ccp, ccp_base, cap,
-                                           out_cnt, overflow,
-                                           cir, cval));
+                                           out_cnt, overflow, cir, cval));
     }
-    if (L.n[kOwnList] > 0) {
-        constexpr size_t sm = (size_t)kOwnWarps * own_rows(sizeof(typename SR::V)) * (sizeof(typename SR::V) + 1);
-        GBC_TRY(set_smem(k_numeric_own<SR>, sm));
-        const int per_sm = resident_blocks(k_numeric_own<SR>, kOwnThreads, sm, 32);
-        GBC_CUDA_TRY(cudaMemsetAsync(P.work + 4, 0, sizeof(unsigned long long), ctx->stream));
-        k_numeric_own<SR><<<grid_for(ctx, L.n[kOwnList], per_sm), kOwnThreads, sm, ctx->stream>>>(
-            P.d, L.l[kOwnList], L.n[kOwnList], ccp, ccp_base, cap, out_cnt, overflow, cir, cval, P.work + 4);
-        note_launch();
+    // (the other semirings never list columns for it)
+    if constexpr (!XAcc<SR>::kUse || std::is_same<SR, PlusTimes<double>>::value) {
+        if (L.n[kOwnList] > 0) {
+            constexpr size_t sm = (size_t)kOwnWarps * own_rows(sizeof(typename SR::V)) * (sizeof(typename SR::V) + 1);
+            GBC_TRY(set_smem(k_numeric_own<SR>, sm));
+            const int per_sm = resident_blocks(k_numeric_own<SR>, kOwnThreads, sm, 32);
+            GBC_CUDA_TRY(cudaMemsetAsync(P.work + 4, 0, sizeof(unsigned long long), ctx->stream));
+            k_numeric_own<SR><<<grid_for(ctx, L.n[kOwnList], per_sm), kOwnThreads, sm, ctx->stream>>>(
+                P.d, L.l[kOwnList], L.n[kOwnList], ccp, ccp_base, cap, out_cnt, overflow, cir, cval, P.work + 4);
+            note_launch();
+        }
     }
     GBC_CUDA_TRY(cudaGetLastError());
     return GBC_OK;
@@ -1563,7 +1577,7 @@ static int spgemm_exact(Context *ctx, const DevMatrix &A, const DevMatrix &B, co
     cudaEventRecord(ctx->ev[0], s);
     Plan P;
     plan_options(P, opt);
-    plan_fold<SR>(ctx, P);
+    plan_fold<SR>(ctx, P, A.nrow, A.ncol);
     GBC_TRY(plan_build(ws, A, B, P));
     const int64_t nb = B.nzc;
     int64_t *cnt = nullptr, *ccp = nullptr;
@@ -1892,7 +1906,7 @@ static int spgemm_phased(Context *ctx, const DevMatrix &A, const DevMatrix &B, i
     Workspace ws(ctx);
     cudaEventRecord(ctx->ev[0], s);
     Plan P;
-    plan_fold<SR>(ctx, P);
+    plan_fold<SR>(ctx, P, A.nrow, A.ncol);
     GBC_TRY(plan_build(ws, A, B, P));
     const int64_t nb = B.nzc;
     int64_t *size = nullptr;  // exact counts, or capacities when learned
@@ -2159,7 +2173,7 @@ int spgemm_learned(Context *ctx, const DevMatrix &A, const DevMatrix &B, const g
     cudaEventRecord(ctx->ev[0], s);
     Plan P;
     plan_options(P, opt);
-    plan_fold<SR>(ctx, P);
+    plan_fold<SR>(ctx, P, A.nrow, A.ncol);
     LearnedOut O;
     GBC_TRY(learned_into_slots<SR>(ctx, ws, A, B, P, O));
     const int64_t nb = O.nb;
@@ -2265,6 +2279,7 @@ int mcl_expand(gbc_context *ctx, const gbc_matrix *Am, float thr, int64_t select
     if (sizing == GBC_SIZING_LEARNED) {
         Plan P;
         LearnedOut O;
+        plan_fold<PlusTimes<float>>(ctx, P, A.nrow, A.ncol);
         GBC_TRY(learned_into_slots<PlusTimes<float>>(ctx, ws, A, A, P, O));
         int64_t *jc = nullptr;
         GBC_TRY(ws.alloc_n(&jc, O.nb + 1));
@@ -2350,7 +2365,12 @@ static int batch_build(Batch &b, const std::vector<DevMatrix> &A, const std::vec
     Context *ctx = b.ctx;
     cudaStream_t s = ctx->stream;
     Workspace &ws = *b.ws;
-    plan_fold<SR>(ctx, b.P);
+    int64_t m = 0, k = 0;
+    for (const DevMatrix &M : A) {
+        m = std::max(m, M.nrow);
+        k = std::max(k, M.ncol);
+    }
+    plan_fold<SR>(ctx, b.P, m, k);
     for (int p = 0; p < b.np; ++p) GBC_TRY(plan_add(ws, b.P, A[p], B[p]));
     GBC_TRY(plan_finalize(ws, b.P));
     const int64_t tc = b.P.total_cols;

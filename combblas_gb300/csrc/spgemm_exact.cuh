@@ -300,13 +300,131 @@ constexpr int kXLight = GBC_XLIGHT;           // runs of at most this many produ
 constexpr int kXDirect = 8192;                // a tile of more products is a visit of its own
 constexpr int64_t kXScap = int64_t(1) << 20;  // bucketed segments of one column, at most (per-block scratch)
 
+// Values of up to 8 bytes travel through the chunk tables as bits.
+template <typename V>
+__device__ __forceinline__ uint64_t x_bits(V v)
+{
+    uint64_t u = 0;
+    memcpy(&u, &v, sizeof(V));
+    return u;
+}
+
+template <typename V>
+__device__ __forceinline__ V x_from(uint64_t u)
+{
+    V v;
+    memcpy(&v, &u, sizeof(V));
+    return v;
+}
+
+// What k_numeric_x keeps in an output row's accumulator, for the semirings
+// whose add does not depend on the order (words 0 when untouched, word i at
+// w[i * R]): PlusTimes<double> is x_add128; whole-number sums are two words
+// with a carry; minima are the complement of an order-preserving key, so that
+// zero is the empty one and a larger key the better; or is a flag.
+template <class SR>
+struct XAcc {
+    static constexpr bool kUse = false;
+};
+
+template <>
+struct XAcc<PlusTimes<double>> {
+    static constexpr bool kUse = true;
+};
+
+template <>
+struct XAcc<PlusTimes<int64_t>> {
+    static constexpr bool kUse = true;
+    static __device__ __forceinline__ bool add(uint32_t *w, int R, int at, int64_t p)
+    {
+        const uint32_t lo = (uint32_t)p, hi = (uint32_t)((uint64_t)p >> 32);
+        const uint32_t old = atomicAdd(w + at, lo);
+        const uint32_t t = hi + (old > ~lo ? 1u : 0u);
+        if (t) atomicAdd(w + R + at, t);
+        return true;
+    }
+    static __device__ __forceinline__ int64_t take(uint32_t *w, int R, int at)
+    {
+        const uint64_t v = w[at] | ((uint64_t)w[R + at] << 32);
+        w[at] = 0;
+        w[R + at] = 0;
+        return (int64_t)v;
+    }
+};
+
+template <>
+struct XAcc<BoolOrAnd> {
+    static constexpr bool kUse = true;
+    static __device__ __forceinline__ bool add(uint32_t *w, int, int at, uint8_t p)
+    {
+        if (p) w[at] = 1;  // every writer writes the same
+        return true;
+    }
+    static __device__ __forceinline__ uint8_t take(uint32_t *w, int, int at)
+    {
+        const uint8_t v = (uint8_t)w[at];
+        w[at] = 0;
+        return v;
+    }
+};
+
+__device__ __forceinline__ void x_max(uint32_t *w, int at, unsigned long long key)
+{
+    unsigned long long *a = reinterpret_cast<unsigned long long *>(w) + at;
+    if (key > *reinterpret_cast<volatile unsigned long long *>(a)) atomicMax(a, key);
+}
+
+__device__ __forceinline__ uint64_t x_take(uint32_t *w, int at)
+{
+    uint64_t *a = reinterpret_cast<uint64_t *>(w) + at;
+    const uint64_t k = *a;
+    *a = 0;
+    return k;
+}
+
+struct XMinI64 {
+    static constexpr bool kUse = true;
+    static __device__ __forceinline__ bool add(uint32_t *w, int, int at, int64_t p)
+    {
+        x_max(w, at, ~((uint64_t)p ^ (1ull << 63)));
+        return true;
+    }
+    static __device__ __forceinline__ int64_t take(uint32_t *w, int, int at)
+    {
+        return (int64_t)(~x_take(w, at) ^ (1ull << 63));
+    }
+};
+
+template <>
+struct XAcc<MinPlus<int64_t>> : XMinI64 {};
+template <>
+struct XAcc<Select2ndMin<int64_t>> : XMinI64 {};
+
+// A NaN or -0.0 among the products makes the fold in order differ from the
+// minimum: add() says so, and the column goes to the ordered kernel.
+template <>
+struct XAcc<MinPlus<double>> {
+    static constexpr bool kUse = true;
+    static __device__ __forceinline__ bool add(uint32_t *w, int, int at, double p)
+    {
+        const uint64_t b = (uint64_t)__double_as_longlong(p);
+        x_max(w, at, ~(b ^ (b >> 63 ? ~0ull : 1ull << 63)));
+        return p == p && b != 1ull << 63;
+    }
+    static __device__ __forceinline__ double take(uint32_t *w, int, int at)
+    {
+        const uint64_t k = ~x_take(w, at);
+        return __longlong_as_double((long long)(k ^ (k >> 63 ? 1ull << 63 : ~0ull)));
+    }
+};
+
 // Shared memory of one k_numeric_x block.
 struct XSmem {
     uint32_t acc[4 * kXRows];              // accumulator words, plane by plane
     uint32_t bm[kXSpanTiles * kXRows / 32];   // touched rows of the visit
     uint16_t pre[kXSpanTiles * kXRows / 32];  // touched rows before each bitmap word
     uint16_t rows[kXRows];                 // row (from the visit's first) of every accumulator
-    double bv[kXSegs];                     // chunk table: B value of each segment,
+    uint64_t bv[kXSegs];                   // chunk table: bits of the B value of each segment,
     uint32_t base[kXSegs];                 //   segment start - products before it (modulo 2^32),
     int32_t off[kXSegs + 1];               //   products before each segment
     int32_t nseg;                          //   segments
@@ -320,7 +438,7 @@ struct XSmem {
     int32_t ebase;    // the column's smallest product exponent
     int64_t bs, be;   // its B entries
     int64_t *oir;     // its output
-    double *oval;
+    void *oval;
     int32_t lim;      // output entries it may write
     SpgemmArgs a;
 };
@@ -351,12 +469,15 @@ static __device__ __noinline__ bool x_has_term(const SpgemmArgs &a, int64_t bs, 
 // other than -0.0 become -0.0.  Called when the visit met a -0.0 product.
 static __device__ __noinline__ void x_fix_zeros(const XSmem &sm, int q0, int q1)
 {
+    double *oval = static_cast<double *>(sm.oval);
     for (int q = q0 + threadIdx.x; q < q1; q += kXThreads)
-        if (sm.oval[q] == 0.0 && !x_has_term(sm.a, sm.bs, sm.be, (int)sm.oir[q])) sm.oval[q] = -0.0;
+        if (oval[q] == 0.0 && !x_has_term(sm.a, sm.bs, sm.be, (int)sm.oir[q])) oval[q] = -0.0;
 }
 
-// Numeric pass for the columns of the big list, one block per column
-// (dynamic counter).  After the column's exponent window is admitted:
+// Numeric pass for the columns of the big list, one block per column (dynamic
+// counter), for PlusTimes<double> under the exact fold and the semirings whose
+// add does not depend on the order (XAcc).  After the column's exponent window
+// is admitted (exact sums):
 //  1. bucketing -- every (B entry, touched row tile of its A column) pair is
 //     counted per tile (segments and products) and written, in any order,
 //     into the block's scratch grouped by tile (a counting sort; the exact
@@ -387,12 +508,18 @@ static __device__ __noinline__ void x_fix_zeros(const XSmem &sm, int q0, int q1)
 // barriers, not by memory (DRAM 9 %).  Against one tile a visit with the
 // segments found by searches and 24-byte accumulators behind flag bytes (322
 // instead of 498 warp instructions per 32 products), R-MAT scale 20 A*A in
-// phases went from 1656 to 998 ms, all passes included (2^14: 1.94 to 1.51 ms).
-static __global__ void __launch_bounds__(kXThreads, 2)
+// phases went from 1656 to 998 ms, all passes included (2^14: 1.94 to 1.51 ms),
+// and a 30011-vertex min-plus product from 8.28 (k_numeric, warp kernels up to
+// 4096 products) to 4.0 ms.
+template <class SR>
+__global__ void __launch_bounds__(kXThreads, 2)
     k_numeric_x(const SpgemmArgs *args, const int64_t *items, int64_t nitems, const int64_t *ccp, int64_t ccp_base,
-                const int64_t *cap, int64_t *out_cnt, int32_t *overflow, int64_t *cir, double *cval,
+                const int64_t *cap, int64_t *out_cnt, int32_t *overflow, int64_t *cir, void *cval_v,
                 unsigned long long *work, int64_t *fb_items, unsigned long long *fb_count, XSeg *scratch_all, int64_t scap)
 {
+    typedef typename SR::V V;
+    typedef XAcc<SR> Acc;
+    constexpr bool EXACT = std::is_same<SR, PlusTimes<double>>::value;
     constexpr int NT = kXThreads, NW = NT / 32, R = kXRows;
     static_assert(kXTMax <= NT && kXSegs == 2 * NT && kXWins == NT && kXSort <= 4096 && kXSort <= 8 * NT, "block shape");
     extern __shared__ __align__(16) unsigned char xsm[];
@@ -449,7 +576,7 @@ static __global__ void __launch_bounds__(kXThreads, 2)
             for (int w = max(0, (p >> 5) + 1); w <= min(kXWins - 1, (p + len) >> 5); ++w) sm.win[w].y = i + 1;
         }
     };
-    auto fill_table = [&](const uint32_t (&st)[2], const int (&ln)[2], const double (&bv)[2], bool compact) -> int {
+    auto fill_table = [&](const uint32_t (&st)[2], const int (&ln)[2], const uint64_t (&bv)[2], bool compact) -> int {
         int tot, cnt = kXSegs;
         sm.win[tid] = make_uint2(0u, 0u);
         int p = block_prefix(ln[0] + ln[1], &tot);
@@ -517,7 +644,7 @@ static __global__ void __launch_bounds__(kXThreads, 2)
         const SpgemmArgs &a = sm.a;
         const int64_t i = item_col(items[ci]);
         const int64_t g = a.col_base + i;
-        const double *bval = static_cast<const double *>(a.bval);
+        const V *bval = static_cast<const V *>(a.bval);
         const int64_t bs = a.bcp[i], be = a.bcp[i + 1];
         int out = 0;  // entries written (a column's output fits its row ids: below 2^31)
         bool over = false, bad = false;
@@ -526,14 +653,20 @@ static __global__ void __launch_bounds__(kXThreads, 2)
             sm.bs = bs;
             sm.be = be;
             sm.oir = cir + out0;
-            sm.oval = cval + out0;
+            sm.oval = static_cast<V *>(cval_v) + out0;
             sm.lim = (int)min(cap ? cap[g] : ccp[g - ccp_base + 1] - out0, (int64_t)INT32_MAX);
         }
 
-        // admission: the exponent window of the column's products; pos: all
-        // of them are positive
-        bool mixed = false;
-        {
+        for (int u = tid; u < kXTMax; u += NT) {
+            sm.segcnt[u] = 0;
+            sm.prodcnt[u] = 0;
+        }
+        // admission (exact sums): the exponent window of the column's
+        // products; pos: all of them are positive
+        bool pos = true;
+        int ebase = 0;
+        if constexpr (EXACT) {
+            bool mixed = false;
             int emin = 1 << 30, emax = -(1 << 30);
             for (int64_t b = bs + tid; b < be; b += NT) {
                 const int32_t ae = a.aexp[a.brow[b]];
@@ -547,20 +680,18 @@ static __global__ void __launch_bounds__(kXThreads, 2)
                 sm.emin[warp] = emin;
                 sm.emax[warp] = emax;
             }
+            pos = !__syncthreads_or(mixed);
+            ebase = __reduce_min_sync(0xffffffffu, sm.emin[lane & (NW - 1)]);
+            const int etop = __reduce_max_sync(0xffffffffu, sm.emax[lane & (NW - 1)]);
+            if (!x_admit(ebase, etop, be - bs)) {
+                if (tid == 0) fb_items[atomicAdd(fb_count, 1ull)] = items[ci];
+                __syncthreads();  // sm.col / sm.a / sm.emin reuse
+                continue;
+            }
+            if (tid == 0) sm.ebase = ebase;  // read behind the barriers of the chunk tables
+        } else {
+            __syncthreads();
         }
-        for (int u = tid; u < kXTMax; u += NT) {
-            sm.segcnt[u] = 0;
-            sm.prodcnt[u] = 0;
-        }
-        const bool pos = !__syncthreads_or(mixed);
-        int ebase = __reduce_min_sync(0xffffffffu, sm.emin[lane & (NW - 1)]);
-        const int etop = __reduce_max_sync(0xffffffffu, sm.emax[lane & (NW - 1)]);
-        if (!x_admit(ebase, etop, be - bs)) {
-            if (tid == 0) fb_items[atomicAdd(fb_count, 1ull)] = items[ci];
-            __syncthreads();  // sm.col / sm.a / sm.emin reuse
-            continue;
-        }
-        if (tid == 0) sm.ebase = ebase;  // read behind the barriers of the chunk tables
         XPROF_LAP(0);
 
         // ---- a ranked visit's steps.  Rows are relative to the visit's first row row0.
@@ -582,13 +713,14 @@ static __global__ void __launch_bounds__(kXThreads, 2)
         // The loads of the warp's next window are issued before the current
         // window's atomics.
         auto accumulate_as = [&](int L, int row0, auto pos_t, auto direct_t) {
-            constexpr bool POS = decltype(pos_t)::value, DIRECT = decltype(direct_t)::value;
+            [[maybe_unused]] constexpr bool POS = decltype(pos_t)::value;
+            constexpr bool DIRECT = decltype(direct_t)::value;
             const int32_t *arow = sm.a.arow;
-            const double *aval = static_cast<const double *>(sm.a.aval);
-            const int ebase = sm.ebase;
+            const V *aval = static_cast<const V *>(sm.a.aval);
+            [[maybe_unused]] const int ebase = sm.ebase;
             rounds(L, true, [&](int q0, int n) {
                 int r_n = -1;
-                double a_n = 0, b_n = 0;
+                V a_n = SR::one(), b_n = SR::one();
                 auto load = [&](int w) {
                     const int p = w * 32 + lane;
                     r_n = -1;
@@ -596,17 +728,17 @@ static __global__ void __launch_bounds__(kXThreads, 2)
                         const int b = seg_of(w);
                         const uint32_t idx = sm.base[b] + (uint32_t)(q0 + p);
                         r_n = arow[idx] - row0;
-                        a_n = aval ? aval[idx] : 1.0;
-                        b_n = sm.bv[b];
+                        a_n = aval ? aval[idx] : SR::one();
+                        b_n = x_from<V>(sm.bv[b]);
                     }
                 };
                 load(warp);
                 for (int w = warp; w * 32 < n; w += NW) {
                     const int r = r_n;
-                    const double av = a_n, bv = b_n;
+                    const V av = a_n, bv = b_n;
                     load(w + NW);
                     if (r >= 0) {
-                        const uint64_t bits = (uint64_t)__double_as_longlong(__dmul_rn(av, bv));
+                        const V prod = SR::mul(av, bv);
                         int at = r;
                         if (DIRECT) {
                             atomicOr(&sm.bm[r >> 5], 1u << (r & 31));
@@ -614,9 +746,14 @@ static __global__ void __launch_bounds__(kXThreads, 2)
                             at = sm.pre[r >> 5] + __popc(sm.bm[r >> 5] & ((1u << (r & 31)) - 1));
                             sm.rows[at] = (uint16_t)r;  // every product of the row writes the same
                         }
-                        if (!POS && (bits << 1) == 0) {
-                            if (bits) sm.negzero = 1;
-                        } else if (!x_add128<POS>(sm.acc + at, R, bits, ebase)) {
+                        if constexpr (EXACT) {
+                            const uint64_t bits = (uint64_t)__double_as_longlong(prod);
+                            if (!POS && (bits << 1) == 0) {
+                                if (bits) sm.negzero = 1;
+                            } else if (!x_add128<POS>(sm.acc + at, R, bits, ebase)) {
+                                bad = true;
+                            }
+                        } else if (!Acc::add(sm.acc, R, at, prod)) {
                             bad = true;
                         }
                     }
@@ -654,24 +791,29 @@ static __global__ void __launch_bounds__(kXThreads, 2)
         };
         // accumulator `at` (row row0 + r) rounded and written as output entry q of the visit, and cleared
         auto write_one = [&](int at, int q, int r, int row0) {
-            uint32_t *w = sm.acc + at;
-            const uint64_t lo = w[0] | ((uint64_t)w[R] << 32), hi = w[2 * R] | ((uint64_t)w[3 * R] << 32);
-            w[0] = 0;
-            w[R] = 0;
-            w[2 * R] = 0;
-            w[3 * R] = 0;
-            const double v = x_round(hi, lo, 2, sm.ebase);
+            V v;
+            if constexpr (EXACT) {
+                uint32_t *w = sm.acc + at;
+                const uint64_t lo = w[0] | ((uint64_t)w[R] << 32), hi = w[2 * R] | ((uint64_t)w[3 * R] << 32);
+                w[0] = 0;
+                w[R] = 0;
+                w[2 * R] = 0;
+                w[3 * R] = 0;
+                v = x_round(hi, lo, 2, sm.ebase);
+            } else {
+                v = Acc::take(sm.acc, R, at);
+            }
             q += out;
             if (q < sm.lim) {
                 sm.oir[q] = row0 + r;
-                sm.oval[q] = v;
+                static_cast<V *>(sm.oval)[q] = v;
             } else {
                 over = true;
             }
         };
         auto end_visit = [&](int n) {
             __syncthreads();
-            if (sm.negzero) {  // block-uniform
+            if (EXACT && sm.negzero) {  // block-uniform
                 x_fix_zeros(sm, out, min(out + n, sm.lim));
                 __syncthreads();
                 if (tid == 0) sm.negzero = 0;  // read again only after another visit's barriers
@@ -712,13 +854,13 @@ static __global__ void __launch_bounds__(kXThreads, 2)
                 for (int64_t cb = bs; cb < be; cb += kXSegs) {
                     uint32_t st[2];
                     int ln[2];
-                    double en[2];  // the entry, carried in the table's value slot
+                    uint64_t en[2];  // the entry, carried in the table's value slot
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
                         const int64_t e = cb + 2 * tid + u;
                         st[u] = 0;
                         ln[u] = 0;
-                        en[u] = __longlong_as_double(e - bs);
+                        en[u] = (uint64_t)(e - bs);
                         if (e < be) {
                             const int k = a.brow[e];
                             const int64_t p0 = a.ktl_ptr[k];
@@ -736,7 +878,7 @@ static __global__ void __launch_bounds__(kXThreads, 2)
                             atomicAdd(&sm.prodcnt[t], len);
                         } else {
                             const int pos = atomicAdd(&sm.tend[t], 1);
-                            scratch[pos] = XSeg{s0, (uint32_t)len, (uint32_t)__double_as_longlong(sm.bv[b])};
+                            scratch[pos] = XSeg{s0, (uint32_t)len, (uint32_t)sm.bv[b]};
                         }
                     });
                     __syncthreads();
@@ -769,11 +911,11 @@ static __global__ void __launch_bounds__(kXThreads, 2)
         auto load_bucket = [&](const XSeg (&sg)[2]) -> int {
             const uint32_t st[2] = {sg[0].start, sg[1].start};
             const int ln[2] = {(int)sg[0].len, (int)sg[1].len};
-            double bv[2];
+            uint64_t bv[2];
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
-                const double *b = static_cast<const double *>(sm.a.bval);
-                bv[u] = b ? b[sm.bs + sg[u].e] : 1.0;
+                const V *b = static_cast<const V *>(sm.a.bval);
+                bv[u] = x_bits<V>(b ? b[sm.bs + sg[u].e] : SR::one());
             }
             return fill_table(st, ln, bv, false);
         };
@@ -896,12 +1038,11 @@ static __global__ void __launch_bounds__(kXThreads, 2)
                         fetch(sg, c0, se);
                         const int L = load_bucket(sg);
                         const int32_t *arow = sm.a.arow;
-                        const double *aval = static_cast<const double *>(sm.a.aval);
+                        const V *aval = static_cast<const V *>(sm.a.aval);
                         for_products(L, false, [&](int b, uint32_t idx, int p) {
                             const int slot = pbase + p;
                             rk0[slot] = ((uint32_t)(arow[idx] - row0) << 12) | (uint32_t)slot;
-                            rval[slot] =
-                                (uint64_t)__double_as_longlong(__dmul_rn(aval ? aval[idx] : 1.0, sm.bv[b]));
+                            rval[slot] = x_bits<V>(SR::mul(aval ? aval[idx] : SR::one(), x_from<V>(sm.bv[b])));
                         });
                         pbase += L;
                         __syncthreads();  // chunk table reuse
@@ -982,17 +1123,30 @@ static __global__ void __launch_bounds__(kXThreads, 2)
                         const int q = out + block_prefix(head ? 1 : 0, &tot);
                         if (head) {
                             const uint32_t row = key >> 12;
-                            uint64_t hi = 0, lo = 0;
-                            uint32_t fl = 0;
-                            for (int v = u; v < prods; ++v) {
-                                const uint32_t kv = src[v];
-                                if ((kv >> 12) != row) break;
-                                if (!x_acc128(hi, lo, fl, __longlong_as_double((long long)rval[kv & 4095]), ebase))
-                                    bad = true;
+                            V val;
+                            if constexpr (EXACT) {
+                                uint64_t hi = 0, lo = 0;
+                                uint32_t fl = 0;
+                                for (int v = u; v < prods; ++v) {
+                                    const uint32_t kv = src[v];
+                                    if ((kv >> 12) != row) break;
+                                    if (!x_acc128(hi, lo, fl, x_from<double>(rval[kv & 4095]), ebase)) bad = true;
+                                }
+                                val = x_round(hi, lo, fl, ebase);
+                            } else {  // any order would do
+                                val = x_from<V>(rval[key & 4095]);
+                                for (int v = u + 1; v < prods && (src[v] >> 12) == row; ++v)
+                                    val = SR::add(x_from<V>(rval[src[v] & 4095]), val);
+                                if constexpr (std::is_same<SR, MinPlus<double>>::value) {
+                                    for (int v = u; v < prods && (src[v] >> 12) == row; ++v) {
+                                        const uint64_t pb = rval[src[v] & 4095];
+                                        if (pb == 1ull << 63 || x_from<double>(pb) != x_from<double>(pb)) bad = true;
+                                    }
+                                }
                             }
                             if (q < sm.lim) {
                                 sm.oir[q] = (int64_t)row0 + (int64_t)row;
-                                sm.oval[q] = x_round(hi, lo, fl, ebase);
+                                static_cast<V *>(sm.oval)[q] = val;
                             } else {
                                 over = true;
                             }
@@ -1025,18 +1179,18 @@ static __global__ void __launch_bounds__(kXThreads, 2)
                 for (int64_t cb = bs; cb < be; cb += kXSegs) {
                     uint32_t st[2];
                     int ln[2];
-                    double bv[2];
+                    uint64_t bv[2];
 #pragma unroll
                     for (int u = 0; u < 2; ++u) {
                         const int64_t e = cb + 2 * tid + u;
                         st[u] = 0;
                         ln[u] = 0;
-                        bv[u] = 1.0;
+                        bv[u] = x_bits<V>(SR::one());
                         if (e < be) {
                             const uint32_t *tp = a.tptr + (int64_t)a.brow[e] * (a.T + 1);
                             st[u] = tp[t];
                             ln[u] = (int)(tp[t + 1] - st[u]);
-                            if (bval) bv[u] = bval[e];
+                            if (bval) bv[u] = x_bits<V>(bval[e]);
                         }
                     }
                     accumulate(fill_table(st, ln, bv, true), row0, std::true_type{});
@@ -1057,7 +1211,8 @@ static __global__ void __launch_bounds__(kXThreads, 2)
                 else
                     atomicOr(a.err, 128);  // exact sizing: counts disagree
             }
-            if (bad) atomicOr(a.err, 512);  // a product outside the admitted window
+            if (bad && EXACT) atomicOr(a.err, 512);  // a product outside the admitted window
+            if (bad && !EXACT) fb_items[atomicAdd(fb_count, 1ull)] = items[ci];  // XAcc: the ordered kernel's
         }
     }
 }

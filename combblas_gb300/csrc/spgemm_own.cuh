@@ -31,8 +31,9 @@ constexpr int64_t kOwnTable = 1ll << 28;    // pointers of a product's range tab
 constexpr int kOwnSmem = 6656 * kOwnWarps;  // accumulators and marks of a block (32 warps per SM)
 
 // Products per B entry and range from which a column is dense enough.  Below,
-// windows are mostly empty: min-plus fp64 on a 30011-vertex R-MAT takes 8.2 ms
-// with 16, 8.6 with 8 and 14.6 with 4 (k_numeric alone 8.3); fp32 ranges are
+// windows are mostly empty: 8-byte values (measured with min-plus, which
+// k_numeric_x has taken over since) on a 30011-vertex R-MAT took 8.2 ms with 16,
+// 8.6 with 8 and 14.6 with 4 (k_numeric alone 8.3); fp32 ranges are
 // nearly twice as wide, an MCL loop takes 263 ms with 8, 280 with 16, 450 without.
 __host__ __device__ constexpr int own_min(int vsize) { return vsize <= 4 ? 8 : 16; }
 

@@ -83,14 +83,16 @@ typedef struct {
     int keep_empty;  /* 1: one output column per stored column of B (SpTuples
                         view); 0: drop empty output columns (SpDCCols view) */
     int tile_rows;   /* rows of the block kernel's accumulator tile: 0 = 4096
-                        up to 2^18 rows of A and 8192 above (4096 for PlusTimes
-                        fp64 under the exact fold), or 4096 / 8192 / 16384
-                        (always 4096 under the exact fold) */
+                        up to 2^18 rows of A and 8192 above, or 4096 / 8192 /
+                        16384; always 4096 for PlusTimes fp64 under the exact
+                        fold and, on ordinary sizes, for the semirings whose
+                        add does not depend on the order */
     int64_t tiny_limit;  /* columns with <= this many multiplications use the
                             smallest warp kernel (<= 256; -1 = default 256) */
     int64_t small_limit; /* ... <= this many the larger warp kernels (<= 4096;
-                            -1 = default: 4096, or 1024 for PlusTimes fp64 under
-                            the exact fold); above it the block kernel */
+                            -1 = default: 1024, or 4096 for PlusTimes fp32 and
+                            for fp64 under the ordered fold); above it the
+                            block kernels */
 } gbc_spgemm_opts;
 
 typedef struct {
@@ -101,9 +103,9 @@ typedef struct {
     double ms_total;        /* device time of the call (CUDA events) */
     double ms_symbolic;
     double ms_numeric;
-    int64_t tile_visits_dense; /* exact-fold big columns: (column, row tile) visits through the
-                                  dense accumulator (gbc_spgemm only; 0 otherwise) */
-    int64_t tile_visits_range; /* ... and runs of light tiles summed through a sorted range */
+    int64_t tile_visits_dense; /* order-free big columns (exact sums, minima, or, whole numbers): visits
+                                  of a single row tile (gbc_spgemm only; 0 otherwise) */
+    int64_t tile_visits_range; /* ... and of runs of tiles, ranked or sorted */
 } gbc_spgemm_stats;
 
 /* ---------------------------------------------------------------- context */
