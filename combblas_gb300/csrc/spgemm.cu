@@ -1375,7 +1375,7 @@ static int launch_small(Context *ctx, Plan &P, const int64_t *items, int64_t n, 
     const size_t sm = WPB * small_warp_smem<FS, V, PACK>();
     GBC_TRY(set_smem(k_small_numeric<SR, FS, WPB, PACK>, sm));
     int per_sm = std::max(1, (int)(ctx->smem_optin / (sm + 1024)));
-    k_small_numeric<SR, FS, WPB, PACK><<<grid_for(ctx, (n + WPB - 1) / WPB, std::min(per_sm, 8)), WPB * 32, sm,
+    k_small_numeric<SR, FS, WPB, PACK><<<grid_for(ctx, (n + WPB - 1) / WPB, std::min(per_sm, std::max(8, 32 / WPB))), WPB * 32, sm,
                                          ctx->stream>>>(P.d, items, n, ccp, ccp_base, cap, out_cnt, overflow, cir,
                                                         cval);
     note_launch();

@@ -7,12 +7,15 @@
 //                   open-addressing table in shared memory (order does not
 //                   matter for a count).
 //  k_small_numeric  gathers the column's products (row, A(row,k)*B(k,j)) in
-//                   k-major order, sorts them by row with a stable LSD radix
-//                   sort (ranks within a 32-item chunk from eight ballots,
-//                   so equal digits keep their order), then folds each run of
-//                   equal rows left to right: acc = add(mrhs, acc) over k
-//                   ascending, the reference's hash-path order.  Rows come out
-//                   ascending.
+//                   k-major order, sorts them by row keeping that order, then
+//                   folds each run of equal rows left to right:
+//                   acc = add(mrhs, acc) over k ascending, the reference's
+//                   hash-path order.  Rows come out ascending.  Up to 1024
+//                   products with rows below 2^20, the keys (row and position
+//                   in one word, all different) are sorted by a bitonic network
+//                   in the warp's registers; else by a stable LSD radix sort in
+//                   shared memory (ranks within a 32-item chunk from eight
+//                   ballots, so equal digits keep their order).
 #pragma once
 
 #include <type_traits>
@@ -177,6 +180,70 @@ __device__ __forceinline__ int warp_gather(const SpgemmArgs &a, const typename S
     return base;
 }
 
+// Shared memory of one warp: values, then the keys (padded where they are
+// sorted in registers; else two buffers, the values twice when they move with
+// the keys, and the digit counts).
+template <int FS, class V, bool PACK>
+constexpr size_t small_warp_smem()
+{
+    const size_t b = PACK && FS <= 1024 ? (size_t)FS * sizeof(V) + (FS + FS / 32) * 4
+                     : PACK            ? (size_t)FS * (8 + sizeof(V)) + 1024
+                                       : (size_t)FS * (8 + 2 * sizeof(V)) + 1024;
+    return (b + 15) & ~size_t(15);
+}
+
+// Sorted keys lie at padded positions, so that lanes with K consecutive ones
+// each meet different banks.
+__device__ __forceinline__ int warp_slot(int p) { return p + (p >> 5); }
+
+// Bitonic sort of keys[0, n), n <= 32 K, in registers: element lane * K + r is
+// held in register r.  15 of the 55 steps for 1024 keys cross lanes; the three
+// 8-bit radix passes it replaces were chains of shared-memory round trips (half
+// a million fp32 columns of about 900 products 14.9 -> 10.5 ms).  The result goes
+// to keys[warp_slot(p)].  For up to 2048 keys the radix sort stays: 64 keys a
+// lane do not stay in registers, and two sorted halves merged by the lanes took
+// 20.0 ms where it takes 14.4.
+template <int K>
+static __device__ __noinline__ void warp_bitonic(uint32_t *keys, int n)
+{
+    const int lane = threadIdx.x & 31;
+    uint32_t x[K];
+#pragma unroll
+    for (int r = 0; r < K; ++r) x[r] = r * 32 + lane < n ? keys[r * 32 + lane] : 0xffffffffu;
+#pragma unroll
+    for (int k = 2; k <= 32 * K; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            if (j >= K) {  // the partner is register r of another lane
+                const bool up = ((lane * K) & k) == 0, low = (lane & (j / K)) == 0;
+#pragma unroll
+                for (int r = 0; r < K; ++r) {
+                    const uint32_t y = __shfl_xor_sync(0xffffffffu, x[r], j / K);
+                    x[r] = low == up ? min(x[r], y) : max(x[r], y);
+                }
+            } else {
+                const bool lane_up = ((lane * K) & k) == 0;  // direction where k spans lanes
+#pragma unroll
+                for (int r = 0; r < K; ++r) {
+                    if (r & j) continue;
+                    const uint32_t a = min(x[r], x[r | j]), b = max(x[r], x[r | j]);
+                    if (k < K) {
+                        x[r] = (r & k) == 0 ? a : b;
+                        x[r | j] = (r & k) == 0 ? b : a;
+                    } else {
+                        x[r] = lane_up ? a : b;
+                        x[r | j] = lane_up ? b : a;
+                    }
+                }
+            }
+        }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < K; ++r) keys[warp_slot(lane * K + r)] = x[r];
+    __syncwarp();
+}
+
 // Numeric for small columns.  `cap` (optional): per-column capacity in the
 // output (learned sizing); when given, the column writes at ccp[i - base]
 // and a column whose distinct rows exceed cap[i] writes nothing and is
@@ -194,13 +261,14 @@ __global__ void __launch_bounds__(WPB * 32) k_small_numeric(const SpgemmArgs *ar
     extern __shared__ __align__(16) unsigned char smem[];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const unsigned lt = (1u << lane) - 1;
-    constexpr size_t per_warp = PACK ? (size_t)FS * (8 + sizeof(V)) + 1024 : (size_t)FS * (8 + 2 * sizeof(V)) + 1024;
-    unsigned char *basep = smem + (size_t)w * ((per_warp + 15) & ~size_t(15));
+    constexpr bool REG = PACK && FS <= 1024;  // keys sorted in registers
+    unsigned char *basep = smem + (size_t)w * small_warp_smem<FS, V, PACK>();
     V *vals0 = reinterpret_cast<V *>(basep);
     V *vals1 = PACK ? vals0 : vals0 + FS;
     uint32_t *keys0 = reinterpret_cast<uint32_t *>(vals0 + (PACK ? FS : 2 * FS));
-    uint32_t *keys1 = keys0 + FS;
+    uint32_t *keys1 = keys0 + (REG ? 0 : FS);
     int32_t *hist = reinterpret_cast<int32_t *>(keys1 + FS);
+    auto slot = [](int p) { return REG ? warp_slot(p) : p; };
     V *cval = static_cast<V *>(cval_v);
     const int shift0 = PACK ? 12 : 0;
 
@@ -221,7 +289,15 @@ __global__ void __launch_bounds__(WPB * 32) k_small_numeric(const SpgemmArgs *ar
         // 2. stable LSD radix sort by row, 8 bits per pass
         uint32_t *ks = keys0, *kd = keys1;
         V *vs = vals0, *vd = vals1;
-        for (int shift = shift0; shift < shift0 + key_bits; shift += 8) {
+        if constexpr (REG) {
+            if (FS == 256 || n <= 256)
+                warp_bitonic<8>(ks, n);
+            else if (n <= 512)
+                warp_bitonic<16>(ks, n);
+            else
+                warp_bitonic<32>(ks, n);
+        }
+        for (int shift = shift0; !REG && shift < shift0 + key_bits; shift += 8) {
             for (int d = lane; d < 256; d += 32) hist[d] = 0;
             __syncwarp();
             for (int p = lane; p < n; p += 32) atomicAdd(&hist[(ks[p] >> shift) & 255], 1);
@@ -300,9 +376,9 @@ __global__ void __launch_bounds__(WPB * 32) k_small_numeric(const SpgemmArgs *ar
         for (int p0 = 0; p0 < n; p0 += 32) {
             const int p = p0 + lane;
             const bool act = p < n;
-            const uint32_t kk = act ? ks[p] : 0u;
+            const uint32_t kk = act ? ks[slot(p)] : 0u;
             const int row = act ? (int)(PACK ? (kk >> 12) : kk) : -1;
-            const bool head = act && (p == 0 || (int)(PACK ? (ks[p - 1] >> 12) : ks[p - 1]) != row);
+            const bool head = act && (p == 0 || (int)(PACK ? (ks[slot(p - 1)] >> 12) : ks[p - 1]) != row);
             const unsigned hm = __ballot_sync(0xffffffffu, head);
             if (head) {
                 V v = PACK ? vs[kk & 4095] : vs[p];
@@ -312,7 +388,7 @@ __global__ void __launch_bounds__(WPB * 32) k_small_numeric(const SpgemmArgs *ar
                     uint32_t fl = 0;
                     bool ok = true;
                     for (int q = p; q < n; ++q) {
-                        const uint32_t kq = ks[q];
+                        const uint32_t kq = ks[slot(q)];
                         if ((int)(PACK ? (kq >> 12) : kq) != row) break;
                         ok &= x_acc128(hi, lo, fl, (double)(PACK ? vs[kq & 4095] : vs[q]), ebase);
                     }
@@ -320,7 +396,7 @@ __global__ void __launch_bounds__(WPB * 32) k_small_numeric(const SpgemmArgs *ar
                     if (!ok) atomicOr(a.err, 512);
                 } else {
                     for (int q = p + 1; q < n; ++q) {
-                        const uint32_t kq = ks[q];
+                        const uint32_t kq = ks[slot(q)];
                         if ((int)(PACK ? (kq >> 12) : kq) != row) break;
                         v = SR::add(PACK ? vs[kq & 4095] : vs[q], v);
                     }
@@ -347,13 +423,6 @@ __global__ void __launch_bounds__(WPB * 32) k_small_numeric(const SpgemmArgs *ar
         }
         __syncwarp();
     }
-}
-
-template <int FS, class V, bool PACK>
-constexpr size_t small_warp_smem()
-{
-    return ((PACK ? (size_t)FS * (8 + sizeof(V)) + 1024 : (size_t)FS * (8 + 2 * sizeof(V)) + 1024) + 15) &
-           ~size_t(15);
 }
 
 }  // namespace gbc
