@@ -223,8 +223,10 @@ __global__ void k_classify(const int64_t *flop, const int64_t *bcp, int64_t own_
     const int64_t i = j0 + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     int cls = -1;
+    unsigned long long fsum = 0;
     if (i < j1 && (!only_flagged || only_flagged[col_base + i])) {
         const int64_t f = flop[i];
+        fsum = f;
         if (f == 0) {
             if (cnt_zero) cnt_zero[col_base + i] = 0;
         } else if (f <= s1) {
@@ -237,6 +239,9 @@ __global__ void k_classify(const int64_t *flop, const int64_t *bcp, int64_t own_
             cls = kWarpClasses + (f > (1ll << 23) ? 0 : f > (1ll << 21) ? 1 : f > (1ll << 19) ? 2 : 3);
         }
     }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) fsum += __shfl_xor_sync(0xffffffffu, fsum, o);
+    if (lane == 0 && fsum) atomicAdd(&counts[kLists], fsum);
 #pragma unroll
     for (int c = 0; c < kLists; ++c) {
         const unsigned m = __ballot_sync(0xffffffffu, cls == c);
@@ -1046,6 +1051,8 @@ int prepare_operands(Workspace &ws, const DevMatrix &A, const DevMatrix &B, Spge
 
 // Everything the passes need, built once: one descriptor per product of a
 // batch (a single product is a batch of one).
+constexpr int64_t kKtlBound = 8192;
+
 struct Plan {
     std::vector<SpgemmArgs> h;        // host copies of the descriptors
     SpgemmArgs *d = nullptr;          // device array
@@ -1106,6 +1113,7 @@ struct Lists {
     // [kOwnList]: big columns for k_numeric_own
     const int64_t *l[kWarpClasses + 2] = {};
     int64_t n[kWarpClasses + 2] = {};
+    int64_t flops = 0;  // multiplications of all columns looked at
     int64_t total() const
     {
         int64_t t = 0;
@@ -1169,8 +1177,11 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
             k_ktl_count<<<(unsigned)((A.ncol + 255) / 256), 256, 0, s>>>(A.ncol, amask, a.mask_words, kptr);
             note_launch();
             GBC_TRY(exclusive_scan_i64(ws, kptr, kptr, A.ncol, s));
-            int64_t nent = 0;
-            GBC_TRY(read_i64(ctx, kptr + A.ncol, &nent));
+            // A column touches at most as many tiles as it has entries: that
+            // bound does where the lists and the scratch stay small (4 KB
+            // per entry over all blocks), and saves the read-back.
+            int64_t nent = A.nnz;
+            if (nent > kKtlBound) GBC_TRY(read_i64(ctx, kptr + A.ncol, &nent));
             P.xscap = std::max(P.xscap, std::min(nent, kXScap));
             uint32_t *kst = nullptr;
             uint16_t *ktt = nullptr;
@@ -1240,7 +1251,7 @@ static int plan_finalize(Workspace &ws, Plan &P)
     GBC_TRY(ws.alloc_n(&P.work, 16));
     GBC_CUDA_TRY(cudaMemsetAsync(P.work, 0, 16 * sizeof(unsigned long long), ws.ctx->stream));
     GBC_TRY(ws.alloc_n(&P.lbuf, kLists * ((size_t)P.total_cols + 1)));
-    GBC_TRY(ws.alloc_n(&P.lcnt, kLists));
+    GBC_TRY(ws.alloc_n(&P.lcnt, kLists + 1));
     if (P.want_x) {
         GBC_TRY(ws.alloc_n(&P.fb_items, (size_t)P.total_cols + 1));
         GBC_TRY(ws.alloc_n(&P.fb_cnt, 1));
@@ -1275,7 +1286,7 @@ static int plan_build(Workspace &ws, const DevMatrix &A, const DevMatrix &B, Pla
 static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j1, Lists &L, int64_t *cnt_zero,
                          const int32_t *flagged = nullptr)
 {
-    constexpr int NL = kLists;
+    constexpr int NL = kLists + 1;  // and the multiplications
     GBC_CUDA_TRY(cudaMemsetAsync(P.lcnt, 0, NL * sizeof(unsigned long long), s));
     const int64_t stride = P.total_cols + 1;
     int64_t *lbig = P.lbuf + kWarpClasses * stride;
@@ -1312,6 +1323,7 @@ static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j
     L.n[kBigList] = nbig;
     L.l[kOwnList] = P.lbuf + kOwnSlot * stride;
     L.n[kOwnList] = (int64_t)h[kOwnSlot];
+    L.flops = (int64_t)h[kLists];
     if (L.n[kOwnList] > 0 && !P.own_built) GBC_TRY(plan_own(P));
     return GBC_OK;
 }
@@ -1507,13 +1519,27 @@ static int run_numeric(Context *ctx, Plan &P, const Lists &L, const int64_t *ccp
     return GBC_OK;
 }
 
-static int check_err(Context *ctx, const Plan &P)
+// The products' error flags, and with `visits` the visit counts of
+// k_numeric_x, behind one synchronisation.
+static int check_err(Context *ctx, const Plan &P, int64_t *visits = nullptr)
 {
-    for (const SpgemmArgs &a : P.h) {
-        int32_t herr = 0;
-        GBC_CUDA_TRY(cudaMemcpyAsync(&herr, a.err, sizeof(herr), cudaMemcpyDeviceToHost, ctx->stream));
+    constexpr size_t kBatch = 512;
+    int32_t *h = static_cast<int32_t *>(ctx->pinned);
+    int64_t *hv = reinterpret_cast<int64_t *>(h + kBatch);
+    if (visits)
+        GBC_CUDA_TRY(cudaMemcpyAsync(hv, P.work + 2, 2 * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+    for (size_t q0 = 0; q0 < P.h.size(); q0 += kBatch) {
+        const size_t n = std::min(P.h.size() - q0, kBatch);
+        for (size_t q = 0; q < n; ++q)
+            GBC_CUDA_TRY(
+                cudaMemcpyAsync(h + q, P.h[q0 + q].err, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
         GBC_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-        if (herr) return fail(GBC_ECUDA, "internal error: numeric and symbolic counts disagree");
+        for (size_t q = 0; q < n; ++q)
+            if (h[q]) return fail(GBC_ECUDA, "internal error: numeric and symbolic counts disagree");
+    }
+    if (visits) {
+        visits[0] = hv[0];
+        visits[1] = hv[1];
     }
     return GBC_OK;
 }
@@ -1604,13 +1630,14 @@ static int spgemm_exact(Context *ctx, const DevMatrix &A, const DevMatrix &B, co
     cudaEventRecord(ctx->ev[3], s);
     if (rc == GBC_OK) rc = finish_columns(ctx, ws, B, opt, nb, cnt, C);
     cudaEventRecord(ctx->ev[4], s);
-    if (rc == GBC_OK) rc = check_err(ctx, P);
+    int64_t visits[2] = {0, 0};
+    if (rc == GBC_OK) rc = check_err(ctx, P, use_exact<SR>(P) ? visits : nullptr);
     if (rc != GBC_OK) {
         gbc_result_free(C);
         return rc;
     }
     if (st) {
-        st->flops = sum_i64(ws, ctx, P.a().flop, nb);
+        st->flops = L.flops;
         st->nnz = nnzc;
         st->overflow_cols = 0;
         st->alloc_entries = nnzc;
@@ -1621,12 +1648,8 @@ static int spgemm_exact(Context *ctx, const DevMatrix &A, const DevMatrix &B, co
         st->ms_total = t04;
         st->ms_symbolic = t12;
         st->ms_numeric = t23;
-        st->tile_visits_dense = 0;
-        st->tile_visits_range = 0;
-        if (use_exact<SR>(P)) {
-            GBC_TRY(read_i64(ctx, reinterpret_cast<const int64_t *>(P.work + 2), &st->tile_visits_dense));
-            GBC_TRY(read_i64(ctx, reinterpret_cast<const int64_t *>(P.work + 3), &st->tile_visits_range));
-        }
+        st->tile_visits_dense = visits[0];
+        st->tile_visits_range = visits[1];
     }
     *Cout = C;
     return GBC_OK;
@@ -2419,7 +2442,12 @@ static int spgemm_entry(gbc_context *ctx, int vt, const gbc_matrix *Am, const gb
     Workspace ws(ctx);
     DevMatrix A, B;
     GBC_TRY(upload(ws, Am, vt, &A));
-    GBC_TRY(upload(ws, Bm, vt, &B));
+    if (Am && Bm && Bm->cp == Am->cp && Bm->jc == Am->jc && Bm->ir == Am->ir && Bm->num == Am->num &&
+        Bm->where == Am->where && Bm->nrow == Am->nrow && Bm->ncol == Am->ncol && Bm->nzc == Am->nzc &&
+        Bm->nnz == Am->nnz)
+        B = A;  // the same arrays: copied once
+    else
+        GBC_TRY(upload(ws, Bm, vt, &B));
     if (opt.sizing == GBC_SIZING_LEARNED) return spgemm_learned<SR>(ctx, A, B, opt, vt, C, st);
     return spgemm_exact<SR>(ctx, A, B, opt, vt, C, st);
 }
@@ -2575,6 +2603,21 @@ static int multiway_merge(Context *ctx, int vt, int nlists, const gbc_matrix *li
 
 using namespace gbc;
 
+// Column pointers from `base` on, rows and values (words of 8, 4 or 1 bytes) of
+// one product.
+template <typename W>
+__global__ void k_batch_out(int64_t nb, const int64_t *ccp, int64_t base, int64_t *cp, int64_t n, const int64_t *ir,
+                            int64_t *oir, const W *num, W *onum)
+{
+    const int64_t i0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, stride = int64_t(gridDim.x) * blockDim.x;
+    if (cp)
+        for (int64_t i = i0; i <= nb; i += stride) cp[i] = ccp[i] - base;
+    if (oir)
+        for (int64_t i = i0; i < n; i += stride) oir[i] = ir[i];
+    if (onum)
+        for (int64_t i = i0; i < n; i += stride) onum[i] = num[i];
+}
+
 extern "C" {
 
 int gbc_spgemm(gbc_context *ctx, int sr, int vt, const gbc_matrix *A, const gbc_matrix *B,
@@ -2724,12 +2767,6 @@ int gbc_batch_info(const gbc_batch *b, int p, int64_t *nzc, int64_t *nnz, int64_
     return GBC_OK;
 }
 
-__global__ void k_rebase(int64_t n, const int64_t *src, int64_t base, int64_t *dst)
-{
-    const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i <= n) dst[i] = src[i] - base;
-}
-
 // Product p of the batch: cp[nzc+1] (one column per stored column of its B),
 // ir[nnz], num[nnz], in host or device memory.
 int gbc_batch_result(const gbc_batch *b, int p, int64_t *cp, int64_t *ir, void *num, int where)
@@ -2739,18 +2776,30 @@ int gbc_batch_result(const gbc_batch *b, int p, int64_t *cp, int64_t *ir, void *
     cudaStream_t s = b->ctx->stream;
     const SpgemmArgs &a = b->P.h[p];
     const int64_t base = b->hccp[a.col_base], n = b->hccp[a.col_base + a.nb] - base;
-    cudaMemcpyKind k = where == GBC_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost;
-    if (cp) {
-        if (where == GBC_DEVICE) {
-            k_rebase<<<(unsigned)((a.nb + 256) / 256), 256, 0, s>>>(a.nb, b->ccp + a.col_base, base, cp);
+    if (where == GBC_DEVICE) {
+        const int grid = (int)std::min<int64_t>((std::max(n, a.nb) + 512) / 512, (int64_t)b->ctx->num_sms * 8);
+        auto out = [&](auto word) {
+            typedef decltype(word) W;
+            k_batch_out<W><<<grid, 512, 0, s>>>(a.nb, b->ccp + a.col_base, base, cp, n, b->ir + base, ir,
+                                                static_cast<const W *>(b->num) + base, static_cast<W *>(num));
             note_launch();
-        } else {
+        };
+        if (b->vsize == 8)
+            out(uint64_t());
+        else if (b->vsize == 4)
+            out(uint32_t());
+        else
+            out(uint8_t());
+        GBC_CUDA_TRY(cudaGetLastError());
+    } else {
+        if (cp)
             for (int64_t j = 0; j <= a.nb; ++j) cp[j] = b->hccp[a.col_base + j] - base;
-        }
+        if (ir && n)
+            GBC_CUDA_TRY(cudaMemcpyAsync(ir, b->ir + base, n * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
+        if (num && n)
+            GBC_CUDA_TRY(cudaMemcpyAsync(num, static_cast<const char *>(b->num) + base * b->vsize, n * b->vsize,
+                                         cudaMemcpyDeviceToHost, s));
     }
-    if (ir && n) GBC_CUDA_TRY(cudaMemcpyAsync(ir, b->ir + base, n * sizeof(int64_t), k, s));
-    if (num && n)
-        GBC_CUDA_TRY(cudaMemcpyAsync(num, static_cast<const char *>(b->num) + base * b->vsize, n * b->vsize, k, s));
     GBC_CUDA_TRY(cudaStreamSynchronize(s));
     return GBC_OK;
 }
