@@ -203,11 +203,23 @@ constexpr int kWarpClasses = 4;
 #define GBC_SMALL2 kSmall2
 #endif
 
-// Big columns are binned by flop (> 2^23, > 2^21, > 2^19, the rest) and
-// listed heaviest bin first, so the longest columns start early and do not
-// run alone at the end of a launch (a scale-20 R-MAT hub column holds up to
-// 2*10^7 products, most of one block's share of a phase).
-constexpr int kBigBins = 4;
+// Big columns are binned by flop (one bin per power of two above 2^15 up to
+// 2^20, then per factor of four) and listed heaviest bin first, so the longest
+// columns start early and do not run alone at the end of a launch: a hub
+// column of a scale-14 R-MAT square holds most of one block's share of the
+// whole product (1.6*10^5 products), one at scale 20 up to 2*10^7.
+constexpr int kBigBins = 8;
+__device__ __forceinline__ int big_bin(int64_t f)
+{
+    return f > (1ll << 22)   ? 0
+           : f > (1ll << 20) ? 1
+           : f > (1ll << 19) ? 2
+           : f > (1ll << 18) ? 3
+           : f > (1ll << 17) ? 4
+           : f > (1ll << 16) ? 5
+           : f > (1ll << 15) ? 6
+                             : 7;
+}
 constexpr int kBigList = kWarpClasses;            // index of the big list in Lists
 constexpr int kOwnList = kBigList + 1;            // ... of the columns for k_numeric_own
 constexpr int kOwnSlot = kWarpClasses + kBigBins; // its slot while classifying
@@ -236,7 +248,7 @@ __global__ void k_classify(const int64_t *flop, const int64_t *bcp, int64_t own_
         } else if (own_need > 0 && f >= own_need * (bcp[i + 1] - bcp[i])) {
             cls = kOwnSlot;
         } else {
-            cls = kWarpClasses + (f > (1ll << 23) ? 0 : f > (1ll << 21) ? 1 : f > (1ll << 19) ? 2 : 3);
+            cls = kWarpClasses + big_bin(f);
         }
     }
 #pragma unroll
