@@ -1750,24 +1750,66 @@ __global__ void k_final_counts(int64_t nb, const int32_t *flag, const int64_t *e
 }
 
 // Gather every column from its region (slots, or the overflow region for
-// flagged columns) into the contiguous result.
+// flagged columns) into the contiguous result: dst holds the column starts
+// (nb + 1).  A warp owns equal pieces of the result, found by a search in dst,
+// instead of columns: one warp copying a hub column was the launch's end (a
+// scale-16 R-MAT square 4.8 -> 1.8 ms, the whole product 18.9 -> 15.8 ms).
+// Bound by its 32 bytes per entry.
+constexpr int kCompactPiece = 1024;
 template <typename V>
-__global__ void k_compact(int64_t nb, const int64_t *cnt, const int64_t *dst, const int32_t *flag,
-                          const int64_t *beg0, const int64_t *ir0, const V *v0, const int64_t *beg1,
-                          const int64_t *ir1, const V *v1, int64_t *oir, V *ov)
+__global__ void k_compact(int64_t nb, const int64_t *dst, const int32_t *flag, const int64_t *beg0,
+                          const int64_t *ir0, const V *v0, const int64_t *beg1, const int64_t *ir1, const V *v1,
+                          int64_t *oir, V *ov)
 {
     const int lane = threadIdx.x & 31;
     const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t i = warp; i < nb; i += nwarps) {
-        const bool o = flag[i] != 0;
-        const int64_t b = o ? beg1[i] : beg0[i];
-        const int64_t *sir = o ? ir1 : ir0;
-        const V *sv = o ? v1 : v0;
-        const int64_t d = dst[i];
-        for (int64_t p = lane; p < cnt[i]; p += 32) {
-            oir[d + p] = sir[b + p];
-            ov[d + p] = sv[b + p];
+    const int64_t n = dst[nb];
+    for (int64_t q = warp * kCompactPiece; q < n; q += nwarps * kCompactPiece) {
+        const int64_t qe = min(q + kCompactPiece, n);
+        // the last column that starts at or before q (it holds entry q)
+        int64_t lo = 0, hi = nb;
+        while (hi - lo > 1) {
+            const int64_t mid = (lo + hi) >> 1;
+            if (dst[mid] <= q)
+                lo = mid;
+            else
+                hi = mid;
+        }
+        for (int64_t i = lo, pos = q; pos < qe;) {
+            // 32 columns' ends at a time; the empty ones cost nothing
+            const int64_t mine = i + lane < nb ? dst[i + lane + 1] : n;
+            unsigned todo = __ballot_sync(0xffffffffu, mine > pos);
+            while (todo && pos < qe) {
+                const int l = __ffs(todo) - 1;
+                const int64_t e = min(__shfl_sync(0xffffffffu, mine, l), qe), c = i + l;
+                const bool o = flag[c] != 0;
+                const int64_t sh = (o ? beg1[c] : beg0[c]) - dst[c];
+                const int64_t *sir = (o ? ir1 : ir0) + sh;
+                const V *sv = (o ? v1 : v0) + sh;
+                int64_t p = pos + lane;
+                for (; p + 96 < e; p += 128) {
+                    int64_t r[4];
+                    V x[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        r[u] = sir[p + 32 * u];
+                        x[u] = sv[p + 32 * u];
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        oir[p + 32 * u] = r[u];
+                        ov[p + 32 * u] = x[u];
+                    }
+                }
+                for (; p < e; p += 32) {
+                    oir[p] = sir[p];
+                    ov[p] = sv[p];
+                }
+                pos = e;
+                todo = __ballot_sync(0xffffffffu, mine > pos);
+            }
+            i += 32;
         }
     }
 }
@@ -2226,9 +2268,9 @@ int spgemm_learned(Context *ctx, const DevMatrix &A, const DevMatrix &B, const g
     C->nnz = nnzc;
     if (rc == GBC_OK) rc = device_alloc(ctx, (void **)&C->ir, (nnzc + 1) * sizeof(int64_t));
     if (rc == GBC_OK) rc = device_alloc(ctx, &C->num, (nnzc + 1) * sizeof(V));
-    if (rc == GBC_OK && nb > 0) {
-        k_compact<V><<<grid_for(ctx, (nb + 7) / 8, 8), 256, 0, s>>>(
-            nb, O.cnt, ccp, O.flag, O.beg0, O.ir0, static_cast<const V *>(O.v0), O.beg1, O.ir1,
+    if (rc == GBC_OK && nnzc > 0) {
+        k_compact<V><<<grid_for(ctx, (nnzc + 8 * kCompactPiece - 1) / (8 * kCompactPiece), 8), 256, 0, s>>>(
+            nb, ccp, O.flag, O.beg0, O.ir0, static_cast<const V *>(O.v0), O.beg1, O.ir1,
             static_cast<const V *>(O.v1), C->ir, static_cast<V *>(C->num));
         note_launch();
     }
