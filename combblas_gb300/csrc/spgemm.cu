@@ -41,55 +41,96 @@
 namespace gbc {
 
 // ----------------------------------------------------------------- prepare
-// One warp per column of A.  tptr[k*(T+1)+t] = first position of column k
-// whose row is >= t*R (t = 0..T); arow = rows as int32.
-__global__ void k_prep_a(int64_t ncol, int64_t nrow, const int64_t *cp, const int64_t *jc, int64_t nzc,
-                         int64_t nnz, const int64_t *ir, int32_t *arow, uint32_t *tptr, int T, int R, int32_t *err)
+// The preparation kernels give every warp a column and the whole block the
+// columns longer than kLongCol, kPrepUnroll loads in flight per thread: one
+// warp alone on a hub column (2*10^3 to 10^5 entries, a chain of loads) was
+// the end of each launch.  The three kernels of a scale-14 R-MAT square 144 ->
+// 51 us (the product 1265 -> 1193), the product of a 30011-vertex one 3760 ->
+// 3614 us.
+constexpr int kLongCol = 256;
+constexpr int kPrepWarps = 8;
+constexpr int kPrepUnroll = 4;
+
+// load(p) and then use(i, p, s, e, loaded) for every entry p of [s, e) =
+// [cp[i], cp[i + 1]) of the columns for which ok(i, s, e, lane) holds.
+template <class Ok, class Load, class Use>
+__device__ __forceinline__ void each_entry(int64_t n, const int64_t *cp, Ok ok, Load load, Use use)
 {
-    int lane = threadIdx.x & 31;
-    int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t i = warp; i < nzc; i += nwarps) {
-        int64_t s = cp[i], e = cp[i + 1];
-        int64_t c = jc ? jc[i] : i;
-        if (e < s || (i == 0 && s != 0) || e > nnz) {
-            if (lane == 0) atomicOr(err, 1);
-            continue;
+    __shared__ int64_t ls[kPrepWarps], le[kPrepWarps];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    auto run = [&](int64_t i, int64_t s, int64_t e, int64_t first, int64_t stride) {
+        for (int64_t p = s + first; p < e; p += kPrepUnroll * stride) {
+            decltype(load(p, s)) v[kPrepUnroll];
+#pragma unroll
+            for (int u = 0; u < kPrepUnroll; ++u)
+                if (p + u * stride < e) v[u] = load(p + u * stride, s);
+#pragma unroll
+            for (int u = 0; u < kPrepUnroll; ++u)
+                if (p + u * stride < e) use(i, p + u * stride, s, e, v[u]);
         }
-        if (c < 0 || c >= ncol || (jc && i > 0 && jc[i - 1] >= c)) {
-            if (lane == 0) atomicOr(err, 2);
-            continue;
+    };
+    for (int64_t i0 = int64_t(blockIdx.x) * kPrepWarps; i0 < n; i0 += int64_t(gridDim.x) * kPrepWarps) {
+        const int64_t i = i0 + w;
+        int64_t s = 0, e = 0;
+        if (i < n) {
+            s = cp[i];
+            e = cp[i + 1];
+            if (!ok(i, s, e, lane)) e = s;
         }
-        uint32_t *tp = tptr + c * (int64_t)(T + 1);
-        int last_t = -1;
-        for (int64_t b = s; b < e; b += 32) {
-            int64_t p = b + lane;
-            int t = -1;
-            int64_t r = -1;
-            if (p < e) {
-                r = ir[p];
-                if (r < 0 || r >= nrow) {
-                    atomicOr(err, 4);
-                    r = 0;
-                }
-                if (p > s && ir[p - 1] >= ir[p]) atomicOr(err, 8);
-                arow[p] = (int32_t)r;
-                t = (int)(r / R);
-            }
-            int tprev = __shfl_up_sync(0xffffffffu, t, 1);
-            if (lane == 0) tprev = last_t;
-            if (p < e) {
-                for (int u = tprev + 1; u <= t; ++u) tp[u] = (uint32_t)p;
-            }
-            // the highest valid lane carries the last tile seen
-            unsigned vm = __ballot_sync(0xffffffffu, p < e);
-            int hi = 31 - __clz(vm);
-            last_t = __shfl_sync(0xffffffffu, t, hi);
-        }
+        const bool is_long = e - s > kLongCol;
         if (lane == 0) {
-            for (int u = last_t + 1; u <= T; ++u) tp[u] = (uint32_t)e;
+            ls[w] = s;
+            le[w] = is_long ? e : s;
         }
+        if (!is_long) run(i, s, e, lane, 32);
+        __syncthreads();
+        for (int q = 0; q < kPrepWarps; ++q) run(i0 + q, ls[q], le[q], threadIdx.x, kPrepWarps * 32);
+        __syncthreads();
     }
+}
+
+struct RowPair {
+    int64_t r, prev;  // an entry's row and the one before it in its column (-1: none)
+};
+
+// tptr[k*(T+1)+t] = first position of column k whose row is >= t*R (t = 0..T;
+// the columns without entries are k_fill_empty_tptr's); arow = rows as int32.
+__global__ void __launch_bounds__(kPrepWarps * 32)
+    k_prep_a(int64_t ncol, int64_t nrow, const int64_t *cp, const int64_t *jc, int64_t nzc, int64_t nnz,
+             const int64_t *ir, int32_t *arow, uint32_t *tptr, int T, int R, int32_t *err)
+{
+    each_entry(
+        nzc, cp,
+        [&](int64_t i, int64_t s, int64_t e, int lane) {
+            const int64_t c = jc ? jc[i] : i;
+            if (e < s || (i == 0 && s != 0) || e > nnz) {
+                if (lane == 0) atomicOr(err, 1);
+                return false;
+            }
+            if (c < 0 || c >= ncol || (jc && i > 0 && jc[i - 1] >= c)) {
+                if (lane == 0) atomicOr(err, 2);
+                return false;
+            }
+            return true;
+        },
+        [&](int64_t p, int64_t s) { return RowPair{ir[p], p > s ? ir[p - 1] : -1}; },
+        [&](int64_t i, int64_t p, int64_t s, int64_t e, RowPair v) {
+            if (p > s && v.prev >= v.r) atomicOr(err, 8);
+            if (v.r < 0 || v.r >= nrow) {
+                atomicOr(err, 4);
+                v.r = 0;
+            }
+            if (v.prev < 0 || v.prev >= nrow) v.prev = 0;  // (reported where it is an entry)
+            arow[p] = (int32_t)v.r;
+            const int t = (int)((uint32_t)v.r / (uint32_t)R);
+            const int tprev = p > s ? (int)((uint32_t)v.prev / (uint32_t)R) : -1;
+            if (tprev != t || p == e - 1) {
+                uint32_t *tp = tptr + (jc ? jc[i] : i) * (int64_t)(T + 1);
+                for (int u = tprev + 1; u <= t; ++u) tp[u] = (uint32_t)p;
+                if (p == e - 1)
+                    for (int u = t + 1; u <= T; ++u) tp[u] = (uint32_t)e;
+            }
+        });
 }
 
 // Dense column pointers of a DCSC matrix (acp[c] = start of column c).
@@ -117,28 +158,24 @@ __global__ void k_fill_empty_tptr(int64_t ncol, const int64_t *acp, uint32_t *tp
     }
 }
 
-__global__ void k_prep_b(int64_t nzc, int64_t nnz, const int64_t *cp, const int64_t *ir, int64_t kdim,
-                         int32_t *brow, int32_t *err)
+__global__ void __launch_bounds__(kPrepWarps * 32)
+    k_prep_b(int64_t nzc, int64_t nnz, const int64_t *cp, const int64_t *ir, int64_t kdim, int32_t *brow,
+             int32_t *err)
 {
-    int lane = threadIdx.x & 31;
-    int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t i = warp; i < nzc; i += nwarps) {
-        int64_t s = cp[i], e = cp[i + 1];
-        if (e < s || (i == 0 && s != 0) || e > nnz) {
-            if (lane == 0) atomicOr(err, 16);
-            continue;
-        }
-        for (int64_t p = s + lane; p < e; p += 32) {
-            int64_t r = ir[p];
-            if (r < 0 || r >= kdim) {
-                atomicOr(err, 32);
-                r = 0;
-            }
-            if (p > s && ir[p - 1] >= ir[p]) atomicOr(err, 64);
-            brow[p] = (int32_t)r;
-        }
-    }
+    each_entry(
+        nzc, cp,
+        [&](int64_t i, int64_t s, int64_t e, int lane) {
+            const bool ok = !(e < s || (i == 0 && s != 0) || e > nnz);
+            if (!ok && lane == 0) atomicOr(err, 16);
+            return ok;
+        },
+        [&](int64_t p, int64_t s) { return RowPair{ir[p], p > s ? ir[p - 1] : -1}; },
+        [&](int64_t, int64_t p, int64_t s, int64_t, RowPair v) {
+            const int64_t r = v.r;
+            if (p > s && v.prev >= r) atomicOr(err, 64);
+            if (r < 0 || r >= kdim) atomicOr(err, 32);
+            brow[p] = r < 0 || r >= kdim ? 0 : (int32_t)r;
+        });
 }
 
 // Row-tile mask of every column of A: bit t set when A(tile t, k) is nonempty.
@@ -160,28 +197,80 @@ __global__ void k_amask(int64_t ncol, const uint32_t *tptr, int T, int mask_word
 // flop[i] = sum over B(:,i) entries k of nnz(A(:,k)) (estimateFLOP), and the
 // column's tile mask = OR of the masks of those A columns (exactly the row
 // tiles the output column touches).
-__global__ void k_flop_mask(int64_t nb, const int64_t *bcp, const int32_t *brow, const int64_t *acp,
-                            const uint64_t *amask, int mask_words, int64_t *flop, uint64_t *tmask)
+__global__ void __launch_bounds__(kPrepWarps * 32)
+    k_flop_mask(int64_t nb, const int64_t *bcp, const int32_t *brow, const int64_t *acp, const uint64_t *amask,
+                int mask_words, int64_t *flop, uint64_t *tmask)
 {
-    const int lane = threadIdx.x & 31;
-    const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-    for (int64_t i = warp; i < nb; i += nwarps) {
-        int64_t f = 0;
-        for (int64_t p = bcp[i] + lane; p < bcp[i + 1]; p += 32) {
-            const int k = brow[p];
-            f += acp[k + 1] - acp[k];
+    constexpr int W = 4;  // mask words of one pass
+    __shared__ int64_t ls[kPrepWarps], le[kPrepWarps];
+    __shared__ uint64_t part[kPrepWarps][W + 1];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // this warp's part of the sum (acc[W]) and of mask words w0.. over [s, e)
+    uint64_t acc[W + 1];
+    auto gather = [&](int64_t s, int64_t e, int64_t first, int64_t stride, int w0) {
+#pragma unroll
+        for (int u = 0; u <= W; ++u) acc[u] = 0;
+        for (int64_t p = s + first; p < e; p += kPrepUnroll * stride) {
+            int k[kPrepUnroll];
+#pragma unroll
+            for (int u = 0; u < kPrepUnroll; ++u) k[u] = p + u * stride < e ? brow[p + u * stride] : -1;
+#pragma unroll
+            for (int u = 0; u < kPrepUnroll; ++u) {
+                if (k[u] < 0) continue;
+                if (w0 == 0) acc[W] += (uint64_t)(acp[k[u] + 1] - acp[k[u]]);
+#pragma unroll
+                for (int x = 0; x < W; ++x)
+                    if (w0 + x < mask_words) acc[x] |= amask[(int64_t)k[u] * mask_words + w0 + x];
+            }
         }
 #pragma unroll
-        for (int o = 16; o; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
-        if (lane == 0) flop[i] = f;
-        for (int w = 0; w < mask_words; ++w) {
-            uint64_t m = 0;
-            for (int64_t p = bcp[i] + lane; p < bcp[i + 1]; p += 32) m |= amask[(int64_t)brow[p] * mask_words + w];
+        for (int o = 16; o; o >>= 1) {
 #pragma unroll
-            for (int o = 16; o; o >>= 1) m |= __shfl_xor_sync(0xffffffffu, m, o);
-            if (lane == 0) tmask[i * mask_words + w] = m;
+            for (int x = 0; x < W; ++x) acc[x] |= __shfl_xor_sync(0xffffffffu, acc[x], o);
+            acc[W] += __shfl_xor_sync(0xffffffffu, acc[W], o);
         }
+    };
+    for (int64_t i0 = int64_t(blockIdx.x) * kPrepWarps; i0 < nb; i0 += int64_t(gridDim.x) * kPrepWarps) {
+        const int64_t i = i0 + wid;
+        const int64_t s = i < nb ? bcp[i] : 0, e = i < nb ? bcp[i + 1] : 0;
+        const bool is_long = e - s > kLongCol;
+        if (lane == 0) {
+            ls[wid] = s;
+            le[wid] = is_long ? e : s;
+        }
+        if (i < nb && !is_long)
+            for (int w0 = 0; w0 == 0 || w0 < mask_words; w0 += W) {
+                gather(s, e, lane, 32, w0);
+                if (lane == 0) {
+                    if (w0 == 0) flop[i] = (int64_t)acc[W];
+#pragma unroll
+                    for (int x = 0; x < W; ++x)
+                        if (w0 + x < mask_words) tmask[i * mask_words + w0 + x] = acc[x];
+                }
+            }
+        __syncthreads();
+        for (int q = 0; q < kPrepWarps; ++q) {
+            if (ls[q] == le[q]) continue;
+            for (int w0 = 0; w0 == 0 || w0 < mask_words; w0 += W) {
+                gather(ls[q], le[q], threadIdx.x, kPrepWarps * 32, w0);
+                if (lane == 0)
+#pragma unroll
+                    for (int u = 0; u <= W; ++u) part[wid][u] = acc[u];
+                __syncthreads();
+                if (threadIdx.x <= W) {
+                    uint64_t m = 0;
+                    for (int y = 0; y < kPrepWarps; ++y)
+                        m = threadIdx.x < W ? m | part[y][threadIdx.x] : m + part[y][threadIdx.x];
+                    if (threadIdx.x == W) {
+                        if (w0 == 0) flop[i0 + q] = (int64_t)m;
+                    } else if (w0 + (int)threadIdx.x < mask_words) {
+                        tmask[(i0 + q) * mask_words + w0 + threadIdx.x] = m;
+                    }
+                }
+                __syncthreads();
+            }
+        }
+        __syncthreads();
     }
 }
 
