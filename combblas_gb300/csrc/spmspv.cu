@@ -98,6 +98,9 @@ enum {
     CTL_DIR = 10,     // 0 top-down, 1 bottom-up
     CTL_E = 11,       // top-down: total frontier edges of this level (scan result)
     CTL_POLICY = 12,  // 0 choose per level, 1 always top-down, 2 always bottom-up
+    CTL_TRIPS = 13,   // trips of the traversal graph's body (policies 0 and 1)
+    CTL_DONE = 14,    // blocks that have finished the level
+    CTL_SOURCE = 15,  // the only vertex that can have a level and no parent
     CTL_N
 };
 // frontier pointer table follows the control words
@@ -239,6 +242,12 @@ __global__ void k_mark_emit(uint32_t *mark, int64_t words, const int64_t *pos, u
 // The direction is chosen on the device per level (frontier edges against
 // unreached edges, as direction-optimizing BFS does), so one captured graph
 // serves every level.
+//
+// A traversal of 2^20 vertices is bound by its launches (2 to 3 us each inside
+// the graph, most levels' work is less): the last block of a level's final
+// kernel advances the level itself, a bottom-up level that follows a top-down
+// one runs in the same trip of the graph, and the bitmaps are written whole or
+// cleared where another pass runs anyway (267 -> 222 us).
 constexpr int kQueue = 4096;
 constexpr int kEdgeChunk = 1024;
 constexpr int kScanTile = 2048;
@@ -260,7 +269,7 @@ __device__ __forceinline__ void queue_flush(int32_t *q, int &s_qn, unsigned long
 
 // Direction of the level about to run (one thread: the end of the previous
 // level, or the traversal's initialisation for the first level).
-__device__ void bfs_direction(int64_t *ctl, int64_t n)
+__device__ void bfs_direction(volatile int64_t *ctl, int64_t n)
 {
     const int64_t nf = ctl[CTL_NF];
     if (nf == 0) return;
@@ -273,11 +282,76 @@ __device__ void bfs_direction(int64_t *ctl, int64_t n)
     ctl[CTL_E] = 0;
 }
 
-// Top-down prefix of frontier degrees, in three fixed-size launches so the
-// graph can be replayed for any frontier size: tile sums, tile scan (one
-// block), rescan.
-__global__ void k_bfs_deg_tiles(const uint32_t *cp32, const int64_t *ctl, int32_t *const *fronts, int64_t *tile)
+// Advance the level (one thread, after every block's part of it): the next
+// frontier becomes current and the next level's direction is chosen.  Inside a
+// traversal graph it also sets the while node's condition: another level while
+// the frontier is nonempty, at most `cap` levels (a level loop over n vertices
+// ends within n + 1 levels, so the cap never cuts a traversal short).  ctl is
+// volatile: other blocks' sums are not to come from this SM's cache.
+__device__ void bfs_advance(volatile int64_t *ctl, int64_t n, int64_t cap, cudaGraphConditionalHandle h, int set_cond)
 {
+    if (ctl[CTL_NF] != 0) {  // else finished: later replays change nothing
+        ctl[CTL_NF] = ctl[CTL_NNEXT];
+        ctl[CTL_NNEXT] = 0;
+        ctl[CTL_WORK] = 0;
+        ctl[CTL_ITER] = ctl[CTL_ITER] + 1;
+        ctl[CTL_CUR] = ctl[CTL_CUR] ^ 1;
+        ctl[CTL_UE] = ctl[CTL_UE] - ctl[CTL_FE_NEXT];
+        ctl[CTL_FE] = ctl[CTL_FE_NEXT];
+        ctl[CTL_FE_NEXT] = 0;
+        bfs_direction(ctl, n);
+    }
+    if (set_cond) cudaGraphSetConditional(h, (ctl[CTL_NF] != 0 && ctl[CTL_ITER] < cap) ? 1u : 0u);
+}
+
+// A block's share of the level's sums, one atomic of each per block: they all go
+// to one address, where 2*10^4 of them (one per warp) took longer than the rest
+// of a bottom-up level.
+__device__ void bfs_block_sums(int64_t *ctl, int64_t deg, int64_t reached, int64_t fdeg)
+{
+    __shared__ unsigned long long s_sum[3];
+    if (threadIdx.x < 3) s_sum[threadIdx.x] = 0;
+    __syncthreads();
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        deg += __shfl_xor_sync(0xffffffffu, deg, o);
+        reached += __shfl_xor_sync(0xffffffffu, reached, o);
+        fdeg += __shfl_xor_sync(0xffffffffu, fdeg, o);
+    }
+    if ((threadIdx.x & 31) == 0 && (fdeg || reached)) {
+        atomicAdd(&s_sum[0], (unsigned long long)deg);
+        atomicAdd(&s_sum[1], (unsigned long long)reached);
+        atomicAdd(&s_sum[2], (unsigned long long)fdeg);
+    }
+    __syncthreads();
+    if (threadIdx.x < 3 && s_sum[threadIdx.x])
+        atomicAdd((unsigned long long *)&ctl[threadIdx.x == 0   ? CTL_EDGES
+                                             : threadIdx.x == 1 ? CTL_REACHED
+                                                                : CTL_FE_NEXT],
+                  s_sum[threadIdx.x]);
+}
+
+// The last of `blocks` blocks to end a level (all of a block's threads call it)
+// advances it.  Nothing waits.
+__device__ void bfs_block_done(int64_t *ctl, unsigned blocks, int64_t n, int64_t cap, cudaGraphConditionalHandle h)
+{
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd((unsigned long long *)&ctl[CTL_DONE], 1ull) != blocks - 1) return;
+    __threadfence();
+    ctl[CTL_DONE] = 0;
+    bfs_advance(ctl, n, cap, h, 1);
+}
+
+// Top-down prefix of frontier degrees, in fixed-size launches so the graph can
+// be replayed for any frontier size: tile sums, tile scan (one block), rescan.
+// With at most kFewTiles tiles every block of the rescan sums the tiles before
+// its own, and the scan in between is left out.
+constexpr int kFewTiles = 2048;
+__global__ void k_bfs_deg_tiles(const uint32_t *cp32, int64_t *ctl, int32_t *const *fronts, int64_t *tile)
+{
+    if (blockIdx.x == 0 && threadIdx.x == 0) ctl[CTL_TRIPS] += 1;
     if (ctl[CTL_DIR] != 0) return;
     const int64_t nf = ctl[CTL_NF];
     const int32_t *front = fronts[ctl[CTL_CUR]];
@@ -310,8 +384,8 @@ __global__ void k_bfs_deg_scan(int64_t *ctl, int64_t *tile)
     if (threadIdx.x == 0) ctl[CTL_E] = carry;
 }
 
-__global__ void k_bfs_deg_rescan(const uint32_t *cp32, const int64_t *ctl, int32_t *const *fronts,
-                                 const int64_t *tile, int64_t *off, int32_t *chunk_f0)
+__global__ void k_bfs_deg_rescan(const uint32_t *cp32, int64_t *ctl, int32_t *const *fronts, const int64_t *tile,
+                                 int scanned, int64_t *off, int32_t *chunk_f0)
 {
     if (ctl[CTL_DIR] != 0) return;
     const int64_t nf = ctl[CTL_NF];
@@ -330,8 +404,15 @@ __global__ void k_bfs_deg_rescan(const uint32_t *cp32, const int64_t *ctl, int32
         }
         sum += d[u];
     }
-    int64_t tot;
-    int64_t run = tile[blockIdx.x] + block_exclusive_sum64(sum, &tot);
+    int64_t tot, before = 0;
+    if (scanned) {
+        before = tile[blockIdx.x];
+    } else {
+        int64_t part = 0;
+        for (int64_t t = threadIdx.x; t < blockIdx.x; t += blockDim.x) part += tile[t];
+        block_exclusive_sum64(part, &before);
+    }
+    int64_t run = before + block_exclusive_sum64(sum, &tot);
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
         const int64_t f = b0 + int64_t(threadIdx.x) * PER + u;
@@ -344,14 +425,17 @@ __global__ void k_bfs_deg_rescan(const uint32_t *cp32, const int64_t *ctl, int32
         }
         run += d[u];
     }
-    if (b0 + kScanTile >= nf && threadIdx.x == kThreads - 1) off[nf] = run;
+    if (b0 + kScanTile >= nf && threadIdx.x == kThreads - 1) {
+        off[nf] = run;
+        ctl[CTL_E] = run;
+    }
 }
 
 // Top-down expansion over fixed edge chunks.
 __global__ void __launch_bounds__(kThreads) k_bfs_td(const uint32_t *cp32, const int32_t *row,
                                                      const uint32_t *visited, int32_t *cand, int64_t *ctl,
                                                      int32_t *const *fronts, const int64_t *off,
-                                                     const int32_t *chunk_f0)
+                                                     const int32_t *chunk_f0, uint32_t *const *fbits, int64_t words)
 {
     __shared__ int64_t s_off[kEdgeChunk + 2];
     __shared__ uint32_t s_st[kEdgeChunk + 2];
@@ -368,6 +452,9 @@ __global__ void __launch_bounds__(kThreads) k_bfs_td(const uint32_t *cp32, const
     int32_t *next = fronts[cur ^ 1];
     const int64_t nf = ctl[CTL_NF];
     const int64_t E = ctl[CTL_E];
+    // the bitmap that k_bfs_finalize fills (not read by top-down levels)
+    for (int64_t w = int64_t(blockIdx.x) * kThreads + tid; w < words; w += int64_t(gridDim.x) * kThreads)
+        fbits[cur ^ 1][w] = 0;
     if (tid == 0) s_qn = 0;
     __syncthreads();
     for (;;) {
@@ -447,16 +534,19 @@ __global__ void __launch_bounds__(kThreads) k_bfs_td(const uint32_t *cp32, const
 }
 
 // Top-down finalize: parents.Set(fringe) for the new frontier, plus visited,
-// levels, next-frontier bitmap and degree sums.
+// levels, next-frontier bitmap and degree sums.  With `advance` the last block
+// that has entries (the first block, if there are none) advances the level; a
+// block that starts after that finds no entries.
 __global__ void k_bfs_finalize(int32_t *cand, uint32_t *visited, int64_t *parents, int64_t *levels,
-                               const int64_t *cp, int64_t *ctl, int32_t *const *fronts, uint32_t *const *fbits)
+                               const uint32_t *cp32, int64_t *ctl, int32_t *const *fronts, uint32_t *const *fbits,
+                               int64_t n, int64_t cap, cudaGraphConditionalHandle h, int advance)
 {
     if (ctl[CTL_NF] == 0 || ctl[CTL_DIR] != 0) return;
     const int cur = (int)ctl[CTL_CUR];
     const int32_t *next = fronts[cur ^ 1];
     uint32_t *nbits = fbits[cur ^ 1];
     const int64_t nn = ctl[CTL_NNEXT];
-    const int64_t iter = ctl[CTL_ITER] + 1;
+    const int64_t iter = ctl[CTL_ITER] + 1, source = ctl[CTL_SOURCE];
     int64_t deg = 0, reached = 0, fdeg = 0;
     for (int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < nn; i += int64_t(gridDim.x) * blockDim.x) {
         const int32_t r = next[i];
@@ -464,32 +554,32 @@ __global__ void k_bfs_finalize(int32_t *cand, uint32_t *visited, int64_t *parent
         cand[r] = kNoCand;
         atomicOr(&visited[r >> 5], 1u << (r & 31));
         atomicOr(&nbits[r >> 5], 1u << (r & 31));
-        const int64_t d = cp[r + 1] - cp[r];
+        const int64_t d = cp32[r + 1] - cp32[r];
         fdeg += d;
-        if (levels[r] < 0) {
+        if (r != source) {
             levels[r] = iter;
             deg += d;
             ++reached;
         }
     }
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        deg += __shfl_xor_sync(0xffffffffu, deg, o);
-        reached += __shfl_xor_sync(0xffffffffu, reached, o);
-        fdeg += __shfl_xor_sync(0xffffffffu, fdeg, o);
-    }
-    if ((threadIdx.x & 31) == 0 && (fdeg || reached)) {
-        atomicAdd((unsigned long long *)&ctl[CTL_EDGES], (unsigned long long)deg);
-        atomicAdd((unsigned long long *)&ctl[CTL_REACHED], (unsigned long long)reached);
-        atomicAdd((unsigned long long *)&ctl[CTL_FE_NEXT], (unsigned long long)fdeg);
+    bfs_block_sums(ctl, deg, reached, fdeg);
+    if (advance) {
+        const int64_t want = (nn + blockDim.x - 1) / blockDim.x;
+        const unsigned blocks = (unsigned)min((int64_t)gridDim.x, max(want, (int64_t)1));
+        if (blockIdx.x < blocks) bfs_block_done(ctl, blocks, n, cap, h);
     }
 }
 
 // Bottom-up level: every vertex without a parent takes its smallest
-// neighbour that is in the current frontier.
-__global__ void __launch_bounds__(kThreads) k_bfs_bu(const int64_t *cp, const int32_t *row, uint32_t *visited,
+// neighbour that is in the current frontier.  A warp's 32 vertices are one word
+// of the bitmaps: the next frontier's word is written whole, and the new
+// vertices go into the visited word at once (only the vertex's own bit of it is
+// read; parents come from frontier bits).  With `advance` the last block
+// advances the level.
+__global__ void __launch_bounds__(kThreads) k_bfs_bu(const uint32_t *cp32, const int32_t *row, uint32_t *visited,
                                                      int64_t *parents, int64_t *levels, int64_t n, int64_t *ctl,
-                                                     int32_t *const *fronts, uint32_t *const *fbits)
+                                                     int32_t *const *fronts, uint32_t *const *fbits, int64_t cap,
+                                                     cudaGraphConditionalHandle h, int advance)
 {
     __shared__ int32_t q[kQueue];
     __shared__ int s_qn;
@@ -500,7 +590,7 @@ __global__ void __launch_bounds__(kThreads) k_bfs_bu(const int64_t *cp, const in
     int32_t *next = fronts[cur ^ 1];
     const uint32_t *fb = fbits[cur];
     uint32_t *nb = fbits[cur ^ 1];
-    const int64_t iter = ctl[CTL_ITER] + 1;
+    const int64_t iter = ctl[CTL_ITER] + 1, source = ctl[CTL_SOURCE];
     if (tid == 0) s_qn = 0;
     __syncthreads();
     int64_t deg = 0, reached = 0, fdeg = 0;
@@ -509,8 +599,8 @@ __global__ void __launch_bounds__(kThreads) k_bfs_bu(const int64_t *cp, const in
         const int64_t v = b + tid;
         bool fresh = false;
         if (v < n && !(visited[v >> 5] & (1u << (v & 31)))) {
-            const int64_t s = cp[v], e = cp[v + 1];
-            for (int64_t p = s; p < e; ++p) {
+            const uint32_t s = cp32[v], e = cp32[v + 1];
+            for (uint32_t p = s; p < e; ++p) {
                 const int32_t u = row[p];
                 if (fb[u >> 5] & (1u << (u & 31))) {
                     parents[v] = u;
@@ -519,9 +609,8 @@ __global__ void __launch_bounds__(kThreads) k_bfs_bu(const int64_t *cp, const in
                 }
             }
             if (fresh) {
-                atomicOr(&nb[v >> 5], 1u << (v & 31));
                 fdeg += e - s;
-                if (levels[v] < 0) {
+                if (v != source) {
                     levels[v] = iter;
                     deg += e - s;
                     ++reached;
@@ -529,7 +618,9 @@ __global__ void __launch_bounds__(kThreads) k_bfs_bu(const int64_t *cp, const in
             }
         }
         const unsigned m = __ballot_sync(0xffffffffu, fresh);
+        if (lane == 0 && v < n) nb[v >> 5] = m;
         if (m) {
+            if (lane == 0) visited[v >> 5] |= m;
             int slot = 0;
             if (lane == __ffs(m) - 1) slot = atomicAdd(&s_qn, __popc(m));
             slot = __shfl_sync(0xffffffffu, slot, __ffs(m) - 1);
@@ -539,84 +630,33 @@ __global__ void __launch_bounds__(kThreads) k_bfs_bu(const int64_t *cp, const in
         if (s_qn > kQueue - kThreads) queue_flush(q, s_qn, s_gbase, ctl, next);
     }
     queue_flush(q, s_qn, s_gbase, ctl, next);
-#pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        deg += __shfl_xor_sync(0xffffffffu, deg, o);
-        reached += __shfl_xor_sync(0xffffffffu, reached, o);
-        fdeg += __shfl_xor_sync(0xffffffffu, fdeg, o);
-    }
-    if (lane == 0 && (fdeg || reached)) {
-        atomicAdd((unsigned long long *)&ctl[CTL_EDGES], (unsigned long long)deg);
-        atomicAdd((unsigned long long *)&ctl[CTL_REACHED], (unsigned long long)reached);
-        atomicAdd((unsigned long long *)&ctl[CTL_FE_NEXT], (unsigned long long)fdeg);
-    }
+    bfs_block_sums(ctl, deg, reached, fdeg);
+    if (advance) bfs_block_done(ctl, gridDim.x, n, cap, h);
 }
 
-// End of a level whose direction may be bottom-up: the current frontier's
-// bitmap (read only by the bottom-up kernel) is cleared, so it can collect
-// the frontier after next; after a bottom-up level the new vertices are
-// marked visited -- after the level, so a vertex found in it is never taken
-// as a parent in it (only frontier bits are read there).
-__global__ void k_bfs_level_end(uint32_t *visited, const int64_t *ctl, int32_t *const *fronts,
-                                uint32_t *const *fbits, int64_t words)
-{
-    if (ctl[CTL_NF] == 0) return;
-    const int cur = (int)ctl[CTL_CUR];
-    const int64_t i0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, stride = int64_t(gridDim.x) * blockDim.x;
-    uint32_t *fb = fbits[cur];
-    for (int64_t w = i0; w < words; w += stride) fb[w] = 0;
-    if (ctl[CTL_DIR] != 1) return;
-    const int32_t *next = fronts[cur ^ 1];
-    const int64_t nn = ctl[CTL_NNEXT];
-    for (int64_t i = i0; i < nn; i += stride) atomicOr(&visited[next[i] >> 5], 1u << (next[i] & 31));
-}
-
-// Advance the level (the next frontier becomes current) and choose the next
-// level's direction.  Inside a traversal graph (set_cond) it also sets the
-// while node's condition: another level while the frontier is nonempty, at
-// most `cap` levels (a level loop over n vertices ends within n + 1 levels,
-// so the cap never cuts a traversal short).
-__global__ void k_bfs_advance(int64_t *ctl, int64_t n, int64_t cap, cudaGraphConditionalHandle h, int set_cond)
-{
-    if (ctl[CTL_NF] != 0) {  // else finished: later replays change nothing
-        ctl[CTL_NF] = ctl[CTL_NNEXT];
-        ctl[CTL_NNEXT] = 0;
-        ctl[CTL_WORK] = 0;
-        ctl[CTL_ITER] += 1;
-        ctl[CTL_CUR] ^= 1;
-        ctl[CTL_UE] -= ctl[CTL_FE_NEXT];
-        ctl[CTL_FE] = ctl[CTL_FE_NEXT];
-        ctl[CTL_FE_NEXT] = 0;
-        bfs_direction(ctl, n);
-    }
-    if (set_cond) cudaGraphSetConditional(h, (ctl[CTL_NF] != 0 && ctl[CTL_ITER] < cap) ? 1u : 0u);
-}
+// The level's end outside a traversal graph (the kernels above cannot advance
+// it there: a replay runs one level).
+__global__ void k_bfs_advance(int64_t *ctl, int64_t n) { bfs_advance(ctl, n, 0, 0, 0); }
 
 __global__ void k_bfs_init(int64_t n, int64_t nnz, int32_t *cand, uint32_t *visited, int64_t *parents,
                            int64_t *levels, int64_t source, const int64_t *cp, int64_t *ctl, int32_t *const *fronts,
-                           uint32_t *const *fbits)
+                           uint32_t *const *fbits, int policy)
 {
     const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     for (int64_t v = i; v < n; v += stride) {
         cand[v] = kNoCand;
         parents[v] = -1;
-        levels[v] = -1;
+        levels[v] = v == source ? 0 : -1;
     }
     for (int64_t w = i; w < (n + 31) / 32; w += stride) {
         visited[w] = 0;
-        fbits[0][w] = 0;
+        fbits[0][w] = w == source >> 5 ? 1u << (source & 31) : 0u;
         fbits[1][w] = 0;
     }
-}
-
-__global__ void k_bfs_init2(int64_t n, int64_t nnz, int64_t *levels, int64_t source, const int64_t *cp,
-                            int64_t *ctl, int32_t *const *fronts, uint32_t *const *fbits, int policy)
-{
+    if (i != 0) return;
     ctl[CTL_POLICY] = policy;
     fronts[0][0] = (int32_t)source;
-    fbits[0][source >> 5] |= 1u << (source & 31);
-    levels[source] = 0;
     const int64_t ds = cp[source + 1] - cp[source];
     ctl[CTL_NF] = 1;
     ctl[CTL_NNEXT] = 0;
@@ -630,6 +670,9 @@ __global__ void k_bfs_init2(int64_t n, int64_t nnz, int64_t *levels, int64_t sou
     ctl[CTL_UE] = nnz;  // the source is still unreached for the reference's loop
     ctl[CTL_DIR] = 0;
     ctl[CTL_E] = 0;
+    ctl[CTL_TRIPS] = 0;
+    ctl[CTL_DONE] = 0;
+    ctl[CTL_SOURCE] = source;
     bfs_direction(ctl, n);  // the first level's
 }
 
@@ -732,35 +775,39 @@ static int occ_grid(const Context *ctx, const void *kernel, int threads, size_t 
 // leaves out the bottom-up kernels (the frontier bitmaps are then never
 // read), always bottom-up leaves out the top-down ones; "auto" launches
 // both sets, the direction flag in the control block enabling one.  In a
-// traversal graph (set_cond) the advance kernel sets the while node's
-// condition h.
+// traversal graph (set_cond) the level's last kernel advances it and sets the
+// while node's condition h; a bottom-up level chosen after a top-down one then
+// follows in the same trip.
 static int launch_level(Graph *g, int64_t *parents, int64_t *levels, cudaStream_t s, cudaGraphConditionalHandle h,
                         int set_cond)
 {
     Context *ctx = g->ctx;
-    const int grid = ctx->num_sms * 4;
-    const int64_t words = (g->n + 31) / 32;
+    const int64_t words = (g->n + 31) / 32, cap = g->n + 2;
     const unsigned tiles = (unsigned)((g->n + kScanTile - 1) / kScanTile);
-    int launched = 1;
+    const int scanned = tiles > kFewTiles ? 1 : 0;
+    int launched = 0;
     if (g->policy != 2) {
         const int grid_td = occ_grid(ctx, (const void *)k_bfs_td, kThreads, 0);
         k_bfs_deg_tiles<<<tiles, kThreads, 0, s>>>(g->cp32, g->ctl, fronts_dev(g), g->tile);
-        k_bfs_deg_scan<<<1, kThreads, 0, s>>>(g->ctl, g->tile);
-        k_bfs_deg_rescan<<<tiles, kThreads, 0, s>>>(g->cp32, g->ctl, fronts_dev(g), g->tile, g->off, g->chunk_f0);
+        if (scanned) k_bfs_deg_scan<<<1, kThreads, 0, s>>>(g->ctl, g->tile);
+        k_bfs_deg_rescan<<<tiles, kThreads, 0, s>>>(g->cp32, g->ctl, fronts_dev(g), g->tile, scanned, g->off,
+                                                    g->chunk_f0);
         k_bfs_td<<<grid_td, kThreads, 0, s>>>(g->cp32, g->row, g->visited, g->cand, g->ctl, fronts_dev(g), g->off,
-                                              g->chunk_f0);
+                                              g->chunk_f0, fbits_dev(g), words);
         k_bfs_finalize<<<occ_grid(ctx, (const void *)k_bfs_finalize, 256, 0), 256, 0, s>>>(
-            g->cand, g->visited, parents, levels, g->cp, g->ctl, fronts_dev(g), fbits_dev(g));
-        launched += 5;
+            g->cand, g->visited, parents, levels, g->cp32, g->ctl, fronts_dev(g), fbits_dev(g), g->n, cap, h, set_cond);
+        launched += 4 + scanned;
     }
     if (g->policy != 1) {
         const int grid_bu = occ_grid(ctx, (const void *)k_bfs_bu, kThreads, 0);
-        k_bfs_bu<<<grid_bu, kThreads, 0, s>>>(g->cp, g->row, g->visited, parents, levels, g->n, g->ctl,
-                                              fronts_dev(g), fbits_dev(g));
-        k_bfs_level_end<<<grid, 256, 0, s>>>(g->visited, g->ctl, fronts_dev(g), fbits_dev(g), words);
-        launched += 2;
+        k_bfs_bu<<<grid_bu, kThreads, 0, s>>>(g->cp32, g->row, g->visited, parents, levels, g->n, g->ctl,
+                                              fronts_dev(g), fbits_dev(g), cap, h, set_cond);
+        launched += 1;
     }
-    k_bfs_advance<<<1, 1, 0, s>>>(g->ctl, g->n, g->n + 2, h, set_cond);
+    if (!set_cond) {
+        k_bfs_advance<<<1, 1, 0, s>>>(g->ctl, g->n);
+        launched += 1;
+    }
     note_launches(launched);
     GBC_CUDA_TRY(cudaGetLastError());
     return GBC_OK;
@@ -816,17 +863,16 @@ static int bfs_device(Graph *g, int64_t source, int64_t *parents, int64_t *level
     GBC_TRY(graph_alloc_bfs(g));
     cudaEventRecord(ctx->ev[5], s);
     k_bfs_init<<<ctx->num_sms * 4, 256, 0, s>>>(g->n, g->nnz, g->cand, g->visited, parents, levels, source, g->cp,
-                                                g->ctl, fronts_dev(g), fbits_dev(g));
-    k_bfs_init2<<<1, 1, 0, s>>>(g->n, g->nnz, levels, source, g->cp, g->ctl, fronts_dev(g), fbits_dev(g),
-                                g->policy);
-    note_launches(2);
+                                                g->ctl, fronts_dev(g), fbits_dev(g), g->policy);
+    note_launch();
     GBC_CUDA_TRY(cudaGetLastError());
     if (use_graph) GBC_TRY(level_graph(g, parents, levels));
     if (use_graph && g->loop_exec) {
         GBC_CUDA_TRY(cudaGraphLaunch(g->loop_exec, s));
         GBC_CUDA_TRY(cudaMemcpyAsync(g->h_ctl, g->ctl, kCtlWords * sizeof(int64_t), cudaMemcpyDeviceToHost, s));
         GBC_CUDA_TRY(cudaStreamSynchronize(s));
-        note_launches(g->loop_kernels * std::max<int64_t>(g->h_ctl[CTL_ITER], 1));
+        note_launches(g->loop_kernels *
+                      std::max<int64_t>(g->h_ctl[g->policy == 2 ? CTL_ITER : CTL_TRIPS], 1));
     }
     // Otherwise levels are replayed in batches; a finished BFS leaves nf == 0
     // and the remaining replays of the batch are empty launches.
