@@ -1153,6 +1153,12 @@ int prepare_operands(Workspace &ws, const DevMatrix &A, const DevMatrix &B, Spge
 // Everything the passes need, built once: one descriptor per product of a
 // batch (a single product is a batch of one).
 constexpr int64_t kKtlBound = 8192;
+// Where k_numeric_x runs, a warp kernel's list above s1 products with at most
+// this many columns per resident block goes to the block kernels: a warp alone
+// takes 70 to 90 us over 1000 products, however few such columns there are, and
+// a block about 8.  A host square of 700 columns 415 -> 314 us, a scale-14 square
+// (2.4*10^3 such columns) 1190 -> 1157 us; from 16 per block on no gain.
+constexpr int64_t kFewColumns = 8;
 
 struct Plan {
     std::vector<SpgemmArgs> h;        // host copies of the descriptors
@@ -1419,6 +1425,11 @@ static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j
     for (int c = 0; c < kWarpClasses; ++c) {
         L.l[c] = P.lbuf + c * stride;
         L.n[c] = (int64_t)h[c];
+        if (c > 0 && P.want_x && !P.s2_set && L.n[c] > 0 && L.n[c] <= kFewColumns * P.x_blocks) {
+            GBC_CUDA_TRY(cudaMemcpyAsync(lbig + nbig, L.l[c], L.n[c] * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
+            nbig += L.n[c];
+            L.n[c] = 0;
+        }
     }
     L.l[kBigList] = lbig;
     L.n[kBigList] = nbig;
