@@ -267,19 +267,15 @@ __device__ __forceinline__ void queue_flush(int32_t *q, int &s_qn, unsigned long
     __syncthreads();
 }
 
-// Direction of the level about to run (one thread: the end of the previous
-// level, or the traversal's initialisation for the first level).
-__device__ void bfs_direction(volatile int64_t *ctl, int64_t n)
+// Direction of a level (0 top-down, 1 bottom-up) whose frontier has nf vertices
+// and fe edges, ue edges being unreached, after a level of direction dir.
+__device__ __forceinline__ int64_t bfs_direction(int64_t dir, int64_t policy, int64_t nf, int64_t fe, int64_t ue,
+                                                 int64_t n)
 {
-    const int64_t nf = ctl[CTL_NF];
-    if (nf == 0) return;
-    int64_t dir = ctl[CTL_DIR];
-    if (dir == 0 && ctl[CTL_FE] * 14 > ctl[CTL_UE]) dir = 1;
-    else if (dir == 1 && nf * 24 < n) dir = 0;
-    if (ctl[CTL_POLICY] == 1) dir = 0;
-    if (ctl[CTL_POLICY] == 2) dir = 1;
-    ctl[CTL_DIR] = dir;
-    ctl[CTL_E] = 0;
+    if (policy != 0) return policy - 1;
+    if (dir == 0 && fe * 14 > ue) return 1;
+    if (dir == 1 && nf * 24 < n) return 0;
+    return dir;
 }
 
 // Advance the level (one thread, after every block's part of it): the next
@@ -287,21 +283,28 @@ __device__ void bfs_direction(volatile int64_t *ctl, int64_t n)
 // traversal graph it also sets the while node's condition: another level while
 // the frontier is nonempty, at most `cap` levels (a level loop over n vertices
 // ends within n + 1 levels, so the cap never cuts a traversal short).  ctl is
-// volatile: other blocks' sums are not to come from this SM's cache.
+// volatile, other blocks' sums are not to come from this SM's cache; all loads
+// come before the first store, so that they are one round trip.
 __device__ void bfs_advance(volatile int64_t *ctl, int64_t n, int64_t cap, cudaGraphConditionalHandle h, int set_cond)
 {
-    if (ctl[CTL_NF] != 0) {  // else finished: later replays change nothing
-        ctl[CTL_NF] = ctl[CTL_NNEXT];
+    const int64_t was = ctl[CTL_NF], nn = ctl[CTL_NNEXT], iter = ctl[CTL_ITER], cur = ctl[CTL_CUR];
+    const int64_t ue = ctl[CTL_UE], fe = ctl[CTL_FE_NEXT], dir = ctl[CTL_DIR], policy = ctl[CTL_POLICY];
+    const bool live = was != 0;  // else finished: later replays change nothing
+    if (live) {
+        ctl[CTL_NF] = nn;
         ctl[CTL_NNEXT] = 0;
         ctl[CTL_WORK] = 0;
-        ctl[CTL_ITER] = ctl[CTL_ITER] + 1;
-        ctl[CTL_CUR] = ctl[CTL_CUR] ^ 1;
-        ctl[CTL_UE] = ctl[CTL_UE] - ctl[CTL_FE_NEXT];
-        ctl[CTL_FE] = ctl[CTL_FE_NEXT];
+        ctl[CTL_ITER] = iter + 1;
+        ctl[CTL_CUR] = cur ^ 1;
+        ctl[CTL_UE] = ue - fe;
+        ctl[CTL_FE] = fe;
         ctl[CTL_FE_NEXT] = 0;
-        bfs_direction(ctl, n);
+        if (nn != 0) {
+            ctl[CTL_DIR] = bfs_direction(dir, policy, nn, fe, ue - fe, n);
+            ctl[CTL_E] = 0;
+        }
     }
-    if (set_cond) cudaGraphSetConditional(h, (ctl[CTL_NF] != 0 && ctl[CTL_ITER] < cap) ? 1u : 0u);
+    if (set_cond) cudaGraphSetConditional(h, (live && nn != 0 && iter + 1 < cap) ? 1u : 0u);
 }
 
 // A block's share of the level's sums, one atomic of each per block: they all go
@@ -668,12 +671,11 @@ __global__ void k_bfs_init(int64_t n, int64_t nnz, int32_t *cand, uint32_t *visi
     ctl[CTL_FE] = ds;
     ctl[CTL_FE_NEXT] = 0;
     ctl[CTL_UE] = nnz;  // the source is still unreached for the reference's loop
-    ctl[CTL_DIR] = 0;
+    ctl[CTL_DIR] = bfs_direction(0, policy, 1, ds, nnz, n);  // the first level's
     ctl[CTL_E] = 0;
     ctl[CTL_TRIPS] = 0;
     ctl[CTL_DONE] = 0;
     ctl[CTL_SOURCE] = source;
-    bfs_direction(ctl, n);  // the first level's
 }
 
 // Condition of a traversal's while node: another level while the frontier
@@ -786,20 +788,25 @@ static int launch_level(Graph *g, int64_t *parents, int64_t *levels, cudaStream_
     const unsigned tiles = (unsigned)((g->n + kScanTile - 1) / kScanTile);
     const int scanned = tiles > kFewTiles ? 1 : 0;
     int launched = 0;
+    // resident blocks, and no more than have work at `per` items a block
+    auto grid = [&](auto kernel, int64_t items, int64_t per) {
+        return (int)std::min<int64_t>(occ_grid(ctx, (const void *)kernel, kThreads, 0),
+                                      std::max<int64_t>((items + per - 1) / per, 1));
+    };
     if (g->policy != 2) {
-        const int grid_td = occ_grid(ctx, (const void *)k_bfs_td, kThreads, 0);
+        const int grid_td = grid(k_bfs_td, g->nnz, kEdgeChunk);
         k_bfs_deg_tiles<<<tiles, kThreads, 0, s>>>(g->cp32, g->ctl, fronts_dev(g), g->tile);
         if (scanned) k_bfs_deg_scan<<<1, kThreads, 0, s>>>(g->ctl, g->tile);
         k_bfs_deg_rescan<<<tiles, kThreads, 0, s>>>(g->cp32, g->ctl, fronts_dev(g), g->tile, scanned, g->off,
                                                     g->chunk_f0);
         k_bfs_td<<<grid_td, kThreads, 0, s>>>(g->cp32, g->row, g->visited, g->cand, g->ctl, fronts_dev(g), g->off,
                                               g->chunk_f0, fbits_dev(g), words);
-        k_bfs_finalize<<<occ_grid(ctx, (const void *)k_bfs_finalize, 256, 0), 256, 0, s>>>(
+        k_bfs_finalize<<<grid(k_bfs_finalize, g->n, kThreads), kThreads, 0, s>>>(
             g->cand, g->visited, parents, levels, g->cp32, g->ctl, fronts_dev(g), fbits_dev(g), g->n, cap, h, set_cond);
         launched += 4 + scanned;
     }
     if (g->policy != 1) {
-        const int grid_bu = occ_grid(ctx, (const void *)k_bfs_bu, kThreads, 0);
+        const int grid_bu = grid(k_bfs_bu, g->n, kThreads);
         k_bfs_bu<<<grid_bu, kThreads, 0, s>>>(g->cp32, g->row, g->visited, parents, levels, g->n, g->ctl,
                                               fronts_dev(g), fbits_dev(g), cap, h, set_cond);
         launched += 1;
