@@ -25,8 +25,9 @@
 // row; the same scan then places every row's products.  A second push writes
 // them (column, product) to their row's place in any order, and each row folds
 // its own in ascending column order: in a thread up to kSxThread products, in a
-// warp up to 32, in a block up to kSxSort.  Longer rows, and all rows of a
-// vector that brings more than 1/kSxPullShare of the matrix, are pulled instead:
+// warp up to 32, in a block up to kSxSort.  Longer rows, all rows of a vector
+// that brings more than 1/kSxPullShare of the matrix, and all rows of a matrix of
+// fewer than kSxPushNnz entries are pulled instead:
 // a warp walks the row's row-major entries (ascending column), tests them
 // against a dense column -> vector position map and folds the hits in order.
 // (Pulling every touched row reads nearly the whole matrix for 2000 entries of
@@ -183,18 +184,18 @@ __device__ __forceinline__ void sx_products(const int64_t *cp, const int32_t *xi
 }
 
 // Push: per product one atomicMax of the column's key into spa[r] (PlusTimes:
-// a count) and the touched mark.
+// a count, where `count` asks for it) and the touched mark.
 template <int SX>
 __global__ void __launch_bounds__(kSxThreads) k_sx_expand(const int64_t *cp, const int32_t *row, const int32_t *xind,
                                                           const int64_t *xval, int64_t nx, int64_t n,
                                                           unsigned long long *spa, uint32_t *mark,
-                                                          unsigned long long *work)
+                                                          unsigned long long *work, bool count)
 {
     sx_products(cp, xind, nx, n, work, [&](int64_t f, int64_t p) {
         const int32_t r = row[p];
-        if (SX == SX_PLUSTIMES)
-            atomicAdd(&spa[r], 1ull);
-        else
+        if (SX == SX_PLUSTIMES) {
+            if (count) atomicAdd(&spa[r], 1ull);
+        } else
             atomicMax(&spa[r], sx_key<SX>(xval[f], xind[f], f));
         const uint32_t bit = 1u << (r & 31);
         if (!(mark[r >> 5] & bit)) atomicOr(&mark[r >> 5], bit);
@@ -291,6 +292,11 @@ __device__ __forceinline__ V sx_add(V a, V b)
 
 constexpr int kSxThread = 8;      // products of a row folded by one thread
 constexpr int kSxPullShare = 4;   // pull when the products times this exceed the matrix
+// Matrices of fewer entries are always pulled: their longest row is a short
+// chain, and the push has five launches more.  R-MAT, pulled / pushed: 1.1*10^5
+// entries, 100 of the vector 114 / 173 us; 1.8*10^6, 1000: 205 / 307; 3.9*10^6,
+// 2000: 238 / 274; 7.9*10^6, 100: 184 / 156, 2000: 261 / 281.
+constexpr int64_t kSxPushNnz = 1 << 22;
 
 // The row's products by one warp over its row-major entries, eight windows of
 // 32 entries in flight; hits are folded left in ascending column order.
@@ -557,19 +563,20 @@ static int sx_run(SpmspvPlan *p, Workspace &ws, const int32_t *dx, const void *d
 {
     Context *ctx = p->ctx;
     cudaStream_t s = ctx->stream;
+    const bool push = SX == SX_PLUSTIMES && p->nnz >= kSxPushNnz;
     GBC_CUDA_TRY(cudaMemsetAsync(p->err, 0, sizeof(int32_t), s));
     GBC_CUDA_TRY(cudaMemsetAsync(p->work, 0, sizeof(unsigned long long), s));
     if (nx > 0) {
         k_sx_xpos<<<(unsigned)((nx + 255) / 256), 256, 0, s>>>(nx, dx, p->n, p->xpos, p->err);
         const int grid = (int)std::min<int64_t>((int64_t)ctx->num_sms * 8, (nx + kSxChunk - 1) / kSxChunk);
         k_sx_expand<SX><<<grid, kSxThreads, 0, s>>>(p->cp, p->row, dx, static_cast<const int64_t *>(dv), nx, p->n,
-                                                    p->spa, p->mark, p->work);
+                                                    p->spa, p->mark, p->work, push);
         note_launches(2);
     }
     int64_t *cnt = nullptr;
     GBC_TRY(ws.alloc_n(&cnt, p->words + 1));
     if (p->words > 0) {
-        if (SX == SX_PLUSTIMES)
+        if (push)
             k_sx_counts_sum<<<(unsigned)((p->words + 255) / 256), 256, 0, s>>>(p->mark, p->words, p->spa, cnt);
         else
             k_sx_counts<<<(unsigned)((p->words + 255) / 256), 256, 0, s>>>(p->mark, p->words, cnt);
@@ -577,15 +584,15 @@ static int sx_run(SpmspvPlan *p, Workspace &ws, const int32_t *dx, const void *d
     }
     GBC_TRY(exclusive_scan_i64(ws, cnt, p->pos, p->words, s));
     GBC_TRY(read_i64(ctx, p->pos + p->words, ny));
-    const int64_t nprod = SX == SX_PLUSTIMES ? (int64_t)((uint64_t)*ny >> 32) : 0;
-    if (SX == SX_PLUSTIMES) *ny &= 0xffffffff;
+    const int64_t nprod = push ? (int64_t)((uint64_t)*ny >> 32) : 0;
+    if (push) *ny &= 0xffffffff;
     if (host_out) {
         GBC_TRY(ws.alloc_n(yi, *ny + 1));
         void *b = nullptr;
         GBC_TRY(ws.alloc(&b, (*ny + 1) * sizeof(V)));
         *yv = b;
     }
-    if (SX == SX_PLUSTIMES && *ny > 0 && nprod * kSxPullShare <= p->nnz) {
+    if (push && *ny > 0 && nprod * kSxPullShare <= p->nnz) {
         uint32_t *off = nullptr;
         int32_t *pcol = nullptr;
         V *pval = nullptr;
