@@ -1159,6 +1159,12 @@ constexpr int64_t kKtlBound = 8192;
 // a block about 8.  A host square of 700 columns 415 -> 314 us, a scale-14 square
 // (2.4*10^3 such columns) 1190 -> 1157 us; from 16 per block on no gain.
 constexpr int64_t kFewColumns = 8;
+// k_numeric_own has a column walked by four warps: with fewer columns per
+// multiprocessor than this (two rounds of its resident blocks) the longest one is
+// the launch's end, and the list goes to k_numeric.  fp32 square of a 2357-vertex
+// R-MAT: 203 us for the kernel against 132, the call 938 -> 826; an MCL loop,
+// whose last dense iteration has few such columns, 262 -> 265 ms.
+constexpr int64_t kFewOwn = 16;
 
 struct Plan {
     std::vector<SpgemmArgs> h;        // host copies of the descriptors
@@ -1170,6 +1176,7 @@ struct Plan {
     int tile_rows = 0;                   // accumulator tile height (0: default)
     unsigned long long *work = nullptr;  // kernel work counters
     int64_t *lbuf = nullptr;             // column lists (kLists x (total_cols + 1))
+    std::vector<int64_t> a_nnz;          // entries of every product's A
     bool s2_set = false;                 // the caller chose s2
     unsigned long long *lcnt = nullptr;  // list lengths
     bool want_x = false;                 // big columns by k_numeric_x
@@ -1312,6 +1319,7 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
     sup_rows = (sup_rows / a.R) * a.R;
     P.max_sym_smem = std::max(P.max_sym_smem, (size_t)sup_rows / 8);
     P.h.push_back(a);
+    P.a_nnz.push_back(A.nnz);
     return GBC_OK;
 }
 
@@ -1323,8 +1331,7 @@ static int plan_own(Plan &P)
     cudaStream_t s = ctx->stream;
     for (SpgemmArgs &a : P.h) {
         if (a.own_T == 0 || a.m == 0) continue;
-        int64_t nnz = 0;
-        GBC_TRY(read_i64(ctx, a.acp + a.kdim, &nnz));
+        const int64_t nnz = P.a_nnz[&a - P.h.data()];
         if (nnz == 0) continue;
         int64_t *w = nullptr;
         uint8_t *range = nullptr;
@@ -1396,7 +1403,6 @@ static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j
     constexpr int NL = kLists + 1;  // and the multiplications
     GBC_CUDA_TRY(cudaMemsetAsync(P.lcnt, 0, NL * sizeof(unsigned long long), s));
     const int64_t stride = P.total_cols + 1;
-    int64_t *lbig = P.lbuf + kWarpClasses * stride;
     for (int q = 0; q < (int)P.h.size(); ++q) {
         if (pid >= 0 && q != pid) continue;
         const SpgemmArgs &a = P.h[q];
@@ -1413,13 +1419,17 @@ static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j
     unsigned long long h[NL];
     GBC_CUDA_TRY(cudaMemcpyAsync(h, P.lcnt, sizeof(h), cudaMemcpyDeviceToHost, s));
     GBC_CUDA_TRY(cudaStreamSynchronize(s));
-    // the big list: bin 0 (heaviest) in place, the other bins appended
-    int64_t nbig = (int64_t)h[kWarpClasses];
-    for (int c = 1; c < kBigBins; ++c) {
+    // the big list: its first part (columns for k_numeric_own that are too few
+    // for it, or bin 0, the heaviest) in place, the other bins appended
+    const bool few_own = h[kOwnSlot] > 0 && !P.s2_set && (int64_t)h[kOwnSlot] <= kFewOwn * P.ws->ctx->num_sms;
+    const int64_t *bins = P.lbuf + kWarpClasses * stride;
+    int64_t *lbig = P.lbuf + (few_own ? kOwnSlot : kWarpClasses) * stride;
+    int64_t nbig = (int64_t)h[few_own ? kOwnSlot : kWarpClasses];
+    for (int c = few_own ? 0 : 1; c < kBigBins; ++c) {
         const int64_t nc = (int64_t)h[kWarpClasses + c];
         if (nc > 0)
             GBC_CUDA_TRY(
-                cudaMemcpyAsync(lbig + nbig, lbig + c * stride, nc * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
+                cudaMemcpyAsync(lbig + nbig, bins + c * stride, nc * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
         nbig += nc;
     }
     for (int c = 0; c < kWarpClasses; ++c) {
@@ -1434,7 +1444,7 @@ static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j
     L.l[kBigList] = lbig;
     L.n[kBigList] = nbig;
     L.l[kOwnList] = P.lbuf + kOwnSlot * stride;
-    L.n[kOwnList] = (int64_t)h[kOwnSlot];
+    L.n[kOwnList] = few_own ? 0 : (int64_t)h[kOwnSlot];
     L.flops = (int64_t)h[kLists];
     if (L.n[kOwnList] > 0 && !P.own_built) GBC_TRY(plan_own(P));
     return GBC_OK;
