@@ -1162,8 +1162,8 @@ constexpr int64_t kFewColumns = 8;
 // k_numeric_own has a column walked by four warps: with fewer columns per
 // multiprocessor than this (two rounds of its resident blocks) the longest one is
 // the launch's end, and the list goes to k_numeric.  fp32 square of a 2357-vertex
-// R-MAT: 203 us for the kernel against 132, the call 938 -> 826; an MCL loop,
-// whose last dense iteration has few such columns, 262 -> 265 ms.
+// R-MAT: 203 us for the kernel against 132, the call 938 -> 826; an MCL
+// loop 262 -> 265 ms.
 constexpr int64_t kFewOwn = 16;
 
 struct Plan {

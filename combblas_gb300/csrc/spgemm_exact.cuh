@@ -293,10 +293,7 @@ constexpr int kXSegs = 1024;                  // segments of one chunk table
 constexpr int kXWins = 512;                   // 32-product windows of one round
 constexpr int kXSpanTiles = 16;               // row tiles of one ranked visit (a 64 K-row bitmap)
 constexpr int kXSort = 4096;                  // products of one sorted range visit (at most)
-#ifndef GBC_XLIGHT
-#define GBC_XLIGHT 512
-#endif
-constexpr int kXLight = GBC_XLIGHT;           // runs of at most this many products go to sorted ranges
+constexpr int kXLight = 512;                  // runs of at most this many products go to sorted ranges
 constexpr int kXDirect = 8192;                // a tile of more products is a visit of its own
 constexpr int64_t kXScap = int64_t(1) << 20;  // bucketed segments of one column, at most (per-block scratch)
 

@@ -10,9 +10,7 @@ namespace gbc {
 
 constexpr int kThreads = 256;            // threads per SpGEMM block
 constexpr int kWarps = kThreads / 32;    // owner warps per block
-constexpr int kBuckets = kWarps;         // one staging bucket per owner warp
 constexpr int kStage = 2048;             // products staged per sub-batch
-constexpr int kRounds = kStage / kThreads;
 constexpr int kTileRows = 8192;          // default rows of the dense accumulator tile (two blocks per SM at fp64)
 constexpr int kSymRows = 1 << 18;        // rows of one symbolic bitmap pass (32 KB: five blocks per SM)
 constexpr int kMaxMaskWords = 64;        // tile-mask words per column (64 tiles each)
@@ -104,7 +102,6 @@ struct ChunkSmemN {
     uint32_t base[NT];
     int32_t off[NT + 1];
 };
-typedef ChunkSmemN<kThreads> ChunkSmem;
 
 // Compact one chunk whose segments are already known per thread (start s,
 // length len, B value bv; len 0 for threads past the chunk), keeping only

@@ -30,8 +30,8 @@
 // fewer than kSxPushNnz entries are pulled instead:
 // a warp walks the row's row-major entries (ascending column), tests them
 // against a dense column -> vector position map and folds the hits in order.
-// (Pulling every touched row reads nearly the whole matrix for 2000 entries of
-// 2^18; it took 0.59 of the call's 0.69 ms.)
+// (One window of 32 entries at a time, the longest pulled row took 0.59 of 0.69 ms
+// over 2000 entries of 2^18; with eight in flight the call takes 0.26 ms pulled.)
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
