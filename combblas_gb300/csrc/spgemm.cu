@@ -32,6 +32,7 @@
 
 #include "gbc_internal.cuh"
 #include "semiring.cuh"
+#include "size_rules.cuh"
 #include "spgemm_kernels.cuh"
 #include "spgemm_small.cuh"
 #include "spgemm_exact.cuh"
@@ -1150,8 +1151,8 @@ int prepare_operands(Workspace &ws, const DevMatrix &A, const DevMatrix &B, Spge
     return GBC_OK;
 }
 
-// Everything the passes need, built once: one descriptor per product of a
-// batch (a single product is a batch of one).
+// Entries of A up to which the exact kernel's tile lists and scratch are sized
+// by bounds.
 constexpr int64_t kKtlBound = 8192;
 // Where k_numeric_x runs, a warp kernel's list above s1 products with at most
 // this many columns per resident block goes to the block kernels: a warp alone
@@ -1166,6 +1167,8 @@ constexpr int64_t kFewColumns = 8;
 // loop 262 -> 265 ms.
 constexpr int64_t kFewOwn = 16;
 
+// Everything the passes need, built once: one descriptor per product of a
+// batch (a single product is a batch of one).
 struct Plan {
     std::vector<SpgemmArgs> h;        // host copies of the descriptors
     SpgemmArgs *d = nullptr;          // device array
@@ -1291,12 +1294,12 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
             k_ktl_count<<<(unsigned)((A.ncol + 255) / 256), 256, 0, s>>>(A.ncol, amask, a.mask_words, kptr);
             note_launch();
             GBC_TRY(exclusive_scan_i64(ws, kptr, kptr, A.ncol, s));
-            // A column touches at most as many tiles as it has entries: that
-            // bound does where the lists and the scratch stay small (4 KB
-            // per entry over all blocks), and saves the read-back.
-            int64_t nent = A.nnz;
-            if (nent > kKtlBound) GBC_TRY(read_i64(ctx, kptr + A.ncol, &nent));
-            P.xscap = std::max(P.xscap, std::min(nent, kXScap));
+            // The bounds do where the scratch stays small (4 KB per entry of
+            // A over all blocks; the lists are smaller than tptr), and save
+            // the read-back.  Segments are touched tiles, without the markers.
+            int64_t nent = ktl_room(A.nnz, A.ncol);
+            if (A.nnz > kKtlBound) GBC_TRY(read_i64(ctx, kptr + A.ncol, &nent));
+            P.xscap = std::max(P.xscap, std::min(std::min(nent, A.nnz), kXScap));
             uint32_t *kst = nullptr;
             uint16_t *ktt = nullptr;
             GBC_TRY(ws.alloc_n(&kst, (size_t)nent + 1));
