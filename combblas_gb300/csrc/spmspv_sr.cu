@@ -184,13 +184,17 @@ __device__ __forceinline__ void sx_products(const int64_t *cp, const int32_t *xi
 }
 
 // Push: per product one atomicMax of the column's key into spa[r] (PlusTimes:
-// a count, where `count` asks for it) and the touched mark.
+// a count, where `count` asks for it) and the touched mark.  A vector that
+// k_sx_xpos found at fault brings nothing: distinct columns keep a row's count,
+// and the total, within the matrix's entries (below 2^31), which the 32-bit
+// places of the products rely on; a column named 2^16 times would pass them.
 template <int SX>
 __global__ void __launch_bounds__(kSxThreads) k_sx_expand(const int64_t *cp, const int32_t *row, const int32_t *xind,
                                                           const int64_t *xval, int64_t nx, int64_t n,
                                                           unsigned long long *spa, uint32_t *mark,
-                                                          unsigned long long *work, bool count)
+                                                          unsigned long long *work, const int32_t *err, bool count)
 {
+    if (*err != 0) return;
     sx_products(cp, xind, nx, n, work, [&](int64_t f, int64_t p) {
         const int32_t r = row[p];
         if (SX == SX_PLUSTIMES) {
@@ -570,7 +574,7 @@ static int sx_run(SpmspvPlan *p, Workspace &ws, const int32_t *dx, const void *d
         k_sx_xpos<<<(unsigned)((nx + 255) / 256), 256, 0, s>>>(nx, dx, p->n, p->xpos, p->err);
         const int grid = (int)std::min<int64_t>((int64_t)ctx->num_sms * 8, (nx + kSxChunk - 1) / kSxChunk);
         k_sx_expand<SX><<<grid, kSxThreads, 0, s>>>(p->cp, p->row, dx, static_cast<const int64_t *>(dv), nx, p->n,
-                                                    p->spa, p->mark, p->work, push);
+                                                    p->spa, p->mark, p->work, p->err, push);
         note_launches(2);
     }
     int64_t *cnt = nullptr;
