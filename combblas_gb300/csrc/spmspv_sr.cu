@@ -23,9 +23,10 @@
 // marking a touched-row bitmap.  Rows come out ascending from a popcount
 // scan of the bitmap.  PlusTimes pushes the marks and counts the products per
 // row; the same scan then places every row's products.  A second push writes
-// them (column, product) to their row's place in any order, and each row folds
-// its own in ascending column order: in a thread up to kSxThread products, in a
-// warp up to 32, in a block up to kSxSort.  Longer rows, all rows of a vector
+// them (entry, product) to their row's place in any order, and each row folds
+// its own in the order of the entries, which is ascending column order (and the
+// stored order where a column holds a row twice): in a thread up to kSxThread
+// products, in a warp up to 32, in a block up to kSxSort.  Longer rows, all rows of a vector
 // that brings more than 1/kSxPullShare of the matrix, and all rows of a matrix of
 // fewer than kSxPushNnz entries are pulled instead:
 // a warp walks the row's row-major entries (ascending column), tests them
@@ -357,21 +358,21 @@ __global__ void __launch_bounds__(256) k_sx_pull(int64_t ny, const int32_t *yind
 template <typename V>
 __global__ void __launch_bounds__(kSxThreads) k_sx_scatter(const int64_t *cp, const int32_t *row, const V *aval,
                                                            const int32_t *xind, const V *xval, int64_t nx, int64_t n,
-                                                           unsigned long long *spa, int32_t *pcol, V *pval,
+                                                           unsigned long long *spa, int32_t *pent, V *pval,
                                                            unsigned long long *work)
 {
     sx_products(cp, xind, nx, n, work, [&](int64_t f, int64_t p) {
         const unsigned long long at = atomicAdd(&spa[row[p]], 1ull);
-        pcol[at] = xind[f];
+        pent[at] = (int32_t)p;
         pval[at] = sx_mul<V>(aval[p], xval[f]);
     });
 }
 
-// Every touched row folds its products in ascending column order; the row's
+// Every touched row folds its products in the order of their entries; the row's
 // cursor goes back to zero.
 template <typename V>
 __global__ void __launch_bounds__(256) k_sx_fold(int64_t ny, const int32_t *yind, const uint32_t *off,
-                                                 const int32_t *pcol, const V *pval, unsigned long long *spa,
+                                                 const int32_t *pent, const V *pval, unsigned long long *spa,
                                                  V *yval, int32_t *longs, unsigned long long *nlong)
 {
     const int lane = threadIdx.x & 31;
@@ -384,12 +385,12 @@ __global__ void __launch_bounds__(256) k_sx_fold(int64_t ny, const int32_t *yind
             spa[yind[i]] = 0;
             if (n <= kSxThread) {
                 V acc = V(0);
-                int32_t done = -1;  // the columns up to this one are folded
+                int32_t done = -1;  // the entries up to this one are folded
                 for (uint32_t k = 0; k < n; ++k) {
                     int32_t next = INT32_MAX;
                     V v = V(0);
                     for (uint32_t q = 0; q < n; ++q) {
-                        const int32_t c = pcol[o + q];
+                        const int32_t c = pent[o + q];
                         if (c > done && c < next) {
                             next = c;
                             v = pval[o + q];
@@ -412,7 +413,7 @@ __global__ void __launch_bounds__(256) k_sx_fold(int64_t ny, const int32_t *yind
                 continue;
             }
             V acc = V(0);
-            unsigned c = lane < (int)rn ? (unsigned)pcol[ro + lane] : 0xffffffffu;
+            unsigned c = lane < (int)rn ? (unsigned)pent[ro + lane] : 0xffffffffu;
             const V v = lane < (int)rn ? pval[ro + lane] : V(0);
             for (uint32_t k = 0; k < rn; ++k) {
                 const unsigned next = __reduce_min_sync(0xffffffffu, c);
@@ -427,13 +428,13 @@ __global__ void __launch_bounds__(256) k_sx_fold(int64_t ny, const int32_t *yind
 }
 
 // Rows of more than 32 products, a block each: the products are sorted by
-// column in shared memory (bitonic) and folded by one thread, the chain that
+// entry in shared memory (bitonic) and folded by one thread, the chain that
 // the order asks for; rows of more than kSxSort are pulled.
 constexpr int kSxSort = 2048;
 
 template <typename V>
 __global__ void __launch_bounds__(256) k_sx_fold_long(const int32_t *longs, const unsigned long long *nlong,
-                                                      const int32_t *yind, const uint32_t *off, const int32_t *pcol,
+                                                      const int32_t *yind, const uint32_t *off, const int32_t *pent,
                                                       const V *pval, const int64_t *rowptr, const int32_t *col,
                                                       const V *aval, const int32_t *xpos, const V *xval, V *yval)
 {
@@ -456,7 +457,7 @@ __global__ void __launch_bounds__(256) k_sx_fold_long(const int32_t *longs, cons
         int N = 64;
         while (N < n) N <<= 1;
         for (int k = tid; k < N; k += 256)
-            key[k] = k < n ? ((uint64_t)(uint32_t)pcol[o + k] << 32) | (uint32_t)k : ~0ull;
+            key[k] = k < n ? ((uint64_t)(uint32_t)pent[o + k] << 32) | (uint32_t)k : ~0ull;
         __syncthreads();
         for (int k2 = 2; k2 <= N; k2 <<= 1) {
             for (int j = k2 >> 1; j > 0; j >>= 1) {
@@ -598,10 +599,10 @@ static int sx_run(SpmspvPlan *p, Workspace &ws, const int32_t *dx, const void *d
     }
     if (push && *ny > 0 && nprod * kSxPullShare <= p->nnz) {
         uint32_t *off = nullptr;
-        int32_t *pcol = nullptr;
+        int32_t *pent = nullptr;
         V *pval = nullptr;
         GBC_TRY(ws.alloc_n(&off, *ny + 1));
-        GBC_TRY(ws.alloc_n(&pcol, nprod));
+        GBC_TRY(ws.alloc_n(&pent, nprod));
         GBC_TRY(ws.alloc_n(&pval, nprod));
         int32_t *longs = nullptr;  // rows of more than 32 products
         unsigned long long *nlong = nullptr;
@@ -612,11 +613,11 @@ static int sx_run(SpmspvPlan *p, Workspace &ws, const int32_t *dx, const void *d
         GBC_CUDA_TRY(cudaMemsetAsync(p->work, 0, sizeof(unsigned long long), s));
         const int grid = (int)std::min<int64_t>((int64_t)ctx->num_sms * 8, (nx + kSxChunk - 1) / kSxChunk);
         k_sx_scatter<V><<<grid, kSxThreads, 0, s>>>(p->cp, p->row, static_cast<const V *>(p->cval), dx,
-                                                    static_cast<const V *>(dv), nx, p->n, p->spa, pcol, pval, p->work);
+                                                    static_cast<const V *>(dv), nx, p->n, p->spa, pent, pval, p->work);
         k_sx_fold<V><<<(int)std::min<int64_t>((*ny + 255) / 256, (int64_t)ctx->num_sms * 8), 256, 0, s>>>(
-            *ny, *yi, off, pcol, pval, p->spa, static_cast<V *>(*yv), longs, nlong);
+            *ny, *yi, off, pent, pval, p->spa, static_cast<V *>(*yv), longs, nlong);
         k_sx_fold_long<V><<<(int)std::min<int64_t>(nprod / 33 + 1, (int64_t)ctx->num_sms * 6), 256, 0, s>>>(
-            longs, nlong, *yi, off, pcol, pval, p->rm.rowptr, p->rm.col, static_cast<const V *>(p->rm.val), p->xpos,
+            longs, nlong, *yi, off, pent, pval, p->rm.rowptr, p->rm.col, static_cast<const V *>(p->rm.val), p->xpos,
             static_cast<const V *>(dv), static_cast<V *>(*yv));
         note_launches(4);
     } else {
