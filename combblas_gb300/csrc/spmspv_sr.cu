@@ -57,7 +57,7 @@ struct SpmspvPlan {
     void *cval = nullptr;    // [nnz] values, column-major (numeric value types only)
     SpmvPlan rm;             // row-major form (numeric value types only)
     bool have_rm = false;
-    // scratch kept between calls: every call leaves it as it found it
+    // scratch kept between calls: every call leaves it as it found it (SxRestore)
     unsigned long long *spa = nullptr;  // [m] per-row key, 0 when untouched
     uint32_t *mark = nullptr;           // [words] touched rows
     int64_t *pos = nullptr;             // [words + 1] output offsets
@@ -562,6 +562,39 @@ static int plan_build(SpmspvPlan *p, const gbc_matrix *Am)
     return GBC_OK;
 }
 
+// A call that ends early, by a failed allocation or launch, clears the plan's
+// scratch on its way out; `done` says that its kernels have.
+struct SxRestore {
+    SpmspvPlan *p;
+    cudaStream_t s;
+    bool done = false;
+    ~SxRestore()
+    {
+        if (done) return;
+        cudaMemsetAsync(p->spa, 0, (p->m + 1) * sizeof(unsigned long long), s);
+        cudaMemsetAsync(p->mark, 0, (p->words + 1) * sizeof(uint32_t), s);
+        cudaMemsetAsync(p->xpos, 0, (p->n + 1) * sizeof(int32_t), s);
+    }
+};
+
+// The pushed products' arrays.
+template <typename V>
+struct SxProducts {
+    uint32_t *off = nullptr;   // [ny + 1] where every touched row's products begin
+    int32_t *pent = nullptr;   // [nprod] their entries
+    V *pval = nullptr;         // [nprod]
+    int32_t *longs = nullptr;  // rows of more than 32 products
+    unsigned long long *nlong = nullptr;
+    int reserve(Workspace &ws, int64_t ny, int64_t nprod)
+    {
+        GBC_TRY(ws.alloc_n(&off, ny + 1));
+        GBC_TRY(ws.alloc_n(&pent, nprod));
+        GBC_TRY(ws.alloc_n(&pval, nprod));
+        GBC_TRY(ws.alloc_n(&longs, nprod / 33 + 1));
+        return ws.alloc_n(&nlong, 1);
+    }
+};
+
 template <int SX, typename V>
 static int sx_run(SpmspvPlan *p, Workspace &ws, const int32_t *dx, const void *dv, int64_t nx, int32_t **yi,
                   void **yv, int64_t *ny, bool host_out)
@@ -571,6 +604,7 @@ static int sx_run(SpmspvPlan *p, Workspace &ws, const int32_t *dx, const void *d
     const bool push = SX == SX_PLUSTIMES && p->nnz >= kSxPushNnz;
     GBC_CUDA_TRY(cudaMemsetAsync(p->err, 0, sizeof(int32_t), s));
     GBC_CUDA_TRY(cudaMemsetAsync(p->work, 0, sizeof(unsigned long long), s));
+    SxRestore restore{p, s};
     if (nx > 0) {
         k_sx_xpos<<<(unsigned)((nx + 255) / 256), 256, 0, s>>>(nx, dx, p->n, p->xpos, p->err);
         const int grid = (int)std::min<int64_t>((int64_t)ctx->num_sms * 8, (nx + kSxChunk - 1) / kSxChunk);
@@ -597,28 +631,19 @@ static int sx_run(SpmspvPlan *p, Workspace &ws, const int32_t *dx, const void *d
         GBC_TRY(ws.alloc(&b, (*ny + 1) * sizeof(V)));
         *yv = b;
     }
-    if (push && *ny > 0 && nprod * kSxPullShare <= p->nnz) {
-        uint32_t *off = nullptr;
-        int32_t *pent = nullptr;
-        V *pval = nullptr;
-        GBC_TRY(ws.alloc_n(&off, *ny + 1));
-        GBC_TRY(ws.alloc_n(&pent, nprod));
-        GBC_TRY(ws.alloc_n(&pval, nprod));
-        int32_t *longs = nullptr;  // rows of more than 32 products
-        unsigned long long *nlong = nullptr;
-        GBC_TRY(ws.alloc_n(&longs, nprod / 33 + 1));
-        GBC_TRY(ws.alloc_n(&nlong, 1));
-        GBC_CUDA_TRY(cudaMemsetAsync(nlong, 0, sizeof(unsigned long long), s));
-        k_sx_places<<<(unsigned)((p->words + 255) / 256), 256, 0, s>>>(p->mark, p->words, p->pos, p->spa, *yi, off);
+    SxProducts<V> q;  // (without room for them the rows are pulled)
+    if (push && *ny > 0 && nprod * kSxPullShare <= p->nnz && q.reserve(ws, *ny, nprod) == GBC_OK) {
+        GBC_CUDA_TRY(cudaMemsetAsync(q.nlong, 0, sizeof(unsigned long long), s));
+        k_sx_places<<<(unsigned)((p->words + 255) / 256), 256, 0, s>>>(p->mark, p->words, p->pos, p->spa, *yi, q.off);
         GBC_CUDA_TRY(cudaMemsetAsync(p->work, 0, sizeof(unsigned long long), s));
         const int grid = (int)std::min<int64_t>((int64_t)ctx->num_sms * 8, (nx + kSxChunk - 1) / kSxChunk);
         k_sx_scatter<V><<<grid, kSxThreads, 0, s>>>(p->cp, p->row, static_cast<const V *>(p->cval), dx,
-                                                    static_cast<const V *>(dv), nx, p->n, p->spa, pent, pval, p->work);
+                                                    static_cast<const V *>(dv), nx, p->n, p->spa, q.pent, q.pval, p->work);
         k_sx_fold<V><<<(int)std::min<int64_t>((*ny + 255) / 256, (int64_t)ctx->num_sms * 8), 256, 0, s>>>(
-            *ny, *yi, off, pent, pval, p->spa, static_cast<V *>(*yv), longs, nlong);
+            *ny, *yi, q.off, q.pent, q.pval, p->spa, static_cast<V *>(*yv), q.longs, q.nlong);
         k_sx_fold_long<V><<<(int)std::min<int64_t>(nprod / 33 + 1, (int64_t)ctx->num_sms * 6), 256, 0, s>>>(
-            longs, nlong, *yi, off, pent, pval, p->rm.rowptr, p->rm.col, static_cast<const V *>(p->rm.val), p->xpos,
-            static_cast<const V *>(dv), static_cast<V *>(*yv));
+            q.longs, q.nlong, *yi, q.off, q.pent, q.pval, p->rm.rowptr, p->rm.col, static_cast<const V *>(p->rm.val),
+            p->xpos, static_cast<const V *>(dv), static_cast<V *>(*yv));
         note_launches(4);
     } else {
         if (p->words > 0) {
@@ -639,6 +664,7 @@ static int sx_run(SpmspvPlan *p, Workspace &ws, const int32_t *dx, const void *d
         note_launch();
     }
     GBC_CUDA_TRY(cudaGetLastError());
+    restore.done = true;
     int32_t herr = 0;
     GBC_CUDA_TRY(cudaMemcpyAsync(&herr, p->err, sizeof(herr), cudaMemcpyDeviceToHost, s));
     GBC_CUDA_TRY(cudaStreamSynchronize(s));
