@@ -23,11 +23,15 @@
 //         two vertex lists, so long thin graphs pay for their frontiers only.
 #pragma once
 
+#include "size_rules.cuh"
+
 namespace gbc {
 
 constexpr int kMbWords = 8;      // 512 roots a pass
 constexpr int kMbChunk = 64;     // neighbours of one pull item
 constexpr int kMbPullShare = 4;  // pull when the active edges times this exceed all edges
+constexpr int kMbPushThreads = 128;  // a block of k_mb_push, and its step over a long vertex
+static_assert(kMbPushThreads <= kMbStep && kMbChunk <= kMbStep, "mb_positions_fit");
 
 enum {
     MB_NF = 0,       // active vertices
@@ -160,7 +164,7 @@ __global__ void k_mb_begin(MbView g)
 
 // Push: a warp per active vertex, the block together for the long ones.
 template <int NW>
-__global__ void __launch_bounds__(128) k_mb_push(MbView g)
+__global__ void __launch_bounds__(kMbPushThreads) k_mb_push(MbView g)
 {
     if (g.ctl[MB_MODE] != 0) return;
     __shared__ int32_t s_long[4];
@@ -204,7 +208,7 @@ __global__ void __launch_bounds__(128) k_mb_push(MbView g)
         if (u >= 0 && !is_long) edges(u, lane, 32);
         __syncthreads();
         for (int k = 0; k < 4; ++k)
-            if (s_long[k] >= 0) edges(s_long[k], threadIdx.x, 128);
+            if (s_long[k] >= 0) edges(s_long[k], threadIdx.x, kMbPushThreads);
         __syncthreads();
     }
 }
@@ -414,6 +418,7 @@ static int mb_prepare(Graph *g)
     MsBits &b = g->mb;
     Context *ctx = g->ctx;
     cudaStream_t s = ctx->stream;
+    if (b.form == 0 && !mb_positions_fit(g->nnz)) b.form = 2;
     if (b.form == 2 || b.list[0]) return GBC_OK;
     if (b.form == 0) {
         Workspace ws(ctx);
@@ -484,7 +489,7 @@ static int mb_pass(Graph *g, int slot, const int64_t *d_roots, int64_t nroots, i
     const MbView v = mb_view(g);
     if (!b.exec[slot]) {
         auto body = [&](cudaStream_t cs, cudaGraphConditionalHandle h) {
-            k_mb_push<NW><<<occ_grid(ctx, (const void *)k_mb_push<NW>, 128, 0), 128, 0, cs>>>(v);
+            k_mb_push<NW><<<occ_grid(ctx, (const void *)k_mb_push<NW>, kMbPushThreads, 0), kMbPushThreads, 0, cs>>>(v);
             k_mb_push_end<NW><<<occ_grid(ctx, (const void *)k_mb_push_end<NW>, 256, 0), 256, 0, cs>>>(v);
             k_mb_pull<NW><<<occ_grid(ctx, (const void *)k_mb_pull<NW>, 256, 0), 256, 0, cs>>>(v);
             k_mb_pull_end<NW><<<occ_grid(ctx, (const void *)k_mb_pull_end<NW>, 256, 0), 256, 0, cs>>>(v);

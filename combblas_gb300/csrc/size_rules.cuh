@@ -11,4 +11,10 @@ namespace gbc {
 // every column, empty ones included, has an end marker.
 constexpr int64_t ktl_room(int64_t nnz, int64_t ncol) { return nnz + ncol; }
 
+// Multi-source BFS with one bit per root holds positions among a graph's nnz
+// entries in 32 bits and walks them in steps of up to kMbStep, one step past the
+// last one included: nnz + kMbStep must not pass 2^32.
+constexpr int64_t kMbStep = 128;
+constexpr bool mb_positions_fit(int64_t nnz) { return nnz + kMbStep <= int64_t(1) << 32; }
+
 }  // namespace gbc

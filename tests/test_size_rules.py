@@ -53,3 +53,16 @@ def test_tile_lists_fit_their_arrays(rule, name):
         n = 2
         rows, cols = np.tile(np.arange(4000), n), np.repeat(np.arange(n), 4000)
     assert tile_list_entries(rows, cols, n) <= rule(f"ktl_room({len(rows)}, {n})")
+
+
+@pytest.mark.parametrize("step", [4, 32, 64, 128])
+def test_positions_of_an_accepted_graph_do_not_wrap(rule, step):
+    """A 32-bit position that walks the last entries in steps ends past them, for the most entries accepted."""
+    lo, hi = 0, (1 << 32) - 1  # most entries that a graph may have at all
+    assert not rule(f"mb_positions_fit({hi})")
+    while hi - lo > 1:
+        mid = (lo + hi) // 2
+        lo, hi = (mid, hi) if rule(f"mb_positions_fit({mid})") else (lo, mid)
+    nnz = lo
+    for first in range(nnz - step, nnz):
+        assert (first + step) & 0xFFFFFFFF >= nnz
