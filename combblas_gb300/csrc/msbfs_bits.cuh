@@ -498,7 +498,8 @@ static int mb_pass(Graph *g, int slot, const int64_t *d_roots, int64_t nroots, i
             GBC_CUDA_TRY(cudaGetLastError());
             return (int)GBC_OK;
         };
-        GBC_TRY(loop_graph(body, true, nullptr, nullptr, 0, &b.exec[slot], &b.kernels));
+        // (a CUDA driver without conditional nodes)
+        if (loop_graph(body, true, nullptr, nullptr, 0, &b.exec[slot], &b.kernels) != GBC_OK) return GBC_EUNSUPPORTED;
     }
     const size_t bytes = (size_t)g->n * NW * sizeof(uint64_t);
     GBC_CUDA_TRY(cudaMemsetAsync(b.seen, 0, bytes, s));
@@ -514,6 +515,7 @@ static int mb_pass(Graph *g, int slot, const int64_t *d_roots, int64_t nroots, i
 }
 
 // parents: device [nroots * n], root-major.  The graph is prepared (form 1).
+// GBC_EUNSUPPORTED: the traversal graph cannot be built.
 static int mb_msbfs(Graph *g, const int64_t *d_roots, int64_t nroots, int64_t *parents, gbc_msbfs_stats *st)
 {
     MsBits &b = g->mb;

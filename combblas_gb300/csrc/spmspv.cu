@@ -1519,13 +1519,16 @@ int gbc_msbfs(gbc_context *ctx, gbc_graph *g, const int64_t *roots, int64_t nroo
     const int64_t cells = nroots * g->n;
     int64_t *dp = parents;
     if (where == GBC_HOST) GBC_TRY(ws.alloc_n(&dp, cells));
-    // One bit per root needs a symmetric pattern with ascending columns (and
-    // the traversal graph); other patterns expand (root, vertex) pairs.
-    GBC_TRY(mb_prepare(g));
-    const int rc = g->mb.form == 1 ? mb_msbfs(g, d_roots, nroots, dp, st) : GBC_EUNSUPPORTED;
-    if (g->mb.form == 1 && rc != GBC_OK && rc != GBC_ECUDA) return rc;
+    // One bit per root needs a symmetric pattern with ascending columns and
+    // the traversal graph; else (root, vertex) pairs are expanded.  They are
+    // for this call where the bits' arrays do not fit: few roots take less as
+    // pairs.
+    int rc = mb_prepare(g);
+    if (rc == GBC_OK) rc = g->mb.form == 1 ? mb_msbfs(g, d_roots, nroots, dp, st) : GBC_EUNSUPPORTED;
+    if (rc == GBC_EUNSUPPORTED) g->mb.form = 2;
     if (rc != GBC_OK) {
-        if (g->mb.form == 1) g->mb.form = 2;  // the driver cannot build the while node
+        mb_free(g);
+        if (rc != GBC_EUNSUPPORTED && rc != GBC_ENOMEM) return rc;
         GBC_TRY(msbfs_device(g, d_roots, nroots, dp, st));
     }
     if (where == GBC_HOST) {

@@ -56,6 +56,13 @@ class SmallPool:
         finally:
             self._ok(self.cu.cuDeviceSetMemPool(self.dev, self.old))
 
+    def leaked(self):
+        """Bytes of the pool that are neither free nor taken here."""
+        self._ok(self.cu.cuCtxSynchronize())
+        used = C.c_uint64()
+        self._ok(self.cu.cuMemPoolGetAttribute(self.pool, 7, C.byref(used)))
+        return used.value - len(self.held) * self.chunk
+
     def close(self):
         self._ok(self.cu.cuCtxSynchronize())
         while self.held:
