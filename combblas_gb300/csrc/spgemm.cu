@@ -1074,7 +1074,7 @@ static int set_smem(K kernel, size_t bytes)
 }
 
 int prepare_operands(Workspace &ws, const DevMatrix &A, const DevMatrix &B, SpgemmArgs &a, int64_t **acp_out,
-                     int tile_rows)
+                     int tile_rows, int max_words)
 {
     Context *ctx = ws.ctx;
     cudaStream_t s = ctx->stream;
@@ -1092,7 +1092,7 @@ int prepare_operands(Workspace &ws, const DevMatrix &A, const DevMatrix &B, Spge
     a.T = (int)((A.nrow + a.R - 1) / a.R);
     if (a.T < 1) a.T = 1;
     a.mask_words = (a.T + 63) / 64;
-    if (a.mask_words > kMaxMaskWords) return fail(GBC_EOVERFLOW, "too many rows for the tile mask");
+    if (a.mask_words > max_words) return fail(GBC_EOVERFLOW, "too many rows for the tile mask");
     if (A.nnz >= (int64_t(1) << 32)) return fail(GBC_EOVERFLOW, "nnz(A) must be below 2^32");
     int32_t *err = nullptr;
     GBC_TRY(ws.alloc_n(&err, 4));
@@ -1177,6 +1177,7 @@ struct Plan {
     size_t max_sym_smem = 0;
     int64_t s1 = kSmall1, s2 = GBC_SMALL2;  // flop thresholds of the column classes
     int tile_rows = 0;                   // accumulator tile height (0: default)
+    int max_words = kMaxMaskWords;       // tile-mask words per column, at most
     unsigned long long *work = nullptr;  // kernel work counters
     int64_t *lbuf = nullptr;             // column lists (kLists x (total_cols + 1))
     std::vector<int64_t> a_nnz;          // entries of every product's A
@@ -1198,7 +1199,7 @@ struct Plan {
 // PlusTimes fp64 under GBC_FOLD_EXACT, and the semirings whose add does not
 // depend on the order, take their big columns to k_numeric_x.  Its row tiles
 // are kXRows high; the tile height is a tuning knob only, so a larger request
-// is lowered.  Columns of more than kSmallMid multiplications go there as well
+// is lowered (and takes as many rows as 8192-row tiles would).  Columns of more than kSmallMid multiplications go there as well
 // (R-MAT s14: 2.1x faster than the larger warp kernels).  The others fold in
 // order, in the columns dense enough for it by k_numeric_own; so do the
 // order-free ones on an A (m x k, the largest of a batch) whose tile pointers
@@ -1211,6 +1212,7 @@ static void plan_fold(Context *ctx, Plan &P, int64_t m, int64_t k)
     if (XAcc<SR>::kUse && (exact ? ctx->fold == GBC_FOLD_EXACT : fits)) {
         P.want_x = true;
         P.want_aexp = exact;
+        if (exact && P.tile_rows != 0 && P.tile_rows != kXRows) P.max_words = 2 * kMaxMaskWords;
         P.tile_rows = kXRows;
         if (!P.s2_set) P.s2 = std::min<int64_t>(P.s2, kSmallMid);
     } else if (!XAcc<SR>::kUse || exact) {
@@ -1246,7 +1248,7 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
     cudaStream_t s = ctx->stream;
     SpgemmArgs a{};
     int64_t *acp = nullptr;
-    GBC_TRY(prepare_operands(ws, A, B, a, &acp, P.tile_rows));
+    GBC_TRY(prepare_operands(ws, A, B, a, &acp, P.tile_rows, P.max_words));
     const int64_t nb = B.nzc;
     int64_t m1 = A.nrow > 1 ? A.nrow - 1 : 0;
     a.key_bits = 0;

@@ -287,7 +287,7 @@ inline size_t numeric_smem_bytes(int R, size_t vsize, int sub)
 }
 
 int prepare_operands(Workspace &ws, const DevMatrix &A, const DevMatrix &B, SpgemmArgs &a, int64_t **acp_out,
-                     int tile_rows = 0);
+                     int tile_rows = 0, int max_words = kMaxMaskWords);
 
 template <class SR>
 int spgemm_learned(Context *ctx, const DevMatrix &A, const DevMatrix &B, const gbc_spgemm_opts &opt, int vt,
