@@ -1199,16 +1199,23 @@ struct Plan {
 // PlusTimes fp64 under GBC_FOLD_EXACT, and the semirings whose add does not
 // depend on the order, take their big columns to k_numeric_x.  Its row tiles
 // are kXRows high; the tile height is a tuning knob only, so a larger request
-// is lowered (and takes as many rows as 8192-row tiles would).  Columns of more than kSmallMid multiplications go there as well
-// (R-MAT s14: 2.1x faster than the larger warp kernels).  The others fold in
-// order, in the columns dense enough for it by k_numeric_own; so do the
-// order-free ones on an A (m x k, the largest of a batch) whose tile pointers
-// kXRows apart would pass 8 GB, where the default tiles need half of that.
+// is lowered (and takes as many rows as 8192-row tiles would).  Columns of more
+// than kSmallMid multiplications go there as well (R-MAT s14: 2.1x faster than
+// the larger warp kernels).  The others fold in order, in the columns dense
+// enough for it by k_numeric_own.
+//
+// Where A (m x k, the largest of a batch) has more row tiles than the kernel
+// buckets (2^20 rows), it visits every touched tile with all of the column's B
+// entries: columns of 1600 products spread over 2^21 rows took 132 ms of min-plus
+// where k_numeric and the larger warp kernels take 3.6, over 2^22 rows 221 and
+// 3.9; a 2^21-vertex R-MAT 91 and 55.  The order-free semirings keep those
+// there, and where the tile pointers kXRows apart would pass 8 GB (the default
+// tiles need half of that).
 template <class SR>
 static void plan_fold(Context *ctx, Plan &P, int64_t m, int64_t k)
 {
     constexpr bool exact = std::is_same<SR, PlusTimes<double>>::value;
-    const bool fits = m < (int64_t)kXRows * 64 * kMaxMaskWords && k * (m / kXRows + 2) <= int64_t(1) << 31;
+    const bool fits = m <= (int64_t)kXRows * kXTMax && k * (m / kXRows + 2) <= int64_t(1) << 31;
     if (XAcc<SR>::kUse && (exact ? ctx->fold == GBC_FOLD_EXACT : fits)) {
         P.want_x = true;
         P.want_aexp = exact;

@@ -1,0 +1,34 @@
+"""Which kernels take a column where A has more row tiles than the exact block
+kernel buckets, told by its visits: the order-free semirings leave it there, the
+oracle's values either way."""
+import numpy as np
+import pytest
+
+from combblas_gb300 import local
+from test_exact_visits_gpu import columns
+from test_spgemm_gpu import SR_NAME
+
+pytestmark = pytest.mark.gpu
+
+BUCKETED = 1 << 20  # rows
+
+
+def product(oracle, m, sr, deg, nb):
+    """Visits of the default product of 40 columns of deg x nb products over m rows."""
+    rng = np.random.default_rng(m + deg)
+    A = columns(m, [np.unique(rng.integers(0, m, deg)) for _ in range(2000)])
+    B = columns(2000, [np.sort(rng.choice(2000, nb, replace=False)) for _ in range(40)])
+    name, dt = SR_NAME[sr]
+    for M in (A, B):
+        M.values = (rng.random(M.nnz) * 100 + 1).astype(dt)
+    R = local.spgemm(A, B, sr=name, dtype=dt)
+    got, exp = R.to_csc(), oracle.port_spgemm(A, B, sr)
+    for g, e in zip(got, exp):
+        assert np.array_equal(g, e)
+    return R.stats.tile_visits_dense + R.stats.tile_visits_range
+
+
+@pytest.mark.parametrize("sr", [2, 3, 4, 5, 6])
+def test_order_free_semirings(gpu_ctx, oracle_lib, sr):
+    assert product(oracle_lib, BUCKETED, sr, 60, 100) > 0
+    assert product(oracle_lib, BUCKETED + 1, sr, 60, 100) == 0
