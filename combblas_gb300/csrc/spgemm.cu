@@ -1199,8 +1199,8 @@ struct Plan {
 // PlusTimes fp64 under GBC_FOLD_EXACT, and the semirings whose add does not
 // depend on the order, take their big columns to k_numeric_x.  Its row tiles
 // are kXRows high; the tile height is a tuning knob only, so a larger request
-// is lowered (and takes as many rows as 8192-row tiles would).  Columns of more
-// than kSmallMid multiplications go there as well (R-MAT s14: 2.1x faster than
+// is lowered (and takes as many rows as 8192-row tiles would).  Columns above
+// x_small_limit() multiplications go there as well (R-MAT s14: 2.1x faster than
 // the larger warp kernels).  The others fold in order, in the columns dense
 // enough for it by k_numeric_own.
 //
@@ -1211,6 +1211,21 @@ struct Plan {
 // 3.9; a 2^21-vertex R-MAT 91 and 55.  The order-free semirings keep those
 // there, and where the tile pointers kXRows apart would pass 8 GB (the default
 // tiles need half of that).
+// Multiplications up to which a column keeps to the warp kernels where
+// k_numeric_x takes the big ones.  A block's time grows with the row tiles that a
+// column touches, a warp's with its products and their bytes.  20000 columns of
+// uniform rows, warps / blocks, ms: 1600 min-plus products over 2^14 rows 2.3 /
+// 1.8, 2^16 2.3 / 2.3, 2^18 2.5 / 3.1, 2^20 2.8 / 4.9; 2560 products 8.9 / 3.5
+// (2^18), 9.2 / 5.7 (2^20), or-and 4.7 / 3.2 and 4.9 / 5.4; R-MAT columns of 2^18
+// rows 2.9 / 2.8.  Above kXTMax tiles (exact sums only) 1600 products over 2^21
+// rows take 4 / 146, 2800 14 / 201.
+static int64_t x_small_limit(int64_t m, bool exact, size_t vsize)
+{
+    if (m > (int64_t)kXRows * kXTMax) return kSmall2;
+    if (exact || m <= (int64_t(1) << 16)) return kSmallMid;
+    return vsize == 1 && m > (int64_t(1) << 19) ? kSmall2 : kSmallMid2;
+}
+
 template <class SR>
 static void plan_fold(Context *ctx, Plan &P, int64_t m, int64_t k)
 {
@@ -1221,7 +1236,7 @@ static void plan_fold(Context *ctx, Plan &P, int64_t m, int64_t k)
         P.want_aexp = exact;
         if (exact && P.tile_rows != 0 && P.tile_rows != kXRows) P.max_words = 2 * kMaxMaskWords;
         P.tile_rows = kXRows;
-        if (!P.s2_set) P.s2 = std::min<int64_t>(P.s2, kSmallMid);
+        if (!P.s2_set) P.s2 = std::min<int64_t>(P.s2, x_small_limit(m, exact, sizeof(typename SR::V)));
     } else if (!XAcc<SR>::kUse || exact) {
         P.own_vsize = (int)sizeof(typename SR::V);
     }

@@ -1193,6 +1193,7 @@ __global__ void __launch_bounds__(kXThreads, 2)
                     accumulate(fill_table(st, ln, bv, true), row0, std::true_type{});
                     __syncthreads();
                 }
+                if (tid == 0) atomicAdd(&work[1], 1ull);
                 write_direct(nw, row0);
                 XPROF_LAP(12);
             }

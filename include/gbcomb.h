@@ -85,14 +85,16 @@ typedef struct {
     int tile_rows;   /* rows of the block kernel's accumulator tile: 0 = 4096
                         up to 2^18 rows of A and 8192 above, or 4096 / 8192 /
                         16384; always 4096 for PlusTimes fp64 under the exact
-                        fold and, on ordinary sizes, for the semirings whose
+                        fold and, up to 2^20 rows, for the semirings whose
                         add does not depend on the order */
     int64_t tiny_limit;  /* columns with <= this many multiplications use the
                             smallest warp kernel (<= 256; -1 = default 256) */
     int64_t small_limit; /* ... <= this many the larger warp kernels (<= 4096;
-                            -1 = default: 1024, or 4096 for PlusTimes fp32 and
-                            for fp64 under the ordered fold); above it the
-                            block kernels */
+                            -1 = default: 4096 for PlusTimes fp32, for fp64
+                            under the ordered fold and above 2^20 rows; else
+                            1024, or 2048 (4096 for booleans above 2^19) from
+                            2^16 rows on for the semirings whose add does not
+                            depend on the order); above it the block kernels */
 } gbc_spgemm_opts;
 
 typedef struct {

@@ -13,16 +13,17 @@ pytestmark = pytest.mark.gpu
 BUCKETED = 1 << 20  # rows
 
 
-def product(oracle, m, sr, deg, nb):
-    """Visits of the default product of 40 columns of deg x nb products over m rows."""
+def product(oracle, m, sr, deg, nb, cols=40):
+    """Visits of the default product of `cols` columns of deg x nb products over m rows."""
     rng = np.random.default_rng(m + deg)
     A = columns(m, [np.unique(rng.integers(0, m, deg)) for _ in range(2000)])
-    B = columns(2000, [np.sort(rng.choice(2000, nb, replace=False)) for _ in range(40)])
+    B = columns(2000, [np.sort(rng.choice(2000, nb, replace=False)) for _ in range(cols)])
     name, dt = SR_NAME[sr]
     for M in (A, B):
         M.values = (rng.random(M.nnz) * 100 + 1).astype(dt)
     R = local.spgemm(A, B, sr=name, dtype=dt)
-    got, exp = R.to_csc(), oracle.port_spgemm(A, B, sr)
+    got = R.to_csc()
+    exp = oracle.port_spgemm(A, B, sr, fold="exact") if sr == 0 else oracle.port_spgemm(A, B, sr)
     for g, e in zip(got, exp):
         assert np.array_equal(g, e)
     return R.stats.tile_visits_dense + R.stats.tile_visits_range
@@ -32,3 +33,11 @@ def product(oracle, m, sr, deg, nb):
 def test_order_free_semirings(gpu_ctx, oracle_lib, sr):
     assert product(oracle_lib, BUCKETED, sr, 60, 100) > 0
     assert product(oracle_lib, BUCKETED + 1, sr, 60, 100) == 0
+
+
+@pytest.mark.parametrize("m,sr,nb,blocks", [
+    (1 << 16, 3, 20, True), ((1 << 16) + 1, 3, 20, False), ((1 << 16) + 1, 3, 40, True),
+    (1 << 19, 5, 40, True), ((1 << 19) + 1, 5, 40, False), ((1 << 19) + 1, 3, 40, True), ((1 << 19) + 1, 5, 100, True),
+    (BUCKETED, 0, 20, True), (BUCKETED + 1, 0, 40, False), (BUCKETED + 1, 0, 100, True)])
+def test_columns_of_1200_2400_and_6000_products(gpu_ctx, oracle_lib, m, sr, nb, blocks):
+    assert (product(oracle_lib, m, sr, 60, nb, cols=3000) > 0) == blocks
