@@ -314,6 +314,8 @@ constexpr int kBigList = kWarpClasses;            // index of the big list in Li
 constexpr int kOwnList = kBigList + 1;            // ... of the columns for k_numeric_own
 constexpr int kOwnSlot = kWarpClasses + kBigBins; // its slot while classifying
 constexpr int kLists = kOwnSlot + 1;              // list slots while classifying
+constexpr int kListSums = kLists + 3;             // their lengths, then all columns' multiplications, and those
+                                                  // and the B entries of the warp classes above s1
 
 // Of the big columns, those with at least own_need products per B entry (0:
 // none), own_min() for every row range, are listed for k_numeric_own: a
@@ -325,7 +327,7 @@ __global__ void k_classify(const int64_t *flop, const int64_t *bcp, int64_t own_
     const int64_t i = j0 + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     int cls = -1;
-    unsigned long long fsum = 0;
+    unsigned long long fsum = 0, msum = 0, esum = 0;
     if (i < j1 && (!only_flagged || only_flagged[col_base + i])) {
         const int64_t f = flop[i];
         fsum = f;
@@ -335,6 +337,8 @@ __global__ void k_classify(const int64_t *flop, const int64_t *bcp, int64_t own_
             cls = 0;
         } else if (f <= s2) {
             cls = f <= kSmallMid ? 1 : f <= kSmallMid2 ? 2 : 3;
+            msum = f;
+            esum = bcp[i + 1] - bcp[i];
         } else if (own_need > 0 && f >= own_need * (bcp[i + 1] - bcp[i])) {
             cls = kOwnSlot;
         } else {
@@ -342,8 +346,16 @@ __global__ void k_classify(const int64_t *flop, const int64_t *bcp, int64_t own_
         }
     }
 #pragma unroll
-    for (int o = 16; o; o >>= 1) fsum += __shfl_xor_sync(0xffffffffu, fsum, o);
+    for (int o = 16; o; o >>= 1) {
+        fsum += __shfl_xor_sync(0xffffffffu, fsum, o);
+        msum += __shfl_xor_sync(0xffffffffu, msum, o);
+        esum += __shfl_xor_sync(0xffffffffu, esum, o);
+    }
     if (lane == 0 && fsum) atomicAdd(&counts[kLists], fsum);
+    if (lane == 0 && msum) {
+        atomicAdd(&counts[kLists + 1], msum);
+        atomicAdd(&counts[kLists + 2], esum);
+    }
 #pragma unroll
     for (int c = 0; c < kLists; ++c) {
         const unsigned m = __ballot_sync(0xffffffffu, cls == c);
@@ -1154,12 +1166,25 @@ int prepare_operands(Workspace &ws, const DevMatrix &A, const DevMatrix &B, Spge
 // Entries of A up to which the exact kernel's tile lists and scratch are sized
 // by bounds.
 constexpr int64_t kKtlBound = 8192;
-// Where k_numeric_x runs, a warp kernel's list above s1 products with at most
-// this many columns per resident block goes to the block kernels: a warp alone
-// takes 70 to 90 us over 1000 products, however few such columns there are, and
-// a block about 8.  A host square of 700 columns 415 -> 314 us, a scale-14 square
-// (2.4*10^3 such columns) 1190 -> 1157 us; from 16 per block on no gain.
-constexpr int64_t kFewColumns = 8;
+// Where k_numeric_x runs, a warp kernel's list above s1 products goes to the
+// block kernels when it has few columns: a warp alone takes 55 to 90 us over 1000
+// products, however few such columns there are, and a block 8 to 15, more the more
+// segments of A and row tiles the column has.  At most this many columns per
+// resident block, for n columns of `prods` products from `entries` entries of B in
+// all; `others`: the block kernels run anyway (else their launches are added).
+// Measured (device us saved, 1 / 4 / 8 columns a block): 280 products of 8-entry
+// segments over 2^14 rows 30 / 0 / -35, 500 45 / 0 / -55, 60-entry segments 50 /
+// 40 / -2; over 2^20 rows -7 at 2 a block and -100 at 4; alone, 1 a block, 280
+// products -6, 960 60.  Above kXTMax tiles a block visits every tile (2400 columns
+// of 500 products over 2^21 rows 10.4 ms, by warps 0.5).  R-MAT segments are long:
+// a host square of 700 columns 415 -> 314 us, a scale-14 square (2.4*10^3 such
+// columns) 1190 -> 1157 us.
+static int64_t few_columns(int tiles, bool others, int64_t n, int64_t prods, int64_t entries)
+{
+    if (tiles > kXTMax) return 0;
+    if (!others) return tiles <= 16 && prods >= 640 * n ? 1 : 0;
+    return tiles > 16 ? 2 : prods >= 32 * entries ? 8 : 4;
+}
 // k_numeric_own has a column walked by four warps: with fewer columns per
 // multiprocessor than this (two rounds of its resident blocks) the longest one is
 // the launch's end, and the list goes to k_numeric.  fp32 square of a 2357-vertex
@@ -1173,7 +1198,7 @@ struct Plan {
     std::vector<SpgemmArgs> h;        // host copies of the descriptors
     SpgemmArgs *d = nullptr;          // device array
     int64_t total_cols = 0;           // stored columns of all B's
-    int max_R = 0, max_key_bits = 0;
+    int max_R = 0, max_T = 0, max_key_bits = 0;
     size_t max_sym_smem = 0;
     int64_t s1 = kSmall1, s2 = GBC_SMALL2;  // flop thresholds of the column classes
     int tile_rows = 0;                   // accumulator tile height (0: default)
@@ -1341,6 +1366,7 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
     a.col_base = P.total_cols;
     P.total_cols += nb;
     P.max_R = std::max(P.max_R, a.R);
+    P.max_T = std::max(P.max_T, a.T);
     P.max_key_bits = std::max(P.max_key_bits, a.key_bits);
     int sup_rows = (int)std::min<int64_t>((int64_t)kSymRows, (int64_t)a.T * a.R);
     sup_rows = (sup_rows / a.R) * a.R;
@@ -1392,7 +1418,7 @@ static int plan_finalize(Workspace &ws, Plan &P)
     GBC_TRY(ws.alloc_n(&P.work, 16));
     GBC_CUDA_TRY(cudaMemsetAsync(P.work, 0, 16 * sizeof(unsigned long long), ws.ctx->stream));
     GBC_TRY(ws.alloc_n(&P.lbuf, kLists * ((size_t)P.total_cols + 1)));
-    GBC_TRY(ws.alloc_n(&P.lcnt, kLists + 1));
+    GBC_TRY(ws.alloc_n(&P.lcnt, kListSums));
     if (P.want_x) {
         GBC_TRY(ws.alloc_n(&P.fb_items, (size_t)P.total_cols + 1));
         GBC_TRY(ws.alloc_n(&P.fb_cnt, 1));
@@ -1427,8 +1453,7 @@ static int plan_build(Workspace &ws, const DevMatrix &A, const DevMatrix &B, Pla
 static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j1, Lists &L, int64_t *cnt_zero,
                          const int32_t *flagged = nullptr)
 {
-    constexpr int NL = kLists + 1;  // and the multiplications
-    GBC_CUDA_TRY(cudaMemsetAsync(P.lcnt, 0, NL * sizeof(unsigned long long), s));
+    GBC_CUDA_TRY(cudaMemsetAsync(P.lcnt, 0, kListSums * sizeof(unsigned long long), s));
     const int64_t stride = P.total_cols + 1;
     for (int q = 0; q < (int)P.h.size(); ++q) {
         if (pid >= 0 && q != pid) continue;
@@ -1443,7 +1468,7 @@ static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j
         }
     }
     GBC_CUDA_TRY(cudaGetLastError());
-    unsigned long long h[NL];
+    unsigned long long h[kListSums];
     GBC_CUDA_TRY(cudaMemcpyAsync(h, P.lcnt, sizeof(h), cudaMemcpyDeviceToHost, s));
     GBC_CUDA_TRY(cudaStreamSynchronize(s));
     // the big list: its first part (columns for k_numeric_own that are too few
@@ -1459,10 +1484,15 @@ static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j
                 cudaMemcpyAsync(lbig + nbig, bins + c * stride, nc * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
         nbig += nc;
     }
+    const int64_t few = P.want_x && !P.s2_set
+                            ? few_columns(P.max_T, nbig > 0, (int64_t)(h[1] + h[2] + h[3]), (int64_t)h[kLists + 1],
+                                          (int64_t)h[kLists + 2]) *
+                                  P.x_blocks
+                            : 0;
     for (int c = 0; c < kWarpClasses; ++c) {
         L.l[c] = P.lbuf + c * stride;
         L.n[c] = (int64_t)h[c];
-        if (c > 0 && P.want_x && !P.s2_set && L.n[c] > 0 && L.n[c] <= kFewColumns * P.x_blocks) {
+        if (c > 0 && L.n[c] > 0 && L.n[c] <= few) {
             GBC_CUDA_TRY(cudaMemcpyAsync(lbig + nbig, L.l[c], L.n[c] * sizeof(int64_t), cudaMemcpyDeviceToDevice, s));
             nbig += L.n[c];
             L.n[c] = 0;

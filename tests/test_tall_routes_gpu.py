@@ -41,3 +41,15 @@ def test_order_free_semirings(gpu_ctx, oracle_lib, sr):
     (BUCKETED, 0, 20, True), (BUCKETED + 1, 0, 40, False), (BUCKETED + 1, 0, 100, True)])
 def test_columns_of_1200_2400_and_6000_products(gpu_ctx, oracle_lib, m, sr, nb, blocks):
     assert (product(oracle_lib, m, sr, 60, nb, cols=3000) > 0) == blocks
+
+
+@pytest.mark.parametrize("sr", [0, 3])
+@pytest.mark.parametrize("m,nb,cols,blocks", [
+    (1 << 14, 5, 40, False), (1 << 14, 15, 40, True), (1 << 14, 15, 3000, False), ((1 << 16) + 1, 15, 40, False)])
+def test_few_columns_of_300_and_900_products(gpu_ctx, oracle_lib, m, nb, cols, blocks, sr):
+    """On their own: to the blocks only where each has one, long enough, over few tiles."""
+    assert (product(oracle_lib, m, sr, 60, nb, cols) > 0) == blocks
+
+
+def test_few_columns_above_the_bucketed_rows(gpu_ctx, oracle_lib):
+    assert product(oracle_lib, BUCKETED + 1, 0, 60, 15) == 0
