@@ -310,6 +310,11 @@ __device__ __forceinline__ int big_bin(int64_t f)
            : f > (1ll << 15) ? 6
                              : 7;
 }
+// The most multiplications of a column in bin c.
+constexpr int64_t big_bin_top(int c)
+{
+    return c == 0 ? INT64_MAX : c == 1 ? int64_t(1) << 22 : int64_t(1) << (22 - c);
+}
 constexpr int kBigList = kWarpClasses;            // index of the big list in Lists
 constexpr int kOwnList = kBigList + 1;            // ... of the columns for k_numeric_own
 constexpr int kOwnSlot = kWarpClasses + kBigBins; // its slot while classifying
@@ -1210,10 +1215,13 @@ struct Plan {
     unsigned long long *lcnt = nullptr;  // list lengths
     bool want_x = false;                 // big columns by k_numeric_x
     bool want_aexp = false;              // ... PlusTimes fp64, exact sums
+    std::vector<uint64_t *> amask;       // row tiles of every product's A columns
+    bool x_built = false;                // k_numeric_x's tile lists and lists of columns are there
     int64_t *fb_items = nullptr;         // big columns the exact kernel hands to the ordered one
     unsigned long long *fb_cnt = nullptr;
-    XSeg *xscratch = nullptr;            // exact kernel: bucketing scratch, xscap segments per block
-    int64_t xscap = 0;                   // (no column has more than its A has tile list entries)
+    XSeg *xscratch = nullptr;            // exact kernel: bucketing scratch, xs_cap segments for each of xs_blocks
+    int64_t xs_cap = 0, xs_blocks = 0;
+    int64_t xscap = 0;                   // segments of a column at most (its A's tile list entries)
     int x_blocks = 0;                    // exact kernel: its grid (resident blocks)
     int own_vsize = 0;                   // value size for k_numeric_own (0: not used)
     bool own_built = false;              // its range tables are there
@@ -1336,30 +1344,6 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
             note_launch();
         }
         a.aexp = aexp;
-        if (a.T <= kXTMax && A.ncol > 0) {
-            // per-column tile lists of A (bucketing in the exact kernel)
-            int64_t *kptr = nullptr;
-            GBC_TRY(ws.alloc_n(&kptr, (size_t)A.ncol + 1));
-            k_ktl_count<<<(unsigned)((A.ncol + 255) / 256), 256, 0, s>>>(A.ncol, amask, a.mask_words, kptr);
-            note_launch();
-            GBC_TRY(exclusive_scan_i64(ws, kptr, kptr, A.ncol, s));
-            // The bounds do where the scratch stays small (4 KB per entry of
-            // A over all blocks; the lists are smaller than tptr), and save
-            // the read-back.  Segments are touched tiles, without the markers.
-            int64_t nent = ktl_room(A.nnz, A.ncol);
-            if (A.nnz > kKtlBound) GBC_TRY(read_i64(ctx, kptr + A.ncol, &nent));
-            P.xscap = std::max(P.xscap, std::min(std::min(nent, A.nnz), kXScap));
-            uint32_t *kst = nullptr;
-            uint16_t *ktt = nullptr;
-            GBC_TRY(ws.alloc_n(&kst, (size_t)nent + 1));
-            GBC_TRY(ws.alloc_n(&ktt, (size_t)nent + 1));
-            k_ktl_fill<<<grid_for(ctx, (A.ncol + 7) / 8, 8), 256, 0, s>>>(A.ncol, a.tptr, a.T, kptr, kst, ktt);
-            note_launch();
-            GBC_CUDA_TRY(cudaGetLastError());
-            a.ktl_ptr = kptr;
-            a.ktl_start = kst;
-            a.ktl_tile = ktt;
-        }
     }
     a.aval = A.num;
     a.bval = B.num;
@@ -1373,6 +1357,66 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
     P.max_sym_smem = std::max(P.max_sym_smem, (size_t)sup_rows / 8);
     P.h.push_back(a);
     P.a_nnz.push_back(A.nnz);
+    P.amask.push_back(amask);
+    return GBC_OK;
+}
+
+// What k_numeric_x needs beside the operands, built when a column first goes
+// there (the counting, a read-back and the fill took a fifth of a product of 300
+// columns that does without): per-column tile lists of every A.
+static int plan_x(Plan &P)
+{
+    Workspace &ws = *P.ws;
+    Context *ctx = ws.ctx;
+    cudaStream_t s = ctx->stream;
+    GBC_TRY(ws.alloc_n(&P.fb_items, (size_t)P.total_cols + 1));
+    GBC_TRY(ws.alloc_n(&P.fb_cnt, 1));
+    for (SpgemmArgs &a : P.h) {
+        if (a.T > kXTMax || a.kdim == 0) continue;
+        const size_t q = &a - P.h.data();
+        const int64_t nnz = P.a_nnz[q];
+        int64_t *kptr = nullptr;
+        GBC_TRY(ws.alloc_n(&kptr, (size_t)a.kdim + 1));
+        k_ktl_count<<<(unsigned)((a.kdim + 255) / 256), 256, 0, s>>>(a.kdim, P.amask[q], a.mask_words, kptr);
+        note_launch();
+        GBC_TRY(exclusive_scan_i64(ws, kptr, kptr, a.kdim, s));
+        // The bounds do where the scratch stays small (4 KB per entry of
+        // A over all blocks; the lists are smaller than tptr), and save
+        // the read-back.  Segments are touched tiles, without the markers.
+        int64_t nent = ktl_room(nnz, a.kdim);
+        if (nnz > kKtlBound) GBC_TRY(read_i64(ctx, kptr + a.kdim, &nent));
+        P.xscap = std::max(P.xscap, std::min(std::min(nent, nnz), kXScap));
+        uint32_t *kst = nullptr;
+        uint16_t *ktt = nullptr;
+        GBC_TRY(ws.alloc_n(&kst, (size_t)nent + 1));
+        GBC_TRY(ws.alloc_n(&ktt, (size_t)nent + 1));
+        k_ktl_fill<<<grid_for(ctx, (a.kdim + 7) / 8, 8), 256, 0, s>>>(a.kdim, a.tptr, a.T, kptr, kst, ktt);
+        note_launch();
+        GBC_CUDA_TRY(cudaGetLastError());
+        a.ktl_ptr = kptr;
+        a.ktl_start = kst;
+        a.ktl_tile = ktt;
+    }
+    GBC_CUDA_TRY(cudaMemcpyAsync(P.d, P.h.data(), P.h.size() * sizeof(SpgemmArgs), cudaMemcpyHostToDevice, s));
+    P.x_built = true;
+    return GBC_OK;
+}
+
+// Bucketing scratch for the blocks that `cols` big columns of at most `flop`
+// multiplications keep busy (a column has no more segments than those).  Columns
+// of more segments than there is room for visit every tile, so less will do.
+static int plan_x_scratch(Plan &P, int64_t cols, int64_t flop)
+{
+    const int64_t blocks = std::max(P.xs_blocks, std::min<int64_t>(cols, P.x_blocks));
+    int64_t cap = std::max(P.xs_cap, std::min(P.xscap, flop));
+    if (blocks == P.xs_blocks && cap == P.xs_cap) return GBC_OK;
+    while (P.ws->alloc_n(&P.xscratch, (size_t)(blocks * cap)) != GBC_OK) {
+        if (cap == 0) return GBC_ENOMEM;
+        cap /= 4;
+        P.xscap = cap;  // nor is more asked for again
+    }
+    P.xs_blocks = blocks;
+    P.xs_cap = cap;
     return GBC_OK;
 }
 
@@ -1419,13 +1463,7 @@ static int plan_finalize(Workspace &ws, Plan &P)
     GBC_CUDA_TRY(cudaMemsetAsync(P.work, 0, 16 * sizeof(unsigned long long), ws.ctx->stream));
     GBC_TRY(ws.alloc_n(&P.lbuf, kLists * ((size_t)P.total_cols + 1)));
     GBC_TRY(ws.alloc_n(&P.lcnt, kListSums));
-    if (P.want_x) {
-        GBC_TRY(ws.alloc_n(&P.fb_items, (size_t)P.total_cols + 1));
-        GBC_TRY(ws.alloc_n(&P.fb_cnt, 1));
-        // bucketing scratch of the exact kernel, per resident block
-        P.x_blocks = ws.ctx->num_sms * 2;  // (the kernels' launch bounds and XSmem)
-        GBC_TRY(ws.alloc_n(&P.xscratch, (size_t)P.x_blocks * P.xscap + 1));
-    }
+    P.x_blocks = ws.ctx->num_sms * 2;  // (k_numeric_x's launch bounds and XSmem)
     GBC_CUDA_TRY(cudaMemcpyAsync(P.d, P.h.data(), P.h.size() * sizeof(SpgemmArgs), cudaMemcpyHostToDevice,
                                  ws.ctx->stream));
     return GBC_OK;
@@ -1504,6 +1542,16 @@ static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j
     L.n[kOwnList] = few_own ? 0 : (int64_t)h[kOwnSlot];
     L.flops = (int64_t)h[kLists];
     if (L.n[kOwnList] > 0 && !P.own_built) GBC_TRY(plan_own(P));
+    if (P.want_x && nbig > 0) {
+        if (!P.x_built) GBC_TRY(plan_x(P));
+        int64_t flop = int64_t(1) << 15;  // of the largest column: the top of the first bin that has one
+        for (int c = 0; c < kBigBins - 1; ++c)
+            if (h[kWarpClasses + c] > 0) {
+                flop = big_bin_top(c);
+                break;
+            }
+        GBC_TRY(plan_x_scratch(P, nbig, flop));
+    }
     return GBC_OK;
 }
 
@@ -1616,13 +1664,13 @@ static int launch_big_exact(Context *ctx, Plan &P, const Lists &L, const int64_t
                             const int64_t *cap, int64_t *out_cnt, int32_t *overflow, int64_t *cir, void *cval)
 {
     cudaStream_t s = ctx->stream;
-    const int grid = (int)std::min<int64_t>(P.x_blocks, L.n[kBigList]);  // the scratch holds P.x_blocks blocks
+    const int grid = (int)std::min<int64_t>(P.xs_blocks, L.n[kBigList]);  // the blocks there is scratch for
     GBC_CUDA_TRY(cudaMemsetAsync(P.work + 1, 0, 3 * sizeof(unsigned long long), s));
     GBC_CUDA_TRY(cudaMemsetAsync(P.fb_cnt, 0, sizeof(unsigned long long), s));
     GBC_TRY(set_smem(k_numeric_x<SR>, sizeof(XSmem)));
     k_numeric_x<SR><<<grid, kXThreads, sizeof(XSmem), s>>>(P.d, L.l[kBigList], L.n[kBigList], ccp, ccp_base, cap, out_cnt,
                                                            overflow, cir, cval, P.work + 1, P.fb_items, P.fb_cnt,
-                                                           P.xscratch, P.xscap);
+                                                           P.xscratch, P.xs_cap);
     note_launch();
     GBC_CUDA_TRY(cudaGetLastError());
     return launch_big_ordered<SR>(ctx, P, P.fb_items, L.n[kBigList], P.fb_cnt, ccp, ccp_base, cap, out_cnt, overflow, cir,
