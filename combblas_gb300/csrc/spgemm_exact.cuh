@@ -75,12 +75,13 @@ extern "C" int gbc_xprof_read(unsigned long long *out, int reset)
 #endif
 
 // Per column of A: smallest and largest biased exponent of its nonzero
-// values, each plus kXBias in 12 bits, and kXMixed when a value is negative or
-// zero.  Subnormal values count as exponent -64 (their products can
+// values, each plus kXBias in 12 bits, kXMixed when a value is negative or
+// zero, and kXZero when one is zero.  Subnormal values count as exponent -64 (their products can
 // underflow: such columns take the ordered kernel); a column without nonzero
 // values gets min > max.
 constexpr int kXBias = 64;
 constexpr uint32_t kXMixed = 1u << 24;
+constexpr uint32_t kXZero = 1u << 25;
 
 static __global__ void k_aexp_f64(int64_t ncol, const int64_t *acp, const double *aval, int32_t *aexp)
 {
@@ -89,12 +90,13 @@ static __global__ void k_aexp_f64(int64_t ncol, const int64_t *acp, const double
     const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
     for (int64_t c = warp; c < ncol; c += nwarps) {
         int lo = 4095 - kXBias, hi = -kXBias;
-        bool mixed = false;
+        bool mixed = false, zeros = false;
         for (int64_t p = acp[c] + lane; p < acp[c + 1]; p += 32) {
             const uint64_t bits = (uint64_t)__double_as_longlong(aval ? aval[p] : 1.0);
             int e = (int)((bits >> 52) & 0x7ff);
             const bool zero = (bits << 1) == 0;
             mixed |= zero || (bits >> 63);
+            zeros |= zero;
             if (e == 0) e = -kXBias;
             if (!zero) {
                 lo = min(lo, e);
@@ -104,8 +106,10 @@ static __global__ void k_aexp_f64(int64_t ncol, const int64_t *acp, const double
         lo = __reduce_min_sync(0xffffffffu, lo);
         hi = __reduce_max_sync(0xffffffffu, hi);
         mixed = __any_sync(0xffffffffu, mixed);
+        zeros = __any_sync(0xffffffffu, zeros);
         if (lane == 0)
-            aexp[c] = (int32_t)((uint32_t)(lo + kXBias) | ((uint32_t)(hi + kXBias) << 12) | (mixed ? kXMixed : 0u));
+            aexp[c] = (int32_t)((uint32_t)(lo + kXBias) | ((uint32_t)(hi + kXBias) << 12) | (mixed ? kXMixed : 0u) |
+                                (zeros ? kXZero : 0u));
     }
 }
 
@@ -421,6 +425,7 @@ struct XSmem {
     uint32_t bm[kXSpanTiles * kXRows / 32];   // touched rows of the visit
     uint16_t pre[kXSpanTiles * kXRows / 32];  // touched rows before each bitmap word
     uint16_t rows[kXRows];                 // row (from the visit's first) of every accumulator
+    uint32_t term[kXRows / 32];            // accumulators with a term other than -0.0 (columns with zeros)
     uint64_t bv[kXSegs];                   // chunk table: bits of the B value of each segment,
     uint32_t base[kXSegs];                 //   segment start - products before it (modulo 2^32),
     int32_t off[kXSegs + 1];               //   products before each segment
@@ -429,9 +434,8 @@ struct XSmem {
                                            //   the segments that start before the window
     int32_t segcnt[kXTMax], prodcnt[kXTMax], tend[kXTMax];
     int32_t wsum[2][kXThreads / 32];
-    int32_t emin[kXThreads / 32], emax[kXThreads / 32];
+    int32_t emin[kXThreads / 32], emax[kXThreads / 32], wzero[kXThreads / 32];
     int64_t col;
-    int32_t negzero;  // a product of the visit was -0.0
     int32_t ebase;    // the column's smallest product exponent
     int64_t bs, be;   // its B entries
     int64_t *oir;     // its output
@@ -439,37 +443,6 @@ struct XSmem {
     int32_t lim;      // output entries it may write
     SpgemmArgs a;
 };
-
-// Does row r of column [bs, be) of B receive a term other than -0.0?
-static __device__ __noinline__ bool x_has_term(const SpgemmArgs &a, int64_t bs, int64_t be, int r)
-{
-    const double *aval = static_cast<const double *>(a.aval), *bval = static_cast<const double *>(a.bval);
-    for (int64_t b = bs; b < be; ++b) {
-        const int k = a.brow[b];
-        int64_t lo = a.acp[k], hi = a.acp[k + 1];
-        const int64_t end = hi;
-        while (lo < hi) {
-            const int64_t mid = (lo + hi) >> 1;
-            if (a.arow[mid] < r)
-                lo = mid + 1;
-            else
-                hi = mid;
-        }
-        if (lo < end && a.arow[lo] == r &&
-            __double_as_longlong(__dmul_rn(aval ? aval[lo] : 1.0, bval ? bval[b] : 1.0)) != (long long)(1ull << 63))
-            return true;
-    }
-    return false;
-}
-
-// Output entries [q0, q1) of the column: sums of exactly zero that got no term
-// other than -0.0 become -0.0.  Called when the visit met a -0.0 product.
-static __device__ __noinline__ void x_fix_zeros(const XSmem &sm, int q0, int q1)
-{
-    double *oval = static_cast<double *>(sm.oval);
-    for (int q = q0 + threadIdx.x; q < q1; q += kXThreads)
-        if (oval[q] == 0.0 && !x_has_term(sm.a, sm.bs, sm.be, (int)sm.oir[q])) oval[q] = -0.0;
-}
 
 // Numeric pass for the columns of the big list, one block per column (dynamic
 // counter), for PlusTimes<double> under the exact fold and the semirings whose
@@ -531,7 +504,7 @@ __global__ void __launch_bounds__(kXThreads, 2)
     XSeg *scratch = scratch_all + (int64_t)blockIdx.x * scap;
     for (int u = tid; u < 4 * R; u += NT) sm.acc[u] = 0;
     for (int u = tid; u < kXSpanTiles * R / 32; u += NT) sm.bm[u] = 0;
-    if (tid == 0) sm.negzero = 0;
+    for (int u = tid; u < R / 32; u += NT) sm.term[u] = 0;
     bool dirty = false;  // the accumulator holds a sorted range's data
     bool first_item = true;
     int par = 0;  // which wsum the next prefix uses
@@ -659,25 +632,30 @@ __global__ void __launch_bounds__(kXThreads, 2)
             sm.prodcnt[u] = 0;
         }
         // admission (exact sums): the exponent window of the column's
-        // products; pos: all of them are positive
+        // products; pos: all of them are positive; zeros: some may be zero
         bool pos = true;
+        [[maybe_unused]] bool zeros = false;
         int ebase = 0;
         if constexpr (EXACT) {
-            bool mixed = false;
+            bool mixed = false, zero = false;
             int emin = 1 << 30, emax = -(1 << 30);
             for (int64_t b = bs + tid; b < be; b += NT) {
                 const int32_t ae = a.aexp[a.brow[b]];
                 const double bv = bval ? bval[b] : 1.0;
                 x_window(ae, bv, bval != nullptr, emin, emax);
                 mixed |= (ae & kXMixed) || !(bv > 0.0);
+                zero |= (ae & kXZero) || bv == 0.0;
             }
             emin = __reduce_min_sync(0xffffffffu, emin);
             emax = __reduce_max_sync(0xffffffffu, emax);
+            zero = __any_sync(0xffffffffu, zero);
             if (lane == 0) {
                 sm.emin[warp] = emin;
                 sm.emax[warp] = emax;
+                sm.wzero[warp] = zero;
             }
             pos = !__syncthreads_or(mixed);
+            zeros = __any_sync(0xffffffffu, sm.wzero[lane & (NW - 1)]);
             ebase = __reduce_min_sync(0xffffffffu, sm.emin[lane & (NW - 1)]);
             const int etop = __reduce_max_sync(0xffffffffu, sm.emax[lane & (NW - 1)]);
             if (!x_admit(ebase, etop, be - bs)) {
@@ -708,9 +686,11 @@ __global__ void __launch_bounds__(kXThreads, 2)
         // Products added into the accumulators: of their row's rank, or of
         // the row itself (DIRECT, one tile: the row is marked here as well).
         // The loads of the warp's next window are issued before the current
-        // window's atomics.
-        auto accumulate_as = [&](int L, int row0, auto pos_t, auto direct_t) {
-            [[maybe_unused]] constexpr bool POS = decltype(pos_t)::value;
+        // window's atomics.  SIGN: 0 the products are positive, 1 of either
+        // sign, 2 some may be zero: then `term` marks the accumulators that got
+        // another term than -0.0, which alone leaves an exact zero -0.0.
+        auto accumulate_as = [&](int L, int row0, auto sign_t, auto direct_t) {
+            [[maybe_unused]] constexpr int SIGN = decltype(sign_t)::value;
             constexpr bool DIRECT = decltype(direct_t)::value;
             const int32_t *arow = sm.a.arow;
             const V *aval = static_cast<const V *>(sm.a.aval);
@@ -745,11 +725,12 @@ __global__ void __launch_bounds__(kXThreads, 2)
                         }
                         if constexpr (EXACT) {
                             const uint64_t bits = (uint64_t)__double_as_longlong(prod);
-                            if (!POS && (bits << 1) == 0) {
-                                if (bits) sm.negzero = 1;
-                            } else if (!x_add128<POS>(sm.acc + at, R, bits, ebase)) {
-                                bad = true;
+                            if (SIGN == 2 && bits != 1ull << 63) {
+                                const uint32_t bit = 1u << (at & 31);
+                                if (!(sm.term[at >> 5] & bit)) atomicOr(&sm.term[at >> 5], bit);
                             }
+                            if ((SIGN < 2 || (bits << 1) != 0) && !x_add128<SIGN == 0>(sm.acc + at, R, bits, ebase))
+                                bad = true;
                         } else if (!Acc::add(sm.acc, R, at, prod)) {
                             bad = true;
                         }
@@ -758,10 +739,12 @@ __global__ void __launch_bounds__(kXThreads, 2)
             });
         };
         auto accumulate = [&](int L, int row0, auto direct_t) {
-            if (pos)
-                accumulate_as(L, row0, std::true_type{}, direct_t);
+            if (!EXACT || pos)
+                accumulate_as(L, row0, std::integral_constant<int, 0>{}, direct_t);
+            else if (!zeros)
+                accumulate_as(L, row0, std::integral_constant<int, EXACT ? 1 : 0>{}, direct_t);
             else
-                accumulate_as(L, row0, std::false_type{}, direct_t);
+                accumulate_as(L, row0, std::integral_constant<int, EXACT ? 2 : 0>{}, direct_t);
         };
         // ranks of the touched rows among the first nw bitmap words (at most
         // 4 per thread); *before(t) is left in pre[]; returns the total
@@ -796,7 +779,7 @@ __global__ void __launch_bounds__(kXThreads, 2)
                 w[R] = 0;
                 w[2 * R] = 0;
                 w[3 * R] = 0;
-                v = x_round(hi, lo, 2, sm.ebase);
+                v = x_round(hi, lo, !zeros || (sm.term[at >> 5] >> (at & 31) & 1) ? 2 : 0, sm.ebase);
             } else {
                 v = Acc::take(sm.acc, R, at);
             }
@@ -810,11 +793,8 @@ __global__ void __launch_bounds__(kXThreads, 2)
         };
         auto end_visit = [&](int n) {
             __syncthreads();
-            if (EXACT && sm.negzero) {  // block-uniform
-                x_fix_zeros(sm, out, min(out + n, sm.lim));
-                __syncthreads();
-                if (tid == 0) sm.negzero = 0;  // read again only after another visit's barriers
-            }
+            if (EXACT && zeros)  // block-uniform; marked again only after another visit's barriers
+                for (int w = tid; w < R / 32; w += NT) sm.term[w] = 0;
             out += n;
         };
         // a ranked visit's n entries; the bitmap's first nw words are cleared
