@@ -143,17 +143,33 @@ __global__ void k_spmv_has(int64_t m, const int64_t *rowptr, int64_t *has)
     if (r < m) has[r] = rowptr[r + 1] > rowptr[r];
 }
 
+// A long row's groups are written by its whole warp: by one thread they took
+// 1.3 ms of a plan with a row of 4*10^6 entries.
 __global__ void k_spmv_mark(int64_t m, const int64_t *rowptr, const int64_t *index, int32_t *rows, uint32_t *starts,
                             int32_t *group_row)
 {
     const int64_t r = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (r >= m) return;
-    const int64_t s = rowptr[r], e = rowptr[r + 1];
-    if (e <= s) return;
-    const int32_t i = (int32_t)index[r];
-    rows[i] = (int32_t)r;
-    atomicOr(&starts[s >> 5], 1u << (s & 31));
-    for (int64_t g = (s + kSpmvPer - 1) / kSpmvPer; g * kSpmvPer < e; ++g) group_row[g] = i;
+    const int lane = threadIdx.x & 31;
+    int64_t s = 0, e = 0;
+    int32_t i = 0;
+    if (r < m) {
+        s = rowptr[r];
+        e = rowptr[r + 1];
+    }
+    if (e > s) {
+        i = (int32_t)index[r];
+        rows[i] = (int32_t)r;
+        atomicOr(&starts[s >> 5], 1u << (s & 31));
+    }
+    const bool is_long = e - s > 32 * kSpmvPer;
+    if (!is_long)
+        for (int64_t g = (s + kSpmvPer - 1) / kSpmvPer; g * kSpmvPer < e; ++g) group_row[g] = i;
+    for (unsigned todo = __ballot_sync(0xffffffffu, is_long); todo; todo &= todo - 1) {
+        const int l = __ffs(todo) - 1;
+        const int64_t ls = __shfl_sync(0xffffffffu, s, l), le = __shfl_sync(0xffffffffu, e, l);
+        const int32_t li = __shfl_sync(0xffffffffu, i, l);
+        for (int64_t g = (ls + kSpmvPer - 1) / kSpmvPer + lane; g * kSpmvPer < le; g += 32) group_row[g] = li;
+    }
 }
 
 // acc + a * x.  Floating sums use a fused multiply-add: one rounding less, and
