@@ -21,6 +21,9 @@
 //   push  the active vertices' edges only: neighbours' words by atomicOr,
 //         parents by atomic minimum.  Everything a push level touches is in its
 //         two vertex lists, so long thin graphs pay for their frontiers only.
+//         A block flattens the edges of a few vertices over its threads; the
+//         hubs, of more than kMbHub neighbours, are listed apart and every block
+//         takes a share of each.
 #pragma once
 
 #include "size_rules.cuh"
@@ -30,8 +33,10 @@ namespace gbc {
 constexpr int kMbWords = 8;      // 512 roots a pass
 constexpr int kMbChunk = 64;     // neighbours of one pull item
 constexpr int kMbPullShare = 4;  // pull when the active edges times this exceed all edges
-constexpr int kMbPushThreads = 128;  // a block of k_mb_push, and its step over a long vertex
-static_assert(kMbPushThreads <= kMbStep && kMbChunk <= kMbStep, "mb_positions_fit");
+static_assert(kMbChunk <= kMbStep, "mb_positions_fit");
+constexpr int kMbQueue = 1024;   // new vertices that a block gathers before it lists them
+constexpr int kMbThreads = 256;  // of a block, and the vertices it pushes at most at a time
+constexpr uint32_t kMbHub = 2048;
 
 enum {
     MB_NF = 0,       // active vertices
@@ -43,9 +48,12 @@ enum {
     MB_CUR = 6,      // which frontier buffer and list is current
     MB_ROOTS = 7,    // roots of this pass
     MB_PARENTS = 8,  // parents of its first root (address)
-    MB_EDGES = 9,    // over all passes: sum of degrees of reached pairs,
-    MB_REACHED = 10, //   reached pairs,
-    MB_LEVELS = 11,  //   the most levels of a pass
+    MB_NHUB = 9,     // hubs among the active vertices
+    MB_NHUB_NEXT = 10,
+    MB_EDGES = 11,   // over all passes: sum of degrees of reached pairs,
+    MB_REACHED = 12, //   reached pairs,
+    MB_LEVELS = 13,  //   the most levels of a pass
+    MB_DONE = 14,    // blocks that have ended the level
     MB_N = 16
 };
 
@@ -57,9 +65,11 @@ struct MbView {
     uint64_t *seen;
     uint64_t *bits0, *bits1;
     int32_t *list0, *list1;
+    int32_t *hubs0, *hubs1;
     uint32_t *touched;
     __device__ __forceinline__ uint64_t *bits(int k) const { return k ? bits1 : bits0; }
     __device__ __forceinline__ int32_t *list(int k) const { return k ? list1 : list0; }
+    __device__ __forceinline__ int32_t *hubs(int k) const { return k ? hubs1 : hubs0; }
     const int32_t *item_v;   // pull chunks of the long vertices
     const uint32_t *item_p;  //   ... and where they start
     int64_t nitems;
@@ -144,78 +154,173 @@ __global__ void k_mb_init(MbView g, const int64_t *roots, int64_t nroots, int64_
     const unsigned long long d = g.cp[v + 1] - g.cp[v];
     if (!(atomicOr(&g.touched[v >> 5], 1u << (v & 31)) & (1u << (v & 31)))) {
         g.list(0)[atomicAdd((unsigned long long *)&g.ctl[MB_NF], 1ull)] = (int32_t)v;
+        if (d > kMbHub) g.hubs(0)[atomicAdd((unsigned long long *)&g.ctl[MB_NHUB], 1ull)] = (int32_t)v;
         atomicAdd((unsigned long long *)&g.ctl[MB_FE], d);
     }
     atomicAdd((unsigned long long *)&g.ctl[MB_EDGES], d);
     atomicAdd((unsigned long long *)&g.ctl[MB_REACHED], 1ull);
 }
 
-__device__ __forceinline__ void mb_mode(int64_t *ctl, int64_t nnz)
-{
-    ctl[MB_MODE] = ctl[MB_FE] * kMbPullShare > nnz ? 1 : 0;
-}
+__device__ __forceinline__ int64_t mb_mode(int64_t fe, int64_t nnz) { return fe * kMbPullShare > nnz ? 1 : 0; }
 
 // The roots' touched marks are cleared, the first level's mode is chosen.
 __global__ void k_mb_begin(MbView g)
 {
     for (int64_t i = threadIdx.x; i < g.ctl[MB_NF]; i += blockDim.x) g.touched[g.list(0)[i] >> 5] = 0;
-    if (threadIdx.x == 0) mb_mode(g.ctl, g.nnz);
+    if (threadIdx.x == 0) g.ctl[MB_MODE] = mb_mode(g.ctl[MB_FE], g.nnz);
 }
 
-// Push: a warp per active vertex, the block together for the long ones.
+// New vertices of a block on their way to the next frontier's list, one atomic on
+// its length per batch (one per warp: 700 x 700 grid with 500 roots 101 -> 81 ms, one
+// root on 2^22 random vertices 1.35 -> 0.88).  Every thread of the block calls add()
+// and step(); step() ends a round of at most NT vertices, end() the kernel.
+template <int NT>
+struct MbQueue {
+    int32_t v[kMbQueue];
+    int n;
+    unsigned long long base;
+    __device__ __forceinline__ void begin()
+    {
+        if (threadIdx.x == 0) n = 0;
+        __syncthreads();
+    }
+    __device__ __forceinline__ void add(bool act, int32_t x)
+    {
+        const int lane = threadIdx.x & 31;
+        const unsigned m = __ballot_sync(0xffffffffu, act);
+        if (m == 0) return;
+        int at = 0;
+        if (lane == __ffs(m) - 1) at = atomicAdd(&n, __popc(m));
+        at = __shfl_sync(0xffffffffu, at, __ffs(m) - 1);
+        if (act) v[at + __popc(m & ((1u << lane) - 1))] = x;
+    }
+    __device__ __forceinline__ void flush(int64_t *ctl, int32_t *list)  // behind a barrier
+    {
+        const int have = n;
+        if (threadIdx.x == 0 && have > 0)
+            base = atomicAdd((unsigned long long *)&ctl[MB_NNEXT], (unsigned long long)have);
+        __syncthreads();
+        for (int k = threadIdx.x; k < have; k += NT) list[base + k] = v[k];
+        __syncthreads();
+    }
+    __device__ __forceinline__ void step(int64_t *ctl, int32_t *list)
+    {
+        // (one thread looks, before the others of the round may have added: all decide alike)
+        if (!__syncthreads_or(threadIdx.x == 0 && n > kMbQueue - 2 * NT)) return;
+        flush(ctl, list);
+        begin();
+    }
+    __device__ __forceinline__ void end(int64_t *ctl, int32_t *list)
+    {
+        __syncthreads();
+        flush(ctl, list);
+    }
+};
+
+// Push.  The vertices that a block takes at a time are as many as share the
+// frontier out evenly, so that thin frontiers keep all blocks busy and wide ones
+// of few neighbours all lanes.  Bound by the latency of an edge's chain (neighbour,
+// its seen word, the atomics).  With a warp per vertex (a block above 512
+// neighbours), an atomic per listed vertex and five launches a level: 700 x 700 grid
+// with 500 roots 112 -> 81 ms, hubs of 300 on a path with 300 roots 228 -> 92, one
+// root on 2^22 vertices with a hub of 10^6 neighbours 16.9 -> 0.58, without the hub
+// 2.08 -> 0.84.
 template <int NW>
-__global__ void __launch_bounds__(kMbPushThreads) k_mb_push(MbView g)
+__device__ __forceinline__ void mb_push(const MbView &g)
 {
-    if (g.ctl[MB_MODE] != 0) return;
-    __shared__ int32_t s_long[4];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int64_t nf = g.ctl[MB_NF];
+    constexpr int NT = kMbThreads;
+    __shared__ int32_t s_u[NT];
+    __shared__ uint32_t s_st[NT];
+    __shared__ int32_t s_off[NT + 1];
+    __shared__ MbQueue<NT> queue;
+    const int tid = threadIdx.x;
+    const int64_t nf = g.ctl[MB_NF], nh = g.ctl[MB_NHUB];
     const int cur = (int)g.ctl[MB_CUR];
     const uint64_t *front = g.bits(cur);
     uint64_t *next = g.bits(cur ^ 1);
     int32_t *nlist = g.list(cur ^ 1);
     unsigned long long *parents = (unsigned long long *)(uintptr_t)g.ctl[MB_PARENTS];
-    auto edges = [&](int32_t u, int first, int step) {
-        uint64_t f[NW];
-#pragma unroll
-        for (int w = 0; w < NW; ++w) f[w] = front[(int64_t)u * NW + w];
-        const uint32_t s = g.cp[u], e = g.cp[u + 1];
-        for (uint32_t p = s + first; p < e; p += step) {
-            const int32_t v = g.row[p];
+    // the edge from u to the entry at p (act: there is one); all threads
+    auto edge = [&](bool act, int32_t u, uint32_t p) {
+        bool fresh = false;
+        int32_t v = 0;
+        if (act) {
+            v = g.row[p];
+            uint64_t x[NW];
             bool any = false;
 #pragma unroll
+            for (int w = 0; w < NW; ++w) x[w] = front[(int64_t)u * NW + w];
+#pragma unroll
+            for (int w = 0; w < NW; ++w)
+                if (x[w]) x[w] &= ~g.seen[(int64_t)v * NW + w];  // (few words, where there are many)
+#pragma unroll
             for (int w = 0; w < NW; ++w) {
-                if (f[w] == 0) continue;
-                uint64_t x = f[w] & ~g.seen[(int64_t)v * NW + w];
-                if (x == 0) continue;
+                if (x[w] == 0) continue;
                 any = true;
-                atomicOr((unsigned long long *)&next[(int64_t)v * NW + w], (unsigned long long)x);
-                while (x) {
-                    const int b = __ffsll((long long)x) - 1;
-                    x &= x - 1;
-                    atomicMin(&parents[(int64_t)(w * 64 + b) * g.n + v], (unsigned long long)u);
-                }
+                atomicOr((unsigned long long *)&next[(int64_t)v * NW + w], (unsigned long long)x[w]);
+                for (uint64_t y = x[w]; y; y &= y - 1)
+                    atomicMin(&parents[(int64_t)(w * 64 + __ffsll((long long)y) - 1) * g.n + v],
+                              (unsigned long long)u);
             }
-            if (any && !(atomicOr(&g.touched[v >> 5], 1u << (v & 31)) & (1u << (v & 31))))
-                nlist[atomicAdd((unsigned long long *)&g.ctl[MB_NNEXT], 1ull)] = v;
+            const uint32_t bit = 1u << (v & 31);
+            fresh = any && !(g.touched[v >> 5] & bit) && !(atomicOr(&g.touched[v >> 5], bit) & bit);
         }
+        queue.add(fresh, v);
+        if (fresh && g.cp[v + 1] - g.cp[v] > kMbHub)
+            g.hubs(cur ^ 1)[atomicAdd((unsigned long long *)&g.ctl[MB_NHUB_NEXT], 1ull)] = v;
+        queue.step(g.ctl, nlist);
     };
-    for (int64_t b = int64_t(blockIdx.x) * 4; b < nf; b += int64_t(gridDim.x) * 4) {
-        int32_t u = -1;
-        if (b + warp < nf) u = g.list(cur)[b + warp];
-        const bool is_long = u >= 0 && g.cp[u + 1] - g.cp[u] > 512;
-        if (lane == 0) s_long[warp] = is_long ? u : -1;
-        if (u >= 0 && !is_long) edges(u, lane, 32);
+    queue.begin();
+    for (int64_t h = 0; h < nh; ++h) {
+        const int32_t u = g.hubs(cur)[h];
+        const uint32_t s = g.cp[u], d = g.cp[u + 1] - s;
+        for (int64_t e0 = int64_t(blockIdx.x) * NT; e0 < d; e0 += int64_t(gridDim.x) * NT)
+            edge(e0 + tid < d, u, s + (uint32_t)(e0 + tid));
+    }
+    const int per = (int)min(max(nf / gridDim.x, (int64_t)1), (int64_t)NT);
+    if (per == 1) {
+        for (int64_t b = blockIdx.x; b < nf; b += gridDim.x) {
+            const int32_t u = g.list(cur)[b];
+            const uint32_t s = g.cp[u], d = g.cp[u + 1] - s;
+            for (uint32_t e0 = 0; e0 < d && d <= kMbHub; e0 += NT) edge(e0 + tid < d, u, s + e0 + tid);
+        }
+        queue.end(g.ctl, nlist);
+        return;
+    }
+    for (int64_t b = int64_t(blockIdx.x) * per; b < nf; b += int64_t(gridDim.x) * per) {
+        const int n = (int)min((int64_t)per, nf - b);
+        int d = 0;
+        if (tid < n) {
+            const int32_t u = g.list(cur)[b + tid];
+            const uint32_t s = g.cp[u], du = g.cp[u + 1] - s;
+            s_u[tid] = u;
+            s_st[tid] = s;
+            d = du > kMbHub ? 0 : (int)du;
+        }
+        int64_t tot;
+        const int off = (int)block_exclusive_sum64<NT>(d, &tot);
+        s_off[tid] = off;
+        if (tid == NT - 1) s_off[NT] = (int)tot;
         __syncthreads();
-        for (int k = 0; k < 4; ++k)
-            if (s_long[k] >= 0) edges(s_long[k], threadIdx.x, kMbPushThreads);
+        for (int e0 = 0; e0 < (int)tot; e0 += NT) {
+            const int e = e0 + tid;
+            int lo = 0;
+#pragma unroll
+            for (int step = NT / 2; step; step >>= 1)
+                if (s_off[lo + step] <= e) lo += step;
+            edge(e < (int)tot, s_u[lo], s_st[lo] + (uint32_t)(e - s_off[lo]));
+        }
         __syncthreads();
     }
+    queue.end(g.ctl, nlist);
 }
 
-__device__ __forceinline__ void mb_count(int64_t *ctl, unsigned long long reached, unsigned long long deg,
-                                         unsigned long long fe)
+// A block's share of the level's sums (all its threads call it).
+__device__ void mb_count(int64_t *ctl, unsigned long long reached, unsigned long long deg, unsigned long long fe)
 {
+    __shared__ unsigned long long s_sum[3];
+    if (threadIdx.x < 3) s_sum[threadIdx.x] = 0;
+    __syncthreads();
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
         reached += __shfl_xor_sync(0xffffffffu, reached, o);
@@ -223,50 +328,49 @@ __device__ __forceinline__ void mb_count(int64_t *ctl, unsigned long long reache
         fe += __shfl_xor_sync(0xffffffffu, fe, o);
     }
     if ((threadIdx.x & 31) == 0 && (reached || fe)) {
-        atomicAdd((unsigned long long *)&ctl[MB_REACHED], reached);
-        atomicAdd((unsigned long long *)&ctl[MB_EDGES], deg);
-        atomicAdd((unsigned long long *)&ctl[MB_FE_NEXT], fe);
+        atomicAdd(&s_sum[0], reached);
+        atomicAdd(&s_sum[1], deg);
+        atomicAdd(&s_sum[2], fe);
     }
+    __syncthreads();
+    if (threadIdx.x < 3 && s_sum[threadIdx.x])
+        atomicAdd((unsigned long long *)&ctl[threadIdx.x == 0   ? MB_REACHED
+                                             : threadIdx.x == 1 ? MB_EDGES
+                                                                : MB_FE_NEXT],
+                  s_sum[threadIdx.x]);
 }
 
 // End of a push level: the new vertices' bits are seen, the old frontier's
 // buffer is zero again.
 template <int NW>
-__global__ void __launch_bounds__(256) k_mb_push_end(MbView g)
+__device__ __forceinline__ void mb_push_end(const MbView &g)
 {
-    if (g.ctl[MB_MODE] != 0) return;
     const int cur = (int)g.ctl[MB_CUR];
     const int64_t i0 = int64_t(blockIdx.x) * blockDim.x + threadIdx.x, stride = int64_t(gridDim.x) * blockDim.x;
     const int64_t nn = g.ctl[MB_NNEXT], nf = g.ctl[MB_NF];
     unsigned long long reached = 0, deg = 0, fe = 0;
-    for (int64_t i = i0; i < nn; i += stride) {
-        const int64_t v = g.list(cur ^ 1)[i];
-        g.touched[v >> 5] = 0;
+    // a lane per word
+    for (int64_t i = i0; i < nn * NW; i += stride) {
+        const int64_t v = g.list(cur ^ 1)[i / NW], at = v * NW + i % NW;
         const unsigned long long d = g.cp[v + 1] - g.cp[v];
-        int c = 0;
-#pragma unroll
-        for (int w = 0; w < NW; ++w) {
-            const uint64_t x = g.bits(cur ^ 1)[v * NW + w];
-            if (x) g.seen[v * NW + w] |= x;
-            c += __popcll(x);
-        }
+        const uint64_t x = g.bits(cur ^ 1)[at];
+        if (x) g.seen[at] |= x;
+        const int c = __popcll(x);
         reached += c;
         deg += c * d;
-        fe += d;
+        if (i % NW == 0) {
+            g.touched[v >> 5] = 0;
+            fe += d;
+        }
     }
-    for (int64_t i = i0; i < nf; i += stride) {
-        const int64_t v = g.list(cur)[i];
-#pragma unroll
-        for (int w = 0; w < NW; ++w) g.bits(cur)[v * NW + w] = 0;
-    }
+    for (int64_t i = i0; i < nf * NW; i += stride) g.bits(cur)[g.list(cur)[i / NW] * (int64_t)NW + i % NW] = 0;
     mb_count(g.ctl, reached, deg, fe);
 }
 
 // Pull: NW lanes per item (a short vertex, or a chunk of a long one).
 template <int NW>
-__global__ void __launch_bounds__(256) k_mb_pull(MbView g)
+__device__ __forceinline__ void mb_pull(const MbView &g)
 {
-    if (g.ctl[MB_MODE] != 1) return;
     constexpr int U = 4;  // neighbours in flight
     const int w = threadIdx.x % NW;
     const int cur = (int)g.ctl[MB_CUR];
@@ -275,8 +379,8 @@ __global__ void __launch_bounds__(256) k_mb_pull(MbView g)
     unsigned long long *parents = (unsigned long long *)(uintptr_t)g.ctl[MB_PARENTS] + (int64_t)w * 64 * g.n;
     const int64_t left = g.ctl[MB_ROOTS] - w * 64;
     const uint64_t valid = left >= 64 ? ~0ull : left > 0 ? (1ull << left) - 1 : 0ull;
-    const int64_t stride = int64_t(gridDim.x) * (256 / NW);
-    for (int64_t i = int64_t(blockIdx.x) * (256 / NW) + threadIdx.x / NW; i < g.nitems + g.n; i += stride) {
+    const int64_t stride = int64_t(gridDim.x) * (kMbThreads / NW);
+    for (int64_t i = int64_t(blockIdx.x) * (kMbThreads / NW) + threadIdx.x / NW; i < g.nitems + g.n; i += stride) {
         const bool chunk = i < g.nitems;
         const int64_t v = chunk ? g.item_v[i] : i - g.nitems;
         uint32_t p = chunk ? g.item_p[i] : g.cp[v], e = g.cp[v + 1];
@@ -316,15 +420,16 @@ __global__ void __launch_bounds__(256) k_mb_pull(MbView g)
     }
 }
 
-// End of a pull level, over all vertices: as k_mb_push_end, and the next
+// End of a pull level, over all vertices: as mb_push_end, and the next
 // frontier's list.
 template <int NW>
-__global__ void __launch_bounds__(256) k_mb_pull_end(MbView g)
+__device__ __forceinline__ void mb_pull_end(const MbView &g)
 {
-    if (g.ctl[MB_MODE] != 1) return;
-    const int cur = (int)g.ctl[MB_CUR], lane = threadIdx.x & 31;
+    __shared__ MbQueue<kMbThreads> queue;
+    const int cur = (int)g.ctl[MB_CUR];
     const int64_t stride = int64_t(gridDim.x) * blockDim.x;
     unsigned long long reached = 0, deg = 0, fe = 0;
+    queue.begin();
     for (int64_t b = int64_t(blockIdx.x) * blockDim.x; b < g.n; b += stride) {
         const int64_t v = b + threadIdx.x;
         int c = 0;
@@ -337,34 +442,61 @@ __global__ void __launch_bounds__(256) k_mb_pull_end(MbView g)
                 g.bits(cur)[v * NW + w] = 0;
             }
         }
-        const unsigned m = __ballot_sync(0xffffffffu, c > 0);
-        if (m) {
-            unsigned long long o = 0;
-            if (lane == 0) o = atomicAdd((unsigned long long *)&g.ctl[MB_NNEXT], (unsigned long long)__popc(m));
-            o = __shfl_sync(0xffffffffu, o, 0);
-            if (c > 0) {
-                const unsigned long long d = g.cp[v + 1] - g.cp[v];
-                g.list(cur ^ 1)[o + __popc(m & ((1u << lane) - 1))] = (int32_t)v;
-                reached += c;
-                deg += c * d;
-                fe += d;
-            }
+        if (c > 0) {
+            const unsigned long long d = g.cp[v + 1] - g.cp[v];
+            if (d > kMbHub) g.hubs(cur ^ 1)[atomicAdd((unsigned long long *)&g.ctl[MB_NHUB_NEXT], 1ull)] = (int32_t)v;
+            reached += c;
+            deg += c * d;
+            fe += d;
         }
+        queue.add(c > 0, (int32_t)v);
+        queue.step(g.ctl, g.list(cur ^ 1));
     }
+    queue.end(g.ctl, g.list(cur ^ 1));
     mb_count(g.ctl, reached, deg, fe);
 }
 
-__global__ void k_mb_advance(int64_t *ctl, int64_t nnz, int64_t cap, cudaGraphConditionalHandle h)
+// A level is two launches, each of them one way or the other: with an idle
+// kernel for the other way, and one to advance, a level of a thin frontier was
+// mostly launches (20000 levels of a path 267 -> 217 ms).
+template <int NW>
+__global__ void __launch_bounds__(kMbThreads) k_mb_level(MbView g)
 {
-    ctl[MB_NF] = ctl[MB_NNEXT];
+    if (g.ctl[MB_MODE] == 0)
+        mb_push<NW>(g);
+    else
+        mb_pull<NW>(g);
+}
+
+// The last block to end the level advances it.  ctl is volatile there, other
+// blocks' sums are not to come from this SM's cache.
+template <int NW>
+__global__ void __launch_bounds__(kMbThreads) k_mb_level_end(MbView g, int64_t cap, cudaGraphConditionalHandle h)
+{
+    if (g.ctl[MB_MODE] == 0)
+        mb_push_end<NW>(g);
+    else
+        mb_pull_end<NW>(g);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    __threadfence();
+    if (atomicAdd((unsigned long long *)&g.ctl[MB_DONE], 1ull) != gridDim.x - 1) return;
+    __threadfence();
+    volatile int64_t *ctl = g.ctl;
+    const int64_t nf = ctl[MB_NNEXT], fe = ctl[MB_FE_NEXT], nh = ctl[MB_NHUB_NEXT], cur = ctl[MB_CUR];
+    const int64_t level = ctl[MB_LEVEL] + 1, levels = ctl[MB_LEVELS];
+    ctl[MB_DONE] = 0;
+    ctl[MB_NF] = nf;
     ctl[MB_NNEXT] = 0;
-    ctl[MB_FE] = ctl[MB_FE_NEXT];
+    ctl[MB_NHUB] = nh;
+    ctl[MB_NHUB_NEXT] = 0;
+    ctl[MB_FE] = fe;
     ctl[MB_FE_NEXT] = 0;
-    ctl[MB_CUR] ^= 1;
-    ctl[MB_LEVEL] += 1;
-    if (ctl[MB_LEVEL] > ctl[MB_LEVELS]) ctl[MB_LEVELS] = ctl[MB_LEVEL];
-    mb_mode(ctl, nnz);
-    cudaGraphSetConditional(h, (ctl[MB_NF] != 0 && ctl[MB_LEVEL] < cap) ? 1u : 0u);
+    ctl[MB_CUR] = cur ^ 1;
+    ctl[MB_LEVEL] = level;
+    if (level > levels) ctl[MB_LEVELS] = level;
+    ctl[MB_MODE] = mb_mode(fe, g.nnz);
+    cudaGraphSetConditional(h, (nf != 0 && level < cap) ? 1u : 0u);
 }
 
 static MbView mb_view(const Graph *g)
@@ -381,6 +513,8 @@ static MbView mb_view(const Graph *g)
     v.bits1 = b.bits[1];
     v.list0 = b.list[0];
     v.list1 = b.list[1];
+    v.hubs0 = b.hubs[0];
+    v.hubs1 = b.hubs[1];
     v.touched = b.touched;
     v.item_v = b.item_v;
     v.item_p = b.item_p;
@@ -401,6 +535,8 @@ static void mb_free(Graph *g)
     device_free(c, b.bits[1]);
     device_free(c, b.list[0]);
     device_free(c, b.list[1]);
+    device_free(c, b.hubs[0]);
+    device_free(c, b.hubs[1]);
     device_free(c, b.touched);
     device_free(c, b.ctl);
     device_free(c, b.item_v);
@@ -452,6 +588,7 @@ static int mb_prepare(Graph *g)
     GBC_CUDA_TRY(cudaMemsetAsync(b.touched, 0, (g->n / 32 + 1) * sizeof(uint32_t), s));
     GBC_TRY(device_alloc(ctx, (void **)&b.ctl, MB_N * sizeof(int64_t)));
     GBC_CUDA_TRY(cudaMallocHost(&b.h_ctl, MB_N * sizeof(int64_t)));
+    for (auto &hubs : b.hubs) GBC_TRY(device_alloc(ctx, (void **)&hubs, (g->nnz / kMbHub + 1) * sizeof(int32_t)));
     GBC_TRY(device_alloc(ctx, (void **)&b.list[1], (g->n + 1) * sizeof(int32_t)));
     GBC_TRY(device_alloc(ctx, (void **)&b.list[0], (g->n + 1) * sizeof(int32_t)));  // last: marks it ready
     return GBC_OK;
@@ -489,12 +626,14 @@ static int mb_pass(Graph *g, int slot, const int64_t *d_roots, int64_t nroots, i
     const MbView v = mb_view(g);
     if (!b.exec[slot]) {
         auto body = [&](cudaStream_t cs, cudaGraphConditionalHandle h) {
-            k_mb_push<NW><<<occ_grid(ctx, (const void *)k_mb_push<NW>, kMbPushThreads, 0), kMbPushThreads, 0, cs>>>(v);
-            k_mb_push_end<NW><<<occ_grid(ctx, (const void *)k_mb_push_end<NW>, 256, 0), 256, 0, cs>>>(v);
-            k_mb_pull<NW><<<occ_grid(ctx, (const void *)k_mb_pull<NW>, 256, 0), 256, 0, cs>>>(v);
-            k_mb_pull_end<NW><<<occ_grid(ctx, (const void *)k_mb_pull_end<NW>, 256, 0), 256, 0, cs>>>(v);
-            k_mb_advance<<<1, 1, 0, cs>>>(v.ctl, v.nnz, v.n + 2, h);
-            note_launches(5);
+            // resident blocks, and no more than have work
+            auto grid = [&](const void *kernel, int64_t items) {
+                return (int)std::min<int64_t>(occ_grid(ctx, kernel, kMbThreads, 0), items / kMbThreads + 1);
+            };
+            k_mb_level<NW><<<grid((const void *)k_mb_level<NW>, std::max((v.n + v.nitems) * NW, v.nnz)), kMbThreads, 0,
+                             cs>>>(v);
+            k_mb_level_end<NW><<<grid((const void *)k_mb_level_end<NW>, v.n * NW), kMbThreads, 0, cs>>>(v, v.n + 2, h);
+            note_launches(2);
             GBC_CUDA_TRY(cudaGetLastError());
             return (int)GBC_OK;
         };

@@ -33,6 +33,7 @@ struct MsBits {
     uint64_t *seen = nullptr;                   // [n * words] roots that have reached a vertex
     uint64_t *bits[2] = {nullptr, nullptr};     // frontier words (current / next)
     int32_t *list[2] = {nullptr, nullptr};      // vertices with a bit in them
+    int32_t *hubs[2] = {nullptr, nullptr};      // ... those of very many neighbours
     uint32_t *touched = nullptr;                // [n / 32] vertices already in the next list (push levels)
     int32_t *item_v = nullptr;                  // chunks of the vertices with many neighbours
     uint32_t *item_p = nullptr;
