@@ -630,9 +630,11 @@ __global__ void __launch_bounds__(kThreads) k_bfs_bu(const uint32_t *cp32, const
             slot = __shfl_sync(0xffffffffu, slot, __ffs(m) - 1);
             if (fresh) q[slot + __popc(m & ((1u << lane) - 1))] = (int32_t)v;
         }
-        __syncthreads();
-        if (s_qn > kQueue - kThreads) queue_flush(q, s_qn, s_gbase, ctl, next);
+        // one thread looks, so that all decide alike: a fast warp may already add
+        // the next round's vertices (kThreads of this round may be missing)
+        if (__syncthreads_or(tid == 0 && s_qn > kQueue - 2 * kThreads)) queue_flush(q, s_qn, s_gbase, ctl, next);
     }
+    __syncthreads();
     queue_flush(q, s_qn, s_gbase, ctl, next);
     bfs_block_sums(ctl, deg, reached, fdeg);
     if (advance) bfs_block_done(ctl, gridDim.x, n, cap, h);
@@ -1014,8 +1016,7 @@ __global__ void __launch_bounds__(kThreads) k_ms_expand(const uint32_t *cp32, co
                 slot = __shfl_sync(0xffffffffu, slot, __ffs(m) - 1);
                 if (fresh) q[slot + __popc(m & ((1u << lane) - 1))] = entry;
             }
-            __syncthreads();
-            if (s_qn > kQueue - kThreads) {
+            if (__syncthreads_or(tid == 0 && s_qn > kQueue - 2 * kThreads)) {  // (as in k_bfs_bu)
                 if (tid == 0) s_gbase = atomicAdd((unsigned long long *)&ctl[MS_NNEXT], (unsigned long long)s_qn);
                 __syncthreads();
                 for (int k = tid; k < s_qn; k += kThreads) next[s_gbase + k] = q[k];
