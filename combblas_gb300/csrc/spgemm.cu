@@ -197,20 +197,28 @@ __global__ void k_amask(int64_t ncol, const uint32_t *tptr, int T, int mask_word
 
 // flop[i] = sum over B(:,i) entries k of nnz(A(:,k)) (estimateFLOP), and the
 // column's tile mask = OR of the masks of those A columns (exactly the row
-// tiles the output column touches).
+// tiles the output column touches).  own[i] (own_need > 0): whether the column's
+// segments suit k_numeric_own.
 __global__ void __launch_bounds__(kPrepWarps * 32)
     k_flop_mask(int64_t nb, const int64_t *bcp, const int32_t *brow, const int64_t *acp, const uint64_t *amask,
-                int mask_words, int64_t *flop, uint64_t *tmask)
+                int mask_words, int64_t *flop, uint64_t *tmask, int64_t own_need, uint8_t *own)
 {
     constexpr int W = 4;  // mask words of one pass
+    constexpr int S = W + 2;
     __shared__ int64_t ls[kPrepWarps], le[kPrepWarps];
-    __shared__ uint64_t part[kPrepWarps][W + 1];
+    __shared__ uint64_t part[kPrepWarps][S];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    // this warp's part of the sum (acc[W]) and of mask words w0.. over [s, e)
-    uint64_t acc[W + 1];
+    // this warp's part of the sums (acc[W] and, cut at own_need a segment,
+    // acc[W + 1]) and of mask words w0.. over [s, e)
+    uint64_t acc[S];
+    auto put = [&](int64_t i, int64_t entries, uint64_t f, uint64_t cut) {
+        flop[i] = (int64_t)f;
+        if (own_need > 0)
+            own[i] = (int64_t)f >= own_need * entries && (int64_t)cut * 8 >= own_need * entries * 7;
+    };
     auto gather = [&](int64_t s, int64_t e, int64_t first, int64_t stride, int w0) {
 #pragma unroll
-        for (int u = 0; u <= W; ++u) acc[u] = 0;
+        for (int u = 0; u < S; ++u) acc[u] = 0;
         for (int64_t p = s + first; p < e; p += kPrepUnroll * stride) {
             int k[kPrepUnroll];
 #pragma unroll
@@ -218,7 +226,11 @@ __global__ void __launch_bounds__(kPrepWarps * 32)
 #pragma unroll
             for (int u = 0; u < kPrepUnroll; ++u) {
                 if (k[u] < 0) continue;
-                if (w0 == 0) acc[W] += (uint64_t)(acp[k[u] + 1] - acp[k[u]]);
+                if (w0 == 0) {
+                    const int64_t len = acp[k[u] + 1] - acp[k[u]];
+                    acc[W] += (uint64_t)len;
+                    acc[W + 1] += (uint64_t)min(len, own_need);
+                }
 #pragma unroll
                 for (int x = 0; x < W; ++x)
                     if (w0 + x < mask_words) acc[x] |= amask[(int64_t)k[u] * mask_words + w0 + x];
@@ -228,7 +240,8 @@ __global__ void __launch_bounds__(kPrepWarps * 32)
         for (int o = 16; o; o >>= 1) {
 #pragma unroll
             for (int x = 0; x < W; ++x) acc[x] |= __shfl_xor_sync(0xffffffffu, acc[x], o);
-            acc[W] += __shfl_xor_sync(0xffffffffu, acc[W], o);
+#pragma unroll
+            for (int x = W; x < S; ++x) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], o);
         }
     };
     for (int64_t i0 = int64_t(blockIdx.x) * kPrepWarps; i0 < nb; i0 += int64_t(gridDim.x) * kPrepWarps) {
@@ -243,7 +256,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32)
             for (int w0 = 0; w0 == 0 || w0 < mask_words; w0 += W) {
                 gather(s, e, lane, 32, w0);
                 if (lane == 0) {
-                    if (w0 == 0) flop[i] = (int64_t)acc[W];
+                    if (w0 == 0) put(i, e - s, acc[W], acc[W + 1]);
 #pragma unroll
                     for (int x = 0; x < W; ++x)
                         if (w0 + x < mask_words) tmask[i * mask_words + w0 + x] = acc[x];
@@ -256,14 +269,16 @@ __global__ void __launch_bounds__(kPrepWarps * 32)
                 gather(ls[q], le[q], threadIdx.x, kPrepWarps * 32, w0);
                 if (lane == 0)
 #pragma unroll
-                    for (int u = 0; u <= W; ++u) part[wid][u] = acc[u];
+                    for (int u = 0; u < S; ++u) part[wid][u] = acc[u];
                 __syncthreads();
                 if (threadIdx.x <= W) {
-                    uint64_t m = 0;
-                    for (int y = 0; y < kPrepWarps; ++y)
+                    uint64_t m = 0, cut = 0;
+                    for (int y = 0; y < kPrepWarps; ++y) {
                         m = threadIdx.x < W ? m | part[y][threadIdx.x] : m + part[y][threadIdx.x];
+                        cut += part[y][W + 1];
+                    }
                     if (threadIdx.x == W) {
-                        if (w0 == 0) flop[i0 + q] = (int64_t)m;
+                        if (w0 == 0) put(i0 + q, le[q] - ls[q], m, cut);
                     } else if (w0 + (int)threadIdx.x < mask_words) {
                         tmask[(i0 + q) * mask_words + w0 + threadIdx.x] = m;
                     }
@@ -319,20 +334,25 @@ constexpr int kBigList = kWarpClasses;            // index of the big list in Li
 constexpr int kOwnList = kBigList + 1;            // ... of the columns for k_numeric_own
 constexpr int kOwnSlot = kWarpClasses + kBigBins; // its slot while classifying
 constexpr int kLists = kOwnSlot + 1;              // list slots while classifying
-constexpr int kListSums = kLists + 3;             // their lengths, then all columns' multiplications, and those
-                                                  // and the B entries of the warp classes above s1
+constexpr int kListSums = kLists + 5;             // their lengths, then all columns' multiplications, those and
+                                                  // the B entries of the warp classes above s1, and the sum and
+                                                  // the most of k_numeric_own's
 
-// Of the big columns, those with at least own_need products per B entry (0:
-// none), own_min() for every row range, are listed for k_numeric_own: a
-// range's segments then fill a good part of a 32-product window.
-__global__ void k_classify(const int64_t *flop, const int64_t *bcp, int64_t own_need, int pid, int64_t col_base, int64_t j0, int64_t j1, int64_t s1,
+// Of the big columns, those that own marks (null: none) are listed for
+// k_numeric_own: they have at least own_need products per B entry, own_min() for
+// every row range, so that a range's segments fill a good part of a 32-product
+// window, and still 7/8 of that with no segment counted for more: a few hubs' long
+// segments do not fill the others' windows (fp32 squares of 20000-vertex R-MATs with
+// 6*10^5 and 1.2*10^6 edges 8.4 -> 5.7 and 17.4 -> 12.0 ms, 15/16 6.0 and 12.0, 3/4
+// 6.0 and 15.9; the MCL loop is the same with all of them).
+__global__ void k_classify(const int64_t *flop, const int64_t *bcp, const uint8_t *own, int pid, int64_t col_base, int64_t j0, int64_t j1, int64_t s1,
                            int64_t s2, int64_t *lbuf, int64_t stride, unsigned long long *counts, int64_t *cnt_zero,
                            const int32_t *only_flagged)
 {
     const int64_t i = j0 + int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     int cls = -1;
-    unsigned long long fsum = 0, msum = 0, esum = 0;
+    unsigned long long fsum = 0, msum = 0, esum = 0, osum = 0;
     if (i < j1 && (!only_flagged || only_flagged[col_base + i])) {
         const int64_t f = flop[i];
         fsum = f;
@@ -344,8 +364,9 @@ __global__ void k_classify(const int64_t *flop, const int64_t *bcp, int64_t own_
             cls = f <= kSmallMid ? 1 : f <= kSmallMid2 ? 2 : 3;
             msum = f;
             esum = bcp[i + 1] - bcp[i];
-        } else if (own_need > 0 && f >= own_need * (bcp[i + 1] - bcp[i])) {
+        } else if (own && own[i]) {
             cls = kOwnSlot;
+            osum = f;
         } else {
             cls = kWarpClasses + big_bin(f);
         }
@@ -355,6 +376,18 @@ __global__ void k_classify(const int64_t *flop, const int64_t *bcp, int64_t own_
         fsum += __shfl_xor_sync(0xffffffffu, fsum, o);
         msum += __shfl_xor_sync(0xffffffffu, msum, o);
         esum += __shfl_xor_sync(0xffffffffu, esum, o);
+    }
+    if (__any_sync(0xffffffffu, cls == kOwnSlot)) {
+        unsigned long long omax = osum;
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            osum += __shfl_xor_sync(0xffffffffu, osum, o);
+            omax = max(omax, __shfl_xor_sync(0xffffffffu, omax, o));
+        }
+        if (lane == 0) {
+            atomicAdd(&counts[kLists + 3], osum);
+            atomicMax(&counts[kLists + 4], omax);
+        }
     }
     if (lane == 0 && fsum) atomicAdd(&counts[kLists], fsum);
     if (lane == 0 && msum) {
@@ -1190,11 +1223,12 @@ static int64_t few_columns(int tiles, bool others, int64_t n, int64_t prods, int
     if (!others) return tiles <= 16 && prods >= 640 * n ? 1 : 0;
     return tiles > 16 ? 2 : prods >= 32 * entries ? 8 : 4;
 }
-// k_numeric_own has a column walked by four warps: with fewer columns per
-// multiprocessor than this (two rounds of its resident blocks) the longest one is
-// the launch's end, and the list goes to k_numeric.  fp32 square of a 2357-vertex
-// R-MAT: 203 us for the kernel against 132, the call 938 -> 826; an MCL
-// loop 262 -> 265 ms.
+// k_numeric_own has a column walked by four warps: where its columns together have
+// less than this many times the longest one's products per multiprocessor (two
+// rounds of its resident blocks, for columns alike), that one is the launch's end,
+// and the list goes to k_numeric.  fp32 squares of R-MATs: 2357 vertices 203 us for
+// the kernel against 132, the call 938 -> 826; 9000 vertices 2.64 -> 2.25 ms.  An MCL
+// loop, whose columns are many and alike: 262 -> 265 ms.
 constexpr int64_t kFewOwn = 16;
 
 // Everything the passes need, built once: one descriptor per product of a
@@ -1224,6 +1258,7 @@ struct Plan {
     int64_t xscap = 0;                   // segments of a column at most (its A's tile list entries)
     int x_blocks = 0;                    // exact kernel: its grid (resident blocks)
     int own_vsize = 0;                   // value size for k_numeric_own (0: not used)
+    std::vector<uint8_t *> own_cols;     // ... every product's columns that suit it
     bool own_built = false;              // its range tables are there
     Workspace *ws = nullptr;
     SpgemmArgs &a() { return h[0]; }
@@ -1320,15 +1355,17 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
         k_amask<<<(unsigned)((A.ncol + 255) / 256), 256, 0, s>>>(A.ncol, a.tptr, a.T, a.mask_words, amask);
         note_launch();
     }
+    a.own_T = P.own_vsize ? own_ranges(A.nrow, A.ncol, P.own_vsize) : 0;
+    uint8_t *own = nullptr;
+    if (a.own_T > 0) GBC_TRY(ws.alloc_n(&own, nb + 1));
     if (nb > 0) {
         k_flop_mask<<<grid_for(ctx, (nb + 7) / 8, 8), 256, 0, s>>>(nb, B.cp, a.brow, acp, amask, a.mask_words, flop,
-                                                                     tmask);
+                                                                     tmask, (int64_t)a.own_T * own_min(P.own_vsize), own);
         note_launch();
     }
     GBC_CUDA_TRY(cudaGetLastError());
     a.flop = flop;
     a.tmask = tmask;
-    a.own_T = P.own_vsize ? own_ranges(A.nrow, A.ncol, P.own_vsize) : 0;
     a.own_ptr = nullptr;
     a.own_rb = nullptr;
     a.aexp = nullptr;
@@ -1358,6 +1395,7 @@ static int plan_add(Workspace &ws, Plan &P, const DevMatrix &A, const DevMatrix 
     P.h.push_back(a);
     P.a_nnz.push_back(A.nnz);
     P.amask.push_back(amask);
+    P.own_cols.push_back(own);
     return GBC_OK;
 }
 
@@ -1498,7 +1536,7 @@ static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j
         const SpgemmArgs &a = P.h[q];
         const int64_t lo = pid >= 0 ? j0 : 0, hi = (pid >= 0 && j1 >= 0) ? j1 : a.nb;
         if (hi > lo) {
-            k_classify<<<(unsigned)((hi - lo + 255) / 256), 256, 0, s>>>(a.flop, a.bcp, (int64_t)a.own_T * own_min(P.own_vsize),
+            k_classify<<<(unsigned)((hi - lo + 255) / 256), 256, 0, s>>>(a.flop, a.bcp, P.own_cols[q],
                                                                          q, a.col_base, lo, hi,
                                                                          P.s1, P.s2,
                                                                          P.lbuf, stride, P.lcnt, cnt_zero, flagged);
@@ -1511,7 +1549,8 @@ static int plan_classify(Plan &P, cudaStream_t s, int pid, int64_t j0, int64_t j
     GBC_CUDA_TRY(cudaStreamSynchronize(s));
     // the big list: its first part (columns for k_numeric_own that are too few
     // for it, or bin 0, the heaviest) in place, the other bins appended
-    const bool few_own = h[kOwnSlot] > 0 && !P.s2_set && (int64_t)h[kOwnSlot] <= kFewOwn * P.ws->ctx->num_sms;
+    const bool few_own = h[kOwnSlot] > 0 && !P.s2_set &&
+                         h[kLists + 3] / h[kLists + 4] <= (unsigned long long)(kFewOwn * P.ws->ctx->num_sms);
     const int64_t *bins = P.lbuf + kWarpClasses * stride;
     int64_t *lbig = P.lbuf + (few_own ? kOwnSlot : kWarpClasses) * stride;
     int64_t nbig = (int64_t)h[few_own ? kOwnSlot : kWarpClasses];
