@@ -42,22 +42,51 @@
 namespace gbc {
 
 // ----------------------------------------------------------------- prepare
-// The preparation kernels give every warp a column and the whole block the
-// columns longer than kLongCol, kPrepUnroll loads in flight per thread: one
-// warp alone on a hub column (2*10^3 to 10^5 entries, a chain of loads) was
+// The preparation kernels give every warp a column and, behind those, the whole
+// block the columns longer than kLongCol, kPrepUnroll loads in flight per thread:
+// one warp alone on a hub column (2*10^3 to 10^5 entries, a chain of loads) was
 // the end of each launch.  The three kernels of a scale-14 R-MAT square 144 ->
 // 51 us (the product 1265 -> 1193), the product of a 30011-vertex one 3760 ->
-// 3614 us.
+// 3614 us.  Short columns meet no barrier: with one for every eight columns, 2*10^5
+// of one entry took k_prep_a 109 us instead of 62, 65536 of 16 entries k_prep_b 30
+// instead of 12 and k_flop_mask 45 instead of 27.
 constexpr int kLongCol = 256;
 constexpr int kPrepWarps = 8;
 constexpr int kPrepUnroll = 4;
+constexpr int kPrepLong = 64;  // long columns that a block puts off (further ones are left to their warps)
+
+// The long columns of a block.  begin() and end() are called by all its threads.
+struct LongCols {
+    int64_t i[kPrepLong];
+    int n;
+    __device__ __forceinline__ void begin()
+    {
+        if (threadIdx.x == 0) n = 0;
+        __syncthreads();
+    }
+    // Column c of this warp put off?  (All its lanes.)
+    __device__ __forceinline__ bool put_off(int64_t c)
+    {
+        int at = 0;
+        if ((threadIdx.x & 31) == 0) {
+            at = atomicAdd(&n, 1);
+            if (at < kPrepLong) i[at] = c;
+        }
+        return __shfl_sync(0xffffffffu, at, 0) < kPrepLong;
+    }
+    __device__ __forceinline__ int end()
+    {
+        __syncthreads();
+        return min(n, kPrepLong);
+    }
+};
 
 // load(p) and then use(i, p, s, e, loaded) for every entry p of [s, e) =
 // [cp[i], cp[i + 1]) of the columns for which ok(i, s, e, lane) holds.
 template <class Ok, class Load, class Use>
 __device__ __forceinline__ void each_entry(int64_t n, const int64_t *cp, Ok ok, Load load, Use use)
 {
-    __shared__ int64_t ls[kPrepWarps], le[kPrepWarps];
+    __shared__ LongCols longs;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     auto run = [&](int64_t i, int64_t s, int64_t e, int64_t first, int64_t stride) {
         for (int64_t p = s + first; p < e; p += kPrepUnroll * stride) {
@@ -70,24 +99,18 @@ __device__ __forceinline__ void each_entry(int64_t n, const int64_t *cp, Ok ok, 
                 if (p + u * stride < e) use(i, p + u * stride, s, e, v[u]);
         }
     };
-    for (int64_t i0 = int64_t(blockIdx.x) * kPrepWarps; i0 < n; i0 += int64_t(gridDim.x) * kPrepWarps) {
-        const int64_t i = i0 + w;
-        int64_t s = 0, e = 0;
-        if (i < n) {
-            s = cp[i];
-            e = cp[i + 1];
-            if (!ok(i, s, e, lane)) e = s;
-        }
-        const bool is_long = e - s > kLongCol;
-        if (lane == 0) {
-            ls[w] = s;
-            le[w] = is_long ? e : s;
-        }
-        if (!is_long) run(i, s, e, lane, 32);
-        __syncthreads();
-        for (int q = 0; q < kPrepWarps; ++q) run(i0 + q, ls[q], le[q], threadIdx.x, kPrepWarps * 32);
-        __syncthreads();
+    longs.begin();
+    for (int64_t i = int64_t(blockIdx.x) * kPrepWarps + w; i < n; i += int64_t(gridDim.x) * kPrepWarps) {
+        const int64_t s = cp[i], e = cp[i + 1];
+        if (!ok(i, s, e, lane) || (e - s > kLongCol && longs.put_off(i))) continue;
+        if (e - s > 32)
+            run(i, s, e, lane, 32);
+        else if (s + lane < e)
+            use(i, s + lane, s, e, load(s + lane, s));
     }
+    const int put_off = longs.end();
+    for (int q = 0; q < put_off; ++q)
+        run(longs.i[q], cp[longs.i[q]], cp[longs.i[q] + 1], threadIdx.x, kPrepWarps * 32);
 }
 
 struct RowPair {
@@ -159,7 +182,7 @@ __global__ void k_fill_empty_tptr(int64_t ncol, const int64_t *acp, uint32_t *tp
     }
 }
 
-__global__ void __launch_bounds__(kPrepWarps * 32)
+__global__ void __launch_bounds__(kPrepWarps * 32, 8)
     k_prep_b(int64_t nzc, int64_t nnz, const int64_t *cp, const int64_t *ir, int64_t kdim, int32_t *brow,
              int32_t *err)
 {
@@ -199,13 +222,13 @@ __global__ void k_amask(int64_t ncol, const uint32_t *tptr, int T, int mask_word
 // column's tile mask = OR of the masks of those A columns (exactly the row
 // tiles the output column touches).  own[i] (own_need > 0): whether the column's
 // segments suit k_numeric_own.
-__global__ void __launch_bounds__(kPrepWarps * 32)
+__global__ void __launch_bounds__(kPrepWarps * 32, 6)
     k_flop_mask(int64_t nb, const int64_t *bcp, const int32_t *brow, const int64_t *acp, const uint64_t *amask,
                 int mask_words, int64_t *flop, uint64_t *tmask, int64_t own_need, uint8_t *own)
 {
     constexpr int W = 4;  // mask words of one pass
     constexpr int S = W + 2;
-    __shared__ int64_t ls[kPrepWarps], le[kPrepWarps];
+    __shared__ LongCols longs;
     __shared__ uint64_t part[kPrepWarps][S];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     // this warp's part of the sums (acc[W] and, cut at own_need a segment,
@@ -219,74 +242,75 @@ __global__ void __launch_bounds__(kPrepWarps * 32)
     auto gather = [&](int64_t s, int64_t e, int64_t first, int64_t stride, int w0) {
 #pragma unroll
         for (int u = 0; u < S; ++u) acc[u] = 0;
-        for (int64_t p = s + first; p < e; p += kPrepUnroll * stride) {
-            int k[kPrepUnroll];
+        auto one = [&](int k) {
+            if (w0 == 0) {
+                const int64_t len = acp[k + 1] - acp[k];
+                acc[W] += (uint64_t)len;
+                acc[W + 1] += (uint64_t)min(len, own_need);
+            }
 #pragma unroll
-            for (int u = 0; u < kPrepUnroll; ++u) k[u] = p + u * stride < e ? brow[p + u * stride] : -1;
+            for (int x = 0; x < W; ++x)
+                if (w0 + x < mask_words) acc[x] |= amask[(int64_t)k * mask_words + w0 + x];
+        };
+        if (e - s <= stride) {
+            if (s + first < e) one(brow[s + first]);
+        } else {
+            for (int64_t p = s + first; p < e; p += kPrepUnroll * stride) {
+                int k[kPrepUnroll];
 #pragma unroll
-            for (int u = 0; u < kPrepUnroll; ++u) {
-                if (k[u] < 0) continue;
-                if (w0 == 0) {
-                    const int64_t len = acp[k[u] + 1] - acp[k[u]];
-                    acc[W] += (uint64_t)len;
-                    acc[W + 1] += (uint64_t)min(len, own_need);
-                }
+                for (int u = 0; u < kPrepUnroll; ++u) k[u] = p + u * stride < e ? brow[p + u * stride] : -1;
 #pragma unroll
-                for (int x = 0; x < W; ++x)
-                    if (w0 + x < mask_words) acc[x] |= amask[(int64_t)k[u] * mask_words + w0 + x];
+                for (int u = 0; u < kPrepUnroll; ++u)
+                    if (k[u] >= 0) one(k[u]);
             }
         }
 #pragma unroll
-        for (int o = 16; o; o >>= 1) {
+        for (int x = 0; x < S; ++x) {
+            if (x < W ? w0 + x >= mask_words : w0 > 0 || (x > W && own_need == 0)) continue;  // block-uniform
 #pragma unroll
-            for (int x = 0; x < W; ++x) acc[x] |= __shfl_xor_sync(0xffffffffu, acc[x], o);
-#pragma unroll
-            for (int x = W; x < S; ++x) acc[x] += __shfl_xor_sync(0xffffffffu, acc[x], o);
+            for (int o = 16; o; o >>= 1) {
+                const uint64_t y = __shfl_xor_sync(0xffffffffu, acc[x], o);
+                acc[x] = x < W ? acc[x] | y : acc[x] + y;
+            }
         }
     };
-    for (int64_t i0 = int64_t(blockIdx.x) * kPrepWarps; i0 < nb; i0 += int64_t(gridDim.x) * kPrepWarps) {
-        const int64_t i = i0 + wid;
-        const int64_t s = i < nb ? bcp[i] : 0, e = i < nb ? bcp[i + 1] : 0;
-        const bool is_long = e - s > kLongCol;
-        if (lane == 0) {
-            ls[wid] = s;
-            le[wid] = is_long ? e : s;
-        }
-        if (i < nb && !is_long)
-            for (int w0 = 0; w0 == 0 || w0 < mask_words; w0 += W) {
-                gather(s, e, lane, 32, w0);
-                if (lane == 0) {
-                    if (w0 == 0) put(i, e - s, acc[W], acc[W + 1]);
+    longs.begin();
+    for (int64_t i = int64_t(blockIdx.x) * kPrepWarps + wid; i < nb; i += int64_t(gridDim.x) * kPrepWarps) {
+        const int64_t s = bcp[i], e = bcp[i + 1];
+        if (e - s > kLongCol && longs.put_off(i)) continue;
+        for (int w0 = 0; w0 == 0 || w0 < mask_words; w0 += W) {
+            gather(s, e, lane, 32, w0);
+            if (lane == 0) {
+                if (w0 == 0) put(i, e - s, acc[W], acc[W + 1]);
 #pragma unroll
-                    for (int x = 0; x < W; ++x)
-                        if (w0 + x < mask_words) tmask[i * mask_words + w0 + x] = acc[x];
-                }
-            }
-        __syncthreads();
-        for (int q = 0; q < kPrepWarps; ++q) {
-            if (ls[q] == le[q]) continue;
-            for (int w0 = 0; w0 == 0 || w0 < mask_words; w0 += W) {
-                gather(ls[q], le[q], threadIdx.x, kPrepWarps * 32, w0);
-                if (lane == 0)
-#pragma unroll
-                    for (int u = 0; u < S; ++u) part[wid][u] = acc[u];
-                __syncthreads();
-                if (threadIdx.x <= W) {
-                    uint64_t m = 0, cut = 0;
-                    for (int y = 0; y < kPrepWarps; ++y) {
-                        m = threadIdx.x < W ? m | part[y][threadIdx.x] : m + part[y][threadIdx.x];
-                        cut += part[y][W + 1];
-                    }
-                    if (threadIdx.x == W) {
-                        if (w0 == 0) put(i0 + q, le[q] - ls[q], m, cut);
-                    } else if (w0 + (int)threadIdx.x < mask_words) {
-                        tmask[(i0 + q) * mask_words + w0 + threadIdx.x] = m;
-                    }
-                }
-                __syncthreads();
+                for (int x = 0; x < W; ++x)
+                    if (w0 + x < mask_words) tmask[i * mask_words + w0 + x] = acc[x];
             }
         }
-        __syncthreads();
+    }
+    const int put_off = longs.end();
+    for (int q = 0; q < put_off; ++q) {
+        const int64_t i = longs.i[q], s = bcp[i], e = bcp[i + 1];
+        for (int w0 = 0; w0 == 0 || w0 < mask_words; w0 += W) {
+            gather(s, e, threadIdx.x, kPrepWarps * 32, w0);
+            if (lane == 0)
+#pragma unroll
+                for (int u = 0; u < S; ++u) part[wid][u] = acc[u];
+            __syncthreads();
+            if (threadIdx.x <= W) {
+                uint64_t m = 0, cut = 0;
+                for (int y = 0; y < kPrepWarps; ++y) {
+                    m = threadIdx.x < W ? m | part[y][threadIdx.x] : m + part[y][threadIdx.x];
+                    cut += part[y][W + 1];
+                }
+                if (threadIdx.x == W) {
+                    if (w0 == 0) put(i, e - s, m, cut);
+                } else if (w0 + (int)threadIdx.x < mask_words) {
+                    tmask[i * mask_words + w0 + threadIdx.x] = m;
+                }
+            }
+            __syncthreads();
+        }
     }
 }
 
@@ -372,10 +396,13 @@ __global__ void k_classify(const int64_t *flop, const int64_t *bcp, const uint8_
         }
     }
 #pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        fsum += __shfl_xor_sync(0xffffffffu, fsum, o);
-        msum += __shfl_xor_sync(0xffffffffu, msum, o);
-        esum += __shfl_xor_sync(0xffffffffu, esum, o);
+    for (int o = 16; o; o >>= 1) fsum += __shfl_xor_sync(0xffffffffu, fsum, o);
+    if (__any_sync(0xffffffffu, msum > 0)) {
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+            msum += __shfl_xor_sync(0xffffffffu, msum, o);
+            esum += __shfl_xor_sync(0xffffffffu, esum, o);
+        }
     }
     if (__any_sync(0xffffffffu, cls == kOwnSlot)) {
         unsigned long long omax = osum;
