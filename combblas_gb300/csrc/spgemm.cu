@@ -1299,13 +1299,74 @@ struct Plan {
 // the larger warp kernels).  The others fold in order, in the columns dense
 // enough for it by k_numeric_own.
 //
-// Where A (m x k, the largest of a batch) has more row tiles than the kernel
-// buckets (2^20 rows), it visits every touched tile with all of the column's B
-// entries: columns of 1600 products spread over 2^21 rows took 132 ms of min-plus
-// where k_numeric and the larger warp kernels take 3.6, over 2^22 rows 221 and
-// 3.9; a 2^21-vertex R-MAT 91 and 55.  The order-free semirings keep those
-// there, and where the tile pointers kXRows apart would pass 8 GB (the default
-// tiles need half of that).
+// Where A has more row tiles than the kernel buckets (2^20 rows), it visits every
+// touched tile with all of the column's B entries: columns of 1600 products spread
+// over 2^21 rows took 132 ms of min-plus where k_numeric and the larger warp
+// kernels take 3.6, over 2^22 rows 221 and 3.9; a 2^21-vertex R-MAT 91 and 55.  The
+// order-free semirings keep those there, and where the tile pointers kXRows apart
+// would pass 8 GB (the default tiles need half of that).
+static bool x_fits(const DevMatrix &A)
+{
+    const int64_t tiles = (A.nrow + kXRows - 1) / kXRows;
+    return tiles <= kXTMax && A.ncol * (tiles + 1) <= int64_t(1) << 31;
+}
+
+// Nor is the kernel worth its lower tiles above 2^18 rows (where the default ones
+// are twice as high) for few products: twice the tile pointers cost 4.5 ps each, in
+// the three passes over them, a product of a big column gains 40 ps and more over
+// the kernels without it.  Min-plus, every 32nd column of R-MATs of 2^20 vertices with 2
+// and 4 entries a column, 0.041 and 0.173 big products per tile pointer: 4.7 and 5.9 ms,
+// without the kernel 4.7 and 7.9; 2^19 vertices, 0.056, 1.75 and 2.16; 10^6 entries of B
+// and no big column, 2^20 columns of A with 2 entries, 2.8 and 1.6.
+constexpr int64_t kXPlainRows = int64_t(1) << 18;
+
+// Multiplications of the columns of A * B above kSmallMid2 (acp: A's dense column
+// pointers).  Malformed operands, which the preparation reports, give any number.
+__global__ void k_big_flops(int64_t nzc, int64_t nnz, const int64_t *cp, const int64_t *ir, int64_t kdim,
+                            const int64_t *acp, unsigned long long *big)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
+    unsigned long long sum = 0;
+    for (int64_t i = warp; i < nzc; i += nwarps) {
+        const int64_t s = max(cp[i], (int64_t)0), e = min(cp[i + 1], nnz);
+        int64_t f = 0;
+        for (int64_t p = s + lane; p < e; p += 32) {
+            const int64_t k = ir[p];
+            if (k >= 0 && k < kdim) f += acp[k + 1] - acp[k];
+        }
+#pragma unroll
+        for (int o = 16; o; o >>= 1) f += __shfl_xor_sync(0xffffffffu, f, o);
+        if (f > kSmallMid2) sum += (unsigned long long)f;
+    }
+    if (lane == 0 && sum) atomicAdd(big, sum);
+}
+
+static int x_worth(Workspace &ws, const DevMatrix &A, const DevMatrix &B, bool *worth)
+{
+    Context *ctx = ws.ctx;
+    cudaStream_t s = ctx->stream;
+    int64_t big = 0, *acp = const_cast<int64_t *>(A.cp);
+    unsigned long long *sum = nullptr;
+    GBC_TRY(ws.alloc_n(&sum, 1));
+    GBC_CUDA_TRY(cudaMemsetAsync(sum, 0, sizeof(*sum), s));
+    if (A.jc) {
+        GBC_TRY(ws.alloc_n(&acp, A.ncol + 1));
+        GBC_CUDA_TRY(cudaMemsetAsync(acp, 0, (A.ncol + 1) * sizeof(int64_t), s));
+        k_dense_colptr<<<(unsigned)((A.nzc + 1 + 255) / 256), 256, 0, s>>>(A.ncol, A.nzc, A.cp, A.jc, acp);
+        note_launch();
+    }
+    if (B.nzc > 0) {
+        k_big_flops<<<grid_for(ctx, (B.nzc + 7) / 8, 8), 256, 0, s>>>(B.nzc, B.nnz, B.cp, B.ir, A.ncol, acp, sum);
+        note_launch();
+    }
+    GBC_CUDA_TRY(cudaGetLastError());
+    GBC_TRY(read_i64(ctx, reinterpret_cast<const int64_t *>(sum), &big));
+    *worth = big * 20 >= A.ncol * ((A.nrow + kXRows - 1) / kXRows);
+    return GBC_OK;
+}
+
 // Multiplications up to which a column keeps to the warp kernels where
 // k_numeric_x takes the big ones.  A block's time grows with the row tiles that a
 // column touches, a warp's with its products and their bytes.  20000 columns of
@@ -1321,12 +1382,20 @@ static int64_t x_small_limit(int64_t m, bool exact, size_t vsize)
     return vsize == 1 && m > (int64_t(1) << 19) ? kSmall2 : kSmallMid2;
 }
 
+// A, B: the operands of the plan's np products.
 template <class SR>
-static void plan_fold(Context *ctx, Plan &P, int64_t m, int64_t k)
+static int plan_fold(Workspace &ws, Plan &P, const DevMatrix *A, const DevMatrix *B, int np)
 {
     constexpr bool exact = std::is_same<SR, PlusTimes<double>>::value;
-    const bool fits = m <= (int64_t)kXRows * kXTMax && k * (m / kXRows + 2) <= int64_t(1) << 31;
-    if (XAcc<SR>::kUse && (exact ? ctx->fold == GBC_FOLD_EXACT : fits)) {
+    int64_t m = 0;
+    for (int p = 0; p < np; ++p) m = std::max(m, A[p].nrow);
+    bool use = XAcc<SR>::kUse && (!exact || ws.ctx->fold == GBC_FOLD_EXACT);
+    if (!exact)
+        for (int p = 0; use && p < np; ++p) {
+            use = x_fits(A[p]);
+            if (use && A[p].nrow > kXPlainRows) GBC_TRY(x_worth(ws, A[p], B[p], &use));
+        }
+    if (use) {
         P.want_x = true;
         P.want_aexp = exact;
         if (exact && P.tile_rows != 0 && P.tile_rows != kXRows) P.max_words = 2 * kMaxMaskWords;
@@ -1335,6 +1404,7 @@ static void plan_fold(Context *ctx, Plan &P, int64_t m, int64_t k)
     } else if (!XAcc<SR>::kUse || exact) {
         P.own_vsize = (int)sizeof(typename SR::V);
     }
+    return GBC_OK;
 }
 
 template <class SR>
@@ -1896,7 +1966,7 @@ static int spgemm_exact(Context *ctx, const DevMatrix &A, const DevMatrix &B, co
     cudaEventRecord(ctx->ev[0], s);
     Plan P;
     plan_options(P, opt);
-    plan_fold<SR>(ctx, P, A.nrow, A.ncol);
+    GBC_TRY(plan_fold<SR>(ws, P, &A, &B, 1));
     GBC_TRY(plan_build(ws, A, B, P));
     const int64_t nb = B.nzc;
     int64_t *cnt = nullptr, *ccp = nullptr;
@@ -2264,7 +2334,7 @@ static int spgemm_phased(Context *ctx, const DevMatrix &A, const DevMatrix &B, i
     Workspace ws(ctx);
     cudaEventRecord(ctx->ev[0], s);
     Plan P;
-    plan_fold<SR>(ctx, P, A.nrow, A.ncol);
+    GBC_TRY(plan_fold<SR>(ws, P, &A, &B, 1));
     GBC_TRY(plan_build(ws, A, B, P));
     const int64_t nb = B.nzc;
     int64_t *size = nullptr;  // exact counts, or capacities when learned
@@ -2531,7 +2601,7 @@ int spgemm_learned(Context *ctx, const DevMatrix &A, const DevMatrix &B, const g
     cudaEventRecord(ctx->ev[0], s);
     Plan P;
     plan_options(P, opt);
-    plan_fold<SR>(ctx, P, A.nrow, A.ncol);
+    GBC_TRY(plan_fold<SR>(ws, P, &A, &B, 1));
     LearnedOut O;
     GBC_TRY(learned_into_slots<SR>(ctx, ws, A, B, P, O));
     const int64_t nb = O.nb;
@@ -2637,7 +2707,7 @@ int mcl_expand(gbc_context *ctx, const gbc_matrix *Am, float thr, int64_t select
     if (sizing == GBC_SIZING_LEARNED) {
         Plan P;
         LearnedOut O;
-        plan_fold<PlusTimes<float>>(ctx, P, A.nrow, A.ncol);
+        GBC_TRY(plan_fold<PlusTimes<float>>(ws, P, &A, &A, 1));
         GBC_TRY(learned_into_slots<PlusTimes<float>>(ctx, ws, A, A, P, O));
         int64_t *jc = nullptr;
         GBC_TRY(ws.alloc_n(&jc, O.nb + 1));
@@ -2723,12 +2793,7 @@ static int batch_build(Batch &b, const std::vector<DevMatrix> &A, const std::vec
     Context *ctx = b.ctx;
     cudaStream_t s = ctx->stream;
     Workspace &ws = *b.ws;
-    int64_t m = 0, k = 0;
-    for (const DevMatrix &M : A) {
-        m = std::max(m, M.nrow);
-        k = std::max(k, M.ncol);
-    }
-    plan_fold<SR>(ctx, b.P, m, k);
+    GBC_TRY(plan_fold<SR>(ws, b.P, A.data(), B.data(), b.np));
     for (int p = 0; p < b.np; ++p) GBC_TRY(plan_add(ws, b.P, A[p], B[p]));
     GBC_TRY(plan_finalize(ws, b.P));
     const int64_t tc = b.P.total_cols;

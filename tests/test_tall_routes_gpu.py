@@ -13,11 +13,11 @@ pytestmark = pytest.mark.gpu
 BUCKETED = 1 << 20  # rows
 
 
-def product(oracle, m, sr, deg, nb, cols=40):
-    """Visits of the default product of `cols` columns of deg x nb products over m rows."""
+def product(oracle, m, sr, deg, nb, cols=40, empty=0):
+    """Visits of the default product of `cols` columns of deg x nb products over m rows, A with `empty` columns more."""
     rng = np.random.default_rng(m + deg)
-    A = columns(m, [np.unique(rng.integers(0, m, deg)) for _ in range(2000)])
-    B = columns(2000, [np.sort(rng.choice(2000, nb, replace=False)) for _ in range(cols)])
+    A = columns(m, [np.unique(rng.integers(0, m, deg)) for _ in range(2000)] + [np.array([], np.int64)] * empty)
+    B = columns(2000 + empty, [np.sort(rng.choice(2000, nb, replace=False)) for _ in range(cols)])
     name, dt = SR_NAME[sr]
     for M in (A, B):
         M.values = (rng.random(M.nnz) * 100 + 1).astype(dt)
@@ -53,3 +53,9 @@ def test_few_columns_of_300_and_900_products(gpu_ctx, oracle_lib, m, nb, cols, b
 
 def test_few_columns_above_the_bucketed_rows(gpu_ctx, oracle_lib):
     assert product(oracle_lib, BUCKETED + 1, 0, 60, 15) == 0
+
+
+@pytest.mark.parametrize("sr", [0, 2, 3, 4, 5, 6])
+def test_hypersparse_operands(gpu_ctx, oracle_lib, sr):
+    """120000 entries in 150000 columns of 2^20 rows: the order-free semirings keep their higher tiles."""
+    assert (product(oracle_lib, BUCKETED, sr, 60, 100, empty=150000) > 0) == (sr == 0)
