@@ -58,12 +58,6 @@ NUMERIC_DRAM_WRITE_PER_ENTRY = 17.65
 # same samples and threads (8 x86 cores): s20 A*A(:, 4096 columns) 4.05 s vs
 # 3.82 s, s14 A*A 0.487 s vs 0.468 s.
 CPU_CALIBRATION = "the compiled reference's hybrid path needs 1.04-1.06x the port's time on the same samples"
-# DRAM bytes of the multi-source BFS kernels per scanned edge (expand +
-# finalize) as last captured, when each level was a separate graph launch
-# (profiles/launches_msbfs22.txt); the traversal is now one graph whose
-# level kernels run inside a conditional while node, which ncu does not
-# list as launches, so the line reports no traffic of its own.
-MSBFS_DRAM_PER_SCANNED_EDGE_LEVEL_REPLAY = 19.5
 MS_ROOTS = 512
 
 
@@ -580,25 +574,21 @@ def bench_msbfs(args, world, A, ctx, stream, hbm, peak_kind, scale, ef):
     launches = _lib.lib().gbc_launch_count() - l0
     ck = clocks.stop()
     value = edges * world / (ms * 1e-3) / 1e9
-    # expand kernel bytes per traversal: per scanned edge a 4-byte row id, a
-    # visited-bit word and a 4-byte candidate read (8-byte frontier entry per
-    # (root, vertex)), parents written once per reached pair
-    scanned = 2 * st.edges
-    bytes_trav = scanned * (4 + 4 + 4) + st.reached * (8 + 8 + 8)
+    # bytes a traversal cannot do without: the pattern (4-byte row ids and
+    # column pointers) once, and a parent per (root, vertex) pair written
+    bytes_trav = A.nnz * 4 + (A.ncol + 1) * 4 + MS_ROOTS * A.ncol * 8
     achieved = bytes_trav / (ms / args.steps * 1e-3) / 1e9
     out = {
         "metric": metric_name(args.workload, scale, ef), "value": value, "unit": "GTEPS",
         "ms_per_step": ms / args.steps, "gpu_launches": launches, "clocks": ck,
         "msbfs": {"roots": MS_ROOTS, "levels": st.levels, "reached_pairs": st.reached, "edges_per_step": st.edges,
-                  "loop": "masked Select2ndMin product into a per-(root, vertex) candidate array; one CUDA "
-                          "graph per traversal (a conditional while node around the captured level)"},
-        "roofline": {"bound": "hbm", "kernel": "k_ms_expand + k_ms_finalize", "achieved": achieved, "peak": hbm,
+                  "loop": "masked Select2ndMin product with one bit per (root, vertex), pushed or pulled per level; "
+                          "one CUDA graph per traversal (a conditional while node around the captured level)"},
+        "roofline": {"bound": "hbm", "kernel": "k_mb_level + k_mb_level_end", "achieved": achieved, "peak": hbm,
                      "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / hbm,
                      "traffic": None, "algorithmic_bytes": bytes_trav,
                      "traffic_note": "the level kernels run inside the traversal graph's while node, which ncu "
-                                     "does not list as launches; the last level-by-level capture measured "
-                                     f"{MSBFS_DRAM_PER_SCANNED_EDGE_LEVEL_REPLAY} DRAM B per scanned edge "
-                                     "(profiles/launches_msbfs22.txt)"},
+                                     "does not list as launches: their DRAM bytes are not measured"},
     }
     # e2e: graph upload from host + traversal + parents read back into pinned host memory
     hp = torch.empty((MS_ROOTS, A.ncol), dtype=torch.int64, pin_memory=True)
