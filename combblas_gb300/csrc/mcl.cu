@@ -17,7 +17,6 @@
 #include <cstring>
 
 #include "gbc_internal.cuh"
-#undef GBC_XPROF  // the phase clocks belong to the SpGEMM unit
 #include "spgemm_exact.cuh"
 
 namespace gbc {

@@ -42,38 +42,6 @@ constexpr int kXOMax = 61;       // largest product exponent above the base
 constexpr int kXRows = 4096;     // rows of a row tile, and output rows of one accumulator pass
 constexpr int kXThreads = 512;   // two blocks per SM
 
-// Phase clocks of k_numeric_x for profiling builds (-DGBC_XPROF): thread 0
-// of every block adds the cycles between two block barriers to a counter.
-#ifdef GBC_XPROF
-__device__ unsigned long long g_xprof[32];
-#define XPROF_T0 long long xp_t = clock64()
-#define XPROF_LAP(id)                                                          \
-    do {                                                                       \
-        if (threadIdx.x == 0) {                                                \
-            const long long xp_n = clock64();                                  \
-            atomicAdd(&g_xprof[id], (unsigned long long)(xp_n - xp_t));        \
-            xp_t = xp_n;                                                       \
-        }                                                                      \
-    } while (0)
-#define XPROF_ADD(id, v)                                                       \
-    do {                                                                       \
-        if (threadIdx.x == 0) atomicAdd(&g_xprof[id], (unsigned long long)(v)); \
-    } while (0)
-extern "C" int gbc_xprof_read(unsigned long long *out, int reset)
-{
-    cudaMemcpyFromSymbol(out, g_xprof, sizeof(g_xprof));
-    if (reset) {
-        static const unsigned long long z[32] = {};
-        cudaMemcpyToSymbol(g_xprof, z, sizeof(z));
-    }
-    return (int)cudaDeviceSynchronize();
-}
-#else
-#define XPROF_T0
-#define XPROF_LAP(id)
-#define XPROF_ADD(id, v)
-#endif
-
 // Per column of A: smallest and largest biased exponent of its nonzero
 // values, each plus kXBias in 12 bits, kXMixed when a value is negative or
 // zero, and kXZero when one is zero.  Subnormal values count as exponent -64 (their products can
@@ -508,7 +476,6 @@ __global__ void __launch_bounds__(kXThreads, 2)
     bool dirty = false;  // the accumulator holds a sorted range's data
     bool first_item = true;
     int par = 0;  // which wsum the next prefix uses
-    XPROF_T0;
 
     // block-wide exclusive prefix of v over the threads (one barrier: two
     // prefixes in a row use different sums); *tot the total
@@ -667,7 +634,6 @@ __global__ void __launch_bounds__(kXThreads, 2)
         } else {
             __syncthreads();
         }
-        XPROF_LAP(0);
 
         // ---- a ranked visit's steps.  Rows are relative to the visit's first row row0.
         auto mark = [&](int L, int row0) {
@@ -873,8 +839,6 @@ __global__ void __launch_bounds__(kXThreads, 2)
                 }
             }
             // tend[t] is now the end of tile t's segments
-            XPROF_LAP(1);
-            XPROF_ADD(bucketed ? 11 : 12, 1);
         }
 
         // segments [c0, min(c0 + kXSegs, se)) of the scratch: this thread's two
@@ -958,14 +922,11 @@ __global__ void __launch_bounds__(kXThreads, 2)
                             if (c0 > sb) __syncthreads();
                             accumulate(load_bucket(sg), row0, std::true_type{});
                         }
-                        XPROF_ADD(20, 1);
-                        XPROF_ADD(21, prods);
                     } else {
                         fetch(sg, sb, sb + segs);
                         int L = load_bucket(sg);
                         mark(L, row0);
                         __syncthreads();
-                        XPROF_LAP(2);
                         n = rank_rows(nw);
                         if (n > R) {
                             // too many rows: keep the first tiles that fit
@@ -977,22 +938,14 @@ __global__ void __launch_bounds__(kXThreads, 2)
                             for (int w = (t1 - t) * (R / 32) + tid; w < nw; w += NT) sm.bm[w] = 0;
                             nw = (t1 - t) * (R / 32);
                         }
-                        XPROF_LAP(3);
                         accumulate(L, row0, std::false_type{});
-                        XPROF_ADD(8, 1);
-                        XPROF_ADD(18, n);
-                        XPROF_ADD(19, L);
                     }
                     if (tid == 0) atomicAdd(&work[t1 - t > 1 ? 2 : 1], 1ull);  // visits of one tile / of a run
                     __syncthreads();
                     if (direct) {
-                        XPROF_LAP(22);
                         write_direct(nw, row0);
-                        XPROF_LAP(23);
                     } else {
-                        XPROF_LAP(4);
                         write_ranks(n, nw, row0);
-                        XPROF_LAP(5);
                     }
                     t = t1;
                     next_run();
@@ -1024,9 +977,6 @@ __global__ void __launch_bounds__(kXThreads, 2)
                         pbase += L;
                         __syncthreads();  // chunk table reuse
                     }
-                    XPROF_LAP(6);
-                    XPROF_ADD(9, 1);
-                    XPROF_ADD(13, prods);
                     if (tid == 0) atomicAdd(&work[2], 1ull);
                     // stable LSD radix sort of the keys by row, 7-bit digits:
                     // warp w owns a contiguous run of keys, counts its digits,
@@ -1084,7 +1034,6 @@ __global__ void __launch_bounds__(kXThreads, 2)
                         src = dst;
                         dst = tmp;
                     }
-                    XPROF_LAP(7);
                     // runs of one row, one sorted key per thread and round:
                     // the thread holding a run's first key sums the run
                     // exactly (runs are short: a range's rows rarely repeat)
@@ -1131,7 +1080,6 @@ __global__ void __launch_bounds__(kXThreads, 2)
                         out += tot;
                     }
                     __syncthreads();
-                    XPROF_LAP(10);
                     t = t1 + 1;
                     next_run();
                 }
@@ -1175,12 +1123,10 @@ __global__ void __launch_bounds__(kXThreads, 2)
                 }
                 if (tid == 0) atomicAdd(&work[1], 1ull);
                 write_direct(nw, row0);
-                XPROF_LAP(12);
             }
         }
         over = __syncthreads_or(over);
         bad = __syncthreads_or(bad);
-        XPROF_LAP(15);
         if (tid == 0) {
             if (out_cnt) out_cnt[g] = out;
             if (over) {

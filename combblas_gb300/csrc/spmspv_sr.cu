@@ -32,7 +32,7 @@
 // a warp walks the row's row-major entries (ascending column), tests them
 // against a dense column -> vector position map and folds the hits in order.
 // (One window of 32 entries at a time, the longest pulled row took 0.59 of 0.69 ms
-// over 2000 entries of 2^18; with eight in flight the call takes 0.26 ms pulled.)
+// over 2000 entries of 2^18; with eight in flight the call is about as fast as pushed.)
 #include <algorithm>
 #include <cstring>
 #include <type_traits>
@@ -298,9 +298,10 @@ __device__ __forceinline__ V sx_add(V a, V b)
 constexpr int kSxThread = 8;      // products of a row folded by one thread
 constexpr int kSxPullShare = 4;   // pull when the products times this exceed the matrix
 // Matrices of fewer entries are always pulled: their longest row is a short
-// chain, and the push has five launches more.  R-MAT, pulled / pushed: 1.1*10^5
-// entries, 100 of the vector 114 / 173 us; 1.8*10^6, 1000: 205 / 307; 3.9*10^6,
-// 2000: 238 / 274; 7.9*10^6, 100: 184 / 156, 2000: 261 / 281.
+// chain, and the push has five launches more.  R-MAT, vectors of 30 / 2000 / 10000
+// entries on the device, us pulled and pushed: 1.8*10^6 entries 84 161 295 and 91 197
+// 344; 3.7*10^6 112 198 330 and 105 250 368; 7.6*10^6 141 204 348 and 115 201 311;
+// 1.5*10^7 175 241 546 and 108 207 402; 3.1*10^7 237 343 662 and 114 193 310.
 constexpr int64_t kSxPushNnz = 1 << 22;
 
 // The row's products by one warp over its row-major entries, eight windows of
