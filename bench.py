@@ -51,8 +51,8 @@ SEED = 1
 BFS_ROOTS = 64
 # DRAM bytes of k_numeric_x measured by ncu on a scale-20 column sample
 # (profiles/k_numeric_x_s20_cols4096.txt), used to scale roofline.traffic
-NUMERIC_DRAM_READ_PER_MULT = 5.91
-NUMERIC_DRAM_WRITE_PER_ENTRY = 17.65
+NUMERIC_DRAM_READ_PER_MULT = 5.95
+NUMERIC_DRAM_WRITE_PER_ENTRY = 17.64
 # The compiled reference's own hybrid path (heap columns below compression
 # ratio 2, hash above, mtSpGEMM.h:310-311) against the restatement timed here,
 # same samples and threads (8 x86 cores): s20 A*A(:, 4096 columns) 4.05 s vs

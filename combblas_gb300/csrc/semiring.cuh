@@ -6,7 +6,8 @@
 // (-0.0 for floating sums, so that a lone -0.0 stays one).
 // Floating-point multiply and add use the _rn intrinsics so that the
 // compiler can never fuse them into an FMA: each product is rounded before
-// it is added, as in the reference's `SR::add(SR::multiply(a, b), acc)`.
+// it is added, as in the reference's `SR::add(SR::multiply(a, b), acc)`.  (The
+// dense-vector SpMV, whose sums have an order of their own, fuses them itself.)
 #pragma once
 
 #include <cuda_runtime.h>

@@ -1792,8 +1792,9 @@ static int launch_big_ordered(Context *ctx, Plan &P, const int64_t *items, int64
     return GBC_OK;
 }
 
-// Exact (order-free) block kernel for PlusTimes fp64 over the big list;
-// the columns it does not admit go to the ordered kernel afterwards
+// The order-free block kernel over the big list (PlusTimes fp64 under the exact
+// fold, min-plus, or-and, whole-number sums, Select2ndMin); the columns it does
+// not admit go to the ordered kernel afterwards
 // (device-side count, no host synchronisation: graph capture stays valid).
 template <class SR>
 static int launch_big_exact(Context *ctx, Plan &P, const Lists &L, const int64_t *ccp, int64_t ccp_base,

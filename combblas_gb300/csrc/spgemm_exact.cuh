@@ -443,9 +443,9 @@ struct XSmem {
 // appended to fb_items for the ordered kernel.
 //
 // Bound by instruction issue and by the latency of a visit's chain of
-// barriers, not by memory (DRAM 9 %).  Against one tile a visit with the
-// segments found by searches and 24-byte accumulators behind flag bytes (322
-// instead of 498 warp instructions per 32 products), R-MAT scale 20 A*A in
+// barriers, not by memory (DRAM 1.4 % of peak).  Against one tile a visit with
+// the segments found by searches and 24-byte accumulators behind flag bytes
+// (209 instead of 498 warp instructions per 32 products), R-MAT scale 20 A*A in
 // phases went from 1656 to 998 ms, all passes included (2^14: 1.94 to 1.51 ms),
 // and a 30011-vertex min-plus product from 8.28 (k_numeric, warp kernels up to
 // 4096 products) to 4.0 ms.
@@ -953,8 +953,10 @@ __global__ void __launch_bounds__(kXThreads, 2)
                     // sorted range of light tiles t .. t1 (at most kXSort products)
                     t1 = t;
                     prods = sm.prodcnt[t];
-                    while (t1 + 1 < a.T && (sm.segcnt[t1 + 1] == 0 || (sm.prodcnt[t1 + 1] <= kXLight &&
-                                                                       prods + sm.prodcnt[t1 + 1] <= kXSort))) {
+                    // (more segments are more products, whose count may have passed 2^31)
+                    while (t1 + 1 < a.T && (sm.segcnt[t1 + 1] == 0 ||
+                                            (sm.segcnt[t1 + 1] <= kXLight && sm.prodcnt[t1 + 1] <= kXLight &&
+                                             prods + sm.prodcnt[t1 + 1] <= kXSort))) {
                         ++t1;
                         prods += sm.prodcnt[t1];
                     }

@@ -203,7 +203,9 @@ int gbc_spgemm_phased(gbc_context *ctx, int sr, int vt, const gbc_matrix *A, con
  * are where-located arrays of the plan's value type.  Rows without entries
  * keep y.  Min-type, boolean and integer semirings give the reference's
  * result exactly; PlusTimes on floating values sums each row in a fixed
- * order (repeatable, within rounding of the reference's column order). */
+ * order by fused multiply-adds (repeatable, within rounding of the
+ * reference's column order; a product is not rounded by itself, so one that
+ * would overflow need not). */
 typedef struct gbc_spmv_plan gbc_spmv_plan;
 int gbc_spmv_plan_create(gbc_context *ctx, int vt, const gbc_matrix *A, gbc_spmv_plan **plan);
 int gbc_spmv_plan_destroy(gbc_spmv_plan *plan);
