@@ -22,8 +22,8 @@
 //         parents by atomic minimum.  Everything a push level touches is in its
 //         two vertex lists, so long thin graphs pay for their frontiers only.
 //         A block flattens the edges of a few vertices over its threads; the
-//         hubs, of more than kMbHub neighbours, are listed apart and every block
-//         takes a share of each.
+//         hubs, of more than kMbHub neighbours, are listed apart and shared out over
+//         groups of blocks.
 #pragma once
 
 #include "size_rules.cuh"
@@ -271,11 +271,16 @@ __device__ __forceinline__ void mb_push(const MbView &g)
         queue.step(g.ctl, nlist);
     };
     queue.begin();
-    for (int64_t h = 0; h < nh; ++h) {
-        const int32_t u = g.hubs(cur)[h];
-        const uint32_t s = g.cp[u], d = g.cp[u + 1] - s;
-        for (int64_t e0 = int64_t(blockIdx.x) * NT; e0 < d; e0 += int64_t(gridDim.x) * NT)
-            edge(e0 + tid < d, u, s + (uint32_t)(e0 + tid));
+    // hubs: groups of at least eight blocks take them in turn, a block its share of each
+    if (nh > 0) {
+        const int groups = (int)min(nh, (int64_t)max(gridDim.x / 8, 1u)), blocks = (int)gridDim.x / groups;
+        const int group = (int)blockIdx.x / blocks, share = (int)blockIdx.x % blocks;
+        for (int64_t h = group; group < groups && h < nh; h += groups) {
+            const int32_t u = g.hubs(cur)[h];
+            const uint32_t s = g.cp[u], d = g.cp[u + 1] - s;
+            for (int64_t e0 = int64_t(share) * NT; e0 < d; e0 += int64_t(blocks) * NT)
+                edge(e0 + tid < d, u, s + (uint32_t)(e0 + tid));
+        }
     }
     const int per = (int)min(max(nf / gridDim.x, (int64_t)1), (int64_t)NT);
     if (per == 1) {

@@ -28,19 +28,28 @@ def graph(name, rng):
         at = np.concatenate([[0], np.cumsum(k + 1)[:-1]])
         leaf = np.concatenate([a + 1 + np.arange(c) for a, c in zip(at, k)])
         return int(k.sum() + len(k)), np.concatenate([np.repeat(at, k), at[:-1]]), np.concatenate([leaf, at[1:]])
+    if name == "many hubs":  # 300 of 2100 leaves in one frontier, beside a part that keeps the level thin
+        hub = 1 + np.arange(300) * 2101
+        leaf = (hub[:, None] + 1 + np.arange(2100)[None, :]).reshape(-1)
+        n = 1 + 300 * 2101
+        u = n + np.arange(1 << 20)
+        return n + (1 << 20) + 3, np.concatenate([np.zeros(300, np.int64), np.repeat(hub, 2100), u, u, u]), \
+            np.concatenate([hub, leaf, u + 1, u + 2, u + 3])
     n = 1300000  # "one level": more new vertices than the grid has threads, several rounds a block
     return n, np.zeros(n - 1, np.int64), np.arange(1, n)
 
 
 @pytest.mark.parametrize("name,nroots", [("hubs", 1), ("hubs", 70), ("hubs", 300), ("wide", 1), ("wide", 40),
                                          ("wide", 130), ("wide", 300), ("stars", 1), ("stars", 100), ("stars", 300),
-                                         ("one level", 1)])
+                                         ("many hubs", 1), ("many hubs", 3), ("one level", 1)])
 def test_thin_levels_match_the_oracle(gpu_ctx, oracle_lib, name, nroots):
     rng = np.random.default_rng(nroots)
     n, u, v = graph(name, rng)
     A = edges(n, u, v)
     roots = rng.integers(0, n, nroots)
-    roots[0] = {"hubs": 7, "one level": 0}.get(name, roots[0])
+    if name == "many hubs":
+        roots %= 600000  # not in the part beside
+    roots[0] = {"hubs": 7, "one level": 0, "many hubs": 0}.get(name, roots[0])
     ref, levels = oracle_lib.port_msbfs(A, roots)
     deg = np.diff(A.colptr)
     g = B.Graph(A)
